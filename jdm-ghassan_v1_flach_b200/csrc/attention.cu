@@ -1,5 +1,7 @@
 // GQA attention: single-token decode over a ring or paged KV cache (split-KV,
-// one pass over K/V for all query heads of a KV group) and causal prefill.
+// one pass over K/V for all query heads of a KV group) and causal prefill.  fp16 caches with
+// head_dim 64 / 128 take attention_decode.cu; the scalar decode kernel here serves the rest
+// (fp32 caches, head_dim 32 / 256, unaligned tensors).
 //
 // Reference arithmetic: core/attn_cpu.cpp:29-94 (prefill, window, segment mask),
 // :151-254 (ring decode, fp32 and fp16 caches); kernels replaced:
@@ -12,6 +14,7 @@
 
 #include <mutex>
 
+#include "attention_decode.cuh"
 #include "common.cuh"
 
 namespace b200 {
@@ -274,6 +277,13 @@ static int decode_ring(const char* who, const float* q, const void* kc, const vo
     a.ring_start = ring_start; a.pinned = pinned; a.ring_cap = ring_cap > 0 ? ring_cap : 1;
     a.scale = scale;
     const int span = cur_len - a.j0;
+    if (half) {
+        DecodeMmaArgs c;
+        c.q = q; c.kc = static_cast<const uint16_t*>(kc); c.vc = static_cast<const uint16_t*>(vc); c.out = out;
+        c.H = H; c.KV = KV; c.hd = hd; c.group = a.group; c.cur_len = cur_len; c.j0 = a.j0;
+        c.ring_start = ring_start; c.pinned = pinned; c.ring_cap = a.ring_cap; c.scale = scale;
+        if (attention_decode_mma_takes(c)) return attention_decode_mma(c, 1, span, fixed_part, fixed_floats);
+    }
     return half ? launch_decode<true, false>(a, 1, span, out, fixed_part, fixed_floats)
                 : launch_decode<false, false>(a, 1, span, out, fixed_part, fixed_floats);
 }
@@ -399,13 +409,17 @@ int b200_attention_decode_paged_fp16(const float* q, const uint16_t* k_pages, co
     B200_REQUIRE(q && k_pages && v_pages && page_table && seq_lens && out, "attention_decode_paged_fp16: null pointer");
     int rc = check_hd("attention_decode_paged_fp16", hd);
     if (rc) return rc;
+    DecodeMmaArgs c;
+    c.q = q; c.kc = k_pages; c.vc = v_pages; c.out = out; c.page_table = page_table; c.seq_lens = seq_lens;
+    c.H = H; c.KV = KV; c.hd = hd; c.group = H / KV; c.max_pages = max_pages; c.page = page; c.scale = scale;
+    // sequence lengths live on the device: size the splits for the longest possible one
+    if (attention_decode_mma_takes(c)) return attention_decode_mma(c, batch, max_pages * page);
     DecodeArgs a{};
     a.q = q; a.kc = k_pages; a.vc = v_pages;
     a.page_table = page_table; a.seq_lens = seq_lens;
     a.H = H; a.KV = KV; a.hd = hd; a.group = H / KV;
     a.max_pages = max_pages; a.page = page; a.ring_cap = 1;
     a.scale = scale;
-    // sequence lengths live on the device: size the splits for the longest possible one
     return launch_decode<true, true>(a, batch, max_pages * page, out);
 }
 

@@ -1,0 +1,349 @@
+// Single-token GQA attention over an fp16 ring or paged KV cache, head_dim 64 / 128, on
+// mma.sync with every fp32 operand cut in two fp16 parts.
+//
+// Reference arithmetic: core/attn_cpu.cpp:151-254; kernels replaced: cuda/attention.cu:614-809.
+//
+// What bounds it: the K and V rows, read once (4 * len * KV * hd bytes).  The scalar form spent
+// 8 FMAs, five shuffles and two exponentials per key and query head and reached 7 % of the copy
+// rate; here a warp takes 16 keys at a time for the up to eight query heads of a KV head:
+//   S[16, 16 keys]  = Q . K^T    rows 0-7 the heads' high parts, rows 8-15 their low parts, so a
+//                                thread's accumulators c0 + c2 are one head's exact score
+//   O[16, hd]      += P . V      the same split of the probabilities; the halves are added at the end
+// q is scaled by a power of two to at most 2^10 before the cut and p runs up to 2^10, so both keep
+// 22 significant bits; K and V are fp16 in memory, products and sums fp32.
+// No shared memory on the way: the contraction over dims is free to permute, so a thread loads 16
+// consecutive bytes of a key (K: dims 32c + 8t ..; V: dims 64w + 8g .. of the four keys its B
+// fragment needs, paired by prmt).  The loads of the next 16 keys are issued as soon as the MMAs
+// have read the registers: 8 KB in flight per warp, 12 warps per SM.
+// 64 sequences of 256 .. 8192 tokens, 32 / 8 heads of 128: 2.50 ms before, 0.295 ms now
+// (1.11 GB: 3.8 TB/s).
+#include <algorithm>
+
+#include "attention_decode.cuh"
+#include "fused_common.cuh"
+
+namespace b200 {
+
+constexpr int AD_WARPS = 4;
+constexpr int AD_HEADS = 8;           // query heads of one KV head per block
+constexpr int AD_TILE = 16;           // keys per warp step
+constexpr int AD_STEP = AD_WARPS * AD_TILE;
+constexpr int AD_MAX_SPLITS = 128;
+constexpr int AD_MAX_COUNTERS = 1 << 16;
+constexpr float AD_LOG2E = 1.4426950408889634f;
+constexpr float AD_P_BIAS = 10.0f;    // probabilities carry a factor 2^10
+
+// Blocks of a (sequence, KV head, head block) that have left their partial result; the last one
+// merges and puts the word back to zero.
+static __device__ unsigned int g_ad_count[AD_MAX_COUNTERS];
+
+__device__ __forceinline__ void ad_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t ad_pack(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+// (a, b) as fp16 pairs: the rounded values and what rounding left
+__device__ __forceinline__ void ad_split(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = ad_pack(a - f.x, b - f.y);
+}
+
+// Row of logical position j: pinned prefix + rolling window (core/attn_cpu.cpp:151-156), or the page.
+template <bool PAGED>
+__device__ __forceinline__ int64_t ad_row(const DecodeMmaArgs& a, const int32_t* pages, int j) {
+    if (PAGED) return (int64_t)pages[j / a.page] * a.page + j % a.page;
+    return j < a.pinned ? j : (int64_t)a.pinned + (a.ring_start + (j - a.pinned)) % a.ring_cap;
+}
+
+// grid (splits, KV * head blocks, batch)
+template <int HD, bool PAGED>
+__global__ void __launch_bounds__(AD_WARPS * 32, 3) attn_decode_mma_kernel(DecodeMmaArgs a) {
+    constexpr int KC = HD / 32, VC = HD / 64;
+    __shared__ uint4 s_q[HD / 16][32];                        // A fragments of Q, one per 16 dims
+    __shared__ float s_o[AD_WARPS][AD_HEADS][HD];
+    __shared__ float s_ml[AD_WARPS][AD_HEADS][2];
+    __shared__ float s_mul[AD_HEADS];                         // score -> log2 units
+    __shared__ int s_last;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int gblocks = (a.group + AD_HEADS - 1) / AD_HEADS;
+    const int kvh = blockIdx.y / gblocks, g0 = (blockIdx.y % gblocks) * AD_HEADS, b = blockIdx.z;
+    const int G = min(AD_HEADS, a.group - g0);
+    const int h0 = kvh * a.group + g0;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int len = PAGED ? __ldcg(a.seq_lens + b) : a.cur_len - a.j0;
+    // this sequence's own cut: even pieces of whole steps, so a short sequence uses few blocks
+    const int chunk = max(AD_STEP, ((len + a.splits - 1) / a.splits + AD_STEP - 1) / AD_STEP * AD_STEP);
+    const int ns = max(1, (len + chunk - 1) / chunk);
+    if (blockIdx.x >= ns) return;
+    const int jbeg = blockIdx.x * chunk, jend = min(len, jbeg + chunk);
+    const int32_t* pages = PAGED ? a.page_table + (int64_t)b * a.max_pages : nullptr;
+    const int jofs = PAGED ? 0 : a.j0;
+    const int64_t stride = (int64_t)a.KV * HD;
+    const uint16_t* kc = a.kc + (int64_t)kvh * HD;
+    const uint16_t* vc = a.vc + (int64_t)kvh * HD;
+
+    auto row_of = [&](int j) { return ad_row<PAGED>(a, pages, jofs + min(j, jend - 1)); };   // past the end: the last key again
+    uint4 kr[2][KC], vr[4][VC];
+    auto load_k = [&](int64_t r) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const uint16_t* p = kc + __shfl_sync(0xffffffffu, r, 8 * n + g) * stride + 8 * t;
+#pragma unroll
+            for (int c = 0; c < KC; ++c) kr[n][c] = __ldcg(reinterpret_cast<const uint4*>(p + 32 * c));
+        }
+    };
+    auto load_v = [&](int64_t r) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const uint16_t* p = vc + __shfl_sync(0xffffffffu, r, 2 * t + (n & 1) + 8 * (n >> 1)) * stride + 8 * g;
+#pragma unroll
+            for (int c = 0; c < VC; ++c) vr[n][c] = __ldcg(reinterpret_cast<const uint4*>(p + 64 * c));
+        }
+    };
+    int j = jbeg + warp * AD_TILE;
+    int64_t row = 0;
+    if (j < jend) {
+        row = row_of(j + (lane & 15));
+        load_k(row);
+        load_v(row);
+    }
+    // Q of head g0 + w, w + 4: scaled by 2^-e to at most 2^10, cut, laid out as A fragments
+    for (int w = warp; w < AD_HEADS; w += AD_WARPS) {
+        const float* q = a.q + ((int64_t)b * a.H + h0 + w) * HD;
+        float v[HD / 32], mx = 0.0f;
+#pragma unroll
+        for (int i = 0; i < HD / 32; ++i) {
+            v[i] = w < G ? __ldcg(q + 32 * i + lane) : 0.0f;
+            mx = fmaxf(mx, fabsf(v[i]));
+        }
+        mx = warp_max(mx);
+        int e = 0;
+        if (mx > 0.0f && isfinite(mx)) frexpf(mx, &e);
+        e = max(e, -100);                                     // a head of denormals stays as it is
+        const float mul = ldexpf(1.0f, 10 - e);
+        if (lane == 0) s_mul[w] = ldexpf(a.scale * AD_LOG2E, e - 10);
+#pragma unroll
+        for (int i = 0; i < HD / 32; ++i) {
+            // dim 32 i + lane belongs to thread t' = lane / 8, step 2 i + (lane & 4 ? 1 : 0), pair (lane & 2), half (lane & 1)
+            const float x = v[i] * mul;
+            const __half hi = __float2half_rn(x);
+            const __half lo = __float2half_rn(x - __half2float(hi));
+            __half* f = reinterpret_cast<__half*>(&s_q[2 * i + ((lane >> 2) & 1)][4 * w + (lane >> 3)]);
+            const int at = ((lane >> 1) & 1) * 4 + (lane & 1);          // a0 | a1 | a2 | a3, two halves each
+            f[at] = hi;
+            f[at + 2] = lo;
+        }
+    }
+    __syncthreads();
+    const float mul = s_mul[g];
+    float o[VC][8][4], m = -INFINITY, l = 0.0f;
+#pragma unroll
+    for (int w = 0; w < VC; ++w)
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[w][n][i] = 0.0f;
+
+    for (; j < jend; j += AD_STEP) {
+        const bool more = j + AD_STEP < jend;
+        int64_t next = 0;
+        if (more) next = row_of(j + AD_STEP + (lane & 15));
+        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < KC; ++c) {
+            const uint4 f0 = s_q[2 * c][lane], f1 = s_q[2 * c + 1][lane];
+            ad_mma(s0, f0.x, f0.y, f0.z, f0.w, kr[0][c].x, kr[0][c].y);
+            ad_mma(s1, f0.x, f0.y, f0.z, f0.w, kr[1][c].x, kr[1][c].y);
+            ad_mma(s0, f1.x, f1.y, f1.z, f1.w, kr[0][c].z, kr[0][c].w);
+            ad_mma(s1, f1.x, f1.y, f1.z, f1.w, kr[1][c].z, kr[1][c].w);
+        }
+        if (more) load_k(next);
+        float x[4] = {(s0[0] + s0[2]) * mul, (s0[1] + s0[3]) * mul, (s1[0] + s1[2]) * mul, (s1[1] + s1[3]) * mul};
+        if (j + AD_TILE > jend) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (j + 2 * t + (i & 1) + 8 * (i >> 1) >= jend) x[i] = -INFINITY;
+        }
+        float mn = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
+        mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+        mn = fmaxf(m, fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2)));
+        if (__any_sync(0xffffffffu, mn != m)) {
+            const float corr = exp2f(m - mn);                 // exp2(-inf) = 0 on the first keys
+            l *= corr;
+#pragma unroll
+            for (int w = 0; w < VC; ++w)
+#pragma unroll
+                for (int n = 0; n < 8; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) o[w][n][i] *= corr;
+            m = mn;
+        }
+        uint32_t hi[2], lo[2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = exp2f(x[i] - (m - AD_P_BIAS));
+        l += (x[0] + x[1]) + (x[2] + x[3]);
+        ad_split(x[0], x[1], hi[0], lo[0]);
+        ad_split(x[2], x[3], hi[1], lo[1]);
+#pragma unroll
+        for (int w = 0; w < VC; ++w) {
+            const uint32_t* v0 = reinterpret_cast<const uint32_t*>(&vr[0][w]);
+            const uint32_t* v1 = reinterpret_cast<const uint32_t*>(&vr[1][w]);
+            const uint32_t* v2 = reinterpret_cast<const uint32_t*>(&vr[2][w]);
+            const uint32_t* v3 = reinterpret_cast<const uint32_t*>(&vr[3][w]);
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+                const uint32_t sel = (n & 1) ? 0x7632u : 0x5410u;
+                ad_mma(o[w][n], hi[0], lo[0], hi[1], lo[1], __byte_perm(v0[n >> 1], v1[n >> 1], sel),
+                       __byte_perm(v2[n >> 1], v3[n >> 1], sel));
+            }
+        }
+        if (more) load_v(next);
+    }
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    if (g < G) {
+        // this thread's dims: 64 w + 16 t + (0 .. 15)
+#pragma unroll
+        for (int w = 0; w < VC; ++w)
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+                s_o[warp][g][64 * w + 16 * t + n] = o[w][n][0] + o[w][n][2];
+                s_o[warp][g][64 * w + 16 * t + 8 + n] = o[w][n][1] + o[w][n][3];
+            }
+        if (t == 0) { s_ml[warp][g][0] = m; s_ml[warp][g][1] = l; }
+    }
+    __syncthreads();
+    constexpr int REC = HD + 4;
+    for (int i = threadIdx.x; i < G * (HD / 4); i += AD_WARPS * 32) {
+        const int hh = i / (HD / 4), c = i % (HD / 4) * 4;
+        float mm = -INFINITY, ll = 0.0f;
+#pragma unroll
+        for (int w = 0; w < AD_WARPS; ++w) mm = fmaxf(mm, s_ml[w][hh][0]);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < AD_WARPS; ++w) {
+            const float mw = s_ml[w][hh][0];
+            const float f = mw == -INFINITY ? 0.0f : exp2f(mw - mm);
+            const float4 v = *reinterpret_cast<const float4*>(&s_o[w][hh][c]);
+            ll += s_ml[w][hh][1] * f;
+            acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
+        }
+        if (ns == 1) {
+            const float inv = ll > 0.0f ? 1.0f / ll : 0.0f;
+            *reinterpret_cast<float4*>(a.out + ((int64_t)b * a.H + h0 + hh) * HD + c) =
+                make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+        } else {
+            float* dst = a.part + (((int64_t)b * a.H + h0 + hh) * a.splits + blockIdx.x) * REC;
+            *reinterpret_cast<float4*>(dst + c) = acc;
+            if (c == 0) { dst[HD] = mm; dst[HD + 1] = ll; }
+        }
+    }
+    if (ns == 1) return;
+    // the block that counts in last merges the pieces
+    __threadfence();
+    __syncthreads();
+    unsigned int* count = g_ad_count + (int64_t)b * gridDim.y + blockIdx.y;
+    if (threadIdx.x == 0) s_last = atomicAdd(count, 1u) == (unsigned)ns - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x == 0) *count = 0;
+    float* s_w = &s_o[0][0][0];                               // [G][ns] weights, then the row sums
+    for (int hh = warp; hh < G; hh += AD_WARPS) {
+        const float* p = a.part + ((int64_t)b * a.H + h0 + hh) * a.splits * REC;
+        float mv[AD_MAX_SPLITS / 32], lv[AD_MAX_SPLITS / 32], mm = -INFINITY, ll = 0.0f;
+#pragma unroll
+        for (int i = 0; i < AD_MAX_SPLITS / 32; ++i) {
+            const int s = 32 * i + lane;
+            mv[i] = s < ns ? __ldcg(p + (int64_t)s * REC + HD) : -INFINITY;
+            lv[i] = s < ns ? __ldcg(p + (int64_t)s * REC + HD + 1) : 0.0f;
+            mm = fmaxf(mm, mv[i]);
+        }
+        mm = warp_max(mm);
+#pragma unroll
+        for (int i = 0; i < AD_MAX_SPLITS / 32; ++i) {
+            const float f = mv[i] == -INFINITY ? 0.0f : exp2f(mv[i] - mm);
+            ll += lv[i] * f;
+            if (32 * i + lane < ns) s_w[hh * AD_MAX_SPLITS + 32 * i + lane] = f;
+        }
+        ll = warp_sum(ll);
+        if (lane == 0) s_ml[0][hh][0] = ll;
+    }
+    __syncthreads();
+    constexpr int COLS = HD / 4, LANES = AD_WARPS * 32 / COLS;          // threads per head row, splits added side by side
+    float4* s_acc = reinterpret_cast<float4*>(s_q);
+    const int col = threadIdx.x % COLS, sl = threadIdx.x / COLS;
+    for (int hh = 0; hh < G; ++hh) {
+        const float* p = a.part + ((int64_t)b * a.H + h0 + hh) * a.splits * REC + 4 * col;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int s = sl; s < ns; s += LANES) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(p + (int64_t)s * REC));
+            const float f = s_w[hh * AD_MAX_SPLITS + s];
+            acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
+        }
+        s_acc[threadIdx.x] = acc;
+        __syncthreads();
+        if (sl == 0) {
+            for (int k = 1; k < LANES; ++k) {
+                const float4 v = s_acc[k * COLS + col];
+                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+            }
+            const float ll = s_ml[0][hh][0], inv = ll > 0.0f ? 1.0f / ll : 0.0f;
+            *reinterpret_cast<float4*>(a.out + ((int64_t)b * a.H + h0 + hh) * HD + 4 * col) =
+                make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+        }
+        __syncthreads();
+    }
+}
+
+bool attention_decode_mma_takes(const DecodeMmaArgs& a) {
+    auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    return (a.hd == 64 || a.hd == 128) && aligned(a.kc) && aligned(a.vc) && aligned(a.out) && aligned(a.q);
+}
+
+// fixed_part: the pieces' results go there (fixed_floats of room), else to the workspace.
+int attention_decode_mma(DecodeMmaArgs a, int batch, int max_len, float* fixed_part, int64_t fixed_floats) {
+    const int rows = a.KV * ceil_div(a.group, AD_HEADS);
+    // About eight rounds of blocks over the SMs: enough pieces that a ragged batch ends evenly and a
+    // lone sequence still covers the chip, none shorter than one step of the four warps.
+    const int64_t want = ceil_div64((int64_t)8 * 3 * num_sms(), (int64_t)rows * batch);
+    a.splits = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, AD_MAX_SPLITS), ceil_div(std::max(max_len, 1), AD_STEP)));
+    const int64_t rec = (int64_t)a.H * (a.hd + 4);
+    if (fixed_part) {
+        a.splits = (int)std::max<int64_t>(1, std::min<int64_t>(a.splits, fixed_floats / (batch * rec)));
+        a.part = fixed_part;
+    } else if (a.splits > 1) {
+        void* wsp;
+        int rc = workspace(WS_ATTN).ensure((size_t)batch * rec * a.splits * sizeof(float), &wsp);
+        if (rc) return rc;
+        a.part = static_cast<float*>(wsp);
+    }
+    // one launch, unless the batch has more (sequence, KV head) pairs than there are counters
+    const int per = std::max(1, std::min(65535, AD_MAX_COUNTERS / rows));
+    for (int b0 = 0; b0 < batch; b0 += per) {
+        const int nb = std::min(per, batch - b0);
+        DecodeMmaArgs c = a;
+        c.q += (int64_t)b0 * a.H * a.hd;
+        c.out += (int64_t)b0 * a.H * a.hd;
+        if (a.page_table) c.page_table += (int64_t)b0 * a.max_pages;
+        if (a.seq_lens) c.seq_lens += b0;
+        if (a.splits > 1) c.part += (int64_t)b0 * rec * a.splits;
+        const dim3 grid(a.splits, rows, nb), block(AD_WARPS * 32);
+        const bool paged = a.page_table != nullptr;
+        int rc;
+        if (a.hd == 64) rc = paged ? launch_pdl(attn_decode_mma_kernel<64, true>, grid, block, 0, c) : launch_pdl(attn_decode_mma_kernel<64, false>, grid, block, 0, c);
+        else rc = paged ? launch_pdl(attn_decode_mma_kernel<128, true>, grid, block, 0, c) : launch_pdl(attn_decode_mma_kernel<128, false>, grid, block, 0, c);
+        if (rc) return rc;
+    }
+    return B200_OK;
+}
+
+}  // namespace b200

@@ -86,6 +86,32 @@ def test_decode_paged_ragged_batch(oracle):
     np.testing.assert_allclose(host(out), want, **TOL)
 
 
+@pytest.mark.parametrize("H,KV,hd", [(1, 1, 64), (12, 4, 128), (18, 2, 64), (16, 2, 128)])
+@pytest.mark.parametrize("n", [15, 16, 17, 63, 64, 65, 127, 129, 1000])
+def test_decode_tile_edges(oracle, H, KV, hd, n):
+    """Around the 16-key tiles and the 64-key steps, with 1, 3, 8 and 9 query heads per KV head, queries
+    and scores of very different sizes, one piece (small capacity) and many (large capacity)."""
+    from gpu_util import dev, empty, host, ops
+    r = np.random.default_rng(n + H)
+    q = (r.standard_normal((H, hd)) * 10.0 ** r.uniform(-4, 1, (H, 1))).astype(np.float32)
+    kc = oracle.f32_to_f16(r.standard_normal((n, KV * hd)).astype(np.float32))
+    vc = oracle.f32_to_f16(r.standard_normal((n, KV * hd)).astype(np.float32))
+    want = oracle.attention_decode_ring(q, kc, vc, 1, H, KV, hd, 0, 0, n, n, 0.3, 0)
+    out = empty((H, hd))
+    ops.attention_decode_ring_fp16(dev(q), dev(kc), dev(vc), out, H, KV, hd, 0, 0, n, n, 0.3, None, 0)
+    np.testing.assert_allclose(host(out), want, **TOL)
+    page = 48                                            # pages that the tiles do not divide
+    np_ = -(-n // page)
+    pages = [np.concatenate([c, np.zeros((np_ * page - n, KV * hd), np.uint16)]).reshape(np_, page, KV * hd) for c in (kc, vc)]
+    for cap in (np_, 400):
+        table = np.zeros((1, cap), np.int32)
+        table[0, :np_] = np.arange(np_)[::-1]
+        out = empty((1, H, hd))
+        ops.attention_decode_paged_fp16(dev(q), dev(pages[0][::-1].copy()), dev(pages[1][::-1].copy()), dev(table),
+                                        dev(np.array([n], np.int32)), out, 1, cap, page, H, KV, hd, 0.3)
+        np.testing.assert_allclose(host(out)[0], want, **TOL)
+
+
 @pytest.mark.parametrize("B,T,H,KV,hd", [(1, 1, 4, 2, 32), (2, 37, 12, 4, 64), (1, 130, 12, 4, 128)])
 def test_prefill(oracle, B, T, H, KV, hd):
     from gpu_util import dev, empty, host, ops
