@@ -11,12 +11,12 @@
 //   O[16, hd]      += P . V      the same split of the probabilities; the halves are added at the end
 // q is scaled by a power of two to at most 2^10 before the cut and p runs up to 2^10, so both keep
 // 22 significant bits; K and V are fp16 in memory, products and sums fp32.
-// No shared memory on the way: the contraction over dims is free to permute, so a thread loads 16
-// consecutive bytes of a key (K: dims 32c + 8t ..; V: dims 64w + 8g .. of the four keys its B
-// fragment needs, paired by prmt).  The loads of the next 16 keys are issued as soon as the MMAs
-// have read the registers: 8 KB in flight per warp, 12 warps per SM.
-// 64 sequences of 256 .. 8192 tokens, 32 / 8 heads of 128: 2.50 ms before, 0.295 ms now
-// (1.11 GB: 3.8 TB/s).
+// Every warp keeps a ring of three 16-key stages of its own in shared memory, filled by cp.async and read
+// by ldmatrix (rows padded by 16 bytes: no bank conflicts), so 17 KB per warp are always under way and no
+// block-wide barrier is on the path.  (The same kernel with the rows in registers, loaded one tile ahead:
+// 0.295 ms on the case below, 57 % of the warps' time in load latency.)
+// 64 sequences of 256 .. 8192 tokens, 32 / 8 heads of 128: 2.50 ms before, 0.22 ms now
+// (1.11 GB: 5.1 TB/s, 78 % of the measured copy rate).
 #include <algorithm>
 
 #include "attention_decode.cuh"
@@ -27,6 +27,7 @@ namespace b200 {
 constexpr int AD_WARPS = 4;
 constexpr int AD_HEADS = 8;           // query heads of one KV head per block
 constexpr int AD_TILE = 16;           // keys per warp step
+constexpr int AD_STAGES = 3;
 constexpr int AD_STEP = AD_WARPS * AD_TILE;
 constexpr int AD_MAX_SPLITS = 128;
 constexpr int AD_MAX_COUNTERS = 1 << 16;
@@ -46,6 +47,17 @@ __device__ __forceinline__ uint32_t ad_pack(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
+__device__ __forceinline__ float ad_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ void ad_ldsm(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ad_ldsm_t(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
 // (a, b) as fp16 pairs: the rounded values and what rounding left
 __device__ __forceinline__ void ad_split(float a, float b, uint32_t& hi, uint32_t& lo) {
     const __half2 h = __floats2half2_rn(a, b);
@@ -61,15 +73,28 @@ __device__ __forceinline__ int64_t ad_row(const DecodeMmaArgs& a, const int32_t*
     return j < a.pinned ? j : (int64_t)a.pinned + (a.ring_start + (j - a.pinned)) % a.ring_cap;
 }
 
+template <int HD>
+struct AdSmem {
+    static constexpr int ROW = HD * 2 + 16;                   // bytes of a staged row
+    static constexpr int STAGE = 2 * AD_TILE * ROW;           // K rows, then V rows
+    static constexpr int WARP = AD_STAGES * STAGE;
+    static constexpr int RING = AD_WARPS * WARP;              // re-used for the merges
+    static constexpr int Q = HD / 16 * 32 * 16;
+    static constexpr int BYTES = RING + Q + AD_WARPS * AD_HEADS * 2 * 4 + AD_HEADS * 4 + 16;
+};
+
 // grid (splits, KV * head blocks, batch)
 template <int HD, bool PAGED>
-__global__ void __launch_bounds__(AD_WARPS * 32, 3) attn_decode_mma_kernel(DecodeMmaArgs a) {
-    constexpr int KC = HD / 32, VC = HD / 64;
-    __shared__ uint4 s_q[HD / 16][32];                        // A fragments of Q, one per 16 dims
-    __shared__ float s_o[AD_WARPS][AD_HEADS][HD];
-    __shared__ float s_ml[AD_WARPS][AD_HEADS][2];
-    __shared__ float s_mul[AD_HEADS];                         // score -> log2 units
-    __shared__ int s_last;
+__global__ void __launch_bounds__(AD_WARPS * 32, 2) attn_decode_mma_kernel(DecodeMmaArgs a) {
+    using S = AdSmem<HD>;
+    constexpr int NT = HD / 8;                                // output tiles of 8 dims
+    constexpr int CH = HD / 8;                                // 16-byte pieces of a row
+    extern __shared__ __align__(128) uint8_t ad_smem[];
+    uint4(*s_q)[32] = reinterpret_cast<uint4(*)[32]>(ad_smem + S::RING);          // A fragments of Q, one per 16 dims
+    float(*s_ml)[AD_HEADS][2] = reinterpret_cast<float(*)[AD_HEADS][2]>(ad_smem + S::RING + S::Q);
+    float* s_mul = reinterpret_cast<float*>(s_ml + AD_WARPS);                     // score -> log2 units
+    int* s_last = reinterpret_cast<int*>(s_mul + AD_HEADS);
+    float(*s_o)[AD_HEADS][HD] = reinterpret_cast<float(*)[AD_HEADS][HD]>(ad_smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int gblocks = (a.group + AD_HEADS - 1) / AD_HEADS;
     const int kvh = blockIdx.y / gblocks, g0 = (blockIdx.y % gblocks) * AD_HEADS, b = blockIdx.z;
@@ -86,34 +111,30 @@ __global__ void __launch_bounds__(AD_WARPS * 32, 3) attn_decode_mma_kernel(Decod
     const int32_t* pages = PAGED ? a.page_table + (int64_t)b * a.max_pages : nullptr;
     const int jofs = PAGED ? 0 : a.j0;
     const int64_t stride = (int64_t)a.KV * HD;
-    const uint16_t* kc = a.kc + (int64_t)kvh * HD;
-    const uint16_t* vc = a.vc + (int64_t)kvh * HD;
+    const uint16_t* kc = a.kc + (int64_t)kvh * HD + lane % CH * 8;
+    const uint16_t* vc = a.vc + (int64_t)kvh * HD + lane % CH * 8;
+    const uint32_t ring = smem_u32(ad_smem) + warp * S::WARP;
 
     auto row_of = [&](int j) { return ad_row<PAGED>(a, pages, jofs + min(j, jend - 1)); };   // past the end: the last key again
-    uint4 kr[2][KC], vr[4][VC];
-    auto load_k = [&](int64_t r) {
+    // one 16-key tile into stage s; lane l brings row (i * 32 + l) / CH, piece l % CH; r: the row of key l % 16
+    auto issue = [&](int s, int64_t r) {
+        const uint32_t dst = ring + s * S::STAGE + lane / CH * S::ROW + lane % CH * 16;
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const uint16_t* p = kc + __shfl_sync(0xffffffffu, r, 8 * n + g) * stride + 8 * t;
-#pragma unroll
-            for (int c = 0; c < KC; ++c) kr[n][c] = __ldcg(reinterpret_cast<const uint4*>(p + 32 * c));
+        for (int i = 0; i < AD_TILE * CH / 32; ++i) {
+            const int64_t at = __shfl_sync(0xffffffffu, r, i * (32 / CH) + lane / CH) * stride;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * (32 / CH) * S::ROW), "l"(kc + at) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + AD_TILE * S::ROW + i * (32 / CH) * S::ROW), "l"(vc + at) : "memory");
         }
     };
-    auto load_v = [&](int64_t r) {
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            const uint16_t* p = vc + __shfl_sync(0xffffffffu, r, 2 * t + (n & 1) + 8 * (n >> 1)) * stride + 8 * g;
-#pragma unroll
-            for (int c = 0; c < VC; ++c) vr[n][c] = __ldcg(reinterpret_cast<const uint4*>(p + 64 * c));
-        }
-    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
     int j = jbeg + warp * AD_TILE;
-    int64_t row = 0;
-    if (j < jend) {
-        row = row_of(j + (lane & 15));
-        load_k(row);
-        load_v(row);
+    int64_t row = 0;                                          // of the next tile to bring
+#pragma unroll
+    for (int s = 0; s < AD_STAGES - 1; ++s) {
+        if (j + s * AD_STEP < jend) issue(s, row_of(j + s * AD_STEP + (lane & 15)));
+        commit();
     }
+    if (j + (AD_STAGES - 1) * AD_STEP < jend) row = row_of(j + (AD_STAGES - 1) * AD_STEP + (lane & 15));
     // Q of head g0 + w, w + 4: scaled by 2^-e to at most 2^10, cut, laid out as A fragments
     for (int w = warp; w < AD_HEADS; w += AD_WARPS) {
         const float* q = a.q + ((int64_t)b * a.H + h0 + w) * HD;
@@ -131,40 +152,45 @@ __global__ void __launch_bounds__(AD_WARPS * 32, 3) attn_decode_mma_kernel(Decod
         if (lane == 0) s_mul[w] = ldexpf(a.scale * AD_LOG2E, e - 10);
 #pragma unroll
         for (int i = 0; i < HD / 32; ++i) {
-            // dim 32 i + lane belongs to thread t' = lane / 8, step 2 i + (lane & 4 ? 1 : 0), pair (lane & 2), half (lane & 1)
-            const float x = v[i] * mul;
-            const __half hi = __float2half_rn(x);
-            const __half lo = __float2half_rn(x - __half2float(hi));
-            __half* f = reinterpret_cast<__half*>(&s_q[2 * i + ((lane >> 2) & 1)][4 * w + (lane >> 3)]);
-            const int at = ((lane >> 1) & 1) * 4 + (lane & 1);          // a0 | a1 | a2 | a3, two halves each
-            f[at] = hi;
-            f[at + 2] = lo;
+            // dim x of a step's 16 belongs to thread (x % 8) / 2, register pair x / 8, half x % 2
+            const int x = lane & 15;
+            const float f = v[i] * mul;
+            const __half hi = __float2half_rn(f);
+            const __half lo = __float2half_rn(f - __half2float(hi));
+            __half* dst = reinterpret_cast<__half*>(&s_q[2 * i + (lane >> 4)][4 * w + (x & 7) / 2]) + (x >> 3) * 4 + (x & 1);
+            dst[0] = hi;                                      // a0 | a1 | a2 | a3, two halves each
+            dst[2] = lo;
         }
     }
     __syncthreads();
     const float mul = s_mul[g];
-    float o[VC][8][4], m = -INFINITY, l = 0.0f;
+    float o[NT][4], m = -INFINITY, l = 0.0f;
 #pragma unroll
-    for (int w = 0; w < VC; ++w)
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int n = 0; n < 8; ++n)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) o[w][n][i] = 0.0f;
+        for (int i = 0; i < 4; ++i) o[n][i] = 0.0f;
+    // ldmatrix row addresses inside a stage: K (keys x dims) as it lies, V transposed
+    const uint32_t k_at = ((lane & 7) + (lane >> 4) * 8) * S::ROW + ((lane >> 3) & 1) * 16;
+    const uint32_t v_at = AD_TILE * S::ROW + (lane & 15) * S::ROW + (lane >> 4) * 16;
 
-    for (; j < jend; j += AD_STEP) {
-        const bool more = j + AD_STEP < jend;
-        int64_t next = 0;
-        if (more) next = row_of(j + AD_STEP + (lane & 15));
+    for (int s = 0; j < jend; j += AD_STEP, s = s + 1 == AD_STAGES ? 0 : s + 1) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(AD_STAGES - 2) : "memory");
+        __syncwarp();                                         // this tile is here, and the tile before it is read
+        if (j + (AD_STAGES - 1) * AD_STEP < jend) {
+            issue(s == 0 ? AD_STAGES - 1 : s - 1, row);
+            if (j + AD_STAGES * AD_STEP < jend) row = row_of(j + AD_STAGES * AD_STEP + (lane & 15));
+        }
+        commit();
+        const uint32_t st = ring + s * S::STAGE;
         float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int c = 0; c < KC; ++c) {
-            const uint4 f0 = s_q[2 * c][lane], f1 = s_q[2 * c + 1][lane];
-            ad_mma(s0, f0.x, f0.y, f0.z, f0.w, kr[0][c].x, kr[0][c].y);
-            ad_mma(s1, f0.x, f0.y, f0.z, f0.w, kr[1][c].x, kr[1][c].y);
-            ad_mma(s0, f1.x, f1.y, f1.z, f1.w, kr[0][c].z, kr[0][c].w);
-            ad_mma(s1, f1.x, f1.y, f1.z, f1.w, kr[1][c].z, kr[1][c].w);
+        for (int c = 0; c < HD / 16; ++c) {
+            const uint4 f = s_q[c][lane];
+            uint32_t kr[4];
+            ad_ldsm(st + k_at + c * 32, kr);
+            ad_mma(s0, f.x, f.y, f.z, f.w, kr[0], kr[1]);
+            ad_mma(s1, f.x, f.y, f.z, f.w, kr[2], kr[3]);
         }
-        if (more) load_k(next);
         float x[4] = {(s0[0] + s0[2]) * mul, (s0[1] + s0[3]) * mul, (s1[0] + s1[2]) * mul, (s1[1] + s1[3]) * mul};
         if (j + AD_TILE > jend) {
 #pragma unroll
@@ -175,48 +201,36 @@ __global__ void __launch_bounds__(AD_WARPS * 32, 3) attn_decode_mma_kernel(Decod
         mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
         mn = fmaxf(m, fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2)));
         if (__any_sync(0xffffffffu, mn != m)) {
-            const float corr = exp2f(m - mn);                 // exp2(-inf) = 0 on the first keys
+            const float corr = ad_exp2(m - mn);               // exp2(-inf) = 0 on the first keys
             l *= corr;
 #pragma unroll
-            for (int w = 0; w < VC; ++w)
+            for (int n = 0; n < NT; ++n)
 #pragma unroll
-                for (int n = 0; n < 8; ++n)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) o[w][n][i] *= corr;
+                for (int i = 0; i < 4; ++i) o[n][i] *= corr;
             m = mn;
         }
         uint32_t hi[2], lo[2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = exp2f(x[i] - (m - AD_P_BIAS));
+        for (int i = 0; i < 4; ++i) x[i] = ad_exp2(x[i] - (m - AD_P_BIAS));
         l += (x[0] + x[1]) + (x[2] + x[3]);
         ad_split(x[0], x[1], hi[0], lo[0]);
         ad_split(x[2], x[3], hi[1], lo[1]);
 #pragma unroll
-        for (int w = 0; w < VC; ++w) {
-            const uint32_t* v0 = reinterpret_cast<const uint32_t*>(&vr[0][w]);
-            const uint32_t* v1 = reinterpret_cast<const uint32_t*>(&vr[1][w]);
-            const uint32_t* v2 = reinterpret_cast<const uint32_t*>(&vr[2][w]);
-            const uint32_t* v3 = reinterpret_cast<const uint32_t*>(&vr[3][w]);
-#pragma unroll
-            for (int n = 0; n < 8; ++n) {
-                const uint32_t sel = (n & 1) ? 0x7632u : 0x5410u;
-                ad_mma(o[w][n], hi[0], lo[0], hi[1], lo[1], __byte_perm(v0[n >> 1], v1[n >> 1], sel),
-                       __byte_perm(v2[n >> 1], v3[n >> 1], sel));
-            }
+        for (int n = 0; n < NT; n += 2) {
+            uint32_t vr[4];
+            ad_ldsm_t(st + v_at + n * 16, vr);
+            ad_mma(o[n], hi[0], lo[0], hi[1], lo[1], vr[0], vr[1]);
+            ad_mma(o[n + 1], hi[0], lo[0], hi[1], lo[1], vr[2], vr[3]);
         }
-        if (more) load_v(next);
     }
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                          // the rings become s_o
     if (g < G) {
-        // this thread's dims: 64 w + 16 t + (0 .. 15)
 #pragma unroll
-        for (int w = 0; w < VC; ++w)
-#pragma unroll
-            for (int n = 0; n < 8; ++n) {
-                s_o[warp][g][64 * w + 16 * t + n] = o[w][n][0] + o[w][n][2];
-                s_o[warp][g][64 * w + 16 * t + 8 + n] = o[w][n][1] + o[w][n][3];
-            }
+        for (int n = 0; n < NT; ++n)
+            *reinterpret_cast<float2*>(&s_o[warp][g][8 * n + 2 * t]) = make_float2(o[n][0] + o[n][2], o[n][1] + o[n][3]);
         if (t == 0) { s_ml[warp][g][0] = m; s_ml[warp][g][1] = l; }
     }
     __syncthreads();
@@ -230,7 +244,7 @@ __global__ void __launch_bounds__(AD_WARPS * 32, 3) attn_decode_mma_kernel(Decod
 #pragma unroll
         for (int w = 0; w < AD_WARPS; ++w) {
             const float mw = s_ml[w][hh][0];
-            const float f = mw == -INFINITY ? 0.0f : exp2f(mw - mm);
+            const float f = mw == -INFINITY ? 0.0f : ad_exp2(mw - mm);
             const float4 v = *reinterpret_cast<const float4*>(&s_o[w][hh][c]);
             ll += s_ml[w][hh][1] * f;
             acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
@@ -250,9 +264,9 @@ __global__ void __launch_bounds__(AD_WARPS * 32, 3) attn_decode_mma_kernel(Decod
     __threadfence();
     __syncthreads();
     unsigned int* count = g_ad_count + (int64_t)b * gridDim.y + blockIdx.y;
-    if (threadIdx.x == 0) s_last = atomicAdd(count, 1u) == (unsigned)ns - 1;
+    if (threadIdx.x == 0) *s_last = atomicAdd(count, 1u) == (unsigned)ns - 1;
     __syncthreads();
-    if (!s_last) return;
+    if (!*s_last) return;
     __threadfence();
     if (threadIdx.x == 0) *count = 0;
     float* s_w = &s_o[0][0][0];                               // [G][ns] weights, then the row sums
@@ -269,7 +283,7 @@ __global__ void __launch_bounds__(AD_WARPS * 32, 3) attn_decode_mma_kernel(Decod
         mm = warp_max(mm);
 #pragma unroll
         for (int i = 0; i < AD_MAX_SPLITS / 32; ++i) {
-            const float f = mv[i] == -INFINITY ? 0.0f : exp2f(mv[i] - mm);
+            const float f = mv[i] == -INFINITY ? 0.0f : ad_exp2(mv[i] - mm);
             ll += lv[i] * f;
             if (32 * i + lane < ns) s_w[hh * AD_MAX_SPLITS + 32 * i + lane] = f;
         }
@@ -309,12 +323,24 @@ bool attention_decode_mma_takes(const DecodeMmaArgs& a) {
     return (a.hd == 64 || a.hd == 128) && aligned(a.kc) && aligned(a.vc) && aligned(a.out) && aligned(a.q);
 }
 
+template <int HD, bool PAGED>
+static int launch_ad(dim3 grid, dim3 block, const DecodeMmaArgs& c) {
+    auto kern = attn_decode_mma_kernel<HD, PAGED>;
+    static bool configured = false;
+    if (!configured) {
+        int rc = allow_smem(kern);
+        if (rc) return rc;
+        configured = true;
+    }
+    return launch_pdl(kern, grid, block, AdSmem<HD>::BYTES, c);
+}
+
 // fixed_part: the pieces' results go there (fixed_floats of room), else to the workspace.
 int attention_decode_mma(DecodeMmaArgs a, int batch, int max_len, float* fixed_part, int64_t fixed_floats) {
     const int rows = a.KV * ceil_div(a.group, AD_HEADS);
     // About eight rounds of blocks over the SMs: enough pieces that a ragged batch ends evenly and a
     // lone sequence still covers the chip, none shorter than one step of the four warps.
-    const int64_t want = ceil_div64((int64_t)8 * 3 * num_sms(), (int64_t)rows * batch);
+    const int64_t want = ceil_div64((int64_t)8 * 2 * num_sms(), (int64_t)rows * batch);
     a.splits = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, AD_MAX_SPLITS), ceil_div(std::max(max_len, 1), AD_STEP)));
     const int64_t rec = (int64_t)a.H * (a.hd + 4);
     if (fixed_part) {
@@ -339,8 +365,8 @@ int attention_decode_mma(DecodeMmaArgs a, int batch, int max_len, float* fixed_p
         const dim3 grid(a.splits, rows, nb), block(AD_WARPS * 32);
         const bool paged = a.page_table != nullptr;
         int rc;
-        if (a.hd == 64) rc = paged ? launch_pdl(attn_decode_mma_kernel<64, true>, grid, block, 0, c) : launch_pdl(attn_decode_mma_kernel<64, false>, grid, block, 0, c);
-        else rc = paged ? launch_pdl(attn_decode_mma_kernel<128, true>, grid, block, 0, c) : launch_pdl(attn_decode_mma_kernel<128, false>, grid, block, 0, c);
+        if (a.hd == 64) rc = paged ? launch_ad<64, true>(grid, block, c) : launch_ad<64, false>(grid, block, c);
+        else rc = paged ? launch_ad<128, true>(grid, block, c) : launch_ad<128, false>(grid, block, c);
         if (rc) return rc;
     }
     return B200_OK;
