@@ -154,43 +154,90 @@ __global__ void __launch_bounds__(256) draw_small_kernel(const float* __restrict
     if (threadIdx.x == 0) next[r] = pick;
 }
 
-// The K largest of a row by K passes (ties to the lower id), as sortable words.
-__global__ void __launch_bounds__(1024) topk_rounds_kernel(const float* __restrict__ logits, int V, int K,
-                                                           uint64_t* __restrict__ keys) {
-    __shared__ uint64_t sm[32];
-    __shared__ uint64_t prev;
-    const float* row = logits + (int64_t)blockIdx.x * V;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (threadIdx.x == 0) prev = ~0ull;
-    __syncthreads();
-    for (int r = 0; r < K; ++r) {
-        const uint64_t p = prev;
-        uint64_t mine = 0;
-        for (int i = threadIdx.x; i < V; i += blockDim.x) {
-            const uint64_t c = cand_key(row[i], i);
-            if (c < p && c > mine) mine = c;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const uint64_t other = __shfl_xor_sync(0xffffffffu, mine, o);
-            mine = other > mine ? other : mine;
-        }
-        if (lane == 0) sm[wid] = mine;
-        __syncthreads();
-        if (wid == 0) {
-            uint64_t t = sm[lane];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const uint64_t other = __shfl_xor_sync(0xffffffffu, t, o);
-                t = other > t ? other : t;
+// The K <= 64 largest of a row (ties to the lower id), as sortable words in descending order: every
+// block takes TOPK_SLICE elements to its own K largest, and what the slices of a row left goes through
+// again until one slice holds it (one pass for any vocabulary up to 2048 * 2048 / K).
+//
+// Bound by shared-memory compare steps, not by the 400 KB a row of 100352 logits is.  A slice is sorted
+// only in runs of k2 = the power of two from K, alternately up and down; two neighbouring runs A
+// (descending) and B (ascending) then give the k2 largest of both as max(A[i], B[i]), a bitonic run that
+// log2(k2) steps put in order, and the slice halves: 21 + 7 steps of a 2048-element sort's 66 at K = 64.
+// (K passes of one block over the row took 972 us for K = 40 of 100352; this takes 10.)
+constexpr int TOPK_SLICE = 2048;
+constexpr int TOPK_THREADS = 512;
+__device__ void topk_slice(uint64_t* keys, int k2) {
+    for (int k = 2; k <= k2; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int q = threadIdx.x; q < TOPK_SLICE / 2; q += TOPK_THREADS) {
+                const int i = 2 * q - (q & (j - 1)), p = i + j;
+                const uint64_t a = keys[i], b = keys[p];
+                if ((i & k) == 0 ? a < b : a > b) {
+                    keys[i] = b;
+                    keys[p] = a;
+                }
             }
-            if (lane == 0) {
-                keys[(int64_t)blockIdx.x * K + r] = t;
-                prev = t;
+            __syncthreads();
+        }
+    for (int n = TOPK_SLICE; n > k2; n >>= 1) {
+        uint64_t best[TOPK_SLICE / 2 / TOPK_THREADS];
+#pragma unroll
+        for (int u = 0; u < TOPK_SLICE / 2 / TOPK_THREADS; ++u) {
+            const int q = u * TOPK_THREADS + threadIdx.x;
+            if (q < n / 2) {
+                const int i = 2 * q - (q & (k2 - 1));
+                best[u] = keys[i] > keys[i + k2] ? keys[i] : keys[i + k2];
             }
         }
         __syncthreads();
+#pragma unroll
+        for (int u = 0; u < TOPK_SLICE / 2 / TOPK_THREADS; ++u) {
+            const int q = u * TOPK_THREADS + threadIdx.x;
+            if (q < n / 2) keys[q] = best[u];
+        }
+        __syncthreads();
+        for (int j = k2 >> 1; j > 0; j >>= 1) {
+            for (int q = threadIdx.x; q < n / 4; q += TOPK_THREADS) {
+                const int i = 2 * q - (q & (j - 1)), p = i + j;
+                const uint64_t a = keys[i], b = keys[p];
+                if ((i & k2) == 0 ? a < b : a > b) {
+                    keys[i] = b;
+                    keys[p] = a;
+                }
+            }
+            __syncthreads();
+        }
     }
+}
+
+// grid (slices, rows): n logits of a row, or n words an earlier pass left, to K words per slice.
+__global__ void __launch_bounds__(TOPK_THREADS) topk_slices_kernel(const float* __restrict__ logits, const uint64_t* __restrict__ in,
+                                                                   int64_t row_stride, int n, int K, int k2, uint64_t* __restrict__ out) {
+    __shared__ uint64_t keys[TOPK_SLICE];
+    const int r = blockIdx.y, i0 = blockIdx.x * TOPK_SLICE;
+#pragma unroll
+    for (int u = 0; u < TOPK_SLICE / TOPK_THREADS; ++u) {
+        const int i = i0 + u * TOPK_THREADS + threadIdx.x;
+        uint64_t k = 0;                                       // below every real candidate
+        if (i < n) k = logits ? cand_key(logits[r * row_stride + i], i) : in[r * row_stride + i];
+        keys[u * TOPK_THREADS + threadIdx.x] = k;
+    }
+    __syncthreads();
+    topk_slice(keys, k2);
+    if (threadIdx.x < K) out[((int64_t)r * gridDim.x + blockIdx.x) * K + threadIdx.x] = keys[threadIdx.x];
+}
+
+// The last pass (n <= TOPK_SLICE words per row) and the draw from the K largest.
+__global__ void __launch_bounds__(TOPK_THREADS) topk_draw_kernel(const uint64_t* __restrict__ in, int n, int K, int k2,
+                                                                 float temperature, float top_p, float min_p,
+                                                                 uint64_t* __restrict__ rng, int32_t* __restrict__ next) {
+    __shared__ uint64_t keys[TOPK_SLICE];
+    __shared__ double probs[SAMPLE_TOPK_MAX];
+    const int r = blockIdx.x;
+    for (int i = threadIdx.x; i < TOPK_SLICE; i += TOPK_THREADS) keys[i] = i < n ? in[(int64_t)r * n + i] : 0ull;
+    __syncthreads();
+    topk_slice(keys, k2);
+    const int pick = draw_sorted(keys, probs, K, temperature, top_p, min_p, rng + 4 * r);
+    if (threadIdx.x == 0) next[r] = pick;
 }
 
 // Whole rows sorted in global scratch (keys [rows, n2]) and drawn from the first K.
@@ -470,7 +517,10 @@ static int pow2_at_least(int v) {
 size_t sample_workspace_bytes(const b200_sampling& c, int V, int rows) {
     if (sampling_is_greedy(c) || no_filter(c, V)) return 256;
     const int k = (c.top_k > 0 && c.top_k < V) ? c.top_k : V;
-    if (k <= SAMPLE_TOPK_ROUNDS_MAX) return (size_t)rows * k * 8 + 256;
+    if (k <= SAMPLE_TOPK_MAX) {
+        const size_t first = (size_t)ceil_div(V, TOPK_SLICE) * k;
+        return (size_t)rows * (first + (size_t)ceil_div((int)first, TOPK_SLICE) * k) * 8 + 256;
+    }
     return (size_t)rows * pow2_at_least(V) * 16 + 256;
 }
 
@@ -495,12 +545,24 @@ int sample_rows(float* logits, int V, int rows, const int32_t* hist, int cap, co
         return B200_OK;
     }
     const int k = (c.top_k > 0 && c.top_k < V) ? c.top_k : V;
-    if (k <= SAMPLE_TOPK_ROUNDS_MAX) {
-        uint64_t* keys = static_cast<uint64_t*>(ws);
-        topk_rounds_kernel<<<rows, 1024, 0, st>>>(logits, V, k, keys);
-        B200_LAUNCH_CHECK("topk_rounds_kernel");
-        draw_small_kernel<<<rows, 256, 0, st>>>(nullptr, nullptr, keys, k, c.temperature, c.top_p, c.min_p, rng, next);
-        B200_LAUNCH_CHECK("draw_small_kernel");
+    if (k <= SAMPLE_TOPK_MAX) {
+        const int k2 = std::max(2, pow2_at_least(k));
+        // the passes write to two areas in turn; the first is the larger one
+        uint64_t* area[2] = {static_cast<uint64_t*>(ws), static_cast<uint64_t*>(ws) + (size_t)rows * ceil_div(V, TOPK_SLICE) * k};
+        const uint64_t* in = nullptr;
+        int n = V;
+        for (int pass = 0; pass == 0 || n > TOPK_SLICE; ++pass) {
+            const int slices = ceil_div(n, TOPK_SLICE);
+            for (int r0 = 0; r0 < rows; r0 += 65535)
+                topk_slices_kernel<<<dim3(slices, std::min(rows - r0, 65535)), TOPK_THREADS, 0, st>>>(
+                    in ? nullptr : logits + (int64_t)r0 * V, in ? in + (int64_t)r0 * n : nullptr, n, n, k, k2,
+                    area[pass & 1] + (int64_t)r0 * slices * k);
+            B200_LAUNCH_CHECK("topk_slices_kernel");
+            in = area[pass & 1];
+            n = slices * k;
+        }
+        topk_draw_kernel<<<rows, TOPK_THREADS, 0, st>>>(in, n, k, k2, c.temperature, c.top_p, c.min_p, rng, next);
+        B200_LAUNCH_CHECK("topk_draw_kernel");
         return B200_OK;
     }
     const int n2 = pow2_at_least(V);

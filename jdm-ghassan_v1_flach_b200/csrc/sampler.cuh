@@ -6,7 +6,7 @@
 
 namespace b200 {
 
-constexpr int SAMPLE_TOPK_ROUNDS_MAX = 64;   // up to this K the K largest are picked by K passes; above, by a full sort
+constexpr int SAMPLE_TOPK_MAX = 64;   // up to this K the K largest are selected slice by slice; above, by a full sort
 
 // Device bytes sample_rows needs for `rows` rows of V logits under cfg (0 for greedy).
 size_t sample_workspace_bytes(const b200_sampling& cfg, int V, int rows);

@@ -111,7 +111,7 @@ def test_sample_logits_reproduces_the_reference_draws(oracle, name):
 
 
 def test_sample_logits_full_vocabulary(oracle):
-    """H-Tiny's vocabulary: the K-pass selection (top-k 40), the full sort (top-k 300 and
+    """H-Tiny's vocabulary: the slice-by-slice selection (top-k 40), the full sort (top-k 300 and
     top-p without top-k) and the unfiltered draw."""
     from gpu_util import dev, empty, host, pkg
     lib = pkg.lib()
@@ -248,3 +248,24 @@ def test_score_tokens(oracle):
     dec.reset()
     assert dec.score_tokens(long[:1]) == (0.0, 0)
     dec.close()
+
+
+@pytest.mark.parametrize("V,k", [(70, 3), (2047, 64), (2048, 2), (2049, 33), (100352, 64)])
+def test_topk_slices(oracle, V, k):
+    """The slice-by-slice selection around its slice of 2048, one and two passes, with equal logits on
+    the boundary (the lower ids are in)."""
+    from gpu_util import dev, empty, host, pkg
+    lib = pkg.lib()
+    rows, draws = 3, 12
+    r = np.random.default_rng(V + k)
+    logits = np.round(r.standard_normal((rows, V)) * 4).astype(np.float32) / 2
+    cfg = oracle.sampling_validate(Sampling(temperature=3.0, top_k=k, top_p=1.0, min_p=0.0, repetition_penalty=1.0))
+    s = B200Sampling.of(cfg)
+    st = _states(lib, 40, rows)
+    states = [oracle.rng_state(40 + i) for i in range(rows)]
+    nxt = empty(rows, torch.int32)
+    for _ in range(draws):
+        lib.b200_sample_logits(dev(logits), V, rows, None, 0, None, C.byref(s), st, nxt)
+        order = [np.lexsort((np.arange(V), -logits[i]))[:k].astype(np.int32) for i in range(rows)]
+        want = [oracle.candidates_with_state(logits[i][order[i]], order[i], cfg, states[i]) for i in range(rows)]
+        assert host(nxt).tolist() == want
