@@ -1,0 +1,469 @@
+// The MoE layer for up to eight tokens and packed weights, three kernels on the digit engine
+// (digit_tile.cuh); arithmetic of cpu::moe_forward_bias, core/moe_cpu.cpp:198-288.
+//
+//   1  a few CTAs: router logits (the reference's exact fp32 order) and, in the one that ends last, softmax,
+//      top-K and mixture weights; all others: the shared expert's gate / up with SwiGLU
+//   2  gate / up of the chosen experts with SwiGLU
+//   3  all down projections as one contraction over [shared | expert k ...], the mixture weights folded into
+//      the activations' scales; residual add or plain store
+//
+// A token moves 10.6 MB of weights through these (H-Tiny shape), 1.6 us at the copy rate: what counts is the
+// chain of dependent steps.  So: a tile is 8 gate rows and the same 8 up rows, which end in one lane pair; the
+// router's group sums are formed by all threads and only the ordered additions - one lane per (expert, token),
+// 384 additions of four cycles - are serial; kernel 2 lets kernel 3 start only after its own wait, which
+// proves the routing of kernel 1 complete, so kernel 3 fetches its experts' rows while kernel 2 runs.
+// One token, H-Tiny shape, in the step's graph: 31 us before, DMSTEP.
+#include "digit_tile.cuh"
+#include "route.cuh"
+
+namespace b200 {
+
+constexpr int DM_ROUTER = 4;                  // experts per router CTA
+
+__host__ __device__ inline int dm_chain_stride(int d) { return ((d >> 2) + 31) / 32 * 32 + 4; }   // floats; 4 mod 32: no bank conflicts
+
+// The tile loop shared by the three kernels: rounds of up to G tiles through `sets` sets of stages, each tile's
+// chunks split over P warps.  issue(r): thread 0 starts round r's copies; dot(tile, part, acc): one warp's
+// share; epilogue(tile index, red): all threads.  Returns false when a bounded wait ran out.
+template <int KIND, int MT, typename Issue, typename Dot, typename Epi>
+__device__ __forceinline__ bool dm_rounds(const MoeFusedArgs& a, int n_my, float* red, uint64_t* bar, Issue issue, Dot dot, Epi epilogue) {
+    const int G = a.n_stages, P = a.parts, rounds = (n_my + G - 1) / G;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    bool ok = true;
+    for (int r = 0; r < rounds; ++r) {
+        const int n = min(G, n_my - r * G), set = a.sets == 1 ? 0 : r & 1;
+        float* rr = red + (size_t)(r & 1) * G * P * dg_red_floats(MT);
+        ok = ok && mbar_wait(&bar[set], (a.sets == 1 ? r : r >> 1) & 1, a.status);
+        if (ok) {
+            for (int u = warp; u < n * P; u += DG_WARPS) {
+                const int tile = u / P, part = u - tile * P;
+                DgAcc<MT> acc;
+                acc.clear();
+                dot(set * G + tile, part, acc);
+                dg_finish<KIND, MT>(acc, rr + u * dg_red_floats(MT), lane);
+            }
+        }
+        if (!__syncthreads_and(ok)) break;
+        if (threadIdx.x == 0 && r + 2 < rounds) issue(r + 2);
+        epilogue(r * G, n, rr);
+    }
+    if (!ok && threadIdx.x == 0)              // no copy of this CTA may be left under way
+        for (int set = 0; set < a.sets; ++set)
+            for (int par = 0; par < 2 && !mbar_wait(&bar[set], par, a.status); ++par) {}
+    return ok;
+}
+
+// Stages tokens [m0, m0 + n) of x [., K] (times norm_w when there is one) as slots 0 ..; per-chunk sums of
+// squares to ssq.  The norm factor itself is applied by the epilogue.
+template <int KIND, int MT>
+__device__ __forceinline__ void dm_stage_norm(const MoeFusedArgs& a, const DgX<MT>& xd, int m0, int n, double* ssq) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunks = dg_chunks(a.d);
+    for (int i = warp; i < chunks * n; i += DG_WARPS) {
+        const int m = i / chunks, c = i - m * chunks;
+        float v[8], nw[8];
+        dg_load8(a.x + (int64_t)(m0 + m) * a.d, c * DG_CHUNK + 8 * lane, a.d, v);
+        double ss = 0.0;
+        if (a.norm_w) {
+            dg_load8(a.norm_w, c * DG_CHUNK + 8 * lane, a.d, nw);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                ss += (double)v[j] * (double)v[j];
+                v[j] *= nw[j];
+            }
+        }
+        dg_stage<KIND, MT>(xd, c, m, v, 1.0f, lane);
+        if (a.norm_w) {
+            ss = warp_sum_d(ss);
+            if (lane == 0) ssq[c * MT + m] = ss;
+        }
+    }
+}
+// After a barrier: the norm factors of n tokens by the last warp (visible after the next barrier).
+template <int MT>
+__device__ __forceinline__ void dm_inv(const MoeFusedArgs& a, int n, const double* ssq, float* inv) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == DG_WARPS - 1 && lane < n) {
+        float f = 1.0f;
+        if (a.norm_w) {
+            double ss = 0.0;
+            for (int c = 0; c < dg_chunks(a.d); ++c) ss += ssq[c * MT + lane];
+            const double d = 1.0 / sqrt(ss / (double)a.d + (double)a.eps);
+            f = isfinite(d) ? (float)d : 0.0f;
+        }
+        inv[lane] = f;
+    }
+}
+
+// ---- kernel 1 ------------------------------------------------------------------
+template <int KIND, int MT>
+__global__ void __launch_bounds__(DG_THREADS, 2) dm_router_shared_kernel(MoeFusedArgs a) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint64_t bar[2];
+    __shared__ double red_d[DG_WARPS * 8];
+    __shared__ float inv[8];
+    __shared__ int s_last;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_router = (a.ne + DM_ROUTER - 1) / DM_ROUTER;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        mbar_fence_init();
+    }
+    if ((int)blockIdx.x < n_router) {
+        const int e0 = blockIdx.x * DM_ROUTER, rows = min(DM_ROUTER, a.ne - e0), groups = a.d >> 2, stride = dm_chain_stride(a.d);
+        float* w_s = reinterpret_cast<float*>(smem);                  // [rows][d]
+        float* gs = w_s + DM_ROUTER * a.d;                            // [token * DM_ROUTER + expert][stride]
+        if (threadIdx.x == 0) {
+            mbar_expect_tx(&bar[0], (uint32_t)rows * a.d * 4);
+            tma_load_1d(w_s, a.router_w + (int64_t)e0 * a.d, (uint32_t)rows * a.d * 4, &bar[0]);
+        }
+        pdl_launch_dependents();
+        pdl_wait();
+        if (a.norm_w) {
+            for (int m = 0; m < a.M; ++m) {
+                double ss = 0.0;
+                for (int g = threadIdx.x; g < groups; g += DG_THREADS) {
+                    const float4 v = *reinterpret_cast<const float4*>(a.x + (int64_t)m * a.d + 4 * g);
+                    ss += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w;
+                }
+                ss = warp_sum_d(ss);
+                if (lane == 0) red_d[m * DG_WARPS + warp] = ss;
+            }
+            __syncthreads();
+            if (threadIdx.x < a.M) {
+                double ss = 0.0;
+                for (int w = 0; w < DG_WARPS; ++w) ss += red_d[threadIdx.x * DG_WARPS + w];
+                const double d = 1.0 / sqrt(ss / (double)a.d + (double)a.eps);
+                inv[threadIdx.x] = isfinite(d) ? (float)d : 0.0f;
+            }
+        }
+        __syncthreads();
+        const bool ok = mbar_wait(&bar[0], 0, a.status);
+        // group sums ((a0 b0 + a1 b1) + a2 b2) + a3 b3 of every (token, expert)
+        for (int i = threadIdx.x; i < groups * a.M; i += DG_THREADS) {
+            const int m = i / groups, g = i - m * groups;
+            float4 x = *reinterpret_cast<const float4*>(a.x + (int64_t)m * a.d + 4 * g);
+            if (a.norm_w) {
+                const float4 nw = *reinterpret_cast<const float4*>(a.norm_w + 4 * g);
+                const float f = inv[m];
+                x = make_float4(x.x * f * nw.x, x.y * f * nw.y, x.z * f * nw.z, x.w * f * nw.w);
+            }
+#pragma unroll
+            for (int e = 0; e < DM_ROUTER; ++e) {
+                if (e < rows) {
+                    const float4 b = *reinterpret_cast<const float4*>(w_s + e * a.d + 4 * g);
+                    float t = __fadd_rn(__fmul_rn(x.x, b.x), __fmul_rn(x.y, b.y));
+                    t = __fadd_rn(t, __fmul_rn(x.z, b.z));
+                    gs[(m * DM_ROUTER + e) * stride + g] = __fadd_rn(t, __fmul_rn(x.w, b.w));
+                }
+            }
+        }
+        __syncthreads();
+        // the ordered additions: one lane per chain
+        if (warp == 0) {
+            const int m = lane / DM_ROUTER, e = lane % DM_ROUTER;
+            if (m < a.M && e < rows) {
+                const float4* p = reinterpret_cast<const float4*>(gs + lane * stride);
+                float s = 0.0f;
+#pragma unroll 8
+                for (int g = 0; g < groups >> 2; ++g) {
+                    const float4 v = p[g];
+                    s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
+                }
+                if (ok) a.logits[(int64_t)m * a.ne + e0 + e] = s;
+                __threadfence();
+            }
+            __syncwarp();
+            if (lane == 0) s_last = atomicAdd(a.route_counter, 1) == n_router - 1;
+        }
+        __syncthreads();
+        // whoever counts last finds every logit published (fence before the count, fence after it)
+        if (!s_last) return;
+        __threadfence();
+        if (threadIdx.x == 0) *a.route_counter = 0;                   // ready for the next layer
+        float* s_p = gs + warp * (2 * a.ne + 32);                     // d / 4 * 4 * M floats hold 8 of these: checked by the host
+        if (warp < a.M)
+            route_finish_fast(a.logits + (int64_t)warp * a.ne, a.router_bias, a.ne, a.K, s_p,
+                              a.idx + (int64_t)warp * a.K, a.w + (int64_t)warp * a.K,
+                              a.probs_out ? a.probs_out + (int64_t)warp * a.ne : nullptr, lane);
+        return;
+    }
+    // shared expert: tiles of 8 gate and 8 up rows
+    const int chunks = dg_chunks(a.d), nsub = a.d >> 5, G = a.n_stages;
+    const uint32_t rb = (uint32_t)row_bytes_of(KIND, a.d);
+    DgX<MT> xd;
+    uint8_t* p = xd.carve(smem + (size_t)a.sets * G * a.stage_bytes, chunks);
+    double* ssq = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
+    float* red = reinterpret_cast<float*>(ssq + chunks * MT);
+    const int first = blockIdx.x - n_router, step = gridDim.x - n_router, num_tiles = a.SH / 8;
+    const int n_my = first < num_tiles ? (num_tiles - first + step - 1) / step : 0;
+    auto issue = [&](int r) {
+        const int n = min(G, n_my - r * G), set = a.sets == 1 ? 0 : r & 1;
+        mbar_expect_tx(&bar[set], n * 16 * rb);
+        for (int i = 0; i < n; ++i) {
+            const int64_t at = (int64_t)(first + (r * G + i) * step) * 8 * rb;
+            uint8_t* dst = smem + (size_t)(set * G + i) * a.stage_bytes;
+            tma_load_1d(dst, a.sh_g + at, 8 * rb, &bar[set]);
+            tma_load_1d(dst + 8 * rb, a.sh_u + at, 8 * rb, &bar[set]);
+        }
+    };
+    if (threadIdx.x == 0)
+        for (int r = 0; r < min((n_my + G - 1) / G, 2); ++r) issue(r);
+    pdl_launch_dependents();
+    pdl_wait();
+    dm_stage_norm<KIND, MT>(a, xd, 0, a.M, ssq);
+    __syncthreads();
+    dm_inv<MT>(a, a.M, ssq, inv);
+    dm_rounds<KIND, MT>(a, n_my, red, bar, issue,
+        [&](int stage, int part, DgAcc<MT>& acc) {
+            const uint32_t at = smem_u32(smem) + stage * a.stage_bytes + (lane >> 2) * rb;
+            for (int c = part; c < chunks; c += a.parts) {
+                const uint32_t ac = at + c * (DG_CHUNK / q_block_elems(KIND)) * q_block_bytes(KIND);
+                dg_chunk<KIND, MT>(acc, ac, ac + 8 * rb, xd, c, min(8, nsub - 8 * c), lane);
+            }
+        },
+        [&](int t0, int n, const float* rr) {
+            for (int e = threadIdx.x; e < n * 8 * MT; e += DG_THREADS) {
+                const int m = e % MT, row = e / MT % 8, i = e / (8 * MT);
+                if (m >= a.M) continue;
+                const float* re = rr + i * a.parts * dg_red_floats(MT);
+                const float gt = dg_value<KIND, MT>(re, a.parts, row, m) * inv[m], up = dg_value<KIND, MT>(re, a.parts, row + 8, m) * inv[m];
+                a.sh_act[(int64_t)m * a.SH + (first + (t0 + i) * step) * 8 + row] = silu_acc(gt) * up;
+            }
+        });
+}
+
+// ---- kernel 2 ------------------------------------------------------------------
+// grid (ctas, M): blockIdx.y is the token.
+template <int KIND>
+__global__ void __launch_bounds__(DG_THREADS, 2) dm_gateup_kernel(MoeFusedArgs a) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint64_t bar[2];
+    __shared__ float inv[8];
+    __shared__ int s_idx[16];
+    const int lane = threadIdx.x & 31, m = blockIdx.y;
+    const int chunks = dg_chunks(a.d), nsub = a.d >> 5, G = a.n_stages;
+    const uint32_t rb = (uint32_t)row_bytes_of(KIND, a.d);
+    DgX<1> xd;
+    uint8_t* p = xd.carve(smem + (size_t)a.sets * G * a.stage_bytes, chunks);
+    double* ssq = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
+    float* red = reinterpret_cast<float*>(ssq + chunks);
+    const int per = a.E / 8, num_tiles = a.K * per, first = blockIdx.x, step = gridDim.x;
+    const int n_my = first < num_tiles ? (num_tiles - first + step - 1) / step : 0;
+    auto issue = [&](int r) {
+        const int n = min(G, n_my - r * G), set = a.sets == 1 ? 0 : r & 1;
+        mbar_expect_tx(&bar[set], n * 16 * rb);
+        for (int i = 0; i < n; ++i) {
+            const int tile = first + (r * G + i) * step, k = tile / per;
+            const int64_t at = ((int64_t)s_idx[k] * a.E + (tile - k * per) * 8) * rb;
+            uint8_t* dst = smem + (size_t)(set * G + i) * a.stage_bytes;
+            tma_load_1d(dst, a.gates + at, 8 * rb, &bar[set]);
+            tma_load_1d(dst + 8 * rb, a.ups + at, 8 * rb, &bar[set]);
+        }
+    };
+    if (threadIdx.x == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        mbar_fence_init();
+    }
+    pdl_wait();
+    pdl_launch_dependents();                  // after the wait: kernel 3 may take kernel 1 for complete
+    if (threadIdx.x < 32) {
+        if (lane < a.K) s_idx[lane] = __ldcg(a.idx + (int64_t)m * a.K + lane);
+        __syncwarp();
+        if (lane == 0)
+            for (int r = 0; r < min((n_my + G - 1) / G, 2); ++r) issue(r);
+        __syncwarp();
+    }
+    dm_stage_norm<KIND, 1>(a, xd, m, 1, ssq);
+    __syncthreads();
+    dm_inv<1>(a, 1, ssq, inv);
+    dm_rounds<KIND, 1>(a, n_my, red, bar, issue,
+        [&](int stage, int part, DgAcc<1>& acc) {
+            const uint32_t at = smem_u32(smem) + stage * a.stage_bytes + (lane >> 2) * rb;
+            for (int c = part; c < chunks; c += a.parts) {
+                const uint32_t ac = at + c * (DG_CHUNK / q_block_elems(KIND)) * q_block_bytes(KIND);
+                dg_chunk<KIND, 1>(acc, ac, ac + 8 * rb, xd, c, min(8, nsub - 8 * c), lane);
+            }
+        },
+        [&](int t0, int n, const float* rr) {
+            for (int e = threadIdx.x; e < n * 8; e += DG_THREADS) {
+                const int row = e % 8, i = e / 8, tile = first + (t0 + i) * step, k = tile / per;
+                const float* re = rr + i * a.parts * dg_red_floats(1);
+                const float gt = dg_value<KIND, 1>(re, a.parts, row, 0) * inv[0], up = dg_value<KIND, 1>(re, a.parts, row + 8, 0) * inv[0];
+                a.act[((int64_t)m * a.K + k) * a.E + (tile - k * per) * 8 + row] = silu_acc(gt) * up;
+            }
+        });
+}
+
+// ---- kernel 3 ------------------------------------------------------------------
+// grid (ctas, M).  A tile is 16 output rows: of sh_down (SH wide), then of each chosen expert's down (E wide).
+template <int KIND>
+__global__ void __launch_bounds__(DG_THREADS, 2) dm_down_kernel(MoeFusedArgs a) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint64_t bar[2];
+    __shared__ int s_idx[16];
+    __shared__ float s_w[16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = blockIdx.y;
+    const int sc = dg_chunks(a.SH), ec = dg_chunks(a.E), chunks = sc + a.K * ec, G = a.n_stages;
+    const uint32_t rb_s = a.SH > 0 ? (uint32_t)row_bytes_of(KIND, a.SH) : 0, rb_e = (uint32_t)row_bytes_of(KIND, a.E);
+    DgX<1> xd;
+    uint8_t* p = xd.carve(smem + (size_t)a.sets * G * a.stage_bytes, chunks);
+    float* red = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
+    const int num_tiles = (a.d + 15) / 16, first = blockIdx.x, step = gridDim.x;
+    const int n_my = first < num_tiles ? (num_tiles - first + step - 1) / step : 0;
+    auto issue = [&](int r) {
+        const int n = min(G, n_my - r * G), set = a.sets == 1 ? 0 : r & 1;
+        uint32_t rows_all = 0;
+        for (int i = 0; i < n; ++i) rows_all += min(16, a.d - (first + (r * G + i) * step) * 16);
+        mbar_expect_tx(&bar[set], rows_all * (rb_s + a.K * rb_e));
+        for (int i = 0; i < n; ++i) {
+            const int r0 = (first + (r * G + i) * step) * 16, rows = min(16, a.d - r0);
+            uint8_t* dst = smem + (size_t)(set * G + i) * a.stage_bytes;
+            if (a.SH > 0) tma_load_1d(dst, a.sh_d + (int64_t)r0 * rb_s, rows * rb_s, &bar[set]);
+            for (int k = 0; k < a.K; ++k)
+                tma_load_1d(dst + 16 * (rb_s + k * rb_e), a.downs + ((int64_t)s_idx[k] * a.d + r0) * rb_e, rows * rb_e, &bar[set]);
+        }
+    };
+    if (threadIdx.x < 32) {
+        // the routing is kernel 1's, complete before kernel 2 let this kernel start
+        if (lane < a.K) {
+            s_idx[lane] = __ldcg(a.idx + (int64_t)m * a.K + lane);
+            s_w[lane] = __ldcg(a.w + (int64_t)m * a.K + lane);
+        }
+        __syncwarp();
+        if (lane == 0) {
+            mbar_init(&bar[0], 1);
+            mbar_init(&bar[1], 1);
+            mbar_fence_init();
+            for (int r = 0; r < min((n_my + G - 1) / G, 2); ++r) issue(r);
+        }
+        __syncwarp();
+    }
+    pdl_launch_dependents();
+    __syncthreads();
+    pdl_wait();
+    for (int i = warp; i < chunks; i += DG_WARPS) {
+        float v[8], mul = 1.0f;
+        if (i < sc) {
+            dg_load8(a.sh_act + (int64_t)m * a.SH, i * DG_CHUNK + 8 * lane, a.SH, v);
+        } else {
+            const int k = (i - sc) / ec;
+            dg_load8(a.act + ((int64_t)m * a.K + k) * a.E, (i - sc - k * ec) * DG_CHUNK + 8 * lane, a.E, v);
+            mul = s_w[k];
+        }
+        dg_stage<KIND, 1>(xd, i, 0, v, mul, lane);
+    }
+    float pre = 0.0f;
+    const int e_n = (first + threadIdx.x / 16 * step) * 16 + (threadIdx.x & 15);      // first element of this thread
+    const bool early = !a.out && threadIdx.x < 16 * (unsigned)min(G, n_my) && e_n < a.d;
+    if (early) pre = a.resid[(int64_t)m * a.d + e_n];
+    __syncthreads();
+    dm_rounds<KIND, 1>(a, n_my, red, bar, issue,
+        [&](int stage, int part, DgAcc<1>& acc) {
+            const uint32_t base = smem_u32(smem) + stage * a.stage_bytes, cb = (DG_CHUNK / q_block_elems(KIND)) * q_block_bytes(KIND);
+            for (int c = part; c < chunks; c += a.parts) {
+                uint32_t at, rb;
+                int cc = c, K = a.SH;
+                if (c < sc) {
+                    at = base;
+                    rb = rb_s;
+                } else {
+                    const int k = (c - sc) / ec;
+                    at = base + 16 * (rb_s + k * rb_e);
+                    rb = rb_e;
+                    cc = c - sc - k * ec;
+                    K = a.E;
+                }
+                at += (lane >> 2) * rb + cc * cb;
+                dg_chunk<KIND, 1>(acc, at, at + 8 * rb, xd, c, min(8, (K >> 5) - 8 * cc), lane);
+            }
+        },
+        [&](int t0, int n, const float* rr) {
+            for (int e = threadIdx.x; e < n * 16; e += DG_THREADS) {
+                const int row = e % 16, i = e / 16, col = (first + (t0 + i) * step) * 16 + row;
+                if (col >= a.d) continue;
+                const float v = dg_value<KIND, 1>(rr + i * a.parts * dg_red_floats(1), a.parts, row, 0);
+                const int64_t at = (int64_t)m * a.d + col;
+                if (a.out) a.out[at] = v;
+                else a.resid[at] = (t0 == 0 && e == (int)threadIdx.x ? pre : a.resid[at]) + v * a.res_mult;
+            }
+        });
+}
+
+// ---- host side -----------------------------------------------------------------
+// Stages and contraction split for `share` tiles per CTA of tile_bytes each: the whole share in half an SM, or two
+// sets of as much as fits there, or the same in a whole SM.  Returns the dynamic shared memory, 0 if nothing fits.
+static size_t dm_plan(MoeFusedArgs& a, int share, size_t tile_bytes, int chunks, int mt, size_t fixed, size_t floor_bytes) {
+    a.stage_bytes = (int)((tile_bytes + 127) / 128 * 128);
+    for (const size_t budget : {(size_t)SMEM_BUDGET - 2048, (size_t)SMEM_BUDGET_FULL - 2048})
+        for (int G = std::max(1, std::min(share, 8)); G >= 1; --G) {
+            a.n_stages = G;
+            a.sets = G >= share ? 1 : 2;
+            int best = 1, cost = 1 << 30;
+            for (int p = 1; p <= std::min(chunks, DG_WARPS); ++p) {
+                const int c = ceil_div(G * p, DG_WARPS) * ceil_div(chunks, p);
+                if (c < cost) { cost = c; best = p; }
+            }
+            a.parts = best;
+            const size_t need = std::max(floor_bytes, (size_t)a.sets * G * a.stage_bytes + dg_x_bytes(chunks, mt) + fixed + 64 +
+                                                          (size_t)2 * G * a.parts * dg_red_floats(mt) * 4);
+            if (need <= budget) return need;
+        }
+    return 0;
+}
+template <typename Kern>
+static int dm_launch(Kern kern, bool& configured, dim3 grid, size_t smem, const MoeFusedArgs& a) {
+    if (!configured) {
+        int rc = allow_smem(kern);
+        if (rc) return rc;
+        configured = true;
+    }
+    return launch_pdl(kern, grid, dim3(DG_THREADS), smem, a);
+}
+
+template <int KIND, int MT>
+static int dm_kernel1(MoeFusedArgs a, size_t smem, int grid) {
+    static bool configured = false;
+    return dm_launch(dm_router_shared_kernel<KIND, MT>, configured, dim3(grid), smem, a);
+}
+
+template <int KIND>
+static int dm_kind(const MoeFusedArgs& a) {
+    const int mt = a.M == 1 ? 1 : a.M == 2 ? 2 : a.M <= 4 ? 4 : 8;
+    const size_t rb_d = row_bytes_of(KIND, a.d), rb_e = row_bytes_of(KIND, a.E), rb_s = a.SH > 0 ? row_bytes_of(KIND, a.SH) : 0;
+    const int per_token = std::max(1, num_sms() / a.M);
+    // all three are planned before the first is launched: a layer runs whole or not at all
+    MoeFusedArgs p1 = a, p2 = a, p3 = a;
+    const int n_router = ceil_div(a.ne, DM_ROUTER), sh_tiles = a.SH / 8;
+    const int sh_ctas = std::min(sh_tiles, std::max(8, num_sms() - n_router));
+    const size_t router_bytes = (size_t)DM_ROUTER * a.d * 4 + std::max<size_t>((size_t)DM_ROUTER * a.M * dm_chain_stride(a.d) * 4, (size_t)a.M * (2 * a.ne + 32) * 4);
+    const size_t s1 = dm_plan(p1, sh_ctas ? ceil_div(sh_tiles, sh_ctas) : 0, sh_ctas ? 16 * rb_d : 0, sh_ctas ? dg_chunks(a.d) : 1, mt,
+                              (size_t)dg_chunks(a.d) * mt * 8, router_bytes);
+    const int t2 = a.K * (a.E / 8), g2 = std::min(t2, per_token);
+    const size_t s2 = dm_plan(p2, ceil_div(t2, g2), 16 * rb_d, dg_chunks(a.d), 1, (size_t)dg_chunks(a.d) * 8, 0);
+    const int t3 = ceil_div(a.d, 16), g3 = std::min(t3, per_token);
+    const size_t s3 = dm_plan(p3, ceil_div(t3, g3), 16 * (rb_s + a.K * rb_e), dg_chunks(a.SH) + a.K * dg_chunks(a.E), 1, 0, 0);
+    if (!s1 || !s2 || !s3) return fail(B200_EUNSUPPORTED, "moe_fused: hidden size %d does not fit the shared-memory staging", a.d);
+    int rc = mt == 1 ? dm_kernel1<KIND, 1>(p1, s1, n_router + sh_ctas) : mt == 2 ? dm_kernel1<KIND, 2>(p1, s1, n_router + sh_ctas)
+             : mt == 4 ? dm_kernel1<KIND, 4>(p1, s1, n_router + sh_ctas) : dm_kernel1<KIND, 8>(p1, s1, n_router + sh_ctas);
+    if (rc) return rc;
+    static bool c2 = false, c3 = false;
+    rc = dm_launch(dm_gateup_kernel<KIND>, c2, dim3(g2, a.M), s2, p2);
+    return rc ? rc : dm_launch(dm_down_kernel<KIND>, c3, dim3(g3, a.M), s3, p3);
+}
+
+// moe_fused() for packed weights (kind 0 .. 3); sizes checked there.
+int moe_digit(const MoeFusedArgs& a, int kind) {
+    auto bad = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
+    if (bad(a.x) || bad(a.norm_w) || bad(a.gates) || bad(a.ups) || bad(a.downs) || (a.SH > 0 && (bad(a.sh_g) || bad(a.sh_u) || bad(a.sh_d))))
+        return fail(B200_EUNSUPPORTED, "moe_fused: tensors must be 16-byte aligned");
+    switch (kind) {
+        case 0: return dm_kind<0>(a);
+        case 1: return dm_kind<1>(a);
+        case 2: return dm_kind<2>(a);
+        default: return dm_kind<3>(a);
+    }
+}
+
+}  // namespace b200

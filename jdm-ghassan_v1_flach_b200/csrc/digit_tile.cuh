@@ -1,0 +1,324 @@
+// The few-token dot engine for packed weights: integer tensor-core products of the weights' own
+// integers with the activations cut into base-256 digits.
+//
+// What bounded the engine before it (mma_tile.cuh on fp16 pairs): instructions.  Turning nibbles into
+// fp16, decoding the 6-bit scales to floats and spreading them with eight shuffles took 137 instructions
+// per 1024 Q4_K weights, 215 in the kernels, on SMs that have about 1500 issue slots for the 1024 * 78
+// weights HBM can deliver in a microsecond.  Here a nibble word needs one AND to become an operand:
+//     x = 2^(e - 30) * sum_j 256^j D_j,   |x| < 2^e,  D_j signed bytes, j = 0 .. 3
+// with e the exponent of the largest of the token's 256 activations (so no activation loses more than
+// 2^-31 of that maximum; the fp16 pairs kept 22 bits of each), and for every 32-weight sub-block one
+// mma.m16n8k32 gives sum_k q_k D_jk exactly, the eight columns being the four digits of two tokens.
+// The 6-bit scale of the sub-block multiplies the integer (exact: at most 63 * 32 * 240 * 128 * 4 in 31
+// bits), so a super-block ends in one conversion and one multiply-add per digit, and the minimum terms of
+// its eight sub-blocks are one mma.m16n8k8 with the sub-block sums.  About 40 instructions per 1024
+// weights for one or two tokens, 85 for eight.
+#pragma once
+
+#include "fused_common.cuh"
+
+namespace b200 {
+
+constexpr int DG_WARPS = 8;
+constexpr int DG_THREADS = DG_WARPS * 32;
+constexpr int DG_CHUNK = 256;                 // activations that share a scale
+
+template <int KIND>
+struct DgKind {
+    static constexpr bool mins = KIND == 3 || KIND == 1;
+    // Q4_0 and Q4_1 pair element j with j + 16 of a block in one byte: their operand words are those of
+    // elements 4t and 16 + 4t; the other kinds use 8t and 8t + 4.
+    static constexpr bool split16 = KIND == 0 || KIND == 1;
+};
+
+__host__ __device__ inline int dg_chunks(int K) { return (K + DG_CHUNK - 1) / DG_CHUNK; }
+// Shared-memory bytes of `tokens` staged token slots of K activations.
+__host__ __device__ inline size_t dg_x_bytes(int chunks, int tokens) {
+    return (size_t)chunks * tokens * (DG_CHUNK * 4 + 32 + 4) + 16;
+}
+
+#ifdef __CUDACC__
+// Staged activations: digits [sub-block][token][slot][32 bytes], slot = (digit + sub-block) & 3 (so that
+// the stores of a warp spread over the banks); sub-block sums * 2^-e as two fp16 parts
+// [chunk][part][token][8]; scales 2^e [chunk][token].
+template <int MT>
+struct DgX {
+    uint32_t dig, sum, scale;                 // shared addresses
+    __device__ __forceinline__ uint8_t* carve(uint8_t* p, int chunks) {
+        dig = smem_u32(p);
+        sum = dig + chunks * MT * DG_CHUNK * 4;
+        scale = sum + chunks * MT * 32;
+        return p + dg_x_bytes(chunks, MT);
+    }
+};
+
+__device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float lds_f32(uint32_t a) { return __uint_as_float(lds_u32(a)); }
+__device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts_u2(uint32_t a, uint32_t x, uint32_t y) {
+    asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void sts_u16(uint32_t a, uint16_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(v) : "memory"); }
+template <bool SIGNED_A>
+__device__ __forceinline__ void dg_mma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b) {
+    if (SIGNED_A)
+        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y), "r"(0));
+    else
+        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y), "r"(0));
+}
+__device__ __forceinline__ void dg_mma_f16k8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(b0));
+}
+
+// Lane l's eight activations 256 * chunk + 8 l .. of token m (zeros past K), staged by one whole warp.
+// mul: a factor of the token's contribution, folded into the scale (a mixture weight).
+template <int KIND, int MT>
+__device__ __forceinline__ void dg_stage(const DgX<MT>& xd, int chunk, int m, const float (&v)[8], float mul, int lane) {
+    float mx = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
+    uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+    int e = (int)(bits >> 23) - 126;                                  // every |v| < 2^e
+    e = max(e, -90);
+    const float to_int = __uint_as_float((uint32_t)(127 + 30 - e) << 23), down = __uint_as_float((uint32_t)(127 - e) << 23);
+    uint32_t w[2][4];
+    float sum = 0.0f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t d[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            // the three low bytes become signed by carrying their top bit into the next digit
+            d[i] = ((uint32_t)__float2int_rn(v[4 * h + i] * to_int) + 0x00808080u) ^ 0x00808080u;
+            sum += v[4 * h + i] * down;
+        }
+        const uint32_t p0 = __byte_perm(d[0], d[1], 0x5140), p1 = __byte_perm(d[2], d[3], 0x5140);      // bytes 0, 1 of each
+        const uint32_t p2 = __byte_perm(d[0], d[1], 0x7362), p3 = __byte_perm(d[2], d[3], 0x7362);      // bytes 2, 3
+        w[h][0] = __byte_perm(p0, p1, 0x5410);
+        w[h][1] = __byte_perm(p0, p1, 0x7632);
+        w[h][2] = __byte_perm(p2, p3, 0x5410);
+        w[h][3] = __byte_perm(p2, p3, 0x7632);
+    }
+    const int sub = 8 * chunk + (lane >> 2), l4 = lane & 3;
+    const uint32_t at = xd.dig + (sub * MT + m) * 128;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t a = at + ((j + sub) & 3) * 32;
+        if (DgKind<KIND>::split16) {
+            const int p = l4 < 2 ? 4 * l4 : 4 * (l4 - 2) + 1;         // words 2 l4, 2 l4 + 1 go to pair positions
+            sts_u32(a + 4 * p, w[0][j]);
+            sts_u32(a + 4 * p + 8, w[1][j]);
+        } else {
+            sts_u2(a + 8 * l4, w[0][j], w[1][j]);
+        }
+    }
+    if (DgKind<KIND>::mins) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if (l4 == 0) {
+            const __half hi = __float2half_rn(sum), lo = __float2half_rn(sum - __half2float(hi));
+            const uint32_t a = xd.sum + (chunk * 2 * MT + m) * 16 + (lane >> 2) * 2;
+            sts_u16(a, __half_as_ushort(hi));
+            sts_u16(a + MT * 16, __half_as_ushort(lo));
+        }
+    }
+    if (lane == 0) sts_u32(xd.scale + (chunk * MT + m) * 4, __float_as_uint(__uint_as_float((uint32_t)(127 + e) << 23) * mul));
+}
+
+// Loads for dg_stage; x 16-byte aligned.
+__device__ __forceinline__ void dg_load8(const float* x, int k, int K, float (&v)[8]) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (k < K) {                                                      // K % 32 == 0: a lane has all eight or none
+        a = *reinterpret_cast<const float4*>(x + k);
+        b = *reinterpret_cast<const float4*>(x + k + 4);
+    }
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+// One warp's accumulators for a 16-row tile: f[q] the digit columns of tokens 2 q, 2 q + 1 (lane
+// (g, t): rows g, g + 8; token 2 q + t / 2, digits 2 (t & 1), + 1), mn the minimum terms (rows g,
+// g + 8; tokens 2 t, 2 t + 1).
+template <int MT>
+struct DgAcc {
+    static constexpr int NT = MT <= 2 ? 1 : MT / 2;
+    float f[NT][4], mn[4];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int q = 0; q < NT; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) f[q][i] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mn[i] = 0.0f;
+    }
+};
+
+// Adds one chunk of 256 weights of 16 rows.  row_a / row_b: shared addresses of the chunk in this lane's
+// rows g and g + 8; xc: the chunk's index among the staged activations; nb: its 32-weight blocks (8, fewer
+// in a tail of kinds 0 .. 2).
+template <int KIND, int MT>
+__device__ __forceinline__ void dg_chunk(DgAcc<MT>& acc, uint32_t row_a, uint32_t row_b, const DgX<MT>& xd, int xc, int nb, int lane) {
+    constexpr int NT = DgAcc<MT>::NT;
+    const int g = lane >> 2, t = lane & 3, dgt = g & 3;
+    const uint32_t xb = xd.dig + xc * 8 * MT * 128 + 8 * t + (MT == 1 ? 0 : (g >> 2) * 128);
+    uint32_t xo[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) xo[s] = xb + ((dgt + s) & 3) * 32;
+    float xs[NT];
+#pragma unroll
+    for (int q = 0; q < NT; ++q) xs[q] = lds_f32(xd.scale + (xc * MT + (MT == 1 ? 0 : 2 * q + (t >> 1))) * 4);
+    auto bfrag = [&](int s, int q) { return lds_u2(xo[s & 3] + (s * MT + 2 * q) * 128); };
+    uint32_t ma = 0, mb = 0;                                          // fp16 pairs of the minima of sub-blocks 2 t, 2 t + 1
+    float da, db, dma = 1.0f, dmb = 1.0f;
+    if (KIND == 3) {
+        const uint4 ha = lds_u4(row_a), hb = lds_u4(row_b);
+        const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&ha.x)), fb = __half22float2(*reinterpret_cast<const __half2*>(&hb.x));
+        da = fa.x; db = fb.x; dma = fa.y; dmb = fb.y;
+        const uint32_t sca[2] = {ha.y & 0x3F3F3F3Fu, (ha.w & 0x0F0F0F0Fu) | ((ha.y >> 2) & 0x30303030u)};
+        const uint32_t scb[2] = {hb.y & 0x3F3F3F3Fu, (hb.w & 0x0F0F0F0Fu) | ((hb.y >> 2) & 0x30303030u)};
+        const uint32_t mna = t < 2 ? ha.z & 0x3F3F3F3Fu : ((ha.w >> 4) & 0x0F0F0F0Fu) | ((ha.z >> 2) & 0x30303030u);
+        const uint32_t mnb = t < 2 ? hb.z & 0x3F3F3F3Fu : ((hb.w >> 4) & 0x0F0F0F0Fu) | ((hb.z >> 2) & 0x30303030u);
+        const uint32_t sel = (t & 1) ? 0x4342u : 0x4140u;
+        const __half2 k1024 = __half2half2(__ushort_as_half(0x6400));
+        const uint32_t pa = __byte_perm(mna, 0x64646464u, sel), pb = __byte_perm(mnb, 0x64646464u, sel);
+        const __half2 qa = __hsub2(*reinterpret_cast<const __half2*>(&pa), k1024), qb = __hsub2(*reinterpret_cast<const __half2*>(&pb), k1024);
+        ma = *reinterpret_cast<const uint32_t*>(&qa);
+        mb = *reinterpret_cast<const uint32_t*>(&qb);
+        int lo[NT][4], hi[NT][4];
+#pragma unroll
+        for (int q = 0; q < NT; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { lo[q][i] = 0; hi[q][i] = 0; }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint2 wa = lds_u2(row_a + 16 + 32 * j + 8 * t), wb = lds_u2(row_b + 16 + 32 * j + 8 * t);
+            const int sa0 = (sca[j >> 1] >> (16 * (j & 1))) & 0xFF, sa1 = (sca[j >> 1] >> (16 * (j & 1) + 8)) & 0xFF;
+            const int sb0 = (scb[j >> 1] >> (16 * (j & 1))) & 0xFF, sb1 = (scb[j >> 1] >> (16 * (j & 1) + 8)) & 0xFF;
+#pragma unroll
+            for (int q = 0; q < NT; ++q) {
+                int c[4];
+                dg_mma<false>(c, wa.x & 0x0F0F0F0Fu, wb.x & 0x0F0F0F0Fu, wa.y & 0x0F0F0F0Fu, wb.y & 0x0F0F0F0Fu, bfrag(2 * j, q));
+                lo[q][0] += sa0 * c[0]; lo[q][1] += sa0 * c[1]; lo[q][2] += sb0 * c[2]; lo[q][3] += sb0 * c[3];
+                dg_mma<false>(c, wa.x & 0xF0F0F0F0u, wb.x & 0xF0F0F0F0u, wa.y & 0xF0F0F0F0u, wb.y & 0xF0F0F0F0u, bfrag(2 * j + 1, q));
+                hi[q][0] += sa1 * c[0]; hi[q][1] += sa1 * c[1]; hi[q][2] += sb1 * c[2]; hi[q][3] += sb1 * c[3];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < NT; ++q) {
+            const float ea = da * xs[q], eb = db * xs[q], ga = ea * 0.0625f, gb = eb * 0.0625f;
+            acc.f[q][0] += ea * (float)lo[q][0] + ga * (float)hi[q][0];
+            acc.f[q][1] += ea * (float)lo[q][1] + ga * (float)hi[q][1];
+            acc.f[q][2] += eb * (float)lo[q][2] + gb * (float)hi[q][2];
+            acc.f[q][3] += eb * (float)lo[q][3] + gb * (float)hi[q][3];
+        }
+    } else {
+        constexpr int BB = q_block_bytes(KIND);
+        if (KIND == 1) {
+            // m of blocks 2 t, 2 t + 1 (zero past the row's end: their sums are zero, but the bits may be anything)
+            auto pair = [&](uint32_t row) {
+                const uint32_t m0 = 2 * t < nb ? lds_u32(row + 2 * t * BB) >> 16 : 0u, m1 = 2 * t + 1 < nb ? lds_u32(row + (2 * t + 1) * BB) & 0xFFFF0000u : 0u;
+                return m0 | m1;
+            };
+            ma = pair(row_a);
+            mb = pair(row_b);
+        }
+        // bytes [a, a + 4) at any even address
+        auto word = [&](uint32_t a) { return __funnelshift_r(lds_u32(a & ~3u), lds_u32((a & ~3u) + 4), (a & 2) * 8); };
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            if (s >= nb) break;
+            uint32_t a0, a1, a2, a3;
+            const uint32_t ra = row_a + s * BB, rb = row_b + s * BB;
+            if (KIND == 2) {
+                auto two = [&](uint32_t a, uint32_t& x, uint32_t& y) {
+                    const uint32_t base = a & ~3u, sh = (a & 2) * 8;
+                    const uint32_t w0 = lds_u32(base), w1 = lds_u32(base + 4), w2 = lds_u32(base + 8);
+                    x = __funnelshift_r(w0, w1, sh);
+                    y = __funnelshift_r(w1, w2, sh);
+                };
+                two(ra + 2 + 8 * t, a0, a2);
+                two(rb + 2 + 8 * t, a1, a3);
+            } else {
+                uint32_t wa = KIND == 0 ? word(ra + 2 + 4 * t) : lds_u32(ra + 4 + 4 * t);
+                uint32_t wb = KIND == 0 ? word(rb + 2 + 4 * t) : lds_u32(rb + 4 + 4 * t);
+                if (KIND == 0) { wa ^= 0x88888888u; wb ^= 0x88888888u; }          // 16 (q - 8) as a signed byte
+                a0 = (wa << 4) & 0xF0F0F0F0u; a1 = (wb << 4) & 0xF0F0F0F0u;
+                a2 = wa & 0xF0F0F0F0u; a3 = wb & 0xF0F0F0F0u;
+            }
+            da = half_bits_to_float((uint16_t)lds_u16(ra));
+            db = half_bits_to_float((uint16_t)lds_u16(rb));
+#pragma unroll
+            for (int q = 0; q < NT; ++q) {
+                int c[4];
+                dg_mma<KIND != 1>(c, a0, a1, a2, a3, bfrag(s, q));
+                const float ea = da * xs[q], eb = db * xs[q];
+                acc.f[q][0] += ea * (float)c[0]; acc.f[q][1] += ea * (float)c[1];
+                acc.f[q][2] += eb * (float)c[2]; acc.f[q][3] += eb * (float)c[3];
+            }
+        }
+    }
+    if (DgKind<KIND>::mins) {
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint32_t at = xd.sum + (xc * 2 * MT + min(g, MT - 1)) * 16 + 4 * t;
+        dg_mma_f16k8(c, ma, mb, lds_u32(at));
+        dg_mma_f16k8(c, ma, mb, lds_u32(at + MT * 16));
+        const float x0 = lds_f32(xd.scale + (xc * MT + min(2 * t, MT - 1)) * 4), x1 = lds_f32(xd.scale + (xc * MT + min(2 * t + 1, MT - 1)) * 4);
+        acc.mn[0] += dma * x0 * c[0]; acc.mn[1] += dma * x1 * c[1];
+        acc.mn[2] += dmb * x0 * c[2]; acc.mn[3] += dmb * x1 * c[3];
+    }
+}
+
+// The warp's sums to red[16 rows][MT] and, for kinds with minima, red[16 * MT + ...] (dg_value adds the two).
+constexpr int dg_red_floats(int MT) { return 2 * 16 * MT; }
+template <int KIND, int MT>
+__device__ __forceinline__ void dg_finish(const DgAcc<MT>& acc, float* red, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    const float scale = ((t & 1) ? 65536.0f : 1.0f) * (DgKind<KIND>::split16 ? 0x1p-34f : 0x1p-30f);
+#pragma unroll
+    for (int q = 0; q < DgAcc<MT>::NT; ++q) {
+        float a = (acc.f[q][0] + 256.0f * acc.f[q][1]) * scale, b = (acc.f[q][2] + 256.0f * acc.f[q][3]) * scale;
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        b += __shfl_xor_sync(0xffffffffu, b, 1);
+        const int tok = 2 * q + (t >> 1);
+        if ((t & 1) == 0 && tok < MT) {
+            red[g * MT + tok] = a;
+            red[(g + 8) * MT + tok] = b;
+        }
+    }
+    if (DgKind<KIND>::mins) {
+        float* r = red + 16 * MT;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (2 * t + i < MT) {
+                r[g * MT + 2 * t + i] = KIND == 3 ? -acc.mn[i] : acc.mn[i];
+                r[(g + 8) * MT + 2 * t + i] = KIND == 3 ? -acc.mn[2 + i] : acc.mn[2 + i];
+            }
+    }
+}
+// Element (row, token) from `parts` warps' results, each dg_red_floats apart.
+template <int KIND, int MT>
+__device__ __forceinline__ float dg_value(const float* red, int parts, int row, int tok) {
+    float v = 0.0f;
+    for (int p = 0; p < parts; ++p, red += dg_red_floats(MT)) {
+        v += red[row * MT + tok];
+        if (DgKind<KIND>::mins) v += red[(16 + row) * MT + tok];
+    }
+    return v;
+}
+#endif
+
+}  // namespace b200

@@ -9,6 +9,7 @@
 // dependent launch: barrier set-up, weight streaming and parameter prefetch run
 // before griddepcontrol.wait and overlap the predecessor's tail.
 #include "fused_common.cuh"
+#include "gemv_epilogue.cuh"
 
 namespace b200 {
 
@@ -121,77 +122,15 @@ __global__ void __launch_bounds__(SG_THREADS, 2) stream_gemv_kernel(SgArgs a) {
         const int n = tile * a.rows_per_tile + e_row;
         const bool owner = e_row < rows && e_m < a.M;
         // epilogue operands are fetched before the dot products so their latency hides
-        float pre = 0.0f, st[4] = {0, 0, 0, 0}, wc[5] = {0, 0, 0, 0, 0};
-        float* dst = nullptr;
-        const bool is_conv = EPI == EPI_INPROJ && n >= a.p.d_inner && n < a.p.d_inner + a.p.conv_dim;
-        if (owner) {
-            if (EPI == EPI_RESIDUAL) {
-                dst = a.resid + (int64_t)e_m * a.y_stride + n;
-                pre = *dst;
-            } else if (is_conv && a.p.k <= 5) {
-                const int c = n - a.p.d_inner, win = a.p.k - 1;
-                const float* sp = a.conv_state + ((int64_t)e_m * a.p.conv_dim + c) * win;
-                const float* wp = a.conv_w + (int64_t)c * a.p.k;
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (j < win) st[j] = sp[j];
-#pragma unroll
-                for (int j = 0; j < 5; ++j)
-                    if (j < a.p.k) wc[j] = wp[j];
-                pre = a.conv_b ? a.conv_b[c] : 0.0f;
-            }
-        }
+        GemvEpilogue<EPI> epi;
+        if (owner) epi.prefetch(a, n, e_m);
         if (!ring.wait_full(i)) break;
         float* red_pass = red + (size_t)(i & 1) * RED_BUF;
         tile_compute<KIND, MT>(ring.stage(i), a.row_bytes, rows, a.K, xa, 0, a.M, red_pass, warp, lane);
         ring.release(i);
         consumer_sync();
         if (owner) {
-            float v = red_value<KIND>(red_pass, e_row, e_m) * in_scale;
-            const int m = e_m;
-            if (EPI == EPI_STORE) {
-                yseg[(int64_t)m * ystride + n] = v * a.out_scale;
-            } else if (EPI == EPI_RESIDUAL) {
-                *dst = pre + v * a.res_mult;
-            } else {
-                // Mamba in_proj row n: gate | conv channel (window of raw inputs, oldest
-                // first; unfused ops in the reference's order) | dt
-                const MambaDims& p = a.p;
-                if (n < p.d_inner) {
-                    a.gate[(int64_t)m * p.d_inner + n] = v;
-                } else if (is_conv) {
-                    const int c = n - p.d_inner, win = p.k - 1;
-                    float* sp = a.conv_state + ((int64_t)m * p.conv_dim + c) * win;
-                    float t;
-                    if (p.k <= 5) {
-                        t = pre;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (j < win) {
-                                t = __fadd_rn(t, __fmul_rn(wc[j], st[j]));
-                                if (j > 0) sp[j - 1] = st[j];
-                            }
-                        float wl = wc[0];
-#pragma unroll
-                        for (int j = 1; j < 5; ++j)
-                            if (j == win) wl = wc[j];
-                        t = __fadd_rn(t, __fmul_rn(wl, v));
-                    } else {
-                        const float* wp = a.conv_w + (int64_t)c * p.k;
-                        t = a.conv_b ? a.conv_b[c] : 0.0f;
-                        for (int j = 0; j < win; ++j) {
-                            const float sv = sp[j];
-                            t = __fadd_rn(t, __fmul_rn(wp[j], sv));
-                            if (j > 0) sp[j - 1] = sv;
-                        }
-                        t = __fadd_rn(t, __fmul_rn(wp[win], v));
-                    }
-                    if (win > 0) sp[win - 1] = v;
-                    a.bc[(int64_t)m * p.conv_dim + c] = silu_acc(t);
-                } else {
-                    a.dt_raw[(int64_t)m * p.n_heads + (n - p.d_inner - p.conv_dim)] = v;
-                }
-            }
+            epi.finish(a, n, e_m, red_value<KIND>(red_pass, e_row, e_m) * in_scale, yseg, ystride);
         }
     }
 }
@@ -307,28 +246,25 @@ static int launch_sg_mt(SgArgs a, int grid) {
 int stream_gemv(SgArgs a, int kind, int pro, int epi) {
     B200_REQUIRE(a.M >= 1 && a.M <= 8, "stream_gemv: 1..8 tokens per launch");
     B200_REQUIRE(a.K % 32 == 0 && (kind != 3 || a.K % 256 == 0), "stream_gemv: K not a multiple of the block size");
-    a.row_bytes = row_bytes_of(kind, a.K);
-    const int R = pick_rows(kind, a.row_bytes, a.row_bytes, a.row_bytes, a.N);
-    if (R < 1) return fail(B200_EUNSUPPORTED, "stream_gemv: row size %lld cannot be tiled to 16 bytes", (long long)a.row_bytes);
-    if ((R * a.row_bytes) % 16 != 0 || !tail_tile_ok(a.N, R, a.row_bytes))
-        return fail(B200_EUNSUPPORTED, "stream_gemv: %d rows of %lld bytes cannot be tiled to 16 bytes", a.N, (long long)a.row_bytes);
-    a.rows_per_tile = R;
-    a.num_tiles = ceil_div(a.N, R);
-    a.t1 = a.t2 = a.num_tiles;
-    if (a.N2 > 0 || a.N3 > 0) {
+    B200_REQUIRE(((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.w2) | reinterpret_cast<uintptr_t>(a.w3)) & 15) == 0,
+                 "stream_gemv: weights must be 16-byte aligned");
+    if (a.N2 > 0 || a.N3 > 0)
         B200_REQUIRE(epi == EPI_STORE && a.N2 > 0 && a.w2 && a.y2 && (a.N3 == 0 || (a.w3 && a.y3)),
                      "stream_gemv: extra matrices need the store epilogue and their pointers");
-        B200_REQUIRE(((reinterpret_cast<uintptr_t>(a.w2) | reinterpret_cast<uintptr_t>(a.w3)) & 15) == 0,
-                     "stream_gemv: weights must be 16-byte aligned");
-        if (!tail_tile_ok(a.N2, R, a.row_bytes) || (a.N3 > 0 && !tail_tile_ok(a.N3, R, a.row_bytes)))
-            return fail(B200_EUNSUPPORTED, "stream_gemv: rows of %lld bytes cannot be tiled to 16 bytes", (long long)a.row_bytes);
-        a.t2 = a.t1 + ceil_div(a.N2, R);
-        a.num_tiles = a.t2 + ceil_div(a.N3, R);
-    }
-    a.stage_bytes = (int)((R * a.row_bytes + 127) / 128 * 128);
+    a.row_bytes = row_bytes_of(kind, a.K);
     a.status = stream_status_ptr();
     B200_REQUIRE(a.status, "stream_gemv: status word allocation failed");
-    B200_REQUIRE((reinterpret_cast<uintptr_t>(a.w) & 15) == 0, "stream_gemv: weights must be 16-byte aligned");
+    // Rows per tile; a bulk copy moves a multiple of 16 bytes, the last tile of each matrix too.
+    const int R = pick_rows(kind, a.row_bytes, a.row_bytes, a.row_bytes, a.N);
+    if (R < 1 || (R * a.row_bytes) % 16 != 0 || !tail_tile_ok(a.N, R, a.row_bytes) || !tail_tile_ok(a.N2, R, a.row_bytes) ||
+        !tail_tile_ok(a.N3, R, a.row_bytes))
+        return fail(B200_EUNSUPPORTED, "stream_gemv: rows of %lld bytes cannot be tiled to 16 bytes", (long long)a.row_bytes);
+    if (kind <= 3) return digit_gemv(a, kind, pro, epi);
+    a.rows_per_tile = R;
+    a.t1 = ceil_div(a.N, R);
+    a.t2 = a.t1 + ceil_div(a.N2, R);
+    a.num_tiles = a.t2 + ceil_div(a.N3, R);
+    a.stage_bytes = (int)((R * a.row_bytes + 127) / 128 * 128);
     const int grid = std::min(a.num_tiles, num_sms());
 #define SG_DISPATCH(KIND)                                                                                   \
     if (pro == PRO_RMS && epi == EPI_STORE) return launch_sg_mt<KIND, PRO_RMS, EPI_STORE>(a, grid);         \
@@ -336,14 +272,8 @@ int stream_gemv(SgArgs a, int kind, int pro, int epi) {
     if (pro == PRO_NONE && epi == EPI_RESIDUAL) return launch_sg_mt<KIND, PRO_NONE, EPI_RESIDUAL>(a, grid); \
     if (pro == PRO_NONE && epi == EPI_STORE) return launch_sg_mt<KIND, PRO_NONE, EPI_STORE>(a, grid);       \
     return fail(B200_EINVAL, "stream_gemv: unsupported prologue/epilogue pair");
-    switch (kind) {
-        case 0: SG_DISPATCH(0)
-        case 1: SG_DISPATCH(1)
-        case 2: SG_DISPATCH(2)
-        case 3: SG_DISPATCH(3)
-        case KIND_F16: SG_DISPATCH(KIND_F16)
-        default: SG_DISPATCH(KIND_F32)
-    }
+    if (kind == KIND_F16) { SG_DISPATCH(KIND_F16) }
+    SG_DISPATCH(KIND_F32)
 #undef SG_DISPATCH
 }
 

@@ -457,14 +457,8 @@ int moe_fused(MoeFusedArgs a, int kind) {
     a.status = stream_status_ptr();
     a.route_counter = a.status ? a.status + 8 : nullptr;      // a word of the same zero-initialised block
     B200_REQUIRE(a.status, "moe_fused: status word allocation failed");
-    switch (kind) {
-        case 0: return moe_fused_kind<0>(a);
-        case 1: return moe_fused_kind<1>(a);
-        case 2: return moe_fused_kind<2>(a);
-        case 3: return moe_fused_kind<3>(a);
-        case KIND_F16: return moe_fused_kind<KIND_F16>(a);
-        default: return moe_fused_kind<KIND_F32>(a);
-    }
+    if (kind <= 3) return moe_digit(a, kind);
+    return kind == KIND_F16 ? moe_fused_kind<KIND_F16>(a) : moe_fused_kind<KIND_F32>(a);
 }
 
 }  // namespace b200

