@@ -6,26 +6,31 @@
 // the tiles' products with the contraction split over the warps, one barrier, the epilogue.  The RMSNorm
 // factor is a scalar of the token and is applied there, so its sum of squares is off that chain.
 // Larger shares go round by round through two sets of stages.
-// In_proj of the H-Tiny shape ([6448, 1536] Q4_K, one token) in the step's graph: DGSTEP.
+// In_proj of the H-Tiny shape ([6448, 1536] Q4_K, one token) in the step's graph:
+// 7.6 us before, 4.5 now, of which 1.5 are the hand-over between the two launches.
 #include "digit_tile.cuh"
 #include "gemv_epilogue.cuh"
 
 namespace b200 {
 
+constexpr int DG_MAX_SETS = 4;
+constexpr size_t DG_SMEM_MAX = 224 * 1024;
+
 template <int KIND, int MT, int PRO, int EPI>
-__global__ void __launch_bounds__(DG_THREADS, 2) dg_gemv_kernel(SgArgs a) {
+__global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dg_gemv_kernel(SgArgs a) {
+    constexpr int W = dg_warps(MT), ELEMS = 16 * MT;
     extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint64_t bar[DG_MAX_SETS];
+    __shared__ float inv[8];
     const int G = a.n_stages, P = a.parts, chunks = dg_chunks(a.K), nsub = a.K >> 5;
-    DgX<MT> xd;
+    DgX<KIND, MT> xd;
     uint8_t* p = xd.carve(smem + (size_t)a.sets * G * a.stage_bytes, chunks);
     double* ssq = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
-    float* inv = reinterpret_cast<float*>(ssq + (PRO == PRO_RMS ? chunks : 1) * MT);
-    float* red = inv + 8;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(red + 2 * G * P * dg_red_floats(MT));
+    float* red = reinterpret_cast<float*>(ssq + (PRO == PRO_RMS ? chunks : 0) * MT);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int first = blockIdx.x, step = gridDim.x;
-    const int n_my = first < a.num_tiles ? (a.num_tiles - first + step - 1) / step : 0;
-    const int rounds = (n_my + G - 1) / G;
+    const int n_my = a.share + (first < a.share_rem ? 1 : 0);        // tiles of this CTA
+    const int rounds = a.sets == 1 ? 1 : (n_my + G - 1) / G;
 
     // tile -> matrix of the launch, first row
     struct Seg { const uint8_t* w; float* y; int N, y_stride, r0; };
@@ -38,37 +43,71 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dg_gemv_kernel(SgArgs a) {
         }
         return s;
     };
-    auto issue = [&](int r) {                                         // one thread: the copies of round r
-        const int n = min(G, n_my - r * G), set = a.sets == 1 ? 0 : r & 1;
+    auto issue = [&](int r, int set) {                                // one thread: the copies of round r
+        const int n = min(G, n_my - r * G);
         uint32_t total = 0;
         for (int i = 0; i < n; ++i) {
             const Seg s = seg_of(first + (r * G + i) * step);
-            total += (uint32_t)(min(a.rows_per_tile, s.N - s.r0) * a.row_bytes);
+            total += (uint32_t)(min(a.rows_per_tile, s.N - s.r0) * (int)a.row_bytes);
         }
         mbar_expect_tx(&bar[set], total);
         for (int i = 0; i < n; ++i) {
             const Seg s = seg_of(first + (r * G + i) * step);
             tma_load_1d(smem + (size_t)(set * G + i) * a.stage_bytes, s.w + (int64_t)s.r0 * a.row_bytes,
-                        (uint32_t)(min(a.rows_per_tile, s.N - s.r0) * a.row_bytes), &bar[set]);
+                        (uint32_t)(min(a.rows_per_tile, s.N - s.r0) * (int)a.row_bytes), &bar[set]);
         }
     };
     if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int i = 0; i < a.sets; ++i) mbar_init(&bar[i], 1);
         mbar_fence_init();
-        for (int r = 0; r < min(rounds, 2); ++r) issue(r);            // the weights do not depend on the previous kernel
+        for (int r = 0; r < min(rounds, a.sets); ++r) issue(r, r);    // the weights do not depend on the previous kernel
     }
     pdl_launch_dependents();
+    // element e of round r: token, output row; false when it does not exist
+    auto element = [&](int r, int e, Seg& s, int& n_out, int& m) {
+        m = e % MT;
+        const int row = e / MT % 16;
+        s = seg_of(first + (r * G + e / ELEMS) * step);
+        n_out = s.r0 + row;
+        return m < a.M && row < a.rows_per_tile && n_out < s.N;
+    };
+    // This thread's first element of round 0: what its epilogue reads is under way before the products.  The
+    // convolution's window and taps are older than the previous kernel, the residual stream is not.
+    GemvEpilogue<EPI> epi;
+    Seg s0;
+    int n0 = 0, m0 = 0;
+    const bool own = (int)threadIdx.x < min(G, n_my) * ELEMS && element(0, threadIdx.x, s0, n0, m0);
+    if (EPI == EPI_INPROJ && own) epi.prefetch(a, n0, m0);
     float nw[8];
-    if (PRO == PRO_RMS) dg_load8(a.norm_w, (warp % chunks) * DG_CHUNK + 8 * lane, a.K, nw);
+    if (PRO == PRO_RMS) {
+        const int c = MT == 1 ? warp : warp - dg_div(warp, a.chunks_inv) * chunks;
+        dg_load8<false>(a.norm_w, c * DG_CHUNK + 8 * lane, a.K, nw);
+    }
     pdl_wait();
 
-    for (int i = warp; i < chunks * a.M; i += DG_WARPS) {
-        const int m = i / chunks, c = i - m * chunks;
+    if (EPI == EPI_RESIDUAL && own) epi.prefetch(a, n0, m0);
+    if (PRO != PRO_RMS && a.in_partials) {
+        // the gated norm's factors from the state update's partial sums, by warps that stage least
+        for (int m = W - 1 - warp; m < a.M; m += W) {
+            const double* q = a.in_partials + (int64_t)m * a.n_partials;
+            double t = 0.0;
+            for (int i0 = 0; i0 < a.n_partials; i0 += 512) {
+                double v[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = i0 + 32 * i + lane < a.n_partials ? __ldcg(q + i0 + 32 * i + lane) : 0.0;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) t += v[i];
+            }
+            t = warp_sum_d(t);
+            if (lane == 0) inv[m] = 1.0f / sqrtf((float)(t / (double)a.in_dim) + a.eps);
+        }
+    }
+    for (int i = warp; i < chunks * a.M; i += W) {
+        const int m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
         float v[8];
-        dg_load8(a.x + (int64_t)m * a.x_stride, c * DG_CHUNK + 8 * lane, a.K, v);
+        dg_load8<true>(a.x + (int64_t)m * a.x_stride, c * DG_CHUNK + 8 * lane, a.K, v);
         if (PRO == PRO_RMS) {
-            if (i != warp || c != warp % chunks) dg_load8(a.norm_w, c * DG_CHUNK + 8 * lane, a.K, nw);
+            if (i != warp) dg_load8<false>(a.norm_w, c * DG_CHUNK + 8 * lane, a.K, nw);
             double ss = 0.0;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -82,17 +121,9 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dg_gemv_kernel(SgArgs a) {
             dg_stage<KIND, MT>(xd, c, m, v, 1.0f, lane);
         }
     }
-    if (PRO != PRO_RMS && a.in_partials) {
-        for (int m = DG_WARPS - 1 - warp; m < a.M; m += DG_WARPS) {
-            double t = 0.0;
-            for (int i = lane; i < a.n_partials; i += 32) t += a.in_partials[(int64_t)m * a.n_partials + i];
-            t = warp_sum_d(t);
-            if (lane == 0) inv[m] = 1.0f / sqrtf((float)(t / (double)a.in_dim) + a.eps);
-        }
-    }
     __syncthreads();
     if (PRO == PRO_RMS) {
-        if (warp == DG_WARPS - 1 && lane < a.M) {
+        if (warp == W - 1 && lane < a.M) {
             double ss = 0.0;
             for (int c = 0; c < chunks; ++c) ss += ssq[c * MT + lane];
             const double d = 1.0 / sqrt(ss / (double)a.K + (double)a.eps);
@@ -102,66 +133,52 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dg_gemv_kernel(SgArgs a) {
         if (threadIdx.x < 8) inv[threadIdx.x] = 1.0f;
     }
 
+    const uint32_t ra = min(lane >> 2, a.rows_per_tile - 1) * (uint32_t)a.row_bytes, rb = min((lane >> 2) + 8, a.rows_per_tile - 1) * (uint32_t)a.row_bytes;
     bool ok = true;
-    for (int r = 0; r < rounds; ++r) {
-        const int n = min(G, n_my - r * G), set = a.sets == 1 ? 0 : r & 1;
+    for (int r = 0, set = 0, parity = 0; r < rounds; ++r) {
+        const int n = min(G, n_my - r * G);
         float* rr = red + (size_t)(r & 1) * G * P * dg_red_floats(MT);
-        // element (tile, row, token) this thread finishes first: its operands before the products
-        auto element = [&](int e, Seg& s, int& n_out, int& m) {
-            m = e % MT;
-            const int row = e / MT % 16;
-            s = seg_of(first + (r * G + e / (16 * MT)) * step);
-            n_out = s.r0 + row;
-            return m < a.M && row < a.rows_per_tile && n_out < s.N;
-        };
-        GemvEpilogue<EPI> epi;
-        Seg s0;
-        int n0 = 0, m0 = 0;
-        const bool own = (int)threadIdx.x < n * 16 * MT && element(threadIdx.x, s0, n0, m0);
-        if (own) epi.prefetch(a, n0, m0);
-        ok = ok && mbar_wait(&bar[set], (a.sets == 1 ? r : r >> 1) & 1, a.status);
+        if (r > 0 && EPI == EPI_RESIDUAL && (int)threadIdx.x < n * ELEMS && element(r, threadIdx.x, s0, n0, m0)) epi.prefetch(a, n0, m0);
+        ok = ok && mbar_wait(&bar[set], parity, a.status);
         if (ok) {
-            for (int u = warp; u < n * P; u += DG_WARPS) {
-                const int tile = u / P, part = u - tile * P;
+            for (int u = warp; u < n * P; u += W) {
+                const int tile = dg_div(u, a.parts_inv), part = u - tile * P;
                 const uint32_t base = smem_u32(smem) + (set * G + tile) * a.stage_bytes;
-                const int ra = min(lane >> 2, a.rows_per_tile - 1), rb = min((lane >> 2) + 8, a.rows_per_tile - 1);
-                DgAcc<MT> acc;
+                DgAcc<KIND, MT> acc;
                 acc.clear();
                 for (int c = part; c < chunks; c += P) {
-                    const uint32_t at = base + c * (DG_CHUNK / q_block_elems(KIND)) * q_block_bytes(KIND);
-                    dg_chunk<KIND, MT>(acc, at + ra * (uint32_t)a.row_bytes, at + rb * (uint32_t)a.row_bytes, xd, c, min(8, nsub - 8 * c), lane);
+                    const uint32_t at = base + c * dg_row_chunk<KIND>();
+                    dg_chunk<KIND, MT>(acc, at + ra, at + rb, xd, c, min(8, nsub - 8 * c), lane);
                 }
                 dg_finish<KIND, MT>(acc, rr + u * dg_red_floats(MT), lane);
             }
         }
         if (!__syncthreads_and(ok)) break;
-        if (threadIdx.x == 0 && r + 2 < rounds) issue(r + 2);
-        for (int e = threadIdx.x; e < n * 16 * MT; e += DG_THREADS) {
-            const float* re = rr + e / (16 * MT) * P * dg_red_floats(MT);
+        if (threadIdx.x == 0 && r + a.sets < rounds) issue(r + a.sets, set);
+        for (int e = threadIdx.x; e < n * ELEMS; e += W * 32) {
+            const float* re = rr + e / ELEMS * P * dg_red_floats(MT);
             const int row = e / MT % 16, m = e % MT;
-            if (e == (int)threadIdx.x) {
-                if (own) epi.finish(a, n0, m0, dg_value<KIND, MT>(re, P, row, m) * inv[m], s0.y, s0.y_stride);
-            } else {
-                GemvEpilogue<EPI> ep;
-                Seg s;
-                int nn, mm;
-                if (!element(e, s, nn, mm)) continue;
-                ep.prefetch(a, nn, mm);
-                ep.finish(a, nn, mm, dg_value<KIND, MT>(re, P, row, m) * inv[m], s.y, s.y_stride);
-            }
+            const bool fetched = e == (int)threadIdx.x && (r == 0 || EPI == EPI_RESIDUAL);
+            if (!element(r, e, s0, n0, m0)) continue;
+            if (!fetched) epi.prefetch(a, n0, m0);
+            epi.finish(a, n0, m0, dg_value<KIND, MT>(re, P, row, m) * inv[m], s0.y, s0.y_stride);
+        }
+        if (++set == a.sets) {
+            set = 0;
+            parity ^= 1;
         }
     }
     // a wait that ran out: no copy of this CTA may be left under way
     if (!ok && threadIdx.x == 0)
-        for (int set = 0; set < a.sets; ++set)
+        for (int set = 0; set < min(a.sets, rounds); ++set)
             for (int par = 0; par < 2 && !mbar_wait(&bar[set], par, a.status); ++par) {}
 }
 
-// Warps per tile's contraction: fewest passes of the eight warps over `tiles` tiles, ties to fewer parts.
-static int dg_parts(int tiles, int chunks) {
+// Warps per tile's contraction: fewest passes of the warps over `tiles` tiles, ties to fewer parts.
+int dg_parts(int tiles, int chunks, int warps) {
     int best = 1, cost = 1 << 30;
-    for (int p = 1; p <= std::min(chunks, DG_WARPS); ++p) {
-        const int c = ceil_div(tiles * p, DG_WARPS) * ceil_div(chunks, p);
+    for (int p = 1; p <= std::min(chunks, warps); ++p) {
+        const int c = ceil_div(tiles * p, warps) * ceil_div(chunks, p);
         if (c < cost) { cost = c; best = p; }
     }
     return best;
@@ -169,13 +186,17 @@ static int dg_parts(int tiles, int chunks) {
 
 template <int KIND, int MT, int PRO, int EPI>
 static int launch_dg(SgArgs a) {
+    constexpr int W = dg_warps(MT);
     const int chunks = dg_chunks(a.K);
-    const size_t fixed = dg_x_bytes(chunks, MT) + 16 + (size_t)(PRO == PRO_RMS ? chunks : 1) * MT * 8 + 32 + 16 + 128;
+    if (chunks > 255) return fail(B200_EUNSUPPORTED, "stream_gemv: K = %d does not fit the shared-memory staging", a.K);
+    a.chunks_inv = dg_inv(chunks);
+    const size_t fixed = dg_x_bytes<KIND>(chunks, MT) + 16 + (size_t)(PRO == PRO_RMS ? chunks : 0) * MT * 8 + 128;
     int grid = 0;
     size_t smem = 0;
     // Rows per tile: 16, fewer only for rows so wide that a tile would not fit.  Stages: the CTA's whole
-    // share when it fits half an SM (the next kernel's CTA fits beside it and streams early), else as much
-    // as does, twice; a whole SM only when half of one holds less than that.
+    // share when it fits half an SM (the next kernel's CTA fits beside it and streams early), else two sets of
+    // as much as does; a whole SM for long shares (an fp16 lm_head: two sets of two tiles, whose products take
+    // less time than their 98 KB - one tile at a time, the barriers between them held the stream at 4.3 TB/s).
     for (int R = TILE_ROWS; R >= 1 && !smem; R >>= 1) {
         if ((R * a.row_bytes) % 16 != 0) break;
         a.rows_per_tile = R;
@@ -184,17 +205,24 @@ static int launch_dg(SgArgs a) {
         a.num_tiles = a.t2 + ceil_div(a.N3, R);
         a.stage_bytes = (int)((R * a.row_bytes + 127) / 128 * 128);
         grid = std::min(a.num_tiles, num_sms());
-        const int share = ceil_div(a.num_tiles, grid);
-        for (const size_t budget : {(size_t)SMEM_BUDGET, (size_t)SMEM_BUDGET_FULL}) {
-            for (int G = std::min(share, 8); G >= 1 && !smem; --G) {
-                a.n_stages = G;
-                a.sets = G >= share ? 1 : 2;
-                a.parts = dg_parts(G, chunks);
-                const size_t need = (size_t)a.sets * G * a.stage_bytes + fixed + (size_t)2 * G * a.parts * dg_red_floats(MT) * 4;
-                if (need <= budget) smem = need;
-            }
-            if (smem) break;
-        }
+        const int most = ceil_div(a.num_tiles, grid);
+        a.share = a.num_tiles / grid;
+        a.share_rem = a.num_tiles % grid;
+        auto fits = [&](int G, int sets, size_t budget) {
+            a.n_stages = G;
+            a.sets = sets;
+            a.parts = dg_parts(G, chunks, W);
+            a.parts_inv = dg_inv(a.parts);
+            const size_t need = (size_t)sets * G * a.stage_bytes + fixed + (size_t)2 * G * a.parts * dg_red_floats(MT) * 4;
+            if (need > budget) return false;
+            smem = need;
+            return true;
+        };
+        if (most <= 8 && fits(most, 1, SMEM_BUDGET)) break;
+        if (most <= 8)
+            for (int G = std::min(most - 1, 4); G >= 1 && !smem; --G) fits(G, 2, SMEM_BUDGET);
+        for (int G = std::min(most, 4); G >= 2 && !smem; --G) fits(G, most > G ? 2 : 1, DG_SMEM_MAX);
+        for (int sets = std::min(most, DG_MAX_SETS); sets >= 1 && !smem; --sets) fits(1, sets, DG_SMEM_MAX);
     }
     if (!smem) return fail(B200_EUNSUPPORTED, "stream_gemv: K = %d does not fit the shared-memory staging", a.K);
     auto kern = dg_gemv_kernel<KIND, MT, PRO, EPI>;
@@ -204,7 +232,7 @@ static int launch_dg(SgArgs a) {
         if (rc) return rc;
         configured = true;
     }
-    return launch_pdl(kern, dim3(grid), dim3(DG_THREADS), smem, a);
+    return launch_pdl(kern, dim3(grid), dim3(W * 32), smem, a);
 }
 
 template <int KIND, int PRO, int EPI>
@@ -223,7 +251,7 @@ static int launch_dg_kind(const SgArgs& a, int pro, int epi) {
     return fail(B200_EINVAL, "stream_gemv: unsupported prologue/epilogue pair");
 }
 
-// stream_gemv() for packed weights (kind 0 .. 3); arguments checked there.
+// stream_gemv() for packed and fp16 weights; arguments checked there.
 int digit_gemv(SgArgs a, int kind, int pro, int epi) {
     if ((reinterpret_cast<uintptr_t>(a.x) & 15) != 0 || (a.x_stride & 3) != 0 || (reinterpret_cast<uintptr_t>(a.norm_w) & 15) != 0)
         return fail(B200_EUNSUPPORTED, "stream_gemv: activations must be 16-byte aligned");
@@ -231,7 +259,8 @@ int digit_gemv(SgArgs a, int kind, int pro, int epi) {
         case 0: return launch_dg_kind<0>(a, pro, epi);
         case 1: return launch_dg_kind<1>(a, pro, epi);
         case 2: return launch_dg_kind<2>(a, pro, epi);
-        default: return launch_dg_kind<3>(a, pro, epi);
+        case 3: return launch_dg_kind<3>(a, pro, epi);
+        default: return launch_dg_kind<KIND_F16>(a, pro, epi);
     }
 }
 

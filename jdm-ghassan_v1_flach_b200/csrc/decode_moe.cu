@@ -12,7 +12,8 @@
 // router's group sums are formed by all threads and only the ordered additions - one lane per (expert, token),
 // 384 additions of four cycles - are serial; kernel 2 lets kernel 3 start only after its own wait, which
 // proves the routing of kernel 1 complete, so kernel 3 fetches its experts' rows while kernel 2 runs.
-// One token, H-Tiny shape, in the step's graph: 31 us before, DMSTEP.
+// One token, H-Tiny shape, in the step's graph: 31 us before,
+// 16 now.
 #include "digit_tile.cuh"
 #include "route.cuh"
 
@@ -23,48 +24,49 @@ constexpr int DM_ROUTER = 4;                  // experts per router CTA
 __host__ __device__ inline int dm_chain_stride(int d) { return ((d >> 2) + 31) / 32 * 32 + 4; }   // floats; 4 mod 32: no bank conflicts
 
 // The tile loop shared by the three kernels: rounds of up to G tiles through `sets` sets of stages, each tile's
-// chunks split over P warps.  issue(r): thread 0 starts round r's copies; dot(tile, part, acc): one warp's
-// share; epilogue(tile index, red): all threads.  Returns false when a bounded wait ran out.
-template <int KIND, int MT, typename Issue, typename Dot, typename Epi>
-__device__ __forceinline__ bool dm_rounds(const MoeFusedArgs& a, int n_my, float* red, uint64_t* bar, Issue issue, Dot dot, Epi epilogue) {
-    const int G = a.n_stages, P = a.parts, rounds = (n_my + G - 1) / G;
+// chunks split over P warps.  issue(r, set): one thread starts round r's copies; dot(stage, part, acc): one warp's
+// share; epilogue(first tile, tiles, red): all threads. prepare() stages the activations, barrier included.
+template <int KIND, int MT, typename Prepare, typename Issue, typename Dot, typename Epi>
+__device__ __forceinline__ void dm_rounds(const MoeFusedArgs& a, int n_my, float* red, uint64_t* bar, Prepare prepare, Issue issue, Dot dot, Epi epilogue) {
+    constexpr int W = dg_warps(MT);
+    const int G = a.n_stages, P = a.parts, rounds = a.sets == 1 ? 1 : (n_my + G - 1) / G;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     bool ok = true;
+    prepare();
     for (int r = 0; r < rounds; ++r) {
         const int n = min(G, n_my - r * G), set = a.sets == 1 ? 0 : r & 1;
         float* rr = red + (size_t)(r & 1) * G * P * dg_red_floats(MT);
         ok = ok && mbar_wait(&bar[set], (a.sets == 1 ? r : r >> 1) & 1, a.status);
         if (ok) {
-            for (int u = warp; u < n * P; u += DG_WARPS) {
-                const int tile = u / P, part = u - tile * P;
-                DgAcc<MT> acc;
+            for (int u = warp; u < n * P; u += W) {
+                const int tile = dg_div(u, a.parts_inv), part = u - tile * P;
+                DgAcc<KIND, MT> acc;
                 acc.clear();
                 dot(set * G + tile, part, acc);
                 dg_finish<KIND, MT>(acc, rr + u * dg_red_floats(MT), lane);
             }
         }
         if (!__syncthreads_and(ok)) break;
-        if (threadIdx.x == 0 && r + 2 < rounds) issue(r + 2);
+        if (warp == W - 1 && lane == 0 && r + 2 < rounds) issue(r + 2, set);
         epilogue(r * G, n, rr);
     }
     if (!ok && threadIdx.x == 0)              // no copy of this CTA may be left under way
-        for (int set = 0; set < a.sets; ++set)
+        for (int set = 0; set < min(a.sets, rounds); ++set)
             for (int par = 0; par < 2 && !mbar_wait(&bar[set], par, a.status); ++par) {}
-    return ok;
 }
 
 // Stages tokens [m0, m0 + n) of x [., K] (times norm_w when there is one) as slots 0 ..; per-chunk sums of
 // squares to ssq.  The norm factor itself is applied by the epilogue.
 template <int KIND, int MT>
-__device__ __forceinline__ void dm_stage_norm(const MoeFusedArgs& a, const DgX<MT>& xd, int m0, int n, double* ssq) {
+__device__ __forceinline__ void dm_stage_norm(const MoeFusedArgs& a, const DgX<KIND, MT>& xd, int m0, int n, double* ssq) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunks = dg_chunks(a.d);
-    for (int i = warp; i < chunks * n; i += DG_WARPS) {
-        const int m = i / chunks, c = i - m * chunks;
+    for (int i = warp; i < chunks * n; i += dg_warps(MT)) {
+        const int m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
         float v[8], nw[8];
-        dg_load8(a.x + (int64_t)(m0 + m) * a.d, c * DG_CHUNK + 8 * lane, a.d, v);
+        dg_load8<true>(a.x + (int64_t)(m0 + m) * a.d, c * DG_CHUNK + 8 * lane, a.d, v);
         double ss = 0.0;
         if (a.norm_w) {
-            dg_load8(a.norm_w, c * DG_CHUNK + 8 * lane, a.d, nw);
+            dg_load8<false>(a.norm_w, c * DG_CHUNK + 8 * lane, a.d, nw);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 ss += (double)v[j] * (double)v[j];
@@ -82,7 +84,7 @@ __device__ __forceinline__ void dm_stage_norm(const MoeFusedArgs& a, const DgX<M
 template <int MT>
 __device__ __forceinline__ void dm_inv(const MoeFusedArgs& a, int n, const double* ssq, float* inv) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (warp == DG_WARPS - 1 && lane < n) {
+    if (warp == dg_warps(MT) - 1 && lane < n) {
         float f = 1.0f;
         if (a.norm_w) {
             double ss = 0.0;
@@ -94,14 +96,69 @@ __device__ __forceinline__ void dm_inv(const MoeFusedArgs& a, int n, const doubl
     }
 }
 
+// ---- the router's logits on their way to the CTA that routes ----------------------
+// A logit is its own flag: the word is zero until it is there (the bits are stored inverted below the sign, and
+// the one NaN that would give zero becomes another), so nothing has to be fenced and counted - a fence, an atomic
+// and a second read took 3 us of this kernel's 12.  Kernel 2 puts the words back to zero.  The CTA that polls is
+// the last of the router's, so those it waits for were scheduled before it; the poll is bounded.
+constexpr int DM_MAX_EXPERTS = 256;
+static __device__ uint32_t g_dm_logits[8 * DM_MAX_EXPERTS];
+constexpr uint32_t DM_POLL_LIMIT = 1u << 20;
+
+__device__ __forceinline__ void dm_post(int m, int e, float logit) {
+    uint32_t u = __float_as_uint(logit);
+    if (u == 0x7FFFFFFFu) u = 0x7FC00000u;
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(g_dm_logits + m * DM_MAX_EXPERTS + e), "r"(u ^ 0x7FFFFFFFu) : "memory");
+}
+template <int PER>
+__device__ __forceinline__ void dm_biases(const MoeFusedArgs& a, float (&bs)[PER], int lane) {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) bs[i] = a.router_bias ? a.router_bias[min(32 * i + lane, a.ne - 1)] : 0.0f;
+}
+// One warp per token: waits for the token's logits, routes it.  real = false: a run of the code without either.
+template <int PER>
+__device__ __noinline__ void dm_route(const MoeFusedArgs& a, float* scratch, const float (&bs)[PER], bool real, int warp, int lane) {
+    if (warp >= a.M) return;
+    float v[PER];
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        uint32_t u = 0x7FFFFFFFu;
+        if (real) {
+            const uint32_t* p = g_dm_logits + warp * DM_MAX_EXPERTS + min(32 * i + lane, a.ne - 1);
+            uint32_t it = 0;
+            do asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(u) : "l"(p) : "memory");
+            while (u == 0 && ++it < DM_POLL_LIMIT);
+            ok = ok && u != 0;
+        }
+        v[i] = __uint_as_float(u ^ 0x7FFFFFFFu);
+    }
+    if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) atomicExch(a.status, 1);
+        return;
+    }
+    int idx;
+    float w;
+    route_pick<PER>(v, bs, a.router_bias != nullptr, a.ne, a.K, scratch + warp * a.ne, lane, idx, w);
+    if (!real) return;
+    if (lane < a.K) {
+        a.idx[(int64_t)warp * a.K + lane] = idx;
+        a.w[(int64_t)warp * a.K + lane] = w;
+    }
+    if (a.probs_out)
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+            if (32 * i + lane < a.ne) a.probs_out[(int64_t)warp * a.ne + 32 * i + lane] = v[i];
+}
+
 // ---- kernel 1 ------------------------------------------------------------------
 template <int KIND, int MT>
-__global__ void __launch_bounds__(DG_THREADS, 2) dm_router_shared_kernel(MoeFusedArgs a) {
+__global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(MoeFusedArgs a) {
+    constexpr int W = dg_warps(MT);
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t bar[2];
-    __shared__ double red_d[DG_WARPS * 8];
+    __shared__ double red_d[W * 8];
     __shared__ float inv[8];
-    __shared__ int s_last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_router = (a.ne + DM_ROUTER - 1) / DM_ROUTER;
     if (threadIdx.x == 0) {
@@ -118,87 +175,105 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dm_router_shared_kernel(MoeFuse
             tma_load_1d(w_s, a.router_w + (int64_t)e0 * a.d, (uint32_t)rows * a.d * 4, &bar[0]);
         }
         pdl_launch_dependents();
+        // the CTA that will route: its biases, and a rehearsal of the code
+        float biases[2], biases8[8];
+        if ((int)blockIdx.x == n_router - 1) {
+            if (a.ne <= 64) {
+                dm_biases(a, biases, lane);
+                dm_route<2>(a, gs, biases, false, warp, lane);
+            } else {
+                dm_biases(a, biases8, lane);
+                dm_route<8>(a, gs, biases8, false, warp, lane);
+            }
+        }
         pdl_wait();
         if (a.norm_w) {
             for (int m = 0; m < a.M; ++m) {
                 double ss = 0.0;
-                for (int g = threadIdx.x; g < groups; g += DG_THREADS) {
-                    const float4 v = *reinterpret_cast<const float4*>(a.x + (int64_t)m * a.d + 4 * g);
+                for (int g = threadIdx.x; g < groups; g += W * 32) {
+                    const float4 v = __ldcg(reinterpret_cast<const float4*>(a.x + (int64_t)m * a.d + 4 * g));
                     ss += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w;
                 }
                 ss = warp_sum_d(ss);
-                if (lane == 0) red_d[m * DG_WARPS + warp] = ss;
+                if (lane == 0) red_d[m * W + warp] = ss;
             }
             __syncthreads();
             if (threadIdx.x < a.M) {
                 double ss = 0.0;
-                for (int w = 0; w < DG_WARPS; ++w) ss += red_d[threadIdx.x * DG_WARPS + w];
+#pragma unroll
+                for (int w = 0; w < W; ++w) ss += red_d[threadIdx.x * W + w];
                 const double d = 1.0 / sqrt(ss / (double)a.d + (double)a.eps);
                 inv[threadIdx.x] = isfinite(d) ? (float)d : 0.0f;
             }
         }
         __syncthreads();
         const bool ok = mbar_wait(&bar[0], 0, a.status);
-        // group sums ((a0 b0 + a1 b1) + a2 b2) + a3 b3 of every (token, expert)
-        for (int i = threadIdx.x; i < groups * a.M; i += DG_THREADS) {
-            const int m = i / groups, g = i - m * groups;
-            float4 x = *reinterpret_cast<const float4*>(a.x + (int64_t)m * a.d + 4 * g);
-            if (a.norm_w) {
-                const float4 nw = *reinterpret_cast<const float4*>(a.norm_w + 4 * g);
-                const float f = inv[m];
-                x = make_float4(x.x * f * nw.x, x.y * f * nw.y, x.z * f * nw.z, x.w * f * nw.w);
-            }
+        // group sums ((a0 b0 + a1 b1) + a2 b2) + a3 b3 of every (token, expert); zeros up to whole runs of 32
+        const int padded = (groups + 31) & ~31;
+        for (int m = 0; m < a.M; ++m) {
+            for (int g = threadIdx.x; g < padded; g += W * 32) {
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (g < groups) {
+                    x = __ldcg(reinterpret_cast<const float4*>(a.x + (int64_t)m * a.d + 4 * g));
+                    if (a.norm_w) {
+                        const float4 nw = *reinterpret_cast<const float4*>(a.norm_w + 4 * g);
+                        const float f = inv[m];
+                        x = make_float4(x.x * f * nw.x, x.y * f * nw.y, x.z * f * nw.z, x.w * f * nw.w);
+                    }
+                }
 #pragma unroll
-            for (int e = 0; e < DM_ROUTER; ++e) {
-                if (e < rows) {
-                    const float4 b = *reinterpret_cast<const float4*>(w_s + e * a.d + 4 * g);
-                    float t = __fadd_rn(__fmul_rn(x.x, b.x), __fmul_rn(x.y, b.y));
-                    t = __fadd_rn(t, __fmul_rn(x.z, b.z));
-                    gs[(m * DM_ROUTER + e) * stride + g] = __fadd_rn(t, __fmul_rn(x.w, b.w));
+                for (int e = 0; e < DM_ROUTER; ++e) {
+                    if (e < rows) {
+                        float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (g < groups) b = *reinterpret_cast<const float4*>(w_s + e * a.d + 4 * g);
+                        float t = __fadd_rn(__fmul_rn(x.x, b.x), __fmul_rn(x.y, b.y));
+                        t = __fadd_rn(t, __fmul_rn(x.z, b.z));
+                        gs[(m * DM_ROUTER + e) * stride + g] = __fadd_rn(t, __fmul_rn(x.w, b.w));
+                    }
                 }
             }
         }
         __syncthreads();
-        // the ordered additions: one lane per chain
+        // the ordered additions: one lane per chain, the next 32 sums on their way while 32 are added
         if (warp == 0) {
             const int m = lane / DM_ROUTER, e = lane % DM_ROUTER;
             if (m < a.M && e < rows) {
                 const float4* p = reinterpret_cast<const float4*>(gs + lane * stride);
                 float s = 0.0f;
-#pragma unroll 8
-                for (int g = 0; g < groups >> 2; ++g) {
-                    const float4 v = p[g];
-                    s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
+                float4 cur[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) cur[i] = p[i];
+                for (int g = 32; g <= padded; g += 32) {
+                    float4 nxt[8];
+                    p += g < padded ? 8 : 0;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) nxt[i] = p[i];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, cur[i].x), cur[i].y), cur[i].z), cur[i].w);
+                        cur[i] = nxt[i];
+                    }
                 }
-                if (ok) a.logits[(int64_t)m * a.ne + e0 + e] = s;
-                __threadfence();
+                if (ok) dm_post(m, e0 + e, s);
             }
-            __syncwarp();
-            if (lane == 0) s_last = atomicAdd(a.route_counter, 1) == n_router - 1;
         }
-        __syncthreads();
-        // whoever counts last finds every logit published (fence before the count, fence after it)
-        if (!s_last) return;
-        __threadfence();
-        if (threadIdx.x == 0) *a.route_counter = 0;                   // ready for the next layer
-        float* s_p = gs + warp * (2 * a.ne + 32);                     // d / 4 * 4 * M floats hold 8 of these: checked by the host
-        if (warp < a.M)
-            route_finish_fast(a.logits + (int64_t)warp * a.ne, a.router_bias, a.ne, a.K, s_p,
-                              a.idx + (int64_t)warp * a.K, a.w + (int64_t)warp * a.K,
-                              a.probs_out ? a.probs_out + (int64_t)warp * a.ne : nullptr, lane);
+        if ((int)blockIdx.x == n_router - 1) {
+            if (a.ne <= 64) dm_route<2>(a, gs, biases, true, warp, lane);
+            else dm_route<8>(a, gs, biases8, true, warp, lane);
+        }
         return;
     }
     // shared expert: tiles of 8 gate and 8 up rows
     const int chunks = dg_chunks(a.d), nsub = a.d >> 5, G = a.n_stages;
     const uint32_t rb = (uint32_t)row_bytes_of(KIND, a.d);
-    DgX<MT> xd;
+    DgX<KIND, MT> xd;
     uint8_t* p = xd.carve(smem + (size_t)a.sets * G * a.stage_bytes, chunks);
     double* ssq = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
     float* red = reinterpret_cast<float*>(ssq + chunks * MT);
-    const int first = blockIdx.x - n_router, step = gridDim.x - n_router, num_tiles = a.SH / 8;
-    const int n_my = first < num_tiles ? (num_tiles - first + step - 1) / step : 0;
-    auto issue = [&](int r) {
-        const int n = min(G, n_my - r * G), set = a.sets == 1 ? 0 : r & 1;
+    const int first = blockIdx.x - n_router, step = gridDim.x - n_router;
+    const int n_my = a.share + (first < a.share_rem ? 1 : 0);
+    auto issue = [&](int r, int set) {
+        const int n = min(G, n_my - r * G);
         mbar_expect_tx(&bar[set], n * 16 * rb);
         for (int i = 0; i < n; ++i) {
             const int64_t at = (int64_t)(first + (r * G + i) * step) * 8 * rb;
@@ -208,22 +283,24 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dm_router_shared_kernel(MoeFuse
         }
     };
     if (threadIdx.x == 0)
-        for (int r = 0; r < min((n_my + G - 1) / G, 2); ++r) issue(r);
+        for (int r = 0; r < a.sets && r * G < n_my; ++r) issue(r, r);
     pdl_launch_dependents();
-    pdl_wait();
-    dm_stage_norm<KIND, MT>(a, xd, 0, a.M, ssq);
-    __syncthreads();
-    dm_inv<MT>(a, a.M, ssq, inv);
-    dm_rounds<KIND, MT>(a, n_my, red, bar, issue,
-        [&](int stage, int part, DgAcc<MT>& acc) {
+    dm_rounds<KIND, MT>(a, n_my, red, bar,
+        [&] {
+            pdl_wait();
+            dm_stage_norm<KIND, MT>(a, xd, 0, a.M, ssq);
+            __syncthreads();
+            dm_inv<MT>(a, a.M, ssq, inv);
+        }, issue,
+        [&](int stage, int part, DgAcc<KIND, MT>& acc) {
             const uint32_t at = smem_u32(smem) + stage * a.stage_bytes + (lane >> 2) * rb;
             for (int c = part; c < chunks; c += a.parts) {
-                const uint32_t ac = at + c * (DG_CHUNK / q_block_elems(KIND)) * q_block_bytes(KIND);
+                const uint32_t ac = at + c * dg_row_chunk<KIND>();
                 dg_chunk<KIND, MT>(acc, ac, ac + 8 * rb, xd, c, min(8, nsub - 8 * c), lane);
             }
         },
         [&](int t0, int n, const float* rr) {
-            for (int e = threadIdx.x; e < n * 8 * MT; e += DG_THREADS) {
+            for (int e = threadIdx.x; e < n * 8 * MT; e += W * 32) {
                 const int m = e % MT, row = e / MT % 8, i = e / (8 * MT);
                 if (m >= a.M) continue;
                 const float* re = rr + i * a.parts * dg_red_floats(MT);
@@ -236,7 +313,8 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dm_router_shared_kernel(MoeFuse
 // ---- kernel 2 ------------------------------------------------------------------
 // grid (ctas, M): blockIdx.y is the token.
 template <int KIND>
-__global__ void __launch_bounds__(DG_THREADS, 2) dm_gateup_kernel(MoeFusedArgs a) {
+__global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_gateup_kernel(MoeFusedArgs a) {
+    constexpr int W = dg_warps(1);
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t bar[2];
     __shared__ float inv[8];
@@ -244,51 +322,55 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dm_gateup_kernel(MoeFusedArgs a
     const int lane = threadIdx.x & 31, m = blockIdx.y;
     const int chunks = dg_chunks(a.d), nsub = a.d >> 5, G = a.n_stages;
     const uint32_t rb = (uint32_t)row_bytes_of(KIND, a.d);
-    DgX<1> xd;
+    DgX<KIND, 1> xd;
     uint8_t* p = xd.carve(smem + (size_t)a.sets * G * a.stage_bytes, chunks);
     double* ssq = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
     float* red = reinterpret_cast<float*>(ssq + chunks);
-    const int per = a.E / 8, num_tiles = a.K * per, first = blockIdx.x, step = gridDim.x;
-    const int n_my = first < num_tiles ? (num_tiles - first + step - 1) / step : 0;
-    auto issue = [&](int r) {
-        const int n = min(G, n_my - r * G), set = a.sets == 1 ? 0 : r & 1;
+    const int per = a.E / 8, first = blockIdx.x, step = gridDim.x;      // tiles per expert
+    const int n_my = a.share + (first < a.share_rem ? 1 : 0);
+    auto issue = [&](int r, int set) {
+        const int n = min(G, n_my - r * G);
         mbar_expect_tx(&bar[set], n * 16 * rb);
         for (int i = 0; i < n; ++i) {
-            const int tile = first + (r * G + i) * step, k = tile / per;
+            const int tile = first + (r * G + i) * step, k = __umulhi(tile, a.per_inv);
             const int64_t at = ((int64_t)s_idx[k] * a.E + (tile - k * per) * 8) * rb;
             uint8_t* dst = smem + (size_t)(set * G + i) * a.stage_bytes;
             tma_load_1d(dst, a.gates + at, 8 * rb, &bar[set]);
             tma_load_1d(dst + 8 * rb, a.ups + at, 8 * rb, &bar[set]);
         }
     };
-    if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_fence_init();
-    }
-    pdl_wait();
-    pdl_launch_dependents();                  // after the wait: kernel 3 may take kernel 1 for complete
-    if (threadIdx.x < 32) {
-        if (lane < a.K) s_idx[lane] = __ldcg(a.idx + (int64_t)m * a.K + lane);
-        __syncwarp();
-        if (lane == 0)
-            for (int r = 0; r < min((n_my + G - 1) / G, 2); ++r) issue(r);
-        __syncwarp();
-    }
-    dm_stage_norm<KIND, 1>(a, xd, m, 1, ssq);
-    __syncthreads();
-    dm_inv<1>(a, 1, ssq, inv);
-    dm_rounds<KIND, 1>(a, n_my, red, bar, issue,
-        [&](int stage, int part, DgAcc<1>& acc) {
+    dm_rounds<KIND, 1>(a, n_my, red, bar,
+        [&] {
+            pdl_wait();
+            pdl_launch_dependents();          // after the wait: kernel 3 may take kernel 1 for complete
+            if ((int)threadIdx.x >= (W - 1) * 32) {
+                // the last warp, which stages nothing here (or last): the chosen experts' rows
+                if (lane < a.K) s_idx[lane] = __ldcg(a.idx + (int64_t)m * a.K + lane);
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_init(&bar[0], 1);
+                    mbar_init(&bar[1], 1);
+                    mbar_fence_init();
+                    for (int r = 0; r < a.sets && r * G < n_my; ++r) issue(r, r);
+                }
+                __syncwarp();
+                if (blockIdx.x == 0)
+                    for (int e = lane; e < a.ne; e += 32) g_dm_logits[m * DM_MAX_EXPERTS + e] = 0;
+            }
+            dm_stage_norm<KIND, 1>(a, xd, m, 1, ssq);
+            __syncthreads();
+            dm_inv<1>(a, 1, ssq, inv);
+        }, issue,
+        [&](int stage, int part, DgAcc<KIND, 1>& acc) {
             const uint32_t at = smem_u32(smem) + stage * a.stage_bytes + (lane >> 2) * rb;
             for (int c = part; c < chunks; c += a.parts) {
-                const uint32_t ac = at + c * (DG_CHUNK / q_block_elems(KIND)) * q_block_bytes(KIND);
+                const uint32_t ac = at + c * dg_row_chunk<KIND>();
                 dg_chunk<KIND, 1>(acc, ac, ac + 8 * rb, xd, c, min(8, nsub - 8 * c), lane);
             }
         },
         [&](int t0, int n, const float* rr) {
-            for (int e = threadIdx.x; e < n * 8; e += DG_THREADS) {
-                const int row = e % 8, i = e / 8, tile = first + (t0 + i) * step, k = tile / per;
+            for (int e = threadIdx.x; e < n * 8; e += W * 32) {
+                const int row = e % 8, i = e / 8, tile = first + (t0 + i) * step, k = __umulhi(tile, a.per_inv);
                 const float* re = rr + i * a.parts * dg_red_floats(1);
                 const float gt = dg_value<KIND, 1>(re, a.parts, row, 0) * inv[0], up = dg_value<KIND, 1>(re, a.parts, row + 8, 0) * inv[0];
                 a.act[((int64_t)m * a.K + k) * a.E + (tile - k * per) * 8 + row] = silu_acc(gt) * up;
@@ -299,7 +381,8 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dm_gateup_kernel(MoeFusedArgs a
 // ---- kernel 3 ------------------------------------------------------------------
 // grid (ctas, M).  A tile is 16 output rows: of sh_down (SH wide), then of each chosen expert's down (E wide).
 template <int KIND>
-__global__ void __launch_bounds__(DG_THREADS, 2) dm_down_kernel(MoeFusedArgs a) {
+__global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_down_kernel(MoeFusedArgs a) {
+    constexpr int W = dg_warps(1);
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t bar[2];
     __shared__ int s_idx[16];
@@ -307,13 +390,13 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dm_down_kernel(MoeFusedArgs a) 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = blockIdx.y;
     const int sc = dg_chunks(a.SH), ec = dg_chunks(a.E), chunks = sc + a.K * ec, G = a.n_stages;
     const uint32_t rb_s = a.SH > 0 ? (uint32_t)row_bytes_of(KIND, a.SH) : 0, rb_e = (uint32_t)row_bytes_of(KIND, a.E);
-    DgX<1> xd;
+    DgX<KIND, 1> xd;
     uint8_t* p = xd.carve(smem + (size_t)a.sets * G * a.stage_bytes, chunks);
     float* red = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
-    const int num_tiles = (a.d + 15) / 16, first = blockIdx.x, step = gridDim.x;
-    const int n_my = first < num_tiles ? (num_tiles - first + step - 1) / step : 0;
-    auto issue = [&](int r) {
-        const int n = min(G, n_my - r * G), set = a.sets == 1 ? 0 : r & 1;
+    const int first = blockIdx.x, step = gridDim.x;
+    const int n_my = a.share + (first < a.share_rem ? 1 : 0);
+    auto issue = [&](int r, int set) {
+        const int n = min(G, n_my - r * G);
         uint32_t rows_all = 0;
         for (int i = 0; i < n; ++i) rows_all += min(16, a.d - (first + (r * G + i) * step) * 16);
         mbar_expect_tx(&bar[set], rows_all * (rb_s + a.K * rb_e));
@@ -336,32 +419,33 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dm_down_kernel(MoeFusedArgs a) 
             mbar_init(&bar[0], 1);
             mbar_init(&bar[1], 1);
             mbar_fence_init();
-            for (int r = 0; r < min((n_my + G - 1) / G, 2); ++r) issue(r);
+            for (int r = 0; r < a.sets && r * G < n_my; ++r) issue(r, r);
         }
         __syncwarp();
     }
     pdl_launch_dependents();
     __syncthreads();
-    pdl_wait();
-    for (int i = warp; i < chunks; i += DG_WARPS) {
-        float v[8], mul = 1.0f;
-        if (i < sc) {
-            dg_load8(a.sh_act + (int64_t)m * a.SH, i * DG_CHUNK + 8 * lane, a.SH, v);
-        } else {
-            const int k = (i - sc) / ec;
-            dg_load8(a.act + ((int64_t)m * a.K + k) * a.E, (i - sc - k * ec) * DG_CHUNK + 8 * lane, a.E, v);
-            mul = s_w[k];
-        }
-        dg_stage<KIND, 1>(xd, i, 0, v, mul, lane);
-    }
     float pre = 0.0f;
-    const int e_n = (first + threadIdx.x / 16 * step) * 16 + (threadIdx.x & 15);      // first element of this thread
-    const bool early = !a.out && threadIdx.x < 16 * (unsigned)min(G, n_my) && e_n < a.d;
-    if (early) pre = a.resid[(int64_t)m * a.d + e_n];
-    __syncthreads();
-    dm_rounds<KIND, 1>(a, n_my, red, bar, issue,
-        [&](int stage, int part, DgAcc<1>& acc) {
-            const uint32_t base = smem_u32(smem) + stage * a.stage_bytes, cb = (DG_CHUNK / q_block_elems(KIND)) * q_block_bytes(KIND);
+    dm_rounds<KIND, 1>(a, n_my, red, bar,
+        [&] {
+            pdl_wait();
+            const int col = (first + threadIdx.x / 16 * step) * 16 + (threadIdx.x & 15);      // this thread's first element
+            if (!a.out && threadIdx.x < 16 * (unsigned)min(G, n_my) && col < a.d) pre = a.resid[(int64_t)m * a.d + col];
+            for (int i = warp; i < chunks; i += W) {
+                float v[8], mul = 1.0f;
+                if (i < sc) {
+                    dg_load8<true>(a.sh_act + (int64_t)m * a.SH, i * DG_CHUNK + 8 * lane, a.SH, v);
+                } else {
+                    const int k = dg_div(i - sc, a.ec_inv);
+                    dg_load8<true>(a.act + ((int64_t)m * a.K + k) * a.E, (i - sc - k * ec) * DG_CHUNK + 8 * lane, a.E, v);
+                    mul = s_w[k];
+                }
+                dg_stage<KIND, 1>(xd, i, 0, v, mul, lane);
+            }
+            __syncthreads();
+        }, issue,
+        [&](int stage, int part, DgAcc<KIND, 1>& acc) {
+            const uint32_t base = smem_u32(smem) + stage * a.stage_bytes, cb = dg_row_chunk<KIND>();
             for (int c = part; c < chunks; c += a.parts) {
                 uint32_t at, rb;
                 int cc = c, K = a.SH;
@@ -369,7 +453,7 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dm_down_kernel(MoeFusedArgs a) 
                     at = base;
                     rb = rb_s;
                 } else {
-                    const int k = (c - sc) / ec;
+                    const int k = dg_div(c - sc, a.ec_inv);
                     at = base + 16 * (rb_s + k * rb_e);
                     rb = rb_e;
                     cc = c - sc - k * ec;
@@ -380,7 +464,7 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dm_down_kernel(MoeFusedArgs a) 
             }
         },
         [&](int t0, int n, const float* rr) {
-            for (int e = threadIdx.x; e < n * 16; e += DG_THREADS) {
+            for (int e = threadIdx.x; e < n * 16; e += W * 32) {
                 const int row = e % 16, i = e / 16, col = (first + (t0 + i) * step) * 16 + row;
                 if (col >= a.d) continue;
                 const float v = dg_value<KIND, 1>(rr + i * a.parts * dg_red_floats(1), a.parts, row, 0);
@@ -394,38 +478,39 @@ __global__ void __launch_bounds__(DG_THREADS, 2) dm_down_kernel(MoeFusedArgs a) 
 // ---- host side -----------------------------------------------------------------
 // Stages and contraction split for `share` tiles per CTA of tile_bytes each: the whole share in half an SM, or two
 // sets of as much as fits there, or the same in a whole SM.  Returns the dynamic shared memory, 0 if nothing fits.
-static size_t dm_plan(MoeFusedArgs& a, int share, size_t tile_bytes, int chunks, int mt, size_t fixed, size_t floor_bytes) {
+template <int KIND>
+static size_t dm_plan(MoeFusedArgs& a, int tiles, int ctas, size_t tile_bytes, int chunks, int mt, size_t fixed, size_t floor_bytes) {
+    const int most = ctas ? ceil_div(tiles, ctas) : 0;
+    a.share = ctas ? tiles / ctas : 0;
+    a.share_rem = ctas ? tiles % ctas : 0;
     a.stage_bytes = (int)((tile_bytes + 127) / 128 * 128);
+    if (chunks > 255) return 0;
     for (const size_t budget : {(size_t)SMEM_BUDGET - 2048, (size_t)SMEM_BUDGET_FULL - 2048})
-        for (int G = std::max(1, std::min(share, 8)); G >= 1; --G) {
+        for (int G = std::max(1, std::min(most, 8)); G >= 1; --G) {
             a.n_stages = G;
-            a.sets = G >= share ? 1 : 2;
-            int best = 1, cost = 1 << 30;
-            for (int p = 1; p <= std::min(chunks, DG_WARPS); ++p) {
-                const int c = ceil_div(G * p, DG_WARPS) * ceil_div(chunks, p);
-                if (c < cost) { cost = c; best = p; }
-            }
-            a.parts = best;
-            const size_t need = std::max(floor_bytes, (size_t)a.sets * G * a.stage_bytes + dg_x_bytes(chunks, mt) + fixed + 64 +
+            a.sets = G >= most ? 1 : 2;
+            a.parts = dg_parts(G, chunks, dg_warps(mt));
+            a.parts_inv = dg_inv(a.parts);
+            const size_t need = std::max(floor_bytes, (size_t)a.sets * G * a.stage_bytes + dg_x_bytes<KIND>(chunks, mt) + fixed + 64 +
                                                           (size_t)2 * G * a.parts * dg_red_floats(mt) * 4);
             if (need <= budget) return need;
         }
     return 0;
 }
 template <typename Kern>
-static int dm_launch(Kern kern, bool& configured, dim3 grid, size_t smem, const MoeFusedArgs& a) {
+static int dm_launch(Kern kern, bool& configured, dim3 grid, int threads, size_t smem, const MoeFusedArgs& a) {
     if (!configured) {
         int rc = allow_smem(kern);
         if (rc) return rc;
         configured = true;
     }
-    return launch_pdl(kern, grid, dim3(DG_THREADS), smem, a);
+    return launch_pdl(kern, grid, dim3(threads), smem, a);
 }
 
 template <int KIND, int MT>
 static int dm_kernel1(MoeFusedArgs a, size_t smem, int grid) {
     static bool configured = false;
-    return dm_launch(dm_router_shared_kernel<KIND, MT>, configured, dim3(grid), smem, a);
+    return dm_launch(dm_router_shared_kernel<KIND, MT>, configured, dim3(grid), dg_warps(MT) * 32, smem, a);
 }
 
 template <int KIND>
@@ -437,20 +522,22 @@ static int dm_kind(const MoeFusedArgs& a) {
     MoeFusedArgs p1 = a, p2 = a, p3 = a;
     const int n_router = ceil_div(a.ne, DM_ROUTER), sh_tiles = a.SH / 8;
     const int sh_ctas = std::min(sh_tiles, std::max(8, num_sms() - n_router));
-    const size_t router_bytes = (size_t)DM_ROUTER * a.d * 4 + std::max<size_t>((size_t)DM_ROUTER * a.M * dm_chain_stride(a.d) * 4, (size_t)a.M * (2 * a.ne + 32) * 4);
-    const size_t s1 = dm_plan(p1, sh_ctas ? ceil_div(sh_tiles, sh_ctas) : 0, sh_ctas ? 16 * rb_d : 0, sh_ctas ? dg_chunks(a.d) : 1, mt,
-                              (size_t)dg_chunks(a.d) * mt * 8, router_bytes);
+    const size_t router_bytes = (size_t)DM_ROUTER * a.d * 4 + std::max<size_t>((size_t)DM_ROUTER * a.M * dm_chain_stride(a.d) * 4, (size_t)a.M * a.ne * 4);
+    p1.chunks_inv = dg_inv(std::min(255, dg_chunks(a.d)));
+    const size_t s1 = dm_plan<KIND>(p1, sh_tiles, sh_ctas, sh_ctas ? 16 * rb_d : 0, sh_ctas ? dg_chunks(a.d) : 1, mt, (size_t)dg_chunks(a.d) * mt * 8, router_bytes);
     const int t2 = a.K * (a.E / 8), g2 = std::min(t2, per_token);
-    const size_t s2 = dm_plan(p2, ceil_div(t2, g2), 16 * rb_d, dg_chunks(a.d), 1, (size_t)dg_chunks(a.d) * 8, 0);
+    p2.per_inv = 0xFFFFFFFFu / (uint32_t)(a.E / 8) + 1u;      // exact quotients below 2^16 (E / 8 >= 4)
+    const size_t s2 = dm_plan<KIND>(p2, t2, g2, 16 * rb_d, dg_chunks(a.d), 1, (size_t)dg_chunks(a.d) * 8, 0);
     const int t3 = ceil_div(a.d, 16), g3 = std::min(t3, per_token);
-    const size_t s3 = dm_plan(p3, ceil_div(t3, g3), 16 * (rb_s + a.K * rb_e), dg_chunks(a.SH) + a.K * dg_chunks(a.E), 1, 0, 0);
+    p3.ec_inv = dg_inv(std::min(255, dg_chunks(a.E)));
+    const size_t s3 = dm_plan<KIND>(p3, t3, g3, 16 * (rb_s + a.K * rb_e), dg_chunks(a.SH) + a.K * dg_chunks(a.E), 1, 0, 0);
     if (!s1 || !s2 || !s3) return fail(B200_EUNSUPPORTED, "moe_fused: hidden size %d does not fit the shared-memory staging", a.d);
     int rc = mt == 1 ? dm_kernel1<KIND, 1>(p1, s1, n_router + sh_ctas) : mt == 2 ? dm_kernel1<KIND, 2>(p1, s1, n_router + sh_ctas)
              : mt == 4 ? dm_kernel1<KIND, 4>(p1, s1, n_router + sh_ctas) : dm_kernel1<KIND, 8>(p1, s1, n_router + sh_ctas);
     if (rc) return rc;
     static bool c2 = false, c3 = false;
-    rc = dm_launch(dm_gateup_kernel<KIND>, c2, dim3(g2, a.M), s2, p2);
-    return rc ? rc : dm_launch(dm_down_kernel<KIND>, c3, dim3(g3, a.M), s3, p3);
+    rc = dm_launch(dm_gateup_kernel<KIND>, c2, dim3(g2, a.M), dg_warps(1) * 32, s2, p2);
+    return rc ? rc : dm_launch(dm_down_kernel<KIND>, c3, dim3(g3, a.M), dg_warps(1) * 32, s3, p3);
 }
 
 // moe_fused() for packed weights (kind 0 .. 3); sizes checked there.

@@ -19,9 +19,13 @@
 
 namespace b200 {
 
-constexpr int DG_WARPS = 8;
-constexpr int DG_THREADS = DG_WARPS * 32;
+// Warps of a CTA: two CTAs of consecutive kernels share an SM, so twelve warps leave 80 registers, which one
+// and two tokens fit; more tokens need the accumulators of eight warps at 128.
+__host__ __device__ constexpr int dg_warps(int MT) { return MT <= 2 ? 12 : 8; }
 constexpr int DG_CHUNK = 256;                 // activations that share a scale
+// a / b for 0 <= a < 4096, 1 <= b < 256, inv = dg_inv(b): no division on the kernels' serial path
+__host__ __device__ constexpr uint32_t dg_inv(int b) { return ((1u << 20) + (uint32_t)b - 1) / (uint32_t)b; }
+__host__ __device__ __forceinline__ int dg_div(int a, uint32_t inv) { return (int)(((uint32_t)a * inv) >> 20); }
 
 template <int KIND>
 struct DgKind {
@@ -32,23 +36,28 @@ struct DgKind {
 };
 
 __host__ __device__ inline int dg_chunks(int K) { return (K + DG_CHUNK - 1) / DG_CHUNK; }
-// Shared-memory bytes of `tokens` staged token slots of K activations.
-__host__ __device__ inline size_t dg_x_bytes(int chunks, int tokens) {
-    return (size_t)chunks * tokens * (DG_CHUNK * 4 + 32 + 4) + 16;
-}
+// Staged activations of a chunk and token: four digit bytes each, the sub-block sums as two fp16 parts and the
+// scale; for fp16 weights the two fp16 parts of each, in columns of their own.
+constexpr int DG_COL = DG_CHUNK * 2 + 64;     // bytes of an fp16 column: two neighbours fall into different halves of the banks
+template <int KIND>
+__host__ __device__ constexpr int dg_chunk_bytes() { return (KIND == KIND_F16 ? 2 * DG_COL : DG_CHUNK * 4 + 32) + 4; }
+template <int KIND>
+__host__ __device__ inline size_t dg_x_bytes(int chunks, int tokens) { return (size_t)chunks * tokens * dg_chunk_bytes<KIND>() + 16; }
+
+int dg_parts(int tiles, int chunks, int warps);      // decode_gemv.cu
 
 #ifdef __CUDACC__
-// Staged activations: digits [sub-block][token][slot][32 bytes], slot = (digit + sub-block) & 3 (so that
-// the stores of a warp spread over the banks); sub-block sums * 2^-e as two fp16 parts
-// [chunk][part][token][8]; scales 2^e [chunk][token].
-template <int MT>
+// Packed weights: digits [sub-block][token][slot][32 bytes], slot = (digit + sub-block) & 3 (so that the stores
+// of a warp spread over the banks); sub-block sums * 2^-e [chunk][part][token][8]; scales [chunk][token].
+// fp16 weights: columns [chunk][token][part][DG_COL bytes]; scales.
+template <int KIND, int MT>
 struct DgX {
     uint32_t dig, sum, scale;                 // shared addresses
     __device__ __forceinline__ uint8_t* carve(uint8_t* p, int chunks) {
         dig = smem_u32(p);
-        sum = dig + chunks * MT * DG_CHUNK * 4;
-        scale = sum + chunks * MT * 32;
-        return p + dg_x_bytes(chunks, MT);
+        sum = dig + chunks * MT * (KIND == KIND_F16 ? 2 * DG_COL : DG_CHUNK * 4);
+        scale = sum + (KIND == KIND_F16 ? 0 : chunks * MT * 32);
+        return p + dg_x_bytes<KIND>(chunks, MT);
     }
 };
 
@@ -88,13 +97,34 @@ __device__ __forceinline__ void dg_mma_f16k8(float (&c)[4], uint32_t a0, uint32_
 // Lane l's eight activations 256 * chunk + 8 l .. of token m (zeros past K), staged by one whole warp.
 // mul: a factor of the token's contribution, folded into the scale (a mixture weight).
 template <int KIND, int MT>
-__device__ __forceinline__ void dg_stage(const DgX<MT>& xd, int chunk, int m, const float (&v)[8], float mul, int lane) {
+__device__ __forceinline__ void dg_stage(const DgX<KIND, MT>& xd, int chunk, int m, const float (&v)[8], float mul, int lane) {
     float mx = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
     uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
     int e = (int)(bits >> 23) - 126;                                  // every |v| < 2^e
-    e = max(e, -90);
+    e = min(max(e, -90), 127);
+    if (lane == 0) {
+        // fp16 parts are kept at up to 2^10
+        const float unit = __uint_as_float((uint32_t)(127 + e - (KIND == KIND_F16 ? 10 : 0)) << 23);
+        sts_u32(xd.scale + (chunk * MT + m) * 4, __float_as_uint(unit * mul));
+    }
+    if (KIND == KIND_F16) {
+        const float up = __uint_as_float((uint32_t)(127 + 10 - e) << 23);
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __half2 h = __floats2half2_rn(v[2 * i] * up, v[2 * i + 1] * up);
+            const float2 f = __half22float2(h);
+            const __half2 l = __floats2half2_rn(v[2 * i] * up - f.x, v[2 * i + 1] * up - f.y);
+            hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+            lo[i] = *reinterpret_cast<const uint32_t*>(&l);
+        }
+        const uint32_t at = xd.dig + (chunk * MT + m) * 2 * DG_COL + 16 * lane;
+        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
+        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(at + DG_COL), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
+        return;
+    }
     const float to_int = __uint_as_float((uint32_t)(127 + 30 - e) << 23), down = __uint_as_float((uint32_t)(127 - e) << 23);
     uint32_t w[2][4];
     float sum = 0.0f;
@@ -137,25 +167,30 @@ __device__ __forceinline__ void dg_stage(const DgX<MT>& xd, int chunk, int m, co
             sts_u16(a + MT * 16, __half_as_ushort(lo));
         }
     }
-    if (lane == 0) sts_u32(xd.scale + (chunk * MT + m) * 4, __float_as_uint(__uint_as_float((uint32_t)(127 + e) << 23) * mul));
 }
 
+// Bytes of a chunk of a row.
+template <int KIND>
+__host__ __device__ constexpr int dg_row_chunk() { return KIND == KIND_F16 ? DG_CHUNK * 2 : DG_CHUNK / q_block_elems(KIND) * q_block_bytes(KIND); }
+
 // Loads for dg_stage; x 16-byte aligned.
+// CG: from L2.
+template <bool CG>
 __device__ __forceinline__ void dg_load8(const float* x, int k, int K, float (&v)[8]) {
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
     if (k < K) {                                                      // K % 32 == 0: a lane has all eight or none
-        a = *reinterpret_cast<const float4*>(x + k);
-        b = *reinterpret_cast<const float4*>(x + k + 4);
+        a = ld_f4<CG>(x + k);
+        b = ld_f4<CG>(x + k + 4);
     }
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-// One warp's accumulators for a 16-row tile: f[q] the digit columns of tokens 2 q, 2 q + 1 (lane
+// One warp's accumulators for a 16-row tile.  Packed: f[q] the digit columns of tokens 2 q, 2 q + 1 (lane
 // (g, t): rows g, g + 8; token 2 q + t / 2, digits 2 (t & 1), + 1), mn the minimum terms (rows g,
-// g + 8; tokens 2 t, 2 t + 1).
-template <int MT>
+// g + 8; tokens 2 t, 2 t + 1).  fp16: f[q] the two parts of token 4 q + t.
+template <int KIND, int MT>
 struct DgAcc {
-    static constexpr int NT = MT <= 2 ? 1 : MT / 2;
+    static constexpr int NT = KIND == KIND_F16 ? (MT <= 4 ? 1 : 2) : (MT <= 2 ? 1 : MT / 2);
     float f[NT][4], mn[4];
     __device__ __forceinline__ void clear() {
 #pragma unroll
@@ -171,9 +206,37 @@ struct DgAcc {
 // rows g and g + 8; xc: the chunk's index among the staged activations; nb: its 32-weight blocks (8, fewer
 // in a tail of kinds 0 .. 2).
 template <int KIND, int MT>
-__device__ __forceinline__ void dg_chunk(DgAcc<MT>& acc, uint32_t row_a, uint32_t row_b, const DgX<MT>& xd, int xc, int nb, int lane) {
-    constexpr int NT = DgAcc<MT>::NT;
+__device__ __forceinline__ void dg_chunk(DgAcc<KIND, MT>& acc, uint32_t row_a, uint32_t row_b, const DgX<KIND, MT>& xd, int xc, int nb, int lane) {
+    constexpr int NT = DgAcc<KIND, MT>::NT;
     const int g = lane >> 2, t = lane & 3, dgt = g & 3;
+    if (KIND == KIND_F16) {
+        uint32_t col[NT];
+        float c[NT][4];
+#pragma unroll
+        for (int q = 0; q < NT; ++q) {
+            col[q] = xd.dig + (xc * MT + min(4 * q + (g >> 1), MT - 1)) * 2 * DG_COL + (g & 1) * DG_COL + 16 * t;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) c[q][i] = 0.0f;
+        }
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            if (s >= nb) break;
+            const uint4 a = lds_u4(row_a + 64 * s + 16 * t), b = lds_u4(row_b + 64 * s + 16 * t);
+#pragma unroll
+            for (int q = 0; q < NT; ++q) {
+                const uint4 x = lds_u4(col[q] + 64 * s);
+                mma_16816(c[q], a.x, b.x, a.y, b.y, x.x, x.y);
+                mma_16816(c[q], a.z, b.z, a.w, b.w, x.z, x.w);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < NT; ++q) {
+            const float xs = lds_f32(xd.scale + (xc * MT + min(4 * q + t, MT - 1)) * 4);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc.f[q][i] += xs * c[q][i];
+        }
+        return;
+    }
     const uint32_t xb = xd.dig + xc * 8 * MT * 128 + 8 * t + (MT == 1 ? 0 : (g >> 2) * 128);
     uint32_t xo[4];
 #pragma unroll
@@ -285,11 +348,20 @@ __device__ __forceinline__ void dg_chunk(DgAcc<MT>& acc, uint32_t row_a, uint32_
 // The warp's sums to red[16 rows][MT] and, for kinds with minima, red[16 * MT + ...] (dg_value adds the two).
 constexpr int dg_red_floats(int MT) { return 2 * 16 * MT; }
 template <int KIND, int MT>
-__device__ __forceinline__ void dg_finish(const DgAcc<MT>& acc, float* red, int lane) {
+__device__ __forceinline__ void dg_finish(const DgAcc<KIND, MT>& acc, float* red, int lane) {
     const int g = lane >> 2, t = lane & 3;
+    if (KIND == KIND_F16) {
+#pragma unroll
+        for (int q = 0; q < DgAcc<KIND, MT>::NT; ++q)
+            if (4 * q + t < MT) {
+                red[g * MT + 4 * q + t] = acc.f[q][0] + acc.f[q][1];
+                red[(g + 8) * MT + 4 * q + t] = acc.f[q][2] + acc.f[q][3];
+            }
+        return;
+    }
     const float scale = ((t & 1) ? 65536.0f : 1.0f) * (DgKind<KIND>::split16 ? 0x1p-34f : 0x1p-30f);
 #pragma unroll
-    for (int q = 0; q < DgAcc<MT>::NT; ++q) {
+    for (int q = 0; q < DgAcc<KIND, MT>::NT; ++q) {
         float a = (acc.f[q][0] + 256.0f * acc.f[q][1]) * scale, b = (acc.f[q][2] + 256.0f * acc.f[q][3]) * scale;
         a += __shfl_xor_sync(0xffffffffu, a, 1);
         b += __shfl_xor_sync(0xffffffffu, b, 1);
@@ -312,12 +384,14 @@ __device__ __forceinline__ void dg_finish(const DgAcc<MT>& acc, float* red, int 
 // Element (row, token) from `parts` warps' results, each dg_red_floats apart.
 template <int KIND, int MT>
 __device__ __forceinline__ float dg_value(const float* red, int parts, int row, int tok) {
-    float v = 0.0f;
-    for (int p = 0; p < parts; ++p, red += dg_red_floats(MT)) {
-        v += red[row * MT + tok];
-        if (DgKind<KIND>::mins) v += red[(16 + row) * MT + tok];
+    const float* at = red + row * MT + tok;
+    float v = 0.0f, w = 0.0f;
+#pragma unroll 4
+    for (int p = 0; p < parts; ++p, at += dg_red_floats(MT)) {
+        v += at[0];
+        if (DgKind<KIND>::mins) w += at[16 * MT];
     }
-    return v;
+    return v + w;
 }
 #endif
 

@@ -58,14 +58,17 @@ struct SgArgs {
     float *conv_state = nullptr, *gate = nullptr, *bc = nullptr, *dt_raw = nullptr;
     // filled by stream_gemv()
     int rows_per_tile = 0, num_tiles = 0, stage_bytes = 0, n_stages = 0;
-    int sets = 1, parts = 1;        // packed weights: sets of n_stages tiles, warps a tile's contraction is split over
+    // digit kernel: sets of n_stages tiles, warps a tile's contraction is split over, tiles per CTA (and how many
+    // CTAs have one more), reciprocals for dg_div
+    int sets = 1, parts = 1, share = 0, share_rem = 0;
+    uint32_t parts_inv = 0, chunks_inv = 0;
     int64_t row_bytes = 0;
     int* status = nullptr;
     bool dry = false;               // validate shapes and tiling, launch nothing
 };
 
 int stream_gemv(SgArgs a, int kind, int pro, int epi);
-int digit_gemv(SgArgs a, int kind, int pro, int epi);   // its form for packed weights (decode_gemv.cu)
+int digit_gemv(SgArgs a, int kind, int pro, int epi);   // its form for packed and fp16 weights (decode_gemv.cu)
 
 // Whole-sequence Mamba-2 layer (mamba.cu).  kind: template tag of the projections'
 // storage.  conv_state_out (optional) [B, conv_dim, k-1] receives the convolution
@@ -103,7 +106,8 @@ struct MoeFusedArgs {
     float res_mult = 1.0f;
     int M = 0, d = 0, E = 0, ne = 0, K = 0, SH = 0;
     // filled per phase
-    int rows_per_tile = 0, stage_bytes = 0, n_stages = 0, sets = 1, parts = 1;
+    int rows_per_tile = 0, stage_bytes = 0, n_stages = 0, sets = 1, parts = 1, share = 0, share_rem = 0;
+    uint32_t parts_inv = 0, chunks_inv = 0, ec_inv = 0, per_inv = 0;
     int* status = nullptr;
     int* route_counter = nullptr;   // router tiles finished so far in this layer (returns to 0)
     bool dry = false;               // validate shapes and tiling, launch nothing

@@ -23,6 +23,7 @@ constexpr int SG_MAX_STAGES = 4;
 constexpr int SMEM_BUDGET = 113 * 1024;            // per CTA: two kernels' CTAs fit one SM, so a
                                                    // dependent kernel can start streaming early
 constexpr int SMEM_BUDGET_FULL = 200 * 1024;       // fallback for wide rows: one CTA per SM
+constexpr int SMEM_OPT_IN = 226 * 1024;            // what the kernels are allowed to ask for
 constexpr int TILE_ROWS = 16;                      // rows of a tile on the tensor-core path (max elsewhere)
 constexpr int RED_TOK = 8;                         // token columns
 constexpr int RED_PASS = TILE_ROWS * RED_TOK;      // floats of one (part, pass)
@@ -481,7 +482,7 @@ static int launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, const Args&
 
 template <typename Kern>
 static int allow_smem(Kern kern) {
-    B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BUDGET_FULL));
+    B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPT_IN));
     return B200_OK;
 }
 

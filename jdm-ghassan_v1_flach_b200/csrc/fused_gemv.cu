@@ -143,12 +143,15 @@ __global__ void __launch_bounds__(SG_THREADS, 2) stream_gemv_kernel(SgArgs a) {
 // out-projection turns the partials into inv = 1/sqrt(mean + eps) and computes
 // inv * (W u) - algebraically the reference's rmsnorm(y*silu(gate))*norm_w -> W.
 constexpr int FS_WARPS = 8;
+// NV: state elements per lane, one vector load (d_state = 32 NV); 0 for any other d_state.
+template <int NV>
 __global__ void __launch_bounds__(FS_WARPS * 32)
 mamba_scan_norm_kernel(const float* __restrict__ bc, const float* __restrict__ dt_raw,
                        const float* __restrict__ gate, const float* __restrict__ dt_bias,
                        const float* __restrict__ a_log, const float* __restrict__ Dv,
                        const float* __restrict__ norm_w, float* __restrict__ ssm_state,
                        float* __restrict__ u_out, double* __restrict__ partials, MambaDims p) {
+    constexpr int N = NV > 0 ? NV : 1;
     __shared__ double wsum[FS_WARPS];
     if (threadIdx.x == 0) pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -156,39 +159,48 @@ mamba_scan_norm_kernel(const float* __restrict__ bc, const float* __restrict__ d
     const int row = blockIdx.x * FS_WARPS + warp;
     const int m = blockIdx.y;
     const bool live = row < rows;
-    const bool vec = (p.d_state == 128);
     const int h = live ? row / p.d_head : 0;
     float* s = ssm_state + ((int64_t)m * rows + (live ? row : 0)) * p.d_state;
+    auto load = [&](const float* q, float (&v)[N]) {
+        if (NV == 4) {
+            const float4 f = *reinterpret_cast<const float4*>(q + lane * 4);
+            v[0] = f.x; v[N > 1 ? 1 : 0] = f.y; v[N > 2 ? 2 : 0] = f.z; v[N > 3 ? 3 : 0] = f.w;
+        } else if (NV == 2) {
+            const float2 f = *reinterpret_cast<const float2*>(q + lane * 2);
+            v[0] = f.x; v[N > 1 ? 1 : 0] = f.y;
+        }
+    };
     // everything that does not depend on this token's projection: before the wait
-    float4 sv = make_float4(0, 0, 0, 0);
-    if (live && vec) sv = *reinterpret_cast<const float4*>(s + lane * 4);
-    const float dtb = dt_bias[h], al = a_log[h], dsk = Dv[h];
+    float sv[N];
+    if (NV > 0) load(s, sv);
+    const float dtb = dt_bias[h], A = -expf(a_log[h]), dsk = Dv[h];
     const float nw = live ? norm_w[row] : 0.0f;
     pdl_wait();
     double sq = 0.0;
     if (live) {
         const float* bcm = bc + (int64_t)m * p.conv_dim;
+        const float* Bv = bcm + p.d_inner;
+        const float* Cv = Bv + p.d_state;
+        float bv[N], cv[N];
+        if (NV > 0) {
+            load(Bv, bv);
+            load(Cv, cv);
+        }
         const float xv = bcm[row];
         const float gt = gate[(int64_t)m * p.d_inner + row];
         const float uu = dt_raw[(int64_t)m * p.n_heads + h] + dtb;
-        const float* Bv = bcm + p.d_inner;
-        const float* Cv = Bv + p.d_state;
         float acc = 0.0f;
-        float4 b4 = make_float4(0, 0, 0, 0), c4 = b4;
-        if (vec) {
-            b4 = *reinterpret_cast<const float4*>(Bv + lane * 4);
-            c4 = *reinterpret_cast<const float4*>(Cv + lane * 4);
-        }
         const float dt = (uu > 20.0f) ? uu : log1pf(expf(uu));
-        const float A = -expf(al);
         const float dA = expf(__fmul_rn(A, dt));
-        if (vec) {
-            sv.x = __fadd_rn(__fmul_rn(dA, sv.x), __fmul_rn(__fmul_rn(dt, b4.x), xv));
-            sv.y = __fadd_rn(__fmul_rn(dA, sv.y), __fmul_rn(__fmul_rn(dt, b4.y), xv));
-            sv.z = __fadd_rn(__fmul_rn(dA, sv.z), __fmul_rn(__fmul_rn(dt, b4.z), xv));
-            sv.w = __fadd_rn(__fmul_rn(dA, sv.w), __fmul_rn(__fmul_rn(dt, b4.w), xv));
-            *reinterpret_cast<float4*>(s + lane * 4) = sv;
-            acc = c4.x * sv.x + c4.y * sv.y + c4.z * sv.z + c4.w * sv.w;
+        const float sg = silu_acc(gt);
+        if (NV > 0) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                sv[i] = __fadd_rn(__fmul_rn(dA, sv[i]), __fmul_rn(__fmul_rn(dt, bv[i]), xv));
+                acc += cv[i] * sv[i];
+            }
+            if (NV == 4) *reinterpret_cast<float4*>(s + lane * 4) = make_float4(sv[0], sv[N > 1 ? 1 : 0], sv[N > 2 ? 2 : 0], sv[N > 3 ? 3 : 0]);
+            else *reinterpret_cast<float2*>(s + lane * 2) = make_float2(sv[0], sv[N > 1 ? 1 : 0]);
         } else {
             for (int j = lane; j < p.d_state; j += 32) {
                 const float sn = __fadd_rn(__fmul_rn(dA, s[j]), __fmul_rn(__fmul_rn(dt, Bv[j]), xv));
@@ -199,7 +211,7 @@ mamba_scan_norm_kernel(const float* __restrict__ bc, const float* __restrict__ d
         acc = warp_sum(acc);
         if (lane == 0) {
             const float y = acc + dsk * xv;
-            const float v = y * silu_acc(gt);
+            const float v = y * sg;
             u_out[(int64_t)m * p.d_inner + row] = v * nw;
             sq = (double)v * v;
         }
@@ -259,7 +271,7 @@ int stream_gemv(SgArgs a, int kind, int pro, int epi) {
     if (R < 1 || (R * a.row_bytes) % 16 != 0 || !tail_tile_ok(a.N, R, a.row_bytes) || !tail_tile_ok(a.N2, R, a.row_bytes) ||
         !tail_tile_ok(a.N3, R, a.row_bytes))
         return fail(B200_EUNSUPPORTED, "stream_gemv: rows of %lld bytes cannot be tiled to 16 bytes", (long long)a.row_bytes);
-    if (kind <= 3) return digit_gemv(a, kind, pro, epi);
+    if (kind != KIND_F32) return digit_gemv(a, kind, pro, epi);
     a.rows_per_tile = R;
     a.t1 = ceil_div(a.N, R);
     a.t2 = a.t1 + ceil_div(a.N2, R);
@@ -272,7 +284,6 @@ int stream_gemv(SgArgs a, int kind, int pro, int epi) {
     if (pro == PRO_NONE && epi == EPI_RESIDUAL) return launch_sg_mt<KIND, PRO_NONE, EPI_RESIDUAL>(a, grid); \
     if (pro == PRO_NONE && epi == EPI_STORE) return launch_sg_mt<KIND, PRO_NONE, EPI_STORE>(a, grid);       \
     return fail(B200_EINVAL, "stream_gemv: unsupported prologue/epilogue pair");
-    if (kind == KIND_F16) { SG_DISPATCH(KIND_F16) }
     SG_DISPATCH(KIND_F32)
 #undef SG_DISPATCH
 }
@@ -291,8 +302,8 @@ int mamba_scan_norm(const float* bc, const float* dt_raw, const float* gate, con
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    B200_CUDA(cudaLaunchKernelEx(&cfg, mamba_scan_norm_kernel, bc, dt_raw, gate, dt_bias, a_log, D, norm_w, ssm_state,
-                                 u_out, partials, p));
+    auto kern = p.d_state == 128 ? mamba_scan_norm_kernel<4> : p.d_state == 64 ? mamba_scan_norm_kernel<2> : mamba_scan_norm_kernel<0>;
+    B200_CUDA(cudaLaunchKernelEx(&cfg, kern, bc, dt_raw, gate, dt_bias, a_log, D, norm_w, ssm_state, u_out, partials, p));
     ++g_kernel_launches;
     return B200_OK;
 }

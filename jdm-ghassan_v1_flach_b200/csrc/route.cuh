@@ -64,55 +64,51 @@ __device__ __forceinline__ void route_finish_warp(const float* __restrict__ logi
     __syncwarp();
 }
 
-// The same result for K <= 16 and ne <= 256 with the candidates in registers: the K rounds are two warp
-// reductions each (the largest value as an ordered word, then the lowest index that has it) instead of ten
-// shuffles and a walk over the taken ones - 1.6 us less at 64 experts, top-6.  s: ne + 16 floats of scratch;
-// idx, w: this token's outputs.
-__device__ __forceinline__ void route_finish_fast(const float* __restrict__ logits, const float* __restrict__ bias, int ne, int K,
-                                                  float* s, int32_t* idx, float* w, float* probs_out, int lane) {
-    constexpr int PER = 8;                                    // ne <= 256
-    float v[PER], mx = __ldcg(logits);
+// The same result for K <= 16 with the candidates in registers (lane holds logits 32 i + lane, i < PER, and
+// their biases; those past ne are repeats of the last and decide nothing): the exponentials side by side, the K
+// rounds two warp reductions each (the largest value as an ordered word, then the lowest index that has it)
+// instead of ten shuffles and a walk over the taken ones.  s: ne floats of shared scratch.  v becomes the
+// probabilities; lane k < K gets choice k and its weight.
+template <int PER>
+__device__ __forceinline__ void route_pick(float (&v)[PER], const float (&bs)[PER], bool biased, int ne, int K, float* s, int lane,
+                                           int& my_idx, float& my_w) {
+    float mx = -INFINITY;
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int e = 32 * i + lane;
-        if (e < ne) {
-            v[i] = __ldcg(logits + e);
-            mx = fmaxf(mx, v[i]);
-        }
-    }
+    for (int i = 0; i < PER; ++i) mx = fmaxf(mx, v[i]);
     mx = warp_max(mx);
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int e = 32 * i + lane;
-        if (e < ne) {
-            v[i] = (float)exp((double)__fsub_rn(v[i], mx));
-            s[e] = v[i];
-        }
-    }
+    for (int i = 0; i < PER; ++i) v[i] = (float)exp((double)__fsub_rn(v[i], mx));
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+        if (32 * i + lane < ne) s[32 * i + lane] = v[i];
     __syncwarp();
     // the sum in index order (every lane the same additions)
     float sum = 0.0f;
-#pragma unroll 8
-    for (int e = 0; e < ne; ++e) sum = __fadd_rn(sum, s[e]);
+    int e0 = 0;
+    for (; e0 + 16 <= ne; e0 += 16) {
+        float p[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) p[i] = s[e0 + i];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum = __fadd_rn(sum, p[i]);
+    }
+    for (; e0 < ne; ++e0) sum = __fadd_rn(sum, s[e0]);
     const float inv = sum > 1e-12f ? __fdiv_rn(1.0f, sum) : 0.0f;
     uint32_t key[PER];                                        // selection value as an ordered word; 0: not a candidate
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-        const int e = 32 * i + lane;
+        v[i] = __fmul_rn(v[i], inv);
+        float sel = biased ? __fadd_rn(v[i], bs[i]) : v[i];
         key[i] = 0;
-        if (e < ne) {
-            v[i] = __fmul_rn(v[i], inv);
-            if (probs_out) probs_out[e] = v[i];
-            float sel = bias ? __fadd_rn(v[i], bias[e]) : v[i];
-            if (sel > -1e30f) {
-                if (sel == 0.0f) sel = 0.0f;                  // -0 ranks as +0
-                const uint32_t u = __float_as_uint(sel);
-                key[i] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-            }
+        if (32 * i + lane < ne && sel > -1e30f) {
+            if (sel == 0.0f) sel = 0.0f;                      // -0 ranks as +0
+            const uint32_t u = __float_as_uint(sel);
+            key[i] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
         }
     }
-    int my_idx = 0;
-    float my_w = 0.0f, sum_w = 0.0f;
+    my_idx = 0;
+    my_w = 0.0f;
+    float sum_w = 0.0f;
     for (int k = 0; k < K; ++k) {
         uint32_t best = 0;
 #pragma unroll
@@ -121,10 +117,9 @@ __device__ __forceinline__ void route_finish_fast(const float* __restrict__ logi
         int at = 0x7fffffff;
 #pragma unroll
         for (int i = PER - 1; i >= 0; --i)
-            if (best != 0 && key[i] == best) at = 32 * i + lane;
+            if (key[i] == best) at = 32 * i + lane;
         at = __reduce_min_sync(0xffffffffu, at);
-        // no candidate left: index 0, as often as it takes
-        const int e = best == 0 ? 0 : at;
+        const int e = best == 0 ? 0 : at;                     // no candidate left: index 0, as often as it takes
         float pw = 0.0f;
 #pragma unroll
         for (int i = 0; i < PER; ++i)
@@ -139,10 +134,7 @@ __device__ __forceinline__ void route_finish_fast(const float* __restrict__ logi
         }
         sum_w = __fadd_rn(sum_w, pw);
     }
-    if (lane < K) {
-        idx[lane] = my_idx;
-        w[lane] = sum_w > 1e-8f ? __fmul_rn(my_w, __fdiv_rn(1.0f, sum_w)) : __fdiv_rn(1.0f, (float)K);
-    }
+    my_w = sum_w > 1e-8f ? __fmul_rn(my_w, __fdiv_rn(1.0f, sum_w)) : __fdiv_rn(1.0f, (float)K);
 }
 #endif
 
