@@ -438,285 +438,6 @@ __global__ void __launch_bounds__(GM_THREADS, 1) umma_gemm_kernel(const __grid_c
 }
 
 // ===========================================================================
-// Packed weights: dequantise inside the GEMM
-// ===========================================================================
-// Same tiling, but B arrives in its packed form: per 256 weights of K (8 blocks of
-// the 32-weight kinds, one Q4_K super-block) a row contributes a fixed number of
-// bytes (144 / 160 / 272 / 144), which one 2-D TMA box brings in for all rows of the
-// tile.  Eight warps expand it, 64 weights of K per row and step, to fp16 - the
-// value the reference's CPU path multiplies with, its dequantised weight rounded to
-// fp16 (core/ops.cpp:313-336, :392), to within one fp16 ulp - and store the result in
-// the swizzled K-major layout the MMA reads.  HBM sees the packed bytes only.
-//
-//   warp 0       TMA: A tile per 64 of K, packed B per 256 of K
-//   warps 6..13  packed B (shared) -> fp16 B tile (shared, 2 buffers)
-//   warp 1       MMA when an A stage and a B tile are both ready
-//   warps 2..5   epilogue
-template <int KIND>
-struct PackedShape {
-    static constexpr int SBB = 8 * (KIND == 3 ? 18 : q_block_bytes(KIND));   // bytes per row per 256 of K
-};
-
-template <int EPI, int KIND>
-struct GemmQShape {
-    static constexpr int UN = GemmShape<EPI>::UN;
-    static constexpr int SBB = PackedShape<KIND>::SBB;
-    static constexpr int B16 = UN * GM_TILE_K * 2;                  // one fp16 B tile
-    static constexpr int PACKED = UN * SBB;                         // one packed stage
-    // fp16 B tiles: enough of them that the expanding warps run ahead of the MMA rather
-    // than in lock-step with it (a hand-off costs a few hundred cycles either way)
-    // A CTA owns 256 rows of A: two 128-row accumulator halves are fed by the same
-    // expanded B tile, which halves the expansion work per flop.  With 128 accumulator
-    // columns per half there is room for two sets (epilogue under the next main loop);
-    // the SwiGLU form (256 columns per half) has one.
-    static constexpr int A_STAGE = 2 * GM_STAGE_A;
-    static constexpr int SA = UN == 128 ? 3 : 2, SB = UN == 128 ? 3 : 2, ACC = UN == 128 ? 2 : 1;
-    static constexpr int FIXED = SA * A_STAGE + SB * B16 + GM_EPI_SCRATCH + 1024 + 256 + GM_SLOT_TABLE;
-    // packed stages: as many as fit (up to 4) - with few rows of A the kernel is a pure
-    // weight stream and needs tens of KB in flight per SM to keep HBM busy
-    static constexpr int ROOM = (227 * 1024 - FIXED) / PACKED;
-    static constexpr int SP = ROOM >= 4 ? 4 : (ROOM >= 1 ? ROOM : 1);
-    static_assert(FIXED + PACKED <= 227 * 1024, "the stages do not fit the shared memory of an SM");
-    static constexpr int SMEM = FIXED + SP * PACKED;
-};
-
-// Half-precision expansion of packed weights, two values per instruction.  A byte
-// b OR-ed into the mantissa of 0x6400 is the fp16 number 1024 + b, so small integers
-// become fp16 without a conversion instruction; __byte_perm interleaves two payload
-// bytes with two 0x64 bytes into one half2.
-__device__ __forceinline__ __half2 magic_pair(uint32_t bytes, uint32_t sel) {
-    const uint32_t v = __byte_perm(bytes, 0x64646464u, sel);
-    return *reinterpret_cast<const __half2*>(&v);
-}
-constexpr uint32_t SEL_01 = 0x5140, SEL_23 = 0x5342;   // (byte0, byte1) / (byte2, byte3) of the first operand
-
-// 32 of the 64 weights of K block j of a row (segment of 256 weights at `seg`):
-// hh = 0 the first 32 of the block, hh = 1 the last 32.  Written as four 16-byte
-// chunks of row r of the swizzled fp16 tile.  Arithmetic in fp16 FMAs:
-//   Q4_0  (q - 8) * d,  Q8_0  q * d       exact (one rounding of an exact product)
-//   Q4_1  q * d + m                        one rounding
-//   Q4_K  (q * sc) * d - fp16(m * dmin)    q * sc exact; the min term rounded first
-// against fp16(fp32 value) of the materialising dequantiser: equal for Q4_0 / Q8_0,
-// within one fp16 ulp otherwise.
-template <int KIND>
-__device__ __forceinline__ void dequant_half_block(const uint8_t* seg, int j, int hh, uint8_t* tile, int r) {
-    uint8_t* rowp = tile + (size_t)(r >> 3) * 1024 + (size_t)(r & 7) * 128;
-    const int sw = r & 7;
-    __half2 out[16];
-    if (KIND == 3) {
-        const uint4 hdr = *reinterpret_cast<const uint4*>(seg);
-        int s, m;
-        q4k_scale_min_regs(2 * j + hh, hdr.y, hdr.z, hdr.w, s, m);
-        const __half d = __ushort_as_half((unsigned short)(hdr.x & 0xFFFF));
-        const float dmin = half_bits_to_float((uint16_t)(hdr.x >> 16));
-        const __half2 sc2 = __half2half2(__int2half_rn(s));
-        const __half2 nsc = __half2half2(__int2half_rn(-1024 * s));          // exact: |1024 * s| <= 64512
-        const __half2 d2 = __half2half2(d);
-        const __half2 nm = __half2half2(__float2half_rn(-__fmul_rn(dmin, (float)m)));
-        const uint4 q0 = *reinterpret_cast<const uint4*>(seg + 16 + 32 * j);
-        const uint4 q1 = *reinterpret_cast<const uint4*>(seg + 32 + 32 * j);
-        const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t x = (words[i] >> (4 * hh)) & 0x0F0F0F0Fu;
-            const __half2 a = __hfma2(magic_pair(x, SEL_01), sc2, nsc);      // q * sc, exact
-            const __half2 b = __hfma2(magic_pair(x, SEL_23), sc2, nsc);
-            out[2 * i] = __hfma2(a, d2, nm);
-            out[2 * i + 1] = __hfma2(b, d2, nm);
-        }
-    } else if (KIND == 2) {
-        const uint16_t* blk = reinterpret_cast<const uint16_t*>(seg + (2 * j + hh) * 34);
-        const __half2 d2 = __half2half2(__ushort_as_half(blk[0]));
-        const __half2 bias = __half2half2(__ushort_as_half((unsigned short)0x6480));   // 1152 = 1024 + 128
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const uint32_t x = (uint32_t)blk[1 + i] ^ 0x8080u;              // int8 + 128 as unsigned bytes
-            out[i] = __hmul2(__hsub2(magic_pair(x, SEL_01), bias), d2);
-        }
-    } else {
-        const int bb = KIND == 0 ? 18 : 20;
-        const uint16_t* blk = reinterpret_cast<const uint16_t*>(seg + (2 * j + hh) * bb);
-        const __half2 d2 = __half2half2(__ushort_as_half(blk[0]));
-        const __half2 m2 = KIND == 1 ? __half2half2(__ushort_as_half(blk[1])) : __half2half2(__ushort_as_half(0));
-        const uint16_t* qs = blk + (KIND == 0 ? 1 : 2);
-        const __half2 off = __half2half2(__ushort_as_half((unsigned short)(KIND == 0 ? 0x6408 : 0x6400)));  // 1032 / 1024
-        // byte i: low nibble = weight i, high nibble = weight 16 + i
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t p = qs[i];
-            const __half2 lo = __hsub2(magic_pair(p & 0x0F0Fu, SEL_01), off);
-            const __half2 hi = __hsub2(magic_pair((p >> 4) & 0x0F0Fu, SEL_01), off);
-            out[i] = KIND == 0 ? __hmul2(lo, d2) : __hfma2(lo, d2, m2);
-            out[8 + i] = KIND == 0 ? __hmul2(hi, d2) : __hfma2(hi, d2, m2);
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<uint4*>(rowp + (((4 * hh + c) ^ sw) << 4)) = *reinterpret_cast<const uint4*>(&out[4 * c]);
-}
-
-
-constexpr int GQ_EXPAND_WARPS = 8;
-constexpr int GQ_FIRST_EXPAND = 6;                 // warps 0, 1: TMA, MMA; 2..5: epilogue; 6..13: expansion
-constexpr int GQ_THREADS = (GQ_FIRST_EXPAND + GQ_EXPAND_WARPS) * 32;
-
-template <int EPI, int KIND>
-__global__ void __launch_bounds__(GQ_THREADS, 1) umma_gemm_q_kernel(const __grid_constant__ GemmArgs a) {
-    using S = GemmQShape<EPI, KIND>;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* sm_a = smem;
-    uint8_t* sm_b = sm_a + S::SA * S::A_STAGE;
-    uint8_t* sm_p = sm_b + S::SB * S::B16;
-    float* epi_scratch = reinterpret_cast<float*>(sm_p + S::SP * S::PACKED);
-    uint64_t* a_full = reinterpret_cast<uint64_t*>(sm_p + S::SP * S::PACKED + GM_EPI_SCRATCH);
-    uint64_t* a_empty = a_full + S::SA;
-    uint64_t* b_full = a_empty + S::SA;
-    uint64_t* b_empty = b_full + S::SB;
-    uint64_t* p_full = b_empty + S::SB;
-    uint64_t* p_empty = p_full + 4;
-    uint64_t* acc_full = p_empty + 4;
-    uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-    int* tab = reinterpret_cast<int*>(sm_p + S::SP * S::PACKED + GM_EPI_SCRATCH + 256);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int total = a.m_slots * a.n_tiles * a.k_splits;
-    const int KB_ALL = a.K / GM_TILE_K;               // K % 256 == 0 (host)
-    gemm_build_slots(a, tab, reinterpret_cast<int*>(epi_scratch));
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < S::SA; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
-        for (int s = 0; s < S::SB; ++s) { mbar_init(&b_full[s], GQ_EXPAND_WARPS); mbar_init(&b_empty[s], 1); }
-        for (int s = 0; s < S::SP; ++s) { mbar_init(&p_full[s], 1); mbar_init(&p_empty[s], GQ_EXPAND_WARPS); }
-        for (int s = 0; s < S::ACC; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], 4); }
-        mbar_fence_init();
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, S::ACC * 2 * S::UN);
-        tmem_relinquish();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            uint32_t it = 0, sbi = 0;                 // K blocks and packed super-blocks issued so far
-            bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-                GemmTile w;
-                if (!gemm_tile_at(a, tab, t, w)) continue;
-                const int kb0 = w.split * a.kb_split, kb1 = min(KB_ALL, kb0 + a.kb_split);
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    if ((kb & 3) == 0) {
-                        const int p = sbi % S::SP;
-                        if (sbi >= S::SP) ok = mbar_wait(&p_empty[p], ((sbi / S::SP) - 1) & 1, a.status);
-                        if (!ok) break;
-                        uint8_t* dst = sm_p + (size_t)p * S::PACKED;
-                        mbar_expect_tx(&p_full[p], S::PACKED);
-                        tma_load_2d(dst, &a.map_b, (kb >> 2) * (S::SBB / 4), w.brow0, &p_full[p]);
-                        if (EPI == GEMM_EPI_SWIGLU)
-                            tma_load_2d(dst + GM_TILE_N * S::SBB, &a.map_b2, (kb >> 2) * (S::SBB / 4), w.brow0, &p_full[p]);
-                        if (EPI == GEMM_EPI_STORE_WIDE)
-                            tma_load_2d(dst + GM_TILE_N * S::SBB, &a.map_b, (kb >> 2) * (S::SBB / 4), w.brow0 + GM_TILE_N,
-                                        &p_full[p]);
-                        ++sbi;
-                    }
-                    const int s = it % S::SA;
-                    if (it >= S::SA) ok = mbar_wait(&a_empty[s], ((it / S::SA) - 1) & 1, a.status);
-                    if (!ok) break;
-                    const bool two = w.row0 + GM_TILE_M < w.row_end;      // second half holds rows of this tile
-                    mbar_expect_tx(&a_full[s], two ? S::A_STAGE : GM_STAGE_A);
-                    tma_load_2d(sm_a + (size_t)s * S::A_STAGE, &a.map_a, kb * GM_TILE_K, w.row0, &a_full[s]);
-                    if (two)
-                        tma_load_2d(sm_a + (size_t)s * S::A_STAGE + GM_STAGE_A, &a.map_a, kb * GM_TILE_K,
-                                    w.row0 + GM_TILE_M, &a_full[s]);
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_f16(GM_TILE_M, S::UN);
-            uint32_t it = 0, ti = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-                GemmTile w;
-                if (!gemm_tile_at(a, tab, t, w)) continue;
-                const int as = ti % S::ACC;
-                if (ti >= S::ACC) ok = mbar_wait(&acc_empty[as], ((ti / S::ACC) - 1) & 1, a.status);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t tacc = tmem + as * (2 * S::UN);
-                const bool two = w.row0 + GM_TILE_M < w.row_end;
-                const int kb0 = w.split * a.kb_split, kb1 = min(KB_ALL, kb0 + a.kb_split);
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = it % S::SA, b = it % S::SB;
-                    ok = mbar_wait(&a_full[s], (it / S::SA) & 1, a.status) &&
-                         mbar_wait(&b_full[b], (it / S::SB) & 1, a.status);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t a_addr = smem_u32(sm_a + (size_t)s * S::A_STAGE);
-                    const uint32_t b_addr = smem_u32(sm_b + (size_t)b * S::B16);
-#pragma unroll
-                    for (int k = 0; k < GM_TILE_K / 16; ++k)
-                        umma_f16(tacc, umma_smem_desc(a_addr + k * 32), umma_smem_desc(b_addr + k * 32), idesc,
-                                 kb > kb0 || k > 0);
-                    if (two) {
-#pragma unroll
-                        for (int k = 0; k < GM_TILE_K / 16; ++k)
-                            umma_f16(tacc + S::UN, umma_smem_desc(a_addr + GM_STAGE_A + k * 32),
-                                     umma_smem_desc(b_addr + k * 32), idesc, kb > kb0 || k > 0);
-                    }
-                    umma_commit(&a_empty[s]);
-                    umma_commit(&b_empty[b]);
-                }
-                if (!ok) break;
-                umma_commit(&acc_full[as]);
-                ++ti;
-            }
-        }
-    } else if (warp < GQ_FIRST_EXPAND) {
-        gemm_epilogue_loop<EPI, S::UN, S::ACC, 2>(a, tmem, acc_full, acc_empty, warp, lane, total, epi_scratch, tab);
-    } else {
-        // eight expanding warps: thread -> (B row, which 32 of the block's 64 weights)
-        const int x = threadIdx.x - GQ_FIRST_EXPAND * 32, row_t = x & 127, hh = x >> 7;
-        uint32_t it = 0, sbi = 0;
-        bool ok = true;
-        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-            GemmTile w;
-            if (!gemm_tile_at(a, tab, t, w)) continue;
-            const int kb0 = w.split * a.kb_split, kb1 = min(KB_ALL, kb0 + a.kb_split);
-            for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                const int j = kb & 3, b = it % S::SB;
-                if (j == 0) ++sbi;                    // sbi - 1 is the super-block in use
-                const int p = (sbi - 1) % S::SP;
-                if (j == 0) ok = mbar_wait(&p_full[p], ((sbi - 1) / S::SP) & 1, a.status);
-                if (ok && it >= S::SB) ok = mbar_wait(&b_empty[b], ((it / S::SB) - 1) & 1, a.status);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                const uint8_t* packed = sm_p + (size_t)p * S::PACKED;
-                uint8_t* tile = sm_b + (size_t)b * S::B16;
-#pragma unroll
-                for (int rr = 0; rr < S::UN / 128; ++rr) {
-                    const int r = row_t + rr * 128;
-                    dequant_half_block<KIND>(packed + (size_t)r * S::SBB, j, hh, tile, r);
-                }
-                fence_proxy_async();                  // generic-proxy stores -> visible to the MMA
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&b_full[b]);
-                    if (j == 3) mbar_arrive(&p_empty[p]);
-                }
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, S::ACC * 2 * S::UN);
-}
-
-// ===========================================================================
 // fp32 rows -> fp16 rows (optionally gathered): the A operand
 // ===========================================================================
 // dst[r, :] = half(src[(row_map ? row_map[r] / div : r), :]), values clamped to the
@@ -811,15 +532,15 @@ int make_tile_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, i
 }
 
 // Tensor map over packed rows viewed as 32-bit words: boxes of (box_bytes / 4) words
-// x GM_TILE_N rows, no swizzle.
-static int make_packed_map(CUtensorMap* out, const void* base, int64_t rows, int64_t row_bytes, int box_bytes) {
+// x box_rows rows, no swizzle.
+int make_packed_map(CUtensorMap* out, const void* base, int64_t rows, int64_t row_bytes, int box_bytes, int box_rows) {
     B200_REQUIRE(base && rows > 0 && row_bytes % 16 == 0 && box_bytes % 16 == 0, "packed map: rows must be 16-byte multiples");
     B200_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, "packed map: base must be 16-byte aligned");
-    typedef std::tuple<const void*, int64_t, int64_t, int> Key;
+    typedef std::tuple<const void*, int64_t, int64_t, int, int> Key;
     static std::map<Key, CUtensorMap> cache;
     static std::mutex mu;
     std::lock_guard<std::mutex> lock(mu);
-    const Key key(base, rows, row_bytes, box_bytes);
+    const Key key(base, rows, row_bytes, box_bytes, box_rows);
     auto it = cache.find(key);
     if (it != cache.end()) {
         *out = it->second;
@@ -829,7 +550,7 @@ static int make_packed_map(CUtensorMap* out, const void* base, int64_t rows, int
     if (!fn) return fail(B200_ECUDA, "packed map: the driver does not export cuTensorMapEncodeTiled");
     const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / 4), (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-    const cuuint32_t box[2] = {(cuuint32_t)(box_bytes / 4), (cuuint32_t)GM_TILE_N};
+    const cuuint32_t box[2] = {(cuuint32_t)(box_bytes / 4), (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -852,102 +573,12 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
     }
 }
 
-template <int EPI, int KIND>
-static int launch_gemm_q(const GemmArgs& a) {
-    using S = GemmQShape<EPI, KIND>;
-    auto kern = umma_gemm_q_kernel<EPI, KIND>;
-    static bool configured = false;
-    if (!configured) {
-        B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
-        configured = true;
-    }
-    GemmArgs b = a;
-    b.tile_m = 2 * GM_TILE_M;
-    b.m_slots = (a.M + b.tile_m - 1) / b.tile_m + (a.offsets ? a.groups : 0);
-    b.tile_n = GemmShape<EPI>::TN;
-    b.n_tiles = (a.N + b.tile_n - 1) / b.tile_n;
-    b.k_splits = 1;
-    b.kb_split = a.K / GM_TILE_K;
-    b.split_stride = 0;
-    // Few tiles (few rows and a narrow matrix: batched decode, the attention projections):
-    // every CTA would stream its 128 weight rows over all of K while most SMs idle, so K is
-    // cut across CTAs and the partial products are added afterwards in a fixed order.
-    const int tiles = b.m_slots * b.n_tiles, sb = a.K / 256;
-    // Not for the grouped form: the reduction pass walks all M rows, but a grouped launch
-    // writes partial sums only for the rows its offsets cover - rows outside them (other
-    // ranks' experts in the expert-parallel layer) must be left exactly as they are.
-    if (EPI == GEMM_EPI_STORE && a.offsets == nullptr && a.allow_split_k && sb >= 2 && tiles * 2 <= num_sms()) {
-        const int want = std::min(sb, num_sms() / tiles);
-        const int per = (sb + want - 1) / want;
-        b.k_splits = (sb + per - 1) / per;
-        b.kb_split = per * 4;
-    }
-    if (b.k_splits > 1) {
-        b.split_stride = (int64_t)a.M * a.ldc;
-        void* wsp;
-        int rc = workspace(WS_SPLITK).ensure((size_t)b.k_splits * b.split_stride * sizeof(float) + 256, &wsp);
-        if (rc) return rc;
-        b.c = static_cast<float*>(wsp);
-    }
-    const int grid = std::min(tiles * b.k_splits, num_sms());
-    kern<<<grid, GQ_THREADS, S::SMEM, stream()>>>(b);
-    B200_LAUNCH_CHECK("umma_gemm_q_kernel");
-    if (b.k_splits > 1) {
-        const int64_t total = (int64_t)a.M * a.N;
-        splitk_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div64(total, 256), (int64_t)num_sms() * 8), 256, 0, stream()>>>(
-            b.c, a.c, b.k_splits, b.split_stride, a.M, a.N, a.ldc);
-        B200_LAUNCH_CHECK("splitk_reduce_kernel");
-    }
+int splitk_reduce(const float* part, float* c, int splits, int64_t stride, int M, int N, int64_t ldc) {
+    const int64_t total = (int64_t)M * N;
+    splitk_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div64(total, 256), (int64_t)num_sms() * 8), 256, 0, stream()>>>(
+        part, c, splits, stride, M, N, ldc);
+    B200_LAUNCH_CHECK("splitk_reduce_kernel");
     return B200_OK;
-}
-
-// As umma_gemm(), with B (and B2) packed in `kind` (0..3), [b_rows, K]; K % 256 == 0.
-int umma_gemm_q(int epi, int kind, const __half* A, int64_t a_rows, const void* B, const void* B2, int64_t b_rows,
-                const int32_t* offsets, int groups, int M, int N, int K, float* c, __half* c16, int64_t ldc,
-                float scale, const int32_t* group_map, float* const* group_c, bool allow_split_k) {
-    if (M <= 0 || N <= 0) return B200_OK;
-    B200_REQUIRE(kind >= 0 && kind <= 3, "umma_gemm_q: unknown kind %d", kind);
-    B200_REQUIRE(!group_c || (offsets && epi == GEMM_EPI_STORE), "umma_gemm_q: per-group outputs need the grouped store form");
-    B200_REQUIRE(A && B && K > 0 && K % 256 == 0, "umma_gemm_q: K must be a positive multiple of 256");
-    B200_REQUIRE(groups >= 1 && (offsets || groups == 1), "umma_gemm_q: groups need a device offsets array");
-    B200_REQUIRE((group_map || b_rows >= (int64_t)groups * N) && a_rows >= M, "umma_gemm_q: operand shapes do not cover the groups");
-    GemmArgs a;
-    int rc = make_tile_map(&a.map_a, A, a_rows, K, GM_TILE_M);
-    if (rc) return rc;
-    const int64_t row_bytes = q_row_bytes(kind, K);
-    const int sbb = 8 * (kind == 3 ? 18 : q_block_bytes(kind));
-    rc = make_packed_map(&a.map_b, B, b_rows, row_bytes, sbb);
-    if (rc) return rc;
-    a.map_b2 = a.map_b;
-    if (epi == GEMM_EPI_SWIGLU) {
-        B200_REQUIRE(B2 && c16 && ldc % 2 == 0, "umma_gemm_q: the SwiGLU form needs the second matrix and an fp16 output");
-        rc = make_packed_map(&a.map_b2, B2, b_rows, row_bytes, sbb);
-        if (rc) return rc;
-    } else {
-        B200_REQUIRE(c || group_c, "umma_gemm_q: null output");
-    }
-    a.offsets = offsets; a.group_map = group_map; a.M = M; a.groups = groups; a.N = N; a.K = K;
-    a.c = c; a.c16 = c16; a.ldc = ldc; a.scale = scale; a.group_c = group_c; a.allow_split_k = allow_split_k;
-    a.status = stream_status_ptr();
-    B200_REQUIRE(a.status, "umma_gemm_q: status word allocation failed");
-    // wide store tiles when they still fill the machine (row slots are an upper bound when
-    // grouped) and K is long: this kernel's wide form has a single accumulator set, so its
-    // epilogue is not hidden, which costs more than the wide MMA gains when a tile has only a
-    // few K steps (measured: the K = 512 expert down-projections lose 20 %, K = 1536 gains 16 %)
-    const int slots256 = (M + 2 * GM_TILE_M - 1) / (2 * GM_TILE_M) + (offsets ? groups / 2 : 0);
-    const bool wide = epi == GEMM_EPI_STORE && N >= 2 * GM_TILE_N && K >= 1024 &&
-                      slots256 * ((N + 2 * GM_TILE_N - 1) / (2 * GM_TILE_N)) >= num_sms();
-#define GQ(KIND_)                                                                        \
-    return epi == GEMM_EPI_SWIGLU ? launch_gemm_q<GEMM_EPI_SWIGLU, KIND_>(a)             \
-           : wide                 ? launch_gemm_q<GEMM_EPI_STORE_WIDE, KIND_>(a)         \
-                                  : launch_gemm_q<GEMM_EPI_STORE, KIND_>(a);
-    switch (kind) {
-        case 0: GQ(0)
-        case 1: GQ(1)
-        case 2: GQ(2)
-        default: GQ(3)
-    }
-#undef GQ
 }
 
 template <int EPI>

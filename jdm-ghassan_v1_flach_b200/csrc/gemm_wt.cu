@@ -1,0 +1,571 @@
+// The many-token GEMM for packed weights:  C[rows, N] = A[rows, K] . W[N, K]^T  on tcgen05 with the
+// dequantised WEIGHTS as the MMA's first operand in TENSOR memory and the token rows as the second in shared
+// memory: the accumulator of a tile is [128 weight rows (lanes) x up to 192 tokens (columns)].
+//
+// What bounded the form before it (weights expanded to fp16 tiles in shared memory, both operands read from
+// there, 256 token rows per tile): shared-memory bandwidth - a 64-wide K step moved 131 KB (1020 cycles at
+// 128 B per cycle) for 524 cycles of tensor work - and, with few tokens, one expanding warp pass per K step
+// and MMA work for 128-row halves that were mostly empty.  Here a thread expands its own weight row in
+// registers and writes it with one tcgen05.st; shared memory sees the token rows once in and once out and the
+// packed bytes (29 + 29 KB per 393 tensor cycles), and the MMA's N is the tile's own token count rounded to 16.
+//
+// Tensor memory: two accumulator sets of 192 columns (the epilogue of a tile under the main loop of the next) and
+// four operand slots of 32 columns (64 fp16 of K).  The SwiGLU form puts 64 gate rows and the same 64 up rows
+// in one tile and exchanges them through shared memory in the epilogue.
+//   warp 0        token rows by TMA (64 of K per stage, boxes of 32 rows)
+//   warp 2        packed rows by TMA (256 of K per stage)
+//   warp 1        MMA issue
+//   warps 4..7    epilogue: a lane holds one weight row, so a warp stores 32 consecutive outputs of a token
+//   warps 8..23   expansion: four groups of four warps, group = operand slot = K step mod 4
+// Group lists (the MoE experts): rows of A cut into consecutive ranges by device offsets; a range is cut into
+// equal token tiles.  All waits are bounded; see gemm_umma.cu for what happens when one runs out.
+//
+// 4096 x 6448 x 1536 Q4_K: 106 us before, WT1.  MoE layer of the H-Tiny shape, 4096 tokens: WT2.
+#include <algorithm>
+
+#include "gemm.cuh"
+#include "linear.cuh"
+#include "umma.cuh"
+
+namespace b200 {
+
+int make_packed_map(CUtensorMap* out, const void* base, int64_t rows, int64_t row_bytes, int box_bytes, int box_rows);
+int splitk_reduce(const float* part, float* c, int splits, int64_t stride, int M, int N, int64_t ldc);
+
+constexpr int WT_TOKENS = 192;                // most tokens of a tile
+constexpr int WT_ROWS = 128;                  // weight rows of a tile
+constexpr int WT_BOX = 32;                    // token rows of a TMA box
+constexpr int WT_X_STAGE = WT_TOKENS * 128;   // 64 fp16 of K per token row
+constexpr int WT_SLOT0 = 2 * WT_TOKENS;       // first tensor-memory column of the operand slots
+constexpr int WT_SLOT = 32, WT_SLOTS = 4;
+constexpr int WT_SWAP = 2 * 2 * 16 * 64 * 4;  // SwiGLU epilogue: [buffer][half][token][row] floats
+constexpr int WT_FIRST_EXPAND = 8;
+constexpr int WT_EXPAND_WARPS = 16;
+constexpr int WT_THREADS = (WT_FIRST_EXPAND + WT_EXPAND_WARPS) * 32;
+constexpr int WT_MAX_GROUPS = 256;            // group lists kept as a prefix table; longer ones are walked
+
+struct alignas(64) WtArgs {
+    CUtensorMap map_x, map_w, map_w2;
+    const int32_t* offsets;                   // device [groups + 1], or null: one group of M rows
+    const int32_t* group_map;                 // device [groups]: block of N weight rows a group uses (negative: skipped)
+    int M, groups, N, K;
+    int slots, n_tiles;                       // upper bound of the token tiles, weight tiles per token tile
+    float* c;
+    float* const* group_c;                    // see GemmArgs
+    __half* c16;
+    int64_t ldc;
+    float scale;
+    int* status;
+    int k_splits, sb_split;                   // K ranges (in units of 256) whose partial products are added afterwards
+    int64_t split_stride;
+};
+
+template <bool SWIGLU, int KIND>
+struct WtShape {
+    static constexpr int SBB = 8 * (KIND == 3 ? 18 : q_block_bytes(KIND));     // bytes of 256 weights
+    static constexpr int PACKED = WT_ROWS * SBB;
+    static constexpr int SX = 5;
+    static constexpr int SP = KIND == 2 ? 2 : 3;
+    static constexpr int TILE_N = SWIGLU ? WT_ROWS / 2 : WT_ROWS;              // output columns of a tile
+    static constexpr int SMEM = SX * WT_X_STAGE + SP * PACKED + (SWIGLU ? WT_SWAP : 0) + 1024 + 256 + (WT_MAX_GROUPS + 2) * 4;
+    static_assert(SMEM <= 227 * 1024, "the stages do not fit the shared memory of an SM");
+};
+
+struct WtTile {
+    int group, row0, rows, n0, brow, split;
+};
+
+__host__ __device__ __forceinline__ int wt_tiles(int rows) { return (rows + WT_TOKENS - 1) / WT_TOKENS; }
+// Tile i of `rows` token rows cut into equal tiles of a multiple of 16.
+__device__ __forceinline__ void wt_cut(int rows, int i, int& first, int& count) {
+    const int n = max(1, wt_tiles(rows)), size = ((rows + n - 1) / n + 15) & ~15;
+    first = i * size;
+    count = max(0, min(size, rows - first));
+}
+
+// first[g] = first token tile of group g; first[groups] = all of them.  All threads.
+__device__ __noinline__ void wt_build(const WtArgs& a, int* first) {
+    if (!a.offsets || a.groups > WT_MAX_GROUPS) return;
+    for (int g = threadIdx.x; g < a.groups; g += blockDim.x)
+        first[g] = (a.group_map && a.group_map[g] < 0) ? 0 : wt_tiles(a.offsets[g + 1] - a.offsets[g]);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int carry = 0;
+        for (int g0 = 0; g0 < a.groups; g0 += 32) {
+            const int g = g0 + threadIdx.x, n = g < a.groups ? first[g] : 0;
+            int incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)threadIdx.x >= o) incl += up;
+            }
+            __syncwarp();
+            if (g < a.groups) first[g] = carry + incl - n;
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (threadIdx.x == 0) first[a.groups] = carry;
+    }
+    __syncthreads();
+}
+
+__device__ __noinline__ bool wt_tile_at(const WtArgs& a, const int* first, int t, WtTile& w) {
+    w.split = 0;
+    if (a.k_splits > 1) {
+        w.split = t % a.k_splits;
+        t /= a.k_splits;
+    }
+    const int slot = t / a.n_tiles;
+    w.n0 = t - slot * a.n_tiles;              // weight tile; scaled by the caller's tile width
+    w.group = 0;
+    int lo = 0, hi = a.M, i = slot;
+    if (a.offsets) {
+        if (a.groups <= WT_MAX_GROUPS) {
+            if (slot >= first[a.groups]) return false;
+            int l = 0, h = a.groups;          // the last group whose first tile is <= slot owns it
+            while (h - l > 1) {
+                const int mid = (l + h) >> 1;
+                if (first[mid] <= slot) l = mid; else h = mid;
+            }
+            w.group = l;
+            i = slot - first[l];
+        } else {
+            int g = 0;
+            for (; g < a.groups; ++g) {
+                const int n = (a.group_map && a.group_map[g] < 0) ? 0 : wt_tiles(a.offsets[g + 1] - a.offsets[g]);
+                if (i < n) break;
+                i -= n;
+            }
+            if (g == a.groups) return false;
+            w.group = g;
+        }
+        lo = a.offsets[w.group];
+        hi = a.offsets[w.group + 1];
+    }
+    wt_cut(hi - lo, i, w.row0, w.rows);
+    w.row0 += lo;
+    w.brow = (a.group_map ? a.group_map[w.group] : w.group) * a.N;
+    return w.rows > 0;
+}
+
+// ---- expansion: 64 weights of a row (K step J of its 256) to 32 fp16 pairs ----------------------
+// fp16 arithmetic, two values per instruction: a byte b OR-ed into the mantissa of 0x6400 is 1024 + b.
+//   Q4_0  (q - 8) * d,  Q8_0  q * d        exact products rounded once
+//   Q4_1  q * d + m                         one rounding
+//   Q4_K  (q * sc) * d - fp16(m * dmin)     q * sc exact; the minimum rounded first
+// against the fp16-rounded value of the materialising dequantiser: equal for Q4_0 / Q8_0, within one ulp else.
+__device__ __forceinline__ __half2 wt_magic(uint32_t bytes, uint32_t sel) {
+    const uint32_t v = __byte_perm(bytes, 0x64646464u, sel);
+    return *reinterpret_cast<const __half2*>(&v);
+}
+constexpr uint32_t WT_SEL_01 = 0x5140, WT_SEL_23 = 0x5342;
+__device__ __forceinline__ uint32_t wt_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ __half2 wt_half2(uint32_t bits16) { return __half2half2(__ushort_as_half((unsigned short)bits16)); }
+
+template <int KIND, int J>
+__device__ __forceinline__ void wt_expand(uint32_t seg, uint32_t (&out)[32]) {
+    auto vec = [&](int i) {
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(seg + 16 * i));
+        return v;
+    };
+    if (KIND == 3) {
+        const uint4 hdr = vec(0), q0 = vec(1 + 2 * J), q1 = vec(2 + 2 * J);
+        const __half2 d2 = wt_half2(hdr.x & 0xFFFFu);
+        const float dmin = half_bits_to_float((uint16_t)(hdr.x >> 16));
+        const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            int s, m;
+            q4k_scale_min_regs(2 * J + hh, hdr.y, hdr.z, hdr.w, s, m);
+            // high nibbles stay where they are: 1024 + 16 q, times s / 16 (exact)
+            const __half2 sc2 = __half2half2(__hmul(__int2half_rn(s), __float2half(hh ? 0.0625f : 1.0f)));
+            const __half2 nsc = __half2half2(__int2half_rn((hh ? -64 : -1024) * s));                    // exact
+            const __half2 nm = __half2half2(__float2half_rn(-__fmul_rn(dmin, (float)m)));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t x = words[i] & (hh ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
+                out[16 * hh + 2 * i] = wt_bits(__hfma2(__hfma2(wt_magic(x, WT_SEL_01), sc2, nsc), d2, nm));
+                out[16 * hh + 2 * i + 1] = wt_bits(__hfma2(__hfma2(wt_magic(x, WT_SEL_23), sc2, nsc), d2, nm));
+            }
+        }
+    } else {
+        // the 16-byte window that covers the two blocks, then words at compile-time places
+        constexpr int WORDS = KIND == 2 ? 17 : KIND == 1 ? 10 : 9, W0 = WORDS * J, V0 = W0 / 4, OFF = W0 % 4, NV = (OFF + WORDS + 3) / 4;
+        uint32_t w[4 * NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const uint4 v = vec(V0 + i);
+            w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+        }
+        auto half_at = [&](int i) { return (w[OFF + (i >> 1)] >> (16 * (i & 1))) & 0xFFFFu; };
+        constexpr int BH = q_block_bytes(KIND) / 2;                   // halfwords per block
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const __half2 d2 = wt_half2(half_at(b * BH));
+            if (KIND == 2) {
+                const __half2 bias = wt_half2(0x6480u);               // 1024 + 128
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int h = b * BH + 1 + i;
+                    const uint32_t x = w[OFF + (h >> 1)] ^ 0x80808080u;          // int8 + 128
+                    out[16 * b + i] = wt_bits(__hmul2(__hsub2(wt_magic(x, (h & 1) ? WT_SEL_23 : WT_SEL_01), bias), d2));
+                }
+            } else {
+                const __half2 off = wt_half2(KIND == 0 ? 0x6408u : 0x6400u);     // 1032 / 1024
+                const __half2 m2 = KIND == 1 ? wt_half2(half_at(b * BH + 1)) : wt_half2(0u);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int h = b * BH + (KIND == 0 ? 1 : 2) + i;
+                    const uint32_t x = w[OFF + (h >> 1)], sel = (h & 1) ? WT_SEL_23 : WT_SEL_01;
+                    const __half2 lo = __hsub2(wt_magic(x & 0x0F0F0F0Fu, sel), off), hi = __hsub2(wt_magic((x >> 4) & 0x0F0F0F0Fu, sel), off);
+                    out[16 * b + i] = wt_bits(KIND == 0 ? __hmul2(lo, d2) : __hfma2(lo, d2, m2));
+                    out[16 * b + 8 + i] = wt_bits(KIND == 0 ? __hmul2(hi, d2) : __hfma2(hi, d2, m2));
+                }
+            }
+        }
+    }
+}
+
+// 32 columns of this warp's 32 tensor-memory lanes from registers.
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
+        "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
+        "r"(r[31])
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+// D[tmem] (+)= A[tmem] * B[smem]^T, one thread issues.
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+}
+// The fast exponential and reciprocal (a few fp32 ulp) are invisible after the rounding to fp16.
+__device__ __forceinline__ float wt_silu(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
+
+template <bool SWIGLU, int KIND>
+__global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_constant__ WtArgs a) {
+    using S = WtShape<SWIGLU, KIND>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* sm_x = smem;
+    uint8_t* sm_p = sm_x + S::SX * WT_X_STAGE;
+    float* swap = reinterpret_cast<float*>(sm_p + S::SP * S::PACKED);
+    uint64_t* x_full = reinterpret_cast<uint64_t*>(sm_p + S::SP * S::PACKED + (SWIGLU ? WT_SWAP : 0));
+    uint64_t* x_empty = x_full + S::SX;
+    uint64_t* p_full = x_empty + S::SX;
+    uint64_t* p_empty = p_full + S::SP;
+    uint64_t* a_full = p_empty + S::SP;
+    uint64_t* a_empty = a_full + WT_SLOTS;
+    uint64_t* acc_full = a_empty + WT_SLOTS;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    int* first = reinterpret_cast<int*>(x_full) + 64;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int total = a.slots * a.n_tiles * a.k_splits, sb_all = a.K / 256;
+    wt_build(a, first);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S::SX; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
+        for (int s = 0; s < S::SP; ++s) { mbar_init(&p_full[s], 1); mbar_init(&p_empty[s], WT_EXPAND_WARPS); }
+        for (int s = 0; s < WT_SLOTS; ++s) { mbar_init(&a_full[s], 4); mbar_init(&a_empty[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], 4); }
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    // every role walks the same tiles; sb0 .. sb1: a tile's range of K in units of 256
+    auto range = [&](const WtTile& w, int& sb0, int& sb1) {
+        sb0 = w.split * a.sb_split;
+        sb1 = min(sb_all, sb0 + a.sb_split);
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t it = 0, s = 0, ph = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+                WtTile w;
+                if (!wt_tile_at(a, first, t, w)) continue;
+                int sb0, sb1;
+                range(w, sb0, sb1);
+                const int boxes = (w.rows + WT_BOX - 1) / WT_BOX;
+                for (int kb = 4 * sb0; kb < 4 * sb1; ++kb, ++it) {
+                    if (it >= S::SX) ok = mbar_wait(&x_empty[s], ph ^ 1, a.status);
+                    if (!ok) break;
+                    mbar_expect_tx(&x_full[s], boxes * WT_BOX * 128);
+                    for (int b = 0; b < boxes; ++b)
+                        tma_load_2d(sm_x + s * WT_X_STAGE + b * WT_BOX * 128, &a.map_x, kb * 64, w.row0 + b * WT_BOX, &x_full[s]);
+                    if (++s == S::SX) { s = 0; ph ^= 1; }
+                }
+            }
+            if (!ok)
+                for (uint32_t j = it > S::SX ? it - S::SX : 0; j < it; ++j)
+                    if (!mbar_wait(&x_full[j % S::SX], (j / S::SX) & 1, a.status)) break;
+        }
+    } else if (warp == 2) {
+        if (lane == 0) {
+            uint32_t it = 0, p = 0, ph = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+                WtTile w;
+                if (!wt_tile_at(a, first, t, w)) continue;
+                int sb0, sb1;
+                range(w, sb0, sb1);
+                const int brow = w.brow + w.n0 * S::TILE_N;
+                for (int sb = sb0; sb < sb1; ++sb, ++it) {
+                    if (it >= S::SP) ok = mbar_wait(&p_empty[p], ph ^ 1, a.status);
+                    if (!ok) break;
+                    uint8_t* dst = sm_p + p * S::PACKED;
+                    mbar_expect_tx(&p_full[p], S::PACKED);
+                    tma_load_2d(dst, &a.map_w, sb * (S::SBB / 4), brow, &p_full[p]);
+                    if (SWIGLU) tma_load_2d(dst + S::PACKED / 2, &a.map_w2, sb * (S::SBB / 4), brow, &p_full[p]);
+                    if (++p == S::SP) { p = 0; ph ^= 1; }
+                }
+            }
+            if (!ok)
+                for (uint32_t j = it > S::SP ? it - S::SP : 0; j < it; ++j)
+                    if (!mbar_wait(&p_full[j % S::SP], (j / S::SP) & 1, a.status)) break;
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            uint32_t it = 0, ti = 0, s = 0, ph = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+                WtTile w;
+                if (!wt_tile_at(a, first, t, w)) continue;
+                int sb0, sb1;
+                range(w, sb0, sb1);
+                const uint32_t idesc = umma_idesc_f16(WT_ROWS, (w.rows + 15) & ~15), as = ti & 1;
+                if (ti > 1) ok = mbar_wait(&acc_empty[as], ((ti >> 1) - 1) & 1, a.status);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t d = tmem + as * WT_TOKENS;
+                for (int kb = 4 * sb0; kb < 4 * sb1; ++kb, ++it) {
+                    const uint32_t slot = it & (WT_SLOTS - 1);
+                    ok = mbar_wait(&x_full[s], ph, a.status) && mbar_wait(&a_full[slot], (it / WT_SLOTS) & 1, a.status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t desc = umma_smem_desc(smem_u32(sm_x + s * WT_X_STAGE));
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)       // 32 bytes of K per step: 2 in the descriptor's units
+                        umma_f16_ts(d, tmem + WT_SLOT0 + slot * WT_SLOT + k * 8, desc + 2 * k, idesc, kb > 4 * sb0 || k > 0);
+                    umma_commit(&a_empty[slot]);
+                    umma_commit(&x_empty[s]);
+                    if (++s == S::SX) { s = 0; ph ^= 1; }
+                }
+                if (!ok) break;
+                umma_commit(&acc_full[as]);
+                ++ti;
+            }
+        }
+    } else if (warp >= 4 && warp < WT_FIRST_EXPAND) {
+        const int q = warp & 3;
+        uint32_t ti = 0;
+        for (int t = blockIdx.x; t < total; t += gridDim.x) {
+            WtTile w;
+            if (!wt_tile_at(a, first, t, w)) continue;
+            const uint32_t as = ti & 1;
+            bool ok = mbar_wait(&acc_full[as], (ti >> 1) & 1, a.status);
+            ok = __all_sync(0xffffffffu, ok && *reinterpret_cast<volatile int*>(a.status) == 0);
+            if (SWIGLU) {
+                // the four warps meet in the exchange: they go on or stop together
+                int all;
+                asm volatile(
+                    "{\n\t.reg .pred p, r;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.and.pred r, 1, 128, p;\n\t"
+                    "selp.b32 %0, 1, 0, r;\n\t}"
+                    : "=r"(all)
+                    : "r"((int)ok)
+                    : "memory");
+                ok = all != 0;
+            }
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t tq = tmem + as * WT_TOKENS + ((uint32_t)(q * 32) << 16);
+            if (SWIGLU) {
+                // lanes of warps 0, 1: gate rows; of 2, 3: up rows.  Of every 32 tokens warps 0, 1 finish the first
+                // 16 and warps 2, 3 the rest: each side leaves the other's half in the exchange buffer.
+                const int side = q >> 1, r = (q & 1) * 32 + lane, n = w.n0 * S::TILE_N + r;
+                __half* dst = a.c16 + ((int64_t)w.row0 + 16 * side) * a.ldc + n;
+                int buf = 0;
+                for (int c0 = 0; c0 < w.rows; c0 += 32, dst += 32 * a.ldc, buf ^= 1) {
+                    float mine[16], give[16];
+                    tmem_ld16(tq + c0 + 16 * side, mine);
+                    tmem_ld16(tq + c0 + 16 * (side ^ 1), give);
+                    float* out = swap + (buf * 2 + side) * 16 * 64 + r;
+                    const float* in = swap + (buf * 2 + (side ^ 1)) * 16 * 64 + r;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) out[i * 64] = give[i];
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    const int left = w.rows - c0 - 16 * side;
+                    if (n < a.N) {
+                        __half* o = dst;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i, o += a.ldc) {
+                            const float other = in[i * 64];
+                            if (i < left) *o = __float2half_rn(side ? wt_silu(other) * mine[i] : wt_silu(mine[i]) * other);
+                        }
+                    }
+                }
+            } else {
+                const int n = w.n0 * S::TILE_N + q * 32 + lane;
+                const int64_t step = a.ldc;
+                float* dst = (a.group_c ? a.group_c[w.group] : a.c + w.split * a.split_stride) + (int64_t)w.row0 * step + n;
+                for (int c0 = 0; c0 < w.rows; c0 += 32) {
+                    float v[32];
+                    tmem_ld32(tq + c0, v);                    // columns past the tile's tokens are not stored
+                    if (n < a.N) {
+                        const int left = w.rows - c0;
+                        if (left >= 32) {
+#pragma unroll
+                            for (int i = 0; i < 32; ++i, dst += step) *dst = v[i] * a.scale;
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 32; ++i, dst += step)
+                                if (i < left) *dst = v[i] * a.scale;
+                        }
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[as]);
+            ++ti;
+        }
+    } else if (warp >= WT_FIRST_EXPAND) {
+        const int slot = (warp - WT_FIRST_EXPAND) >> 2, q = warp & 3;
+        const uint32_t dst = tmem + WT_SLOT0 + slot * WT_SLOT + ((uint32_t)(q * 32) << 16);
+        const uint32_t row_at = smem_u32(sm_p) + (q * 32 + lane) * S::SBB;
+        uint32_t it = 0, p = 0, ph = 0;                   // stages of 256 = K steps of this slot
+        bool ok = true;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+            WtTile w;
+            if (!wt_tile_at(a, first, t, w)) continue;
+            int sb0, sb1;
+            range(w, sb0, sb1);
+            for (int sb = sb0; sb < sb1; ++sb, ++it) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&p_full[p], ph, a.status));
+                if (!ok) break;
+                const uint32_t seg = row_at + p * S::PACKED;
+                uint32_t out[32];
+                if (slot == 0) wt_expand<KIND, 0>(seg, out);
+                else if (slot == 1) wt_expand<KIND, 1>(seg, out);
+                else if (slot == 2) wt_expand<KIND, 2>(seg, out);
+                else wt_expand<KIND, 3>(seg, out);
+                if (lane == 0) mbar_arrive(&p_empty[p]);
+                if (++p == S::SP) { p = 0; ph ^= 1; }
+                if (it > 0) ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[slot], (it - 1) & 1, a.status));
+                if (!ok) break;
+                tc_fence_after();
+                tmem_st32(dst, out);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&a_full[slot]);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, 512);
+}
+
+// ---- host side ------------------------------------------------------------------
+template <bool SWIGLU, int KIND>
+static int launch_wt(WtArgs& a, bool allow_split) {
+    using S = WtShape<SWIGLU, KIND>;
+    auto kern = umma_wt_kernel<SWIGLU, KIND>;
+    static bool configured = false;
+    if (!configured) {
+        B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
+        configured = true;
+    }
+    a.n_tiles = ceil_div(a.N, S::TILE_N);
+    a.slots = wt_tiles(a.M) + (a.offsets ? a.groups : 0);
+    const int tiles = a.slots * a.n_tiles, sb = a.K / 256;
+    a.k_splits = 1;
+    a.sb_split = sb;
+    // Few tiles (a decode batch, the attention projections): K is cut across CTAs and the partial products are
+    // added in a fixed order.  Not for group lists: the sum walks all M rows, a list may leave some untouched.
+    if (!SWIGLU && !a.offsets && allow_split && sb >= 2 && tiles * 2 <= num_sms()) {
+        const int per = ceil_div(sb, std::min(sb, num_sms() / tiles));
+        a.k_splits = ceil_div(sb, per);
+        a.sb_split = per;
+    }
+    float* c = a.c;
+    if (a.k_splits > 1) {
+        a.split_stride = (int64_t)a.M * a.ldc;
+        void* wsp;
+        int rc = workspace(WS_SPLITK).ensure((size_t)a.k_splits * a.split_stride * sizeof(float) + 256, &wsp);
+        if (rc) return rc;
+        a.c = static_cast<float*>(wsp);
+    }
+    kern<<<std::min(tiles * a.k_splits, num_sms()), WT_THREADS, S::SMEM, stream()>>>(a);
+    B200_LAUNCH_CHECK("umma_wt_kernel");
+    return a.k_splits > 1 ? splitk_reduce(a.c, c, a.k_splits, a.split_stride, a.M, a.N, a.ldc) : B200_OK;
+}
+
+// See gemm.cuh.
+int umma_gemm_q(int epi, int kind, const __half* A, int64_t a_rows, const void* B, const void* B2, int64_t b_rows,
+                const int32_t* offsets, int groups, int M, int N, int K, float* c, __half* c16, int64_t ldc,
+                float scale, const int32_t* group_map, float* const* group_c, bool allow_split_k) {
+    if (M <= 0 || N <= 0) return B200_OK;
+    B200_REQUIRE(kind >= 0 && kind <= 3, "umma_gemm_q: unknown kind %d", kind);
+    B200_REQUIRE(!group_c || (offsets && epi == GEMM_EPI_STORE), "umma_gemm_q: per-group outputs need the grouped store form");
+    B200_REQUIRE(A && B && K > 0 && K % 256 == 0, "umma_gemm_q: K must be a positive multiple of 256");
+    B200_REQUIRE(groups >= 1 && (offsets || groups == 1), "umma_gemm_q: groups need a device offsets array");
+    B200_REQUIRE((group_map || b_rows >= (int64_t)groups * N) && a_rows >= M, "umma_gemm_q: operand shapes do not cover the groups");
+    WtArgs a;
+    int rc = make_tile_map(&a.map_x, A, a_rows, K, WT_BOX);
+    if (rc) return rc;
+    const int64_t row_bytes = q_row_bytes(kind, K);
+    const int sbb = 8 * (kind == 3 ? 18 : q_block_bytes(kind));
+    const bool swiglu = epi == GEMM_EPI_SWIGLU;
+    const int box_rows = swiglu ? WT_ROWS / 2 : WT_ROWS;
+    rc = make_packed_map(&a.map_w, B, b_rows, row_bytes, sbb, box_rows);
+    if (rc) return rc;
+    a.map_w2 = a.map_w;
+    if (swiglu) {
+        B200_REQUIRE(B2 && c16 && ldc % 2 == 0, "umma_gemm_q: the SwiGLU form needs the second matrix and an fp16 output");
+        rc = make_packed_map(&a.map_w2, B2, b_rows, row_bytes, sbb, box_rows);
+        if (rc) return rc;
+    } else {
+        B200_REQUIRE(c || group_c, "umma_gemm_q: null output");
+    }
+    a.offsets = offsets; a.group_map = group_map; a.M = M; a.groups = groups; a.N = N; a.K = K;
+    a.c = c; a.group_c = group_c; a.c16 = c16; a.ldc = ldc; a.scale = scale; a.split_stride = 0;
+    a.status = stream_status_ptr();
+    B200_REQUIRE(a.status, "umma_gemm_q: status word allocation failed");
+    switch (kind) {
+        case 0: return swiglu ? launch_wt<true, 0>(a, allow_split_k) : launch_wt<false, 0>(a, allow_split_k);
+        case 1: return swiglu ? launch_wt<true, 1>(a, allow_split_k) : launch_wt<false, 1>(a, allow_split_k);
+        case 2: return swiglu ? launch_wt<true, 2>(a, allow_split_k) : launch_wt<false, 2>(a, allow_split_k);
+        default: return swiglu ? launch_wt<true, 3>(a, allow_split_k) : launch_wt<false, 3>(a, allow_split_k);
+    }
+}
+
+}  // namespace b200
