@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     int* first = reinterpret_cast<int*>(x_full) + 64;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int total = a.slots * a.n_tiles * a.k_splits, sb_all = a.K / 256;
     wt_build(a, first);
     if (threadIdx.x == 0) {
@@ -306,83 +306,82 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
     };
 
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t it = 0, s = 0, ph = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-                WtTile w;
-                if (!wt_tile_at(a, first, t, w)) continue;
-                int sb0, sb1;
-                range(w, sb0, sb1);
-                const int boxes = (w.rows + WT_BOX - 1) / WT_BOX;
-                for (int kb = 4 * sb0; kb < 4 * sb1; ++kb, ++it) {
-                    if (it >= S::SX) ok = mbar_wait(&x_empty[s], ph ^ 1, a.status);
-                    if (!ok) break;
+        uint32_t it = 0, s = 0, ph = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+            WtTile w;
+            if (!wt_tile_at(a, first, t, w)) continue;
+            int sb0, sb1;
+            range(w, sb0, sb1);
+            const int boxes = (w.rows + WT_BOX - 1) / WT_BOX;
+            for (int kb = 4 * sb0; kb < 4 * sb1; ++kb, ++it) {
+                if (it >= S::SX) ok = mbar_wait_warp(&x_empty[s], ph ^ 1, a.status);
+                if (!ok) break;
+                if (elect_one()) {
                     mbar_expect_tx(&x_full[s], boxes * WT_BOX * 128);
                     for (int b = 0; b < boxes; ++b)
                         tma_load_2d(sm_x + s * WT_X_STAGE + b * WT_BOX * 128, &a.map_x, kb * 64, w.row0 + b * WT_BOX, &x_full[s]);
-                    if (++s == S::SX) { s = 0; ph ^= 1; }
                 }
+                if (++s == S::SX) { s = 0; ph ^= 1; }
             }
-            if (!ok)
-                for (uint32_t j = it > S::SX ? it - S::SX : 0; j < it; ++j)
-                    if (!mbar_wait(&x_full[j % S::SX], (j / S::SX) & 1, a.status)) break;
         }
+        if (!ok)
+            for (uint32_t j = it > S::SX ? it - S::SX : 0; j < it; ++j)
+                if (!mbar_wait_warp(&x_full[j % S::SX], (j / S::SX) & 1, a.status)) break;
     } else if (warp == 2) {
-        if (lane == 0) {
-            uint32_t it = 0, p = 0, ph = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-                WtTile w;
-                if (!wt_tile_at(a, first, t, w)) continue;
-                int sb0, sb1;
-                range(w, sb0, sb1);
-                const int brow = w.brow + w.n0 * S::TILE_N;
-                for (int sb = sb0; sb < sb1; ++sb, ++it) {
-                    if (it >= S::SP) ok = mbar_wait(&p_empty[p], ph ^ 1, a.status);
-                    if (!ok) break;
+        uint32_t it = 0, p = 0, ph = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+            WtTile w;
+            if (!wt_tile_at(a, first, t, w)) continue;
+            int sb0, sb1;
+            range(w, sb0, sb1);
+            const int brow = w.brow + w.n0 * S::TILE_N;
+            for (int sb = sb0; sb < sb1; ++sb, ++it) {
+                if (it >= S::SP) ok = mbar_wait_warp(&p_empty[p], ph ^ 1, a.status);
+                if (!ok) break;
+                if (elect_one()) {
                     uint8_t* dst = sm_p + p * S::PACKED;
                     mbar_expect_tx(&p_full[p], S::PACKED);
                     tma_load_2d(dst, &a.map_w, sb * (S::SBB / 4), brow, &p_full[p]);
                     if (SWIGLU) tma_load_2d(dst + S::PACKED / 2, &a.map_w2, sb * (S::SBB / 4), brow, &p_full[p]);
-                    if (++p == S::SP) { p = 0; ph ^= 1; }
                 }
+                if (++p == S::SP) { p = 0; ph ^= 1; }
             }
-            if (!ok)
-                for (uint32_t j = it > S::SP ? it - S::SP : 0; j < it; ++j)
-                    if (!mbar_wait(&p_full[j % S::SP], (j / S::SP) & 1, a.status)) break;
         }
+        if (!ok)
+            for (uint32_t j = it > S::SP ? it - S::SP : 0; j < it; ++j)
+                if (!mbar_wait_warp(&p_full[j % S::SP], (j / S::SP) & 1, a.status)) break;
     } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t it = 0, ti = 0, s = 0, ph = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-                WtTile w;
-                if (!wt_tile_at(a, first, t, w)) continue;
-                int sb0, sb1;
-                range(w, sb0, sb1);
-                const uint32_t idesc = umma_idesc_f16(WT_ROWS, (w.rows + 15) & ~15), as = ti & 1;
-                if (ti > 1) ok = mbar_wait(&acc_empty[as], ((ti >> 1) - 1) & 1, a.status);
+        uint32_t it = 0, ti = 0, s = 0, ph = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+            WtTile w;
+            if (!wt_tile_at(a, first, t, w)) continue;
+            int sb0, sb1;
+            range(w, sb0, sb1);
+            const uint32_t idesc = umma_idesc_f16(WT_ROWS, (w.rows + 15) & ~15), as = ti & 1;
+            if (ti > 1) ok = mbar_wait_warp(&acc_empty[as], ((ti >> 1) - 1) & 1, a.status);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t d = tmem + as * WT_TOKENS;
+            for (int kb = 4 * sb0; kb < 4 * sb1; ++kb, ++it) {
+                const uint32_t slot = it & (WT_SLOTS - 1);
+                ok = mbar_wait_warp(&x_full[s], ph, a.status) && mbar_wait_warp(&a_full[slot], (it / WT_SLOTS) & 1, a.status);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t d = tmem + as * WT_TOKENS;
-                for (int kb = 4 * sb0; kb < 4 * sb1; ++kb, ++it) {
-                    const uint32_t slot = it & (WT_SLOTS - 1);
-                    ok = mbar_wait(&x_full[s], ph, a.status) && mbar_wait(&a_full[slot], (it / WT_SLOTS) & 1, a.status);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint64_t desc = umma_smem_desc(smem_u32(sm_x + s * WT_X_STAGE));
+                const uint64_t desc = umma_smem_desc(smem_u32(sm_x + s * WT_X_STAGE));
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k)       // 32 bytes of K per step: 2 in the descriptor's units
                         umma_f16_ts(d, tmem + WT_SLOT0 + slot * WT_SLOT + k * 8, desc + 2 * k, idesc, kb > 4 * sb0 || k > 0);
                     umma_commit(&a_empty[slot]);
                     umma_commit(&x_empty[s]);
-                    if (++s == S::SX) { s = 0; ph ^= 1; }
+                    if (kb == 4 * sb1 - 1) umma_commit(&acc_full[as]);
                 }
-                if (!ok) break;
-                umma_commit(&acc_full[as]);
-                ++ti;
+                if (++s == S::SX) { s = 0; ph ^= 1; }
             }
+            ++ti;
         }
     } else if (warp >= 4 && warp < WT_FIRST_EXPAND) {
         const int q = warp & 3;
@@ -469,7 +468,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
             int sb0, sb1;
             range(w, sb0, sb1);
             for (int sb = sb0; sb < sb1; ++sb, ++it) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&p_full[p], ph, a.status));
+                ok = mbar_wait_warp(&p_full[p], ph, a.status);
                 if (!ok) break;
                 const uint32_t seg = row_at + p * S::PACKED;
                 uint32_t out[32];
@@ -479,7 +478,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
                 else wt_expand<KIND, 3>(seg, out);
                 if (lane == 0) mbar_arrive(&p_empty[p]);
                 if (++p == S::SP) { p = 0; ph ^= 1; }
-                if (it > 0) ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[slot], (it - 1) & 1, a.status));
+                if (it > 0) ok = mbar_wait_warp(&a_empty[slot], (it - 1) & 1, a.status);
                 if (!ok) break;
                 tc_fence_after();
                 tmem_st32(dst, out);

@@ -92,6 +92,32 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
         ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
+// ---- warp-uniform roles ---------------------------------------------------------------
+// The tcgen05 and TMA instructions take descriptors and addresses in uniform registers.  A role run by one lane
+// of a divergent branch moves every operand there by hand, and its waits are divergent loops: 1150 cycles per
+// K step of four MMAs, whatever their size, with all operands ready (measured with clock stamps).  So a role's
+// whole warp walks its loop and only the issuing instructions are elected.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// Bounded wait of a whole warp, with the same result in every lane.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n"
+        "WAIT:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE;\n\t"
+        "sub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra WAIT;\n"
+        "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "n"(MBAR_SPIN_LIMIT)
+        : "memory");
+    const bool all = __all_sync(0xffffffffu, ok != 0);
+    if (!all && elect_one()) atomicExch(status, 1);
+    return all;
+}
 // Makes shared-memory writes of this thread visible to the async proxy (TMA, tcgen05).
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 #endif
