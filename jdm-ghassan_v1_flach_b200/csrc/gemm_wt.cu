@@ -12,7 +12,7 @@
 // Tensor memory: two accumulator sets of 192 columns (the epilogue of a tile under the main loop of the next) and
 // four operand slots of 32 columns (64 fp16 of K).  The SwiGLU form puts 64 gate rows and the same 64 up rows
 // in one tile and exchanges them through shared memory in the epilogue.
-//   warp 0        token rows by TMA (64 of K per stage, boxes of 32 rows)
+//   warp 0        token rows by TMA (64 of K per stage, boxes of 96 and 32 rows)
 //   warp 2        packed rows by TMA (256 of K per stage)
 //   warp 1        MMA issue
 //   warps 4..7    epilogue: a lane holds one weight row, so a warp stores 32 consecutive outputs of a token
@@ -20,7 +20,10 @@
 // Group lists (the MoE experts): rows of A cut into consecutive ranges by device offsets; a range is cut into
 // equal token tiles.  All waits are bounded; see gemm_umma.cu for what happens when one runs out.
 //
-// 4096 x 6448 x 1536 Q4_K: 106 us before, WT1.  MoE layer of the H-Tiny shape, 4096 tokens: WT2.
+// 4096 x 6448 x 1536 Q4_K: 106 us before, 90 now (both
+// with the 13 us that round the activations), a K step 600 cycles: what is left is the token rows' way from L2, 29 KB
+// per step and SM, where 256 weight rows per CTA would halve it but leave no room for a second accumulator set
+// (tried: the exposed epilogue cost more than the traffic).
 #include <algorithm>
 
 #include "gemm.cuh"
@@ -34,7 +37,7 @@ int splitk_reduce(const float* part, float* c, int splits, int64_t stride, int M
 
 constexpr int WT_TOKENS = 192;                // most tokens of a tile
 constexpr int WT_ROWS = 128;                  // weight rows of a tile
-constexpr int WT_BOX = 32;                    // token rows of a TMA box
+constexpr int WT_BOX = 32, WT_BIG_BOX = 96;   // token rows of a TMA box; one big box instead of three small ones: 5 %
 constexpr int WT_X_STAGE = WT_TOKENS * 128;   // 64 fp16 of K per token row
 constexpr int WT_SLOT0 = 2 * WT_TOKENS;       // first tensor-memory column of the operand slots
 constexpr int WT_SLOT = 32, WT_SLOTS = 4;
@@ -42,10 +45,11 @@ constexpr int WT_SWAP = 2 * 2 * 16 * 64 * 4;  // SwiGLU epilogue: [buffer][half]
 constexpr int WT_FIRST_EXPAND = 8;
 constexpr int WT_EXPAND_WARPS = 16;
 constexpr int WT_THREADS = (WT_FIRST_EXPAND + WT_EXPAND_WARPS) * 32;
+constexpr int WT_TABLE = 64;                  // a CTA's tiles worked out in advance; later ones on the way
 constexpr int WT_MAX_GROUPS = 256;            // group lists kept as a prefix table; longer ones are walked
 
 struct alignas(64) WtArgs {
-    CUtensorMap map_x, map_w, map_w2;
+    CUtensorMap map_x, map_x_big, map_w, map_w2;
     const int32_t* offsets;                   // device [groups + 1], or null: one group of M rows
     const int32_t* group_map;                 // device [groups]: block of N weight rows a group uses (negative: skipped)
     int M, groups, N, K;
@@ -67,7 +71,7 @@ struct WtShape {
     static constexpr int SX = 5;
     static constexpr int SP = KIND == 2 ? 2 : 3;
     static constexpr int TILE_N = SWIGLU ? WT_ROWS / 2 : WT_ROWS;              // output columns of a tile
-    static constexpr int SMEM = SX * WT_X_STAGE + SP * PACKED + (SWIGLU ? WT_SWAP : 0) + 1024 + 256 + (WT_MAX_GROUPS + 2) * 4;
+    static constexpr int SMEM = SX * WT_X_STAGE + SP * PACKED + (SWIGLU ? WT_SWAP : 0) + 1024 + 256 + (WT_MAX_GROUPS + 2) * 4 + WT_TABLE * 24;
     static_assert(SMEM <= 227 * 1024, "the stages do not fit the shared memory of an SM");
 };
 
@@ -108,7 +112,7 @@ __device__ __noinline__ void wt_build(const WtArgs& a, int* first) {
     __syncthreads();
 }
 
-__device__ __noinline__ bool wt_tile_at(const WtArgs& a, const int* first, int t, WtTile& w) {
+__device__ __noinline__ bool wt_find(const WtArgs& a, const int* first, int t, WtTile& w) {
     w.split = 0;
     if (a.k_splits > 1) {
         w.split = t % a.k_splits;
@@ -144,6 +148,24 @@ __device__ __noinline__ bool wt_tile_at(const WtArgs& a, const int* first, int t
     wt_cut(hi - lo, i, w.row0, w.rows);
     w.row0 += lo;
     w.brow = (a.group_map ? a.group_map[w.group] : w.group) * a.N;
+    return w.rows > 0;
+}
+
+// Tile number i of this CTA.  The search (divisions, bisection) takes over a thousand cycles, which every role would
+// otherwise spend between two tiles of a few thousand: one thread per tile does it when the kernel starts.
+__device__ __forceinline__ void wt_fill(const WtArgs& a, const int* first, int* table, int total) {
+    const int t = blockIdx.x + threadIdx.x * gridDim.x;
+    if (threadIdx.x < WT_TABLE && t < total) {
+        WtTile w{0, 0, 0, 0, 0, 0};
+        if (!wt_find(a, first, t, w)) w.rows = 0;
+        int* e = table + 6 * threadIdx.x;
+        e[0] = w.group; e[1] = w.row0; e[2] = w.rows; e[3] = w.n0; e[4] = w.brow; e[5] = w.split;
+    }
+}
+__device__ __forceinline__ bool wt_tile_at(const WtArgs& a, const int* first, const int* table, int i, WtTile& w) {
+    if (i >= WT_TABLE) return wt_find(a, first, blockIdx.x + i * gridDim.x, w);
+    const int* e = table + 6 * i;
+    w.group = e[0]; w.row0 = e[1]; w.rows = e[2]; w.n0 = e[3]; w.brow = e[4]; w.split = e[5];
     return w.rows > 0;
 }
 
@@ -281,9 +303,11 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     int* first = reinterpret_cast<int*>(x_full) + 64;
+    int* table = first + WT_MAX_GROUPS + 2;
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int total = a.slots * a.n_tiles * a.k_splits, sb_all = a.K / 256;
     wt_build(a, first);
+    wt_fill(a, first, table, total);
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::SX; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
         for (int s = 0; s < S::SP; ++s) { mbar_init(&p_full[s], 1); mbar_init(&p_empty[s], WT_EXPAND_WARPS); }
@@ -299,6 +323,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    const int mine = ((int)blockIdx.x < total ? total - (int)blockIdx.x + (int)gridDim.x - 1 : 0) / (int)gridDim.x;
     // every role walks the same tiles; sb0 .. sb1: a tile's range of K in units of 256
     auto range = [&](const WtTile& w, int& sb0, int& sb1) {
         sb0 = w.split * a.sb_split;
@@ -308,9 +333,9 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
     if (warp == 0) {
         uint32_t it = 0, s = 0, ph = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        for (int i = 0; i < mine && ok; ++i) {
             WtTile w;
-            if (!wt_tile_at(a, first, t, w)) continue;
+            if (!wt_tile_at(a, first, table, i, w)) continue;
             int sb0, sb1;
             range(w, sb0, sb1);
             const int boxes = (w.rows + WT_BOX - 1) / WT_BOX;
@@ -319,7 +344,10 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
                 if (!ok) break;
                 if (elect_one()) {
                     mbar_expect_tx(&x_full[s], boxes * WT_BOX * 128);
-                    for (int b = 0; b < boxes; ++b)
+                    int b = 0;
+                    for (; b + 3 <= boxes; b += 3)
+                        tma_load_2d(sm_x + s * WT_X_STAGE + b * WT_BOX * 128, &a.map_x_big, kb * 64, w.row0 + b * WT_BOX, &x_full[s]);
+                    for (; b < boxes; ++b)
                         tma_load_2d(sm_x + s * WT_X_STAGE + b * WT_BOX * 128, &a.map_x, kb * 64, w.row0 + b * WT_BOX, &x_full[s]);
                 }
                 if (++s == S::SX) { s = 0; ph ^= 1; }
@@ -331,9 +359,9 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
     } else if (warp == 2) {
         uint32_t it = 0, p = 0, ph = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        for (int i = 0; i < mine && ok; ++i) {
             WtTile w;
-            if (!wt_tile_at(a, first, t, w)) continue;
+            if (!wt_tile_at(a, first, table, i, w)) continue;
             int sb0, sb1;
             range(w, sb0, sb1);
             const int brow = w.brow + w.n0 * S::TILE_N;
@@ -353,11 +381,11 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
             for (uint32_t j = it > S::SP ? it - S::SP : 0; j < it; ++j)
                 if (!mbar_wait_warp(&p_full[j % S::SP], (j / S::SP) & 1, a.status)) break;
     } else if (warp == 1) {
-        uint32_t it = 0, ti = 0, s = 0, ph = 0;
+        uint32_t it = 0, ti = 0, s = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        for (int i = 0; i < mine && ok; ++i) {
             WtTile w;
-            if (!wt_tile_at(a, first, t, w)) continue;
+            if (!wt_tile_at(a, first, table, i, w)) continue;
             int sb0, sb1;
             range(w, sb0, sb1);
             const uint32_t idesc = umma_idesc_f16(WT_ROWS, (w.rows + 15) & ~15), as = ti & 1;
@@ -365,11 +393,18 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
             if (!ok) break;
             tc_fence_after();
             const uint32_t d = tmem + as * WT_TOKENS;
+            // a slot's barrier stands for both operands (an expanding warp waits for the token rows before it
+            // arrives), and the next slot's is looked at before this one's MMAs are issued: a wait costs this warp
+            // some 200 cycles even when there is nothing to wait for, half a K step
+            uint32_t ready = mbar_peek(&a_full[it & (WT_SLOTS - 1)], (it / WT_SLOTS) & 1);
             for (int kb = 4 * sb0; kb < 4 * sb1; ++kb, ++it) {
-                const uint32_t slot = it & (WT_SLOTS - 1);
-                ok = mbar_wait_warp(&x_full[s], ph, a.status) && mbar_wait_warp(&a_full[slot], (it / WT_SLOTS) & 1, a.status);
-                if (!ok) break;
+                const uint32_t slot = it & (WT_SLOTS - 1), nxt = it + 1;
+                if (!__all_sync(0xffffffffu, ready != 0)) {
+                    ok = mbar_wait_warp(&a_full[slot], (it / WT_SLOTS) & 1, a.status);
+                    if (!ok) break;
+                }
                 tc_fence_after();
+                ready = mbar_peek(&a_full[nxt & (WT_SLOTS - 1)], (nxt / WT_SLOTS) & 1);
                 const uint64_t desc = umma_smem_desc(smem_u32(sm_x + s * WT_X_STAGE));
                 if (elect_one()) {
 #pragma unroll
@@ -379,16 +414,16 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
                     umma_commit(&x_empty[s]);
                     if (kb == 4 * sb1 - 1) umma_commit(&acc_full[as]);
                 }
-                if (++s == S::SX) { s = 0; ph ^= 1; }
+                if (++s == S::SX) s = 0;
             }
             ++ti;
         }
     } else if (warp >= 4 && warp < WT_FIRST_EXPAND) {
         const int q = warp & 3;
         uint32_t ti = 0;
-        for (int t = blockIdx.x; t < total; t += gridDim.x) {
+        for (int i = 0; i < mine; ++i) {
             WtTile w;
-            if (!wt_tile_at(a, first, t, w)) continue;
+            if (!wt_tile_at(a, first, table, i, w)) continue;
             const uint32_t as = ti & 1;
             bool ok = mbar_wait(&acc_full[as], (ti >> 1) & 1, a.status);
             ok = __all_sync(0xffffffffu, ok && *reinterpret_cast<volatile int*>(a.status) == 0);
@@ -461,10 +496,11 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
         const uint32_t dst = tmem + WT_SLOT0 + slot * WT_SLOT + ((uint32_t)(q * 32) << 16);
         const uint32_t row_at = smem_u32(sm_p) + (q * 32 + lane) * S::SBB;
         uint32_t it = 0, p = 0, ph = 0;                   // stages of 256 = K steps of this slot
+        uint32_t xs = slot, xph = 0;                      // the token rows' stage of its K step
         bool ok = true;
-        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        for (int i = 0; i < mine && ok; ++i) {
             WtTile w;
-            if (!wt_tile_at(a, first, t, w)) continue;
+            if (!wt_tile_at(a, first, table, i, w)) continue;
             int sb0, sb1;
             range(w, sb0, sb1);
             for (int sb = sb0; sb < sb1; ++sb, ++it) {
@@ -483,6 +519,10 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
                 tc_fence_after();
                 tmem_st32(dst, out);
                 tc_fence_before();
+                if (q == 0) ok = mbar_wait_warp(&x_full[xs], xph, a.status);
+                if (!ok) break;
+                xs += WT_SLOTS;
+                if (xs >= S::SX) { xs -= S::SX; xph ^= 1; }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&a_full[slot]);
             }
@@ -540,6 +580,8 @@ int umma_gemm_q(int epi, int kind, const __half* A, int64_t a_rows, const void* 
     B200_REQUIRE((group_map || b_rows >= (int64_t)groups * N) && a_rows >= M, "umma_gemm_q: operand shapes do not cover the groups");
     WtArgs a;
     int rc = make_tile_map(&a.map_x, A, a_rows, K, WT_BOX);
+    if (rc) return rc;
+    rc = make_tile_map(&a.map_x_big, A, a_rows, K, WT_BIG_BOX);
     if (rc) return rc;
     const int64_t row_bytes = q_row_bytes(kind, K);
     const int sbb = 8 * (kind == 3 ? 18 : q_block_bytes(kind));
