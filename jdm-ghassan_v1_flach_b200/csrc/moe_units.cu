@@ -124,10 +124,13 @@ __device__ __forceinline__ bool unit_tiles(const MoeUnitArgs& a, const int4 unit
             }
         }
         if (!__syncthreads_and(ok)) break;
-        if (threadIdx.x == 0 && r + 2 < rounds) issue(r + 2, set);
+        // The next copies and the outputs are the last warps' work: with one tile in six parts two warps have none of
+        // the products, and the others go on to the next tile (by the first warps, a round of 1220 cycles of products
+        // had 1900 more of this behind it).
+        if (threadIdx.x == (W - 1) * 32 && r + 2 < rounds) issue(r + 2, set);
         // (row, token) with the row fastest: neighbouring threads store neighbouring outputs
         const int per = DOWN ? 16 : 8;
-        for (int i = threadIdx.x; i < n * per * MT; i += W * 32) {
+        for (int i = (threadIdx.x + 64) & (W * 32 - 1); i < n * per * MT; i += W * 32) {       // 0 at the last two warps' first thread
             const int row = i % per, m = i / per % MT, tile = i / (per * MT), at = (t0 + r * G + tile) * R + row;
             if (m >= M || row >= R || at >= N) continue;
             const float* re = rr + tile * P * dg_red_floats(MT);
