@@ -345,8 +345,9 @@ __device__ __forceinline__ void dg_chunk(DgAcc<KIND, MT>& acc, uint32_t row_a, u
     }
 }
 
-// The warp's sums to red[16 rows][MT] and, for kinds with minima, red[16 * MT + ...] (dg_value adds the two).
-constexpr int dg_red_floats(int MT) { return 2 * 16 * MT; }
+// The warp's sums to red[16 rows][MT].  The minimum terms lie in other lanes than the products: they go first, the
+// products' lanes add theirs (so the threads that add the parts up read one value per part).
+constexpr int dg_red_floats(int MT) { return 16 * MT; }
 template <int KIND, int MT>
 __device__ __forceinline__ void dg_finish(const DgAcc<KIND, MT>& acc, float* red, int lane) {
     const int g = lane >> 2, t = lane & 3;
@@ -359,6 +360,15 @@ __device__ __forceinline__ void dg_finish(const DgAcc<KIND, MT>& acc, float* red
             }
         return;
     }
+    if (DgKind<KIND>::mins) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (2 * t + i < MT) {
+                red[g * MT + 2 * t + i] = KIND == 3 ? -acc.mn[i] : acc.mn[i];
+                red[(g + 8) * MT + 2 * t + i] = KIND == 3 ? -acc.mn[2 + i] : acc.mn[2 + i];
+            }
+        __syncwarp();
+    }
     const float scale = ((t & 1) ? 65536.0f : 1.0f) * (DgKind<KIND>::split16 ? 0x1p-34f : 0x1p-30f);
 #pragma unroll
     for (int q = 0; q < DgAcc<KIND, MT>::NT; ++q) {
@@ -367,31 +377,20 @@ __device__ __forceinline__ void dg_finish(const DgAcc<KIND, MT>& acc, float* red
         b += __shfl_xor_sync(0xffffffffu, b, 1);
         const int tok = 2 * q + (t >> 1);
         if ((t & 1) == 0 && tok < MT) {
-            red[g * MT + tok] = a;
-            red[(g + 8) * MT + tok] = b;
+            float *ra = red + g * MT + tok, *rb = red + (g + 8) * MT + tok;
+            *ra = DgKind<KIND>::mins ? *ra + a : a;
+            *rb = DgKind<KIND>::mins ? *rb + b : b;
         }
-    }
-    if (DgKind<KIND>::mins) {
-        float* r = red + 16 * MT;
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-            if (2 * t + i < MT) {
-                r[g * MT + 2 * t + i] = KIND == 3 ? -acc.mn[i] : acc.mn[i];
-                r[(g + 8) * MT + 2 * t + i] = KIND == 3 ? -acc.mn[2 + i] : acc.mn[2 + i];
-            }
     }
 }
 // Element (row, token) from `parts` warps' results, each dg_red_floats apart.
 template <int KIND, int MT>
 __device__ __forceinline__ float dg_value(const float* red, int parts, int row, int tok) {
     const float* at = red + row * MT + tok;
-    float v = 0.0f, w = 0.0f;
+    float v = 0.0f;
 #pragma unroll 4
-    for (int p = 0; p < parts; ++p, at += dg_red_floats(MT)) {
-        v += at[0];
-        if (DgKind<KIND>::mins) w += at[16 * MT];
-    }
-    return v + w;
+    for (int p = 0; p < parts; ++p, at += dg_red_floats(MT)) v += *at;
+    return v;
 }
 #endif
 

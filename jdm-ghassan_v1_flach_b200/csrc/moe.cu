@@ -426,6 +426,30 @@ static int launch_experts(const MoeArgs& a) {
 // ---------------------------------------------------------------------------
 constexpr int RT_K = 64, RT_LD = RT_K + 4;
 
+// One warp routes token t from its logits; s: ne floats of shared scratch.
+template <int PER>
+__device__ __forceinline__ void route_token(const float* __restrict__ logits, const float* __restrict__ router_bias, float* __restrict__ probs_out,
+                                            int32_t* __restrict__ idx_out, float* __restrict__ w_out, int64_t t, int ne, int K, float* s, int lane) {
+    float v[PER], bs[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int e = min(32 * i + lane, ne - 1);
+        v[i] = __ldcg(logits + t * ne + e);
+        bs[i] = router_bias ? router_bias[e] : 0.0f;
+    }
+    int idx;
+    float w;
+    route_pick<PER>(v, bs, router_bias != nullptr, ne, K, s, lane, idx, w);
+    if (lane < K) {
+        idx_out[t * K + lane] = idx;
+        w_out[t * K + lane] = w;
+    }
+    if (probs_out)
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+            if (32 * i + lane < ne) probs_out[t * ne + 32 * i + lane] = v[i];
+}
+
 template <int TPT, int EPT>
 __global__ void __launch_bounds__(256)
 route_logits_kernel(const float* __restrict__ x, const float* __restrict__ router_w, float* __restrict__ logits,
@@ -478,7 +502,7 @@ route_logits_kernel(const float* __restrict__ x, const float* __restrict__ route
         park();
         __syncthreads();
         if (k0 + RT_K < d) fetch(k0 + RT_K);
-        for (int g = 0; g < kc; g += 4) {
+        auto group = [&](int g) {
             float4 a[TPT], b[EPT];
 #pragma unroll
             for (int i = 0; i < TPT; ++i) a[i] = *reinterpret_cast<const float4*>(&xs[TPT * ty + i][g]);
@@ -493,6 +517,13 @@ route_logits_kernel(const float* __restrict__ x, const float* __restrict__ route
                     s = __fadd_rn(s, __fmul_rn(a[i].w, b[j].w));
                     acc[i][j] = __fadd_rn(acc[i][j], s);
                 }
+        };
+        // whole chunks with the loads of later groups under the additions of earlier ones (the chains are serial)
+        if (kc == RT_K) {
+#pragma unroll 8
+            for (int g = 0; g < RT_K; g += 4) group(g);
+        } else {
+            for (int g = 0; g < kc; g += 4) group(g);
         }
     }
 #pragma unroll
@@ -591,18 +622,11 @@ route_logits_chains_kernel(const float* __restrict__ x, const float* __restrict_
     __threadfence();
     {
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        float* s_p = rc_smem + (size_t)warp * (2 * MOE_MAX_NE + 2 * MOE_MAX_K);      // the tiles are dead
-        float* s_sel = s_p + MOE_MAX_NE;
-        float* s_w = s_sel + MOE_MAX_NE;
-        int* s_idx = reinterpret_cast<int*>(s_w + MOE_MAX_K);
         const int64_t t = t0 + warp;
         if (warp < RC_TOK && t < N) {
-            route_finish_warp(logits + t * ne, router_bias, ne, K, s_p, s_sel, s_idx, s_w,
-                              probs_out ? probs_out + t * ne : nullptr, lane);
-            if (lane < K) {
-                idx_out[t * K + lane] = s_idx[lane];
-                w_out[t * K + lane] = s_w[lane];
-            }
+            float* s_p = rc_smem + (size_t)warp * MOE_MAX_NE;                         // the tiles are dead
+            if (ne <= 64) route_token<2>(logits, router_bias, probs_out, idx_out, w_out, t, ne, K, s_p, lane);
+            else route_token<8>(logits, router_bias, probs_out, idx_out, w_out, t, ne, K, s_p, lane);
         }
         if (threadIdx.x == 0) counters[blockIdx.x] = 0;       // ready for the next call
     }
@@ -626,20 +650,14 @@ static int* route_counters() {
 }
 
 constexpr int RF_WARPS = 8;
+template <int PER>
 __global__ void __launch_bounds__(RF_WARPS * 32)
 route_finish_kernel(const float* __restrict__ logits, const float* __restrict__ router_bias, float* __restrict__ probs_out,
                     int32_t* __restrict__ idx_out, float* __restrict__ w_out, int64_t N, int ne, int K) {
-    __shared__ float s_p[RF_WARPS][MOE_MAX_NE], s_sel[RF_WARPS][MOE_MAX_NE], s_w[RF_WARPS][MOE_MAX_K];
-    __shared__ int s_idx[RF_WARPS][MOE_MAX_K];
+    __shared__ float s_p[RF_WARPS][32 * PER];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t t = (int64_t)blockIdx.x * RF_WARPS + warp;
-    if (t >= N) return;
-    route_finish_warp(logits + t * ne, router_bias, ne, K, s_p[warp], s_sel[warp], s_idx[warp], s_w[warp],
-                      probs_out ? probs_out + t * ne : nullptr, lane);
-    if (lane < K) {
-        idx_out[t * K + lane] = s_idx[warp][lane];
-        w_out[t * K + lane] = s_w[warp][lane];
-    }
+    if (t < N) route_token<PER>(logits, router_bias, probs_out, idx_out, w_out, t, ne, K, s_p[warp], lane);
 }
 
 int moe_route(const float* x, const float* router_w, const float* router_bias, float* probs,
@@ -672,8 +690,10 @@ int moe_route(const float* x, const float* router_w, const float* router_bias, f
             route_logits_kernel<4, 1><<<grid, 256, 0, stream()>>>(x, router_w, logits, N, d, ne);
         }
         B200_LAUNCH_CHECK("route_logits_kernel");
-        route_finish_kernel<<<(unsigned)ceil_div64(N, RF_WARPS), RF_WARPS * 32, 0, stream()>>>(logits, router_bias, probs,
-                                                                                                  idx, w, N, ne, K);
+        const unsigned blocks = (unsigned)ceil_div64(N, RF_WARPS);
+        if (ne <= 64) route_finish_kernel<2><<<blocks, RF_WARPS * 32, 0, stream()>>>(logits, router_bias, probs, idx, w, N, ne, K);
+        else if (ne <= 128) route_finish_kernel<4><<<blocks, RF_WARPS * 32, 0, stream()>>>(logits, router_bias, probs, idx, w, N, ne, K);
+        else route_finish_kernel<8><<<blocks, RF_WARPS * 32, 0, stream()>>>(logits, router_bias, probs, idx, w, N, ne, K);
         B200_LAUNCH_CHECK("route_finish_kernel");
         return B200_OK;
     }
