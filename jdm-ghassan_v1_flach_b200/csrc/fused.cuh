@@ -20,7 +20,9 @@ struct SeqLayout {
     const int32_t* seq_off = nullptr;     // [n_seq + 1] first row of each sequence
     const int32_t* pos = nullptr;         // [rows] position of a row inside its sequence
     const int32_t* seq = nullptr;         // [rows] sequence a row belongs to
-    const int2* chunks = nullptr;         // [n_chunks] (first row, steps <= SSD_Q); no chunk crosses a sequence boundary
+    // [n_chunks] (first row, steps <= SSD_Q | (1 + sequence) << 8 where it is the sequence's only chunk); no chunk
+    // crosses a sequence boundary
+    const int2* chunks = nullptr;
     const int32_t* seq_chunk0 = nullptr;  // [n_seq + 1] first chunk of each sequence
     const int32_t* host_off = nullptr;    // host copy of seq_off
 };

@@ -20,8 +20,8 @@
 //
 //   ssd_cb_kernel           G[b,c] = C B^T                         [Q, Q]
 //   ssd_chunk_state_kernel  dt, cum per step; S_c per (b, c, h)   [d_head, d_state]
-//   ssd_carry_kernel        S_c -> S_prev(c) in place, final state out
-//   ssd_chunk_out_kernel    y = intra + inter + D x
+//   ssd_carry_kernel        S_c -> S_prev(c) in place, final state out (sequences of several chunks)
+//   ssd_chunk_out_kernel    y = intra + inter + D x; the final state of a sequence of one chunk
 #include "fused.cuh"
 
 namespace b200 {
@@ -37,6 +37,7 @@ struct SsdChunk {
     int64_t ci;        // index into the per-chunk arrays (G, chunk_state, decay)
     int64_t dt0;       // index of the chunk's first (dt, cum) pair for head h
     int nt;            // steps in the chunk
+    int whole;         // the sequence, if this is its only chunk; else -1
 };
 __device__ __forceinline__ SsdChunk ssd_chunk(const int2* __restrict__ tab, int64_t NT, int c, int b, int h, int T, int NC,
                                               int H) {
@@ -44,17 +45,35 @@ __device__ __forceinline__ SsdChunk ssd_chunk(const int2* __restrict__ tab, int6
     if (tab) {
         const int2 e = tab[c];
         k.row0 = e.x;
-        k.nt = e.y;
+        k.nt = e.y & 0xFF;
+        k.whole = (e.y >> 8) - 1;
         k.ci = c;
         k.dt0 = (int64_t)h * NT + e.x;
     } else {
         const int t0 = c * SSD_Q;
         k.row0 = (int64_t)b * T + t0;
         k.nt = min(SSD_Q, T - t0);
+        k.whole = NC == 1 ? b : -1;
         k.ci = (int64_t)b * NC + c;
         k.dt0 = ((int64_t)b * H + h) * T + t0;
     }
     return k;
+}
+
+// Four elements of the state before the chunk.  A sequence of one chunk has no carry: its block reads the sequence's
+// state here and leaves the state after the chunk in its place (each element by one thread).
+__device__ __forceinline__ float4 ssd_prev4(const float* own, float* state, float decay, bool whole) {
+    const float4 o = __ldcs(reinterpret_cast<const float4*>(own));
+    if (!whole) return o;
+    const bool wide = (reinterpret_cast<uintptr_t>(state) & 15) == 0;       // the caller's own buffer
+    const float4 s = wide ? __ldcs(reinterpret_cast<const float4*>(state)) : make_float4(state[0], state[1], state[2], state[3]);
+    const float4 n = make_float4(decay * s.x + o.x, decay * s.y + o.y, decay * s.z + o.z, decay * s.w + o.w);
+    if (wide) {
+        __stcs(reinterpret_cast<float4*>(state), n);
+    } else {
+        state[0] = n.x; state[1] = n.y; state[2] = n.z; state[3] = n.w;
+    }
+    return s;
 }
 
 __device__ __forceinline__ float softplus_dt(float u) { return (u > 20.0f) ? u : log1pf(expf(u)); }
@@ -260,6 +279,7 @@ ssd_carry_kernel(float* __restrict__ chunk_state, const float* __restrict__ deca
     // the sequence's chunks are consecutive entries of the per-chunk arrays
     const int64_t c_first = seq_chunk0 ? seq_chunk0[b] : (int64_t)b * NC;
     const int nc = seq_chunk0 ? seq_chunk0[b + 1] - seq_chunk0[b] : NC;
+    if (nc == 1) return;                   // the chunk's output block carries the state itself
     float* cs = chunk_state + (c_first * p.n_heads + h) * per + e;
     const float* dc = decay + c_first * p.n_heads + h;
     float s = state[i];
@@ -291,7 +311,8 @@ ssd_carry_kernel(float* __restrict__ chunk_state, const float* __restrict__ deca
 template <bool X3>
 __global__ void __launch_bounds__(SSD_THREADS, 2)
 ssd_chunk_out_kernel(const float* __restrict__ bc, const float* __restrict__ G, const float* __restrict__ dtcum,
-                     const float* __restrict__ chunk_state, const float* __restrict__ Dv, float* __restrict__ y, int T,
+                     const float* __restrict__ chunk_state, const float* __restrict__ decay, float* __restrict__ state,
+                     const float* __restrict__ Dv, float* __restrict__ y, int T,
                      int NC, MambaDims p, const int2* __restrict__ tab, int64_t NT) {
     extern __shared__ float sm[];
     constexpr int P = SSD_P, LDM = SSD_Q + 4;
@@ -337,9 +358,12 @@ ssd_chunk_out_kernel(const float* __restrict__ bc, const float* __restrict__ G, 
             *reinterpret_cast<float4*>(sC + t * ldc + n) = v;
         }
         const float* sp = chunk_state + ((ck.ci) * p.n_heads + h) * P * N;
+        const bool whole = ck.whole >= 0;
+        float* st = whole ? state + ((int64_t)ck.whole * p.n_heads + h) * P * N : nullptr;
+        const float dk = whole ? decay[ck.ci * p.n_heads + h] : 0.0f;
         for (int e = threadIdx.x; e < P * n4; e += SSD_THREADS) {
             const int i = e / n4, n = (e - i * n4) * 4;
-            const float4 v = __ldcs(reinterpret_cast<const float4*>(sp + i * N + n));
+            const float4 v = ssd_prev4(sp + i * N + n, st + i * N + n, dk, whole);
             *reinterpret_cast<float4*>(sS + i * ldc + n) = v;
         }
         __syncthreads();
@@ -562,7 +586,8 @@ ssd_chunk_state16_kernel(const float* __restrict__ proj, const float* __restrict
 // As ssd_chunk_out_kernel; d_state a multiple of 16.
 __global__ void __launch_bounds__(SSD_THREADS, 4)
 ssd_chunk_out16_kernel(const float* __restrict__ bc, const float* __restrict__ G, const float* __restrict__ dtcum,
-                       const float* __restrict__ chunk_state, const float* __restrict__ Dv, float* __restrict__ y, int T,
+                       const float* __restrict__ chunk_state, const float* __restrict__ decay, float* __restrict__ state,
+                     const float* __restrict__ Dv, float* __restrict__ y, int T,
                        int NC, MambaDims p, const int2* __restrict__ tab, int64_t NT) {
     extern __shared__ __align__(16) uint8_t sm16[];
     constexpr int P = SSD_P;
@@ -609,9 +634,12 @@ ssd_chunk_out16_kernel(const float* __restrict__ bc, const float* __restrict__ G
             store_half4(sC + t * ldc + n, v);
         }
         const float* sp = chunk_state + ((ck.ci) * p.n_heads + h) * P * N;
+        const bool whole = ck.whole >= 0;
+        float* st = whole ? state + ((int64_t)ck.whole * p.n_heads + h) * P * N : nullptr;
+        const float dk = whole ? decay[ck.ci * p.n_heads + h] : 0.0f;
         for (int e = threadIdx.x; e < P * n4; e += SSD_THREADS) {
             const int i = e / n4, n = (e - i * n4) * 4;
-            store_half4(sS + i * ldc + n, __ldcs(reinterpret_cast<const float4*>(sp + i * N + n)));
+            store_half4(sS + i * ldc + n, ssd_prev4(sp + i * N + n, st + i * N + n, dk, whole));
         }
         __syncthreads();
         for (int ks = 0; ks < (N >> 4); ++ks) {
@@ -750,15 +778,24 @@ int mamba_ssd_scan(const float* proj, const float* bc, const float* dt_bias, con
     else
         ssd_chunk_state_kernel<false><<<grid, SSD_THREADS, smem_st, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
     B200_LAUNCH_CHECK("ssd_chunk_state_kernel");
-    ssd_carry_kernel<<<dim3((unsigned)ceil_div(p.d_head * p.d_state, 256), (unsigned)p.n_heads, (unsigned)B), 256, 0, stream()>>>(
-        cstate, decay, state, B, NC, p, lay ? lay->seq_chunk0 : nullptr);
-    B200_LAUNCH_CHECK("ssd_carry_kernel");
+    // 64 sequences of one chunk: 295 us in the carry, its blocks each a chain of three dependent loads, and a second
+    // way of the chunk states through memory
+    bool carry = NC > 1;
+    if (lay && lay->host_off) {
+        carry = false;
+        for (int b = 0; b < B && !carry; ++b) carry = lay->host_off[b + 1] - lay->host_off[b] > SSD_Q;
+    }
+    if (carry) {
+        ssd_carry_kernel<<<dim3((unsigned)ceil_div(p.d_head * p.d_state, 256), (unsigned)p.n_heads, (unsigned)B), 256, 0, stream()>>>(
+            cstate, decay, state, B, NC, p, lay ? lay->seq_chunk0 : nullptr);
+        B200_LAUNCH_CHECK("ssd_carry_kernel");
+    }
     if (half_tiles)
-        ssd_chunk_out16_kernel<<<grid, SSD_THREADS, smem_out16, stream()>>>(bc, G, dtcum, cstate, D, y, T, NC, p, tab, NT);
+        ssd_chunk_out16_kernel<<<grid, SSD_THREADS, smem_out16, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
     else if (precise)
-        ssd_chunk_out_kernel<true><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, D, y, T, NC, p, tab, NT);
+        ssd_chunk_out_kernel<true><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
     else
-        ssd_chunk_out_kernel<false><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, D, y, T, NC, p, tab, NT);
+        ssd_chunk_out_kernel<false><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
     B200_LAUNCH_CHECK("ssd_chunk_out_kernel");
     return B200_OK;
 }

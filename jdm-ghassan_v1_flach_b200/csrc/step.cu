@@ -1247,7 +1247,7 @@ int b200_decoder_prefill_ragged(b200_decoder* dec, const int32_t* tokens_dev, co
             }
             for (int t = 0; t < n; t += SSD_Q, ++c) {
                 h[o_chunks + 2 * c] = (int32_t)(r + t);
-                h[o_chunks + 2 * c + 1] = std::min(SSD_Q, n - t);
+                h[o_chunks + 2 * c + 1] = std::min(SSD_Q, n - t) | (n <= SSD_Q ? (b + 1) << 8 : 0);
             }
             r += n;
         }
