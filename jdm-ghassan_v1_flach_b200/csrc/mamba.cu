@@ -208,7 +208,9 @@ mamba_conv_step_kernel(const float* __restrict__ proj, const float* __restrict__
 // PER: values of the row a thread keeps in registers (d_inner <= PER * 256), 0 = two passes
 // through `out`.  Six CTAs per SM: the kernel is a chain of load -> block reduction -> store
 // per row, so resident rows are what hides its latencies.
-template <int PER>
+// VEC (rows, pointers and strides of 16 bytes): four neighbours per load, all of a thread's loads under way before the
+// first exponential.  GN_TIMES
+template <int PER, bool VEC = false>
 __global__ void __launch_bounds__(256, 6)
 mamba_gated_norm_kernel(const float* y, const float* __restrict__ gate, int64_t gate_stride,
                         const float* __restrict__ norm_w, float* out, int d_inner, float eps,
@@ -219,7 +221,47 @@ mamba_gated_norm_kernel(const float* y, const float* __restrict__ gate, int64_t 
     const float* gr = gate + r * gate_stride;
     float* o = out + r * d_inner;
     double var = 0.0;
-    if (PER > 0) {
+    if constexpr (VEC) {
+        constexpr int NV = PER / 4;
+        float4 v[NV], z[NV];
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int c = 4 * (j * 256 + threadIdx.x);
+            v[j] = z[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c < d_inner) {
+                v[j] = *reinterpret_cast<const float4*>(yr + c);
+                z[j] = __ldg(reinterpret_cast<const float4*>(gr + c));
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            v[j].x *= silu_acc(z[j].x);
+            v[j].y *= silu_acc(z[j].y);
+            v[j].z *= silu_acc(z[j].z);
+            v[j].w *= silu_acc(z[j].w);
+            var += (double)v[j].x * v[j].x;
+            var += (double)v[j].y * v[j].y;
+            var += (double)v[j].z * v[j].z;
+            var += (double)v[j].w * v[j].w;
+        }
+        var = block_sum_d(var, red) / (double)d_inner;
+        const float inv = 1.0f / sqrtf((float)var + eps);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int c = 4 * (j * 256 + threadIdx.x);
+            if (c < d_inner) {
+                const float4 w = __ldg(reinterpret_cast<const float4*>(norm_w + c));
+                const float4 res = make_float4(v[j].x * inv * w.x, v[j].y * inv * w.y, v[j].z * inv * w.z, v[j].w * inv * w.w);
+                if (out16) {
+                    auto clamp = [](float f) { return fminf(fmaxf(f, -65504.0f), 65504.0f); };
+                    __half2 h[2] = {__floats2half2_rn(clamp(res.x), clamp(res.y)), __floats2half2_rn(clamp(res.z), clamp(res.w))};
+                    *reinterpret_cast<uint2*>(out16 + r * d_inner + c) = *reinterpret_cast<uint2*>(h);
+                } else {
+                    *reinterpret_cast<float4*>(o + c) = res;
+                }
+            }
+        }
+    } else if (PER > 0) {
         float v[PER > 0 ? PER : 1];
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
@@ -253,10 +295,16 @@ mamba_gated_norm_kernel(const float* y, const float* __restrict__ gate, int64_t 
 static void launch_gated_norm(const float* y, const float* gate, int64_t gate_stride, const float* norm_w, float* out,
                               int d_inner, float eps, __half* out16, int64_t rows) {
     const unsigned g = (unsigned)rows;
-    if (d_inner <= 1024) mamba_gated_norm_kernel<4><<<g, 256, 0, stream()>>>(y, gate, gate_stride, norm_w, out, d_inner, eps, out16);
-    else if (d_inner <= 2048) mamba_gated_norm_kernel<8><<<g, 256, 0, stream()>>>(y, gate, gate_stride, norm_w, out, d_inner, eps, out16);
-    else if (d_inner <= 3072) mamba_gated_norm_kernel<12><<<g, 256, 0, stream()>>>(y, gate, gate_stride, norm_w, out, d_inner, eps, out16);
-    else if (d_inner <= 4096) mamba_gated_norm_kernel<16><<<g, 256, 0, stream()>>>(y, gate, gate_stride, norm_w, out, d_inner, eps, out16);
+    const uintptr_t at = (uintptr_t)y | (uintptr_t)gate | (uintptr_t)norm_w | (out16 ? (uintptr_t)out16 : (uintptr_t)out);
+    const bool vec = d_inner % 4 == 0 && gate_stride % 4 == 0 && at % 16 == 0;
+#define B200_GATED(PER)                                                                                                                       \
+    (vec ? mamba_gated_norm_kernel<PER, true><<<g, 256, 0, stream()>>>(y, gate, gate_stride, norm_w, out, d_inner, eps, out16)                \
+         : mamba_gated_norm_kernel<PER><<<g, 256, 0, stream()>>>(y, gate, gate_stride, norm_w, out, d_inner, eps, out16))
+    if (d_inner <= 1024) B200_GATED(4);
+    else if (d_inner <= 2048) B200_GATED(8);
+    else if (d_inner <= 3072) B200_GATED(12);
+    else if (d_inner <= 4096) B200_GATED(16);
+#undef B200_GATED
     else mamba_gated_norm_kernel<0><<<g, 256, 0, stream()>>>(y, gate, gate_stride, norm_w, out, d_inner, eps, nullptr);
 }
 

@@ -418,13 +418,15 @@ static int launch_experts(const MoeArgs& a) {
 
 // ---------------------------------------------------------------------------
 // Router for many tokens.  The logit of (token, expert) keeps the reference's
-// sequential fp32 chain over groups of four, but the chains of a 32-token x
-// 64-expert tile advance together: activations and router rows are staged in
-// shared memory 64 columns at a time and every thread carries TPT x EPT chains in
-// registers (4 x 2 for prompts; 1 x 1 for a batch of decode tokens, so that the few
-// chains spread over many SMs).  A second kernel finishes each token with one warp.
+// sequential fp32 chain over groups of four (products and sums rounded one by one, so two
+// instructions per multiply-add: 22 us for 4096 tokens of 1536 x 64 experts), but the chains
+// of a tile advance together: token and router rows come through a ring of asynchronous copies,
+// 64 columns at a time, and a thread carries TPT tokens of one expert - a warp reads its
+// lanes' 32 expert rows (four wavefronts per group of columns) for TPT token rows (one each, the
+// same for all lanes), so at 8 tokens shared memory needs 12 cycles where the arithmetic needs 16.
+// RT_TIMES  A second kernel finishes each token with one warp.
 // ---------------------------------------------------------------------------
-constexpr int RT_K = 64, RT_LD = RT_K + 4;
+constexpr int RT_K = 64, RT_LD = RT_K + 4, RT_WARPS = 4, RT_THREADS = 32 * RT_WARPS, RT_STAGES = 3;
 
 // One warp routes token t from its logits; s: ne floats of shared scratch.
 template <int PER>
@@ -450,90 +452,81 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
             if (32 * i + lane < ne) probs_out[t * ne + 32 * i + lane] = v[i];
 }
 
-template <int TPT, int EPT>
-__global__ void __launch_bounds__(256)
+template <int TPT>
+__global__ void __launch_bounds__(RT_THREADS)
 route_logits_kernel(const float* __restrict__ x, const float* __restrict__ router_w, float* __restrict__ logits,
                     int64_t N, int d, int ne) {
-    constexpr int RT_TOK = 8 * TPT, RT_EXP = 32 * EPT;
-    __shared__ __align__(16) float xs[RT_TOK][RT_LD];
-    __shared__ __align__(16) float ws[RT_EXP][RT_LD];
+    constexpr int TOK = RT_WARPS * TPT, ROWS = TOK + 32, STAGE = ROWS * RT_LD;
+    extern __shared__ __align__(16) float rt_sm[];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t t0 = (int64_t)blockIdx.x * RT_TOK;
-    const int e0 = blockIdx.y * RT_EXP;
-    float acc[TPT][EPT] = {};
-    // The next 64 columns of the tile are fetched into registers while the current ones
-    // are consumed from shared memory, so the global-memory latency of a chunk is paid
-    // once, not once per chunk.
-    constexpr int ITEMS = (RT_TOK + RT_EXP) * (RT_K / 4);
-    constexpr int PER = (ITEMS + 255) / 256;
-    float4 pre[PER];
-    auto fetch = [&](int k0) {
-        const int kc = min(RT_K, d - k0);
+    const int64_t t0 = (int64_t)blockIdx.x * TOK;
+    const int e0 = blockIdx.y * 32;
+    // rows 0 .. TOK-1: tokens, then 32 experts; rows past the ends repeat the last one, columns past d are not read
+    const int c4 = (threadIdx.x % (RT_K / 4)) * 4, r0 = threadIdx.x / (RT_K / 4);
+    constexpr int STEP = RT_THREADS / (RT_K / 4), PER = ROWS / STEP;
+    static_assert(ROWS % STEP == 0, "rows of a stage per copying thread");
+    const int chunks = (d + RT_K - 1) / RT_K;
+    auto fetch = [&](int k) {
+        if (k < chunks) {
+            float* st = rt_sm + (k % RT_STAGES) * STAGE;
+            if (k * RT_K + c4 < d)
 #pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            const int i = u * 256 + threadIdx.x;
-            const int row = i / (RT_K / 4), c4 = (i % (RT_K / 4)) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < ITEMS && c4 < kc) {
-                if (row < RT_TOK) {
-                    if (t0 + row < N) v = *reinterpret_cast<const float4*>(x + (t0 + row) * d + k0 + c4);
-                } else if (e0 + row - RT_TOK < ne) {
-                    v = *reinterpret_cast<const float4*>(router_w + (int64_t)(e0 + row - RT_TOK) * d + k0 + c4);
+                for (int u = 0; u < PER; ++u) {
+                    const int row = r0 + u * STEP;
+                    const float* src = row < TOK ? x + min(t0 + row, N - 1) * d : router_w + (int64_t)min(e0 + row - TOK, ne - 1) * d;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(st + row * RT_LD + c4)), "l"(src + k * RT_K + c4) : "memory");
                 }
-            }
-            pre[u] = v;
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto park = [&]() {
+    float acc[TPT] = {};
 #pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            const int i = u * 256 + threadIdx.x;
-            if (i < ITEMS) {
-                const int row = i / (RT_K / 4), c4 = (i % (RT_K / 4)) * 4;
-                float* dst = row < RT_TOK ? &xs[row][c4] : &ws[row - RT_TOK][c4];
-                *reinterpret_cast<float4*>(dst) = pre[u];
-            }
-        }
-    };
-    fetch(0);
-    for (int k0 = 0; k0 < d; k0 += RT_K) {
-        const int kc = min(RT_K, d - k0);              // a multiple of 4
-        __syncthreads();                               // the previous chunk has been consumed
-        park();
-        __syncthreads();
-        if (k0 + RT_K < d) fetch(k0 + RT_K);
+    for (int k = 0; k < RT_STAGES - 1; ++k) fetch(k);
+    for (int k = 0; k < chunks; ++k) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(RT_STAGES - 2) : "memory");
+        __syncthreads();                               // the stage is here, and the one before it is free
+        fetch(k + RT_STAGES - 1);
+        const float* xs = rt_sm + (k % RT_STAGES) * STAGE + TPT * ty * RT_LD;
+        const float* ws = rt_sm + (k % RT_STAGES) * STAGE + (TOK + tx) * RT_LD;
+        const int kc = min(RT_K, d - k * RT_K);        // a multiple of 4
         auto group = [&](int g) {
-            float4 a[TPT], b[EPT];
+            const float4 b = *reinterpret_cast<const float4*>(ws + g);
 #pragma unroll
-            for (int i = 0; i < TPT; ++i) a[i] = *reinterpret_cast<const float4*>(&xs[TPT * ty + i][g]);
-#pragma unroll
-            for (int j = 0; j < EPT; ++j) b[j] = *reinterpret_cast<const float4*>(&ws[tx + 32 * j][g]);
-#pragma unroll
-            for (int i = 0; i < TPT; ++i)
-#pragma unroll
-                for (int j = 0; j < EPT; ++j) {
-                    float s = __fadd_rn(__fmul_rn(a[i].x, b[j].x), __fmul_rn(a[i].y, b[j].y));
-                    s = __fadd_rn(s, __fmul_rn(a[i].z, b[j].z));
-                    s = __fadd_rn(s, __fmul_rn(a[i].w, b[j].w));
-                    acc[i][j] = __fadd_rn(acc[i][j], s);
-                }
+            for (int i = 0; i < TPT; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(xs + i * RT_LD + g);
+                float s = __fadd_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+                s = __fadd_rn(s, __fmul_rn(a.z, b.z));
+                s = __fadd_rn(s, __fmul_rn(a.w, b.w));
+                acc[i] = __fadd_rn(acc[i], s);
+            }
         };
         // whole chunks with the loads of later groups under the additions of earlier ones (the chains are serial)
         if (kc == RT_K) {
-#pragma unroll 8
+#pragma unroll
             for (int g = 0; g < RT_K; g += 4) group(g);
         } else {
             for (int g = 0; g < kc; g += 4) group(g);
         }
     }
+    const int e = e0 + tx;
 #pragma unroll
-    for (int i = 0; i < TPT; ++i)
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) {
-            const int64_t t = t0 + TPT * ty + i;
-            const int e = e0 + tx + 32 * j;
-            if (t < N && e < ne) logits[t * ne + e] = acc[i][j];
-        }
+    for (int i = 0; i < TPT; ++i) {
+        const int64_t t = t0 + TPT * ty + i;
+        if (t < N && e < ne) logits[t * ne + e] = acc[i];
+    }
+}
+template <int TPT>
+static int launch_route_logits(const float* x, const float* router_w, float* logits, int64_t N, int d, int ne) {
+    constexpr int SMEM = RT_STAGES * (RT_WARPS * TPT + 32) * RT_LD * 4;
+    static bool configured = false;
+    if (!configured) {
+        B200_CUDA(cudaFuncSetAttribute(route_logits_kernel<TPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        configured = true;
+    }
+    const dim3 grid((unsigned)ceil_div64(N, RT_WARPS * TPT), ceil_div(ne, 32));
+    route_logits_kernel<TPT><<<grid, RT_THREADS, SMEM, stream()>>>(x, router_w, logits, N, d, ne);
+    B200_LAUNCH_CHECK("route_logits_kernel");
+    return B200_OK;
 }
 
 // A decode batch (tens of tokens): the tiled kernel above would occupy N / 8 x ne / 32 blocks -
@@ -680,16 +673,16 @@ int moe_route(const float* x, const float* router_w, const float* router_bias, f
                                                                          w, K, counters);
             B200_LAUNCH_CHECK("route_logits_chains_kernel");
             if (counters) return B200_OK;
-        } else if (N <= 1024) {
-            const dim3 grid((unsigned)ceil_div64(N, 8), ceil_div(ne, 32));
-            route_logits_kernel<1, 1><<<grid, 256, 0, stream()>>>(x, router_w, logits, N, d, ne);
         } else {
-            // 32 tokens x 32 experts per block: twice the blocks of a 32 x 64 tile, which
-            // measured 15 % faster at 4096 tokens x 64 experts (more resident warps per SM)
-            const dim3 grid((unsigned)ceil_div64(N, 32), ceil_div(ne, 32));
-            route_logits_kernel<4, 1><<<grid, 256, 0, stream()>>>(x, router_w, logits, N, d, ne);
+            // the smallest token tile that one wave of blocks covers: a thread's chains run side by side, so few
+            // tokens want many blocks and many tokens want each expert row read for as many of them as there are
+            const int e_tiles = ceil_div(ne, 32);
+            auto blocks = [&](int tpt) { return ceil_div64(N, RT_WARPS * tpt) * e_tiles; };
+            rc = blocks(2) <= num_sms()   ? launch_route_logits<2>(x, router_w, logits, N, d, ne)
+                 : blocks(4) <= num_sms() ? launch_route_logits<4>(x, router_w, logits, N, d, ne)
+                                          : launch_route_logits<8>(x, router_w, logits, N, d, ne);
+            if (rc) return rc;
         }
-        B200_LAUNCH_CHECK("route_logits_kernel");
         const unsigned blocks = (unsigned)ceil_div64(N, RF_WARPS);
         if (ne <= 64) route_finish_kernel<2><<<blocks, RF_WARPS * 32, 0, stream()>>>(logits, router_bias, probs, idx, w, N, ne, K);
         else if (ne <= 128) route_finish_kernel<4><<<blocks, RF_WARPS * 32, 0, stream()>>>(logits, router_bias, probs, idx, w, N, ne, K);
