@@ -484,36 +484,49 @@ constexpr int SSD_LDM16 = SSD_Q + 8;       // M tile [Q][Q + 8] halfs
 
 // As ssd_chunk_state_kernel; d_state a multiple of 32.  S[p][n] = sum_s Xw[s][p] B[s][n]:
 // both operands are stored step-major, so both fragments come from transposing loads.
+template <int N_>
 __global__ void __launch_bounds__(SSD_THREADS, 4)
 ssd_chunk_state16_kernel(const float* __restrict__ proj, const float* __restrict__ bc, const float* __restrict__ dt_bias,
                          const float* __restrict__ a_log, float* __restrict__ dtcum, float* __restrict__ chunk_state,
                          float* __restrict__ decay, int T, int NC, MambaDims p, const int2* __restrict__ tab, int64_t NT) {
     extern __shared__ __align__(16) uint8_t sm16[];
     constexpr int P = SSD_P;
-    const int N = p.d_state, ldb = N + 8;
+    const int N = N_ ? N_ : p.d_state, ldb = N + 8;
     __half* sB = reinterpret_cast<__half*>(sm16);      // [Q][N + 8]
     __half* sX = sB + SSD_Q * ldb;                      // [Q][P + 8]   (already multiplied by w_s)
     float* sDt = reinterpret_cast<float*>(sX + SSD_Q * SSD_LDX16);   // [Q]
-    float* sCum = sDt + SSD_Q;                          // [Q]
+    float* sW = sDt + SSD_Q;                            // [Q]   e^{cum_last - cum_s} dt_s
     const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
     const SsdChunk ck = ssd_chunk(tab, NT, c, b, h, T, NC, p.n_heads);
     const int nt = ck.nt;
     const float A = -expf(a_log[h]);
-    if (threadIdx.x < SSD_Q) {
-        float dt = 0.0f;
-        if (threadIdx.x < nt) {
-            const float u = proj[(ck.row0 + threadIdx.x) * p.proj + p.proj - p.n_heads + h] + dt_bias[h];
-            dt = softplus_dt(u);
-        }
-        sDt[threadIdx.x] = dt;
+    float u = 0.0f;
+    if (threadIdx.x < nt) u = proj[(ck.row0 + threadIdx.x) * p.proj + p.proj - p.n_heads + h] + dt_bias[h];
+    // the rows of x wait in registers for their factors, so that all loads of the block are under way together
+    float4 xr[SSD_Q * (P / 4) / SSD_THREADS];
+#pragma unroll
+    for (int i = 0; i < SSD_Q * (P / 4) / SSD_THREADS; ++i) {
+        const int e = i * SSD_THREADS + threadIdx.x, t = e / (P / 4), c4 = (e % (P / 4)) * 4;
+        xr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < nt) xr[i] = *reinterpret_cast<const float4*>(bc + (ck.row0 + t) * p.conv_dim + h * P + c4);
     }
+    const int n4 = N >> 2;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < SSD_Q * n4; e += SSD_THREADS) {
+        const int t = e / n4, n = (e - t * n4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < nt) v = *reinterpret_cast<const float4*>(bc + (ck.row0 + t) * p.conv_dim + p.d_inner + n);
+        store_half4(sB + t * ldb + n, v);
+    }
+    if (threadIdx.x < SSD_Q) sDt[threadIdx.x] = threadIdx.x < nt ? softplus_dt(u) : 0.0f;
     __syncthreads();
     if (threadIdx.x < 32) {                 // running sum of A dt over the chunk: 4 steps per lane
         const int l = threadIdx.x;
-        float v[4], run = 0.0f;
+        float v[4], dt[4], run = 0.0f;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            run += __fmul_rn(A, sDt[l * 4 + i]);
+            dt[i] = sDt[l * 4 + i];
+            run += __fmul_rn(A, dt[i]);
             v[i] = run;
         }
         float incl = run;
@@ -522,34 +535,21 @@ ssd_chunk_state16_kernel(const float* __restrict__ proj, const float* __restrict
             const float up = __shfl_up_sync(0xffffffffu, incl, o);
             if (l >= o) incl += up;
         }
-        const float before = incl - run;
+        const float before = incl - run, last = __shfl_sync(0xffffffffu, before + v[3], 31);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sCum[l * 4 + i] = before + v[i];
+        for (int i = 0; i < 4; ++i) {
+            const float cum = before + v[i];
+            sW[l * 4 + i] = expf(last - cum) * dt[i];
+            if (l * 4 + i < nt) *reinterpret_cast<float2*>(dtcum + (ck.dt0 + l * 4 + i) * 2) = make_float2(dt[i], cum);
+        }
+        if (l == 31) decay[(ck.ci) * p.n_heads + h] = expf(last);
     }
     __syncthreads();
-    const float cum_last = sCum[SSD_Q - 1];
-    if (threadIdx.x < nt) {
-        float* o = dtcum + (ck.dt0 + threadIdx.x) * 2;
-        o[0] = sDt[threadIdx.x];
-        o[1] = sCum[threadIdx.x];
-    }
-    if (threadIdx.x == 0) decay[(ck.ci) * p.n_heads + h] = expf(cum_last);
-    const int n4 = N >> 2;
-    for (int e = threadIdx.x; e < SSD_Q * n4; e += SSD_THREADS) {
-        const int t = e / n4, n = (e - t * n4) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t < nt) v = *reinterpret_cast<const float4*>(bc + (ck.row0 + t) * p.conv_dim + p.d_inner + n);
-        store_half4(sB + t * ldb + n, v);
-    }
-    for (int e = threadIdx.x; e < SSD_Q * (P / 4); e += SSD_THREADS) {
-        const int t = e / (P / 4), i = (e - t * (P / 4)) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t < nt) {
-            const float w = expf(cum_last - sCum[t]) * sDt[t];
-            v = *reinterpret_cast<const float4*>(bc + (ck.row0 + t) * p.conv_dim + h * P + i);
-            v = make_float4(w * v.x, w * v.y, w * v.z, w * v.w);
-        }
-        store_half4(sX + t * SSD_LDX16 + i, v);
+#pragma unroll
+    for (int i = 0; i < SSD_Q * (P / 4) / SSD_THREADS; ++i) {
+        const int e = i * SSD_THREADS + threadIdx.x, t = e / (P / 4), c4 = (e % (P / 4)) * 4;
+        const float w = sW[t];
+        store_half4(sX + t * SSD_LDX16 + c4, make_float4(w * xr[i].x, w * xr[i].y, w * xr[i].z, w * xr[i].w));
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
@@ -584,6 +584,7 @@ ssd_chunk_state16_kernel(const float* __restrict__ proj, const float* __restrict
 }
 
 // As ssd_chunk_out_kernel; d_state a multiple of 16.
+template <int N_>
 __global__ void __launch_bounds__(SSD_THREADS, 4)
 ssd_chunk_out16_kernel(const float* __restrict__ bc, const float* __restrict__ G, const float* __restrict__ dtcum,
                        const float* __restrict__ chunk_state, const float* __restrict__ decay, float* __restrict__ state,
@@ -591,13 +592,14 @@ ssd_chunk_out16_kernel(const float* __restrict__ bc, const float* __restrict__ G
                        int NC, MambaDims p, const int2* __restrict__ tab, int64_t NT) {
     extern __shared__ __align__(16) uint8_t sm16[];
     constexpr int P = SSD_P;
-    const int N = p.d_state, ldc = N + 8;
+    const int N = N_ ? N_ : p.d_state, ldc = N + 8;
     const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
     const SsdChunk ck = ssd_chunk(tab, NT, c, b, h, T, NC, p.n_heads);
     const int nt = ck.nt;
     float* sDt = reinterpret_cast<float*>(sm16);        // [Q]
     float* sCum = sDt + SSD_Q;                          // [Q]
-    __half* buf = reinterpret_cast<__half*>(sCum + SSD_Q);
+    float* sE = sCum + SSD_Q;                           // [Q]   e^{cum_t}
+    __half* buf = reinterpret_cast<__half*>(sE + SSD_Q);
     if (threadIdx.x < SSD_Q) {
         float dt = 0.0f, cum = 0.0f;
         if (threadIdx.x < nt) {
@@ -607,6 +609,7 @@ ssd_chunk_out16_kernel(const float* __restrict__ bc, const float* __restrict__ G
         }
         sDt[threadIdx.x] = dt;
         sCum[threadIdx.x] = cum;
+        sE[threadIdx.x] = expf(cum);
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
@@ -623,11 +626,12 @@ ssd_chunk_out16_kernel(const float* __restrict__ bc, const float* __restrict__ G
         __half* sC = buf;                   // [Q][N + 8]
         __half* sS = buf + SSD_Q * ldc;     // [P][N + 8]
         const int n4 = N >> 2;
+#pragma unroll 4
         for (int e = threadIdx.x; e < SSD_Q * n4; e += SSD_THREADS) {
             const int t = e / n4, n = (e - t * n4) * 4;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (t < nt) {
-                const float w = expf(sCum[t]);
+                const float w = sE[t];
                 v = *reinterpret_cast<const float4*>(bc + (ck.row0 + t) * p.conv_dim + p.d_inner + N + n);
                 v = make_float4(w * v.x, w * v.y, w * v.z, w * v.w);
             }
@@ -637,6 +641,7 @@ ssd_chunk_out16_kernel(const float* __restrict__ bc, const float* __restrict__ G
         const bool whole = ck.whole >= 0;
         float* st = whole ? state + ((int64_t)ck.whole * p.n_heads + h) * P * N : nullptr;
         const float dk = whole ? decay[ck.ci * p.n_heads + h] : 0.0f;
+#pragma unroll 4
         for (int e = threadIdx.x; e < P * n4; e += SSD_THREADS) {
             const int i = e / n4, n = (e - i * n4) * 4;
             store_half4(sS + i * ldc + n, ssd_prev4(sp + i * N + n, st + i * N + n, dk, whole));
@@ -665,19 +670,30 @@ ssd_chunk_out16_kernel(const float* __restrict__ bc, const float* __restrict__ G
         __half* sM = buf;                   // [Q][Q + 8]
         __half* sX = buf + SSD_Q * SSD_LDM16;   // [Q][P + 8]
         const float* gm = G + (ck.ci) * SSD_Q * SSD_Q;
-        for (int e = threadIdx.x; e < SSD_Q * (SSD_Q / 4); e += SSD_THREADS) {
-            const int t = e / (SSD_Q / 4), s = (e - t * (SSD_Q / 4)) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (s <= t && t < nt) {
+        // a row has t / 4 + 1 groups of four on and below the diagonal: rows t and 123 - t fill the lanes of a warp
+        // exactly, rows 124 .. 127 alone
+#pragma unroll 3
+        for (int pr = warp; pr < 66; pr += SSD_THREADS / 32) {
+            const int ta = pr < 62 ? pr : pr + 62;
+            const bool low = lane <= (ta >> 2);
+            const int t = low ? ta : 123 - ta, s = 4 * (low ? lane : 31 - lane);
+            if (t < nt) {
                 const float4 gv = *reinterpret_cast<const float4*>(gm + t * SSD_Q + s);
+                const float4 cs = *reinterpret_cast<const float4*>(sCum + s), dt = *reinterpret_cast<const float4*>(sDt + s);
                 const float ct = sCum[t];
-                v.x = gv.x * expf(ct - sCum[s]) * sDt[s];
-                if (s + 1 <= t) v.y = gv.y * expf(ct - sCum[s + 1]) * sDt[s + 1];
-                if (s + 2 <= t) v.z = gv.z * expf(ct - sCum[s + 2]) * sDt[s + 2];
-                if (s + 3 <= t) v.w = gv.w * expf(ct - sCum[s + 3]) * sDt[s + 3];
+                float4 v;
+                v.x = gv.x * expf(ct - cs.x) * dt.x;
+                v.y = s + 1 <= t ? gv.y * expf(ct - cs.y) * dt.y : 0.0f;
+                v.z = s + 2 <= t ? gv.z * expf(ct - cs.z) * dt.z : 0.0f;
+                v.w = s + 3 <= t ? gv.w * expf(ct - cs.w) * dt.w : 0.0f;
+                store_half4(sM + t * SSD_LDM16 + s, v);
             }
-            store_half4(sM + t * SSD_LDM16 + s, v);
         }
+        if (threadIdx.x < SSD_Q) {            // the rest of the diagonal's tile of 16
+            const int t = threadIdx.x;
+            for (int q = (t >> 2) + 1; q < (t >> 4) * 4 + 4; ++q) *reinterpret_cast<uint2*>(sM + t * SSD_LDM16 + 4 * q) = make_uint2(0u, 0u);
+        }
+#pragma unroll 4
         for (int e = threadIdx.x; e < SSD_Q * (P / 4); e += SSD_THREADS) {
             const int t = e / (P / 4), i = (e - t * (P / 4)) * 4;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -757,8 +773,10 @@ int mamba_ssd_scan(const float* proj, const float* bc, const float* dt_bias, con
         B200_CUDA(cudaFuncSetAttribute(ssd_chunk_state_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
         B200_CUDA(cudaFuncSetAttribute(ssd_chunk_out_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
         B200_CUDA(cudaFuncSetAttribute(ssd_chunk_out_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-        B200_CUDA(cudaFuncSetAttribute(ssd_chunk_state16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-        B200_CUDA(cudaFuncSetAttribute(ssd_chunk_out16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        B200_CUDA(cudaFuncSetAttribute(ssd_chunk_state16_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        B200_CUDA(cudaFuncSetAttribute(ssd_chunk_state16_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        B200_CUDA(cudaFuncSetAttribute(ssd_chunk_out16_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        B200_CUDA(cudaFuncSetAttribute(ssd_chunk_out16_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
         configured = true;
     }
     B200_REQUIRE(smem_cb <= 160 * 1024 && smem_st <= 160 * 1024 && smem_out <= 160 * 1024, "mamba_ssd_scan: shared memory");
@@ -770,9 +788,10 @@ int mamba_ssd_scan(const float* proj, const float* bc, const float* dt_bias, con
     const dim3 grid(NC, p.n_heads, gz);
     const bool half_tiles = !precise && N % 32 == 0;
     const size_t smem_st16 = (size_t)(SSD_Q * (N + 8) + SSD_Q * SSD_LDX16) * 2 + 2 * SSD_Q * 4;
-    const size_t smem_out16 = (size_t)std::max(SSD_Q * (N + 8) + P * (N + 8), SSD_Q * SSD_LDM16 + SSD_Q * SSD_LDX16) * 2 + 2 * SSD_Q * 4;
+    const size_t smem_out16 = (size_t)std::max(SSD_Q * (N + 8) + P * (N + 8), SSD_Q * SSD_LDM16 + SSD_Q * SSD_LDX16) * 2 + 3 * SSD_Q * 4;
     if (half_tiles)
-        ssd_chunk_state16_kernel<<<grid, SSD_THREADS, smem_st16, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
+        N == 128 ? ssd_chunk_state16_kernel<128><<<grid, SSD_THREADS, smem_st16, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT)
+                 : ssd_chunk_state16_kernel<0><<<grid, SSD_THREADS, smem_st16, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
     else if (precise)
         ssd_chunk_state_kernel<true><<<grid, SSD_THREADS, smem_st, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
     else
@@ -791,7 +810,8 @@ int mamba_ssd_scan(const float* proj, const float* bc, const float* dt_bias, con
         B200_LAUNCH_CHECK("ssd_carry_kernel");
     }
     if (half_tiles)
-        ssd_chunk_out16_kernel<<<grid, SSD_THREADS, smem_out16, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
+        N == 128 ? ssd_chunk_out16_kernel<128><<<grid, SSD_THREADS, smem_out16, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT)
+                 : ssd_chunk_out16_kernel<0><<<grid, SSD_THREADS, smem_out16, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
     else if (precise)
         ssd_chunk_out_kernel<true><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
     else
