@@ -54,6 +54,10 @@ size_t moe_units_table_bytes(int64_t NK, int ne);
 int moe_units_forward(const float* x, const int32_t* grouped, const int32_t* offsets, const void* gates, const void* ups,
                       const void* downs, float* act, float* y, void* units_scratch, int64_t N, int d, int E, int ne, int K,
                       int kind);
+// moe_exact.cu: the same for Q4_K on the large tensor cores; scratch: moe_exact_bytes.
+size_t moe_exact_bytes(int64_t NK, int d, int E);
+int moe_exact_forward(const float* x, const int32_t* grouped, const int32_t* offsets, const void* gates, const void* ups,
+                      const void* downs, float* act, float* y, void* scratch, int64_t N, int d, int E, int ne, int K);
 int moe_dispatch_perm(const int32_t* idx, int64_t N, int ne, int K, int32_t* grouped, int32_t* inv, int32_t* offsets);
 size_t moe_shared_scratch_bytes(int64_t N, int d, int SH);
 int moe_shared_expert(const float* x, const void* sh_g, const void* sh_u, const void* sh_d, float* out, int64_t N, int d,

@@ -174,10 +174,11 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
                       int ne, int K, int SH, int kind) {
     const bool shared = sh_g && sh_u && sh_d && SH > 0;
     const size_t NK = (size_t)N * K;
+    const bool exact = kind == 3;                 // EXACT_RULE
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
     const size_t o_idx = take(NK * 4), o_w = take(NK * 4), o_grp = take(NK * 4), o_inv = take(NK * 4),
-                 o_off = take((size_t)(ne + 1) * 4), o_units = take(moe_units_table_bytes((int64_t)NK, ne)),
+                 o_off = take((size_t)(ne + 1) * 4), o_units = take(exact ? moe_exact_bytes((int64_t)NK, d, E) : moe_units_table_bytes((int64_t)NK, ne)),
                  o_act = take(NK * E * 4), o_y = take(NK * d * 4),
                  o_sh = shared ? take(moe_shared_scratch_bytes(N, d, SH)) : 0;
     void* wsp;
@@ -202,7 +203,8 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
     if (rc) return rc;
     rc = moe_dispatch_perm(idx, N, ne, K, grouped, inv, offsets);
     if (rc) return rc;
-    rc = moe_units_forward(x, grouped, offsets, gates, ups, downs, act, y, base + o_units, N, d, E, ne, K, kind);
+    rc = exact ? moe_exact_forward(x, grouped, offsets, gates, ups, downs, act, y, base + o_units, N, d, E, ne, K)
+               : moe_units_forward(x, grouped, offsets, gates, ups, downs, act, y, base + o_units, N, d, E, ne, K, kind);
     if (rc) return rc;
     if (shared && (rc = side_wait())) return rc;
     return moe_combine(y, inv, w, out, N, d, K, shared);

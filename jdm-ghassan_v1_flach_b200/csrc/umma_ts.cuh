@@ -1,0 +1,43 @@
+// tcgen05.mma with the first operand in tensor memory, and the fp16 arithmetic that expands packed weights into it.
+#pragma once
+
+#include "linear.cuh"
+#include "umma.cuh"
+
+namespace b200 {
+
+#ifdef __CUDACC__
+// A byte b OR-ed into the mantissa of 0x6400 is 1024 + b: two values per instruction.
+__device__ __forceinline__ __half2 wt_magic(uint32_t bytes, uint32_t sel) {
+    const uint32_t v = __byte_perm(bytes, 0x64646464u, sel);
+    return *reinterpret_cast<const __half2*>(&v);
+}
+constexpr uint32_t WT_SEL_01 = 0x5140, WT_SEL_23 = 0x5342;
+__device__ __forceinline__ uint32_t wt_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ __half2 wt_half2(uint32_t bits16) { return __half2half2(__ushort_as_half((unsigned short)bits16)); }
+
+// 32 columns of this warp's 32 tensor-memory lanes from registers.
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
+        "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
+        "r"(r[31])
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem]^T, one thread issues.
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+}
+#endif
+
+}  // namespace b200
