@@ -168,6 +168,11 @@ int linear(const float* x, const void* w, int kind, float* y, int M, int K, int 
         }
         return umma_gemm(GEMM_EPI_STORE, a16, M, b16, nullptr, N, nullptr, 1, M, N, K, y, nullptr, N, 1.0f);
     }
+    // More tokens than one pass of the few-token kernels, fewer than the rounding path takes: Q4_K goes to the exact
+    // tensor-core form, each weight read once (20 tokens of 6448 x 1536: LX_TIMES).
+    if (M > 8 && kind == 3 && K % 256 == 0 && N % 4 == 0 && N < (1 << 26) &&
+        ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 && M < GEMM_MIN_ROWS)
+        return linear_exact(x, w, y, M, K, N);
     // Preferred path: the TMA-streamed kernel (tensor-core dot for Q4_K / fp16 weights),
     // eight tokens per pass.  Shapes it cannot tile fall through to the plain kernel.
     if ((reinterpret_cast<uintptr_t>(w) & 15) == 0 && (kind != 3 || K % 256 == 0)) {

@@ -542,8 +542,9 @@ int mamba2_step(const float* x, const void* w_in, const float* conv_w, const flo
     float* y = dt_raw + (((size_t)batch * p.n_heads + 3) & ~(size_t)3);
     const int win = p.k - 1;
     const int rows = p.n_heads * p.d_head;
-    if (batch >= GEMM_MIN_ROWS && kind != KIND_F32) {
-        // many sequences: both projections as tensor-core GEMMs, the conv step on its own
+    if (batch > 2 && kind != KIND_F32) {
+        // several sequences: both projections as products of their own (the fused kernel below, which multiplies on the
+        // fp32 units, took 50 us for eight of them where the tensor cores take 15), the conv step by itself
         void* wsp2;
         const bool out_gemm = p.d_inner % 8 == 0 && p.d_inner <= 4096 && linear_uses_gemm(w_out, kind, out, batch, p.d_inner, p.d);
         const size_t f32_bytes = ((per + p.proj) * batch * sizeof(float) + 255) & ~(size_t)255;

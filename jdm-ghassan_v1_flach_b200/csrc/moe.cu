@@ -655,7 +655,7 @@ route_finish_kernel(const float* __restrict__ logits, const float* __restrict__ 
 
 int moe_route(const float* x, const float* router_w, const float* router_bias, float* probs,
               int32_t* idx, float* w, int64_t N, int d, int ne, int K) {
-    if (N >= 16 && d % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    if (d % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
         void* wsp;
         int rc = workspace(WS_ROUTE).ensure((size_t)N * ne * 4 + 256, &wsp);
         if (rc) return rc;

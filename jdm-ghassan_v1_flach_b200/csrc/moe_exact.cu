@@ -24,6 +24,7 @@
 
 namespace b200 {
 
+int splitk_reduce(const float* part, float* c, int splits, int64_t stride, int M, int N, int64_t ldc);
 int make_packed_map(CUtensorMap* out, const void* base, int64_t rows, int64_t row_bytes, int box_bytes, int box_rows);
 
 constexpr int WX_CAP = 24;                    // slots of a tile
@@ -50,10 +51,12 @@ static_assert(WX_SMEM <= 227 * 1024, "the stages do not fit the shared memory of
 
 struct alignas(64) WxArgs {
     CUtensorMap map_x, map_w, map_w2;
-    const int32_t* offsets;                   // device [ne + 1]: sorted slots of each expert
+    const int32_t* offsets;                   // device [ne + 1]: sorted slots of each expert; null: one of M rows
     const float* aux;                         // [NK, K / 256, WX_AUX]
     float* c;                                 // [NK, N]
-    int ne, N, K, n_tiles;
+    int ne, M, N, K, n_tiles;
+    int k_splits, per_split;                  // ranges of K (in units of 256) whose partial sums are added afterwards
+    int64_t split_stride;
     int* status;
 };
 
@@ -103,9 +106,18 @@ wx_split_kernel(const float* __restrict__ x, const int32_t* __restrict__ grouped
 // ---- tiles ------------------------------------------------------------------------
 struct WxTile {
     int slot0, slots, n0, brow;
+    int sb0, sb1;                             // its range of K in units of 256
 };
 // first[e] = first token tile of expert e; first[ne] = all of them.  All threads.
 __device__ __forceinline__ void wx_build(const WxArgs& a, int* first) {
+    if (!a.offsets) {
+        if (threadIdx.x == 0) {
+            first[0] = 0;
+            first[1] = (a.M + WX_CAP - 1) / WX_CAP;
+        }
+        __syncthreads();
+        return;
+    }
     if (threadIdx.x < 32) {
         int carry = 0;
         for (int e0 = 0; e0 < a.ne; e0 += 32) {
@@ -126,6 +138,10 @@ __device__ __forceinline__ void wx_build(const WxArgs& a, int* first) {
 }
 __device__ __noinline__ WxTile wx_find(const WxArgs& a, const int* first, int t) {
     WxTile w;
+    const int split = t % a.k_splits;
+    t /= a.k_splits;
+    w.sb0 = split * a.per_split;
+    w.sb1 = min(a.K >> 8, w.sb0 + a.per_split);
     const int tile = t / a.n_tiles;
     w.n0 = t - tile * a.n_tiles;
     int l = 0, h = a.ne;                      // the last expert whose first tile is <= tile owns it
@@ -133,7 +149,7 @@ __device__ __noinline__ WxTile wx_find(const WxArgs& a, const int* first, int t)
         const int mid = (l + h) >> 1;
         if (first[mid] <= tile) l = mid; else h = mid;
     }
-    const int lo = a.offsets[l], rows = a.offsets[l + 1] - lo, n = first[l + 1] - first[l], i = tile - first[l];
+    const int lo = a.offsets ? a.offsets[l] : 0, rows = (a.offsets ? a.offsets[l + 1] : a.M) - lo, n = first[l + 1] - first[l], i = tile - first[l];
     const int size = ((rows + n - 1) / n + 7) & ~7;                // equal tiles of whole groups of eight
     w.slot0 = lo + i * size;
     w.slots = max(0, min(size, rows - i * size));
@@ -143,7 +159,8 @@ __device__ __noinline__ WxTile wx_find(const WxArgs& a, const int* first, int t)
 __device__ __forceinline__ WxTile wx_tile_at(const WxArgs& a, const int* first, const int4* table, int i) {
     if (i >= WX_TABLE) return wx_find(a, first, blockIdx.x + i * gridDim.x);
     const int4 e = table[i];
-    return WxTile{e.x, e.y, e.z, e.w};
+    const int sb0 = (e.z >> 20) * a.per_split;
+    return WxTile{e.x, e.y, e.z & 0xFFFFF, e.w, sb0, min(a.K >> 8, sb0 + a.per_split)};
 }
 
 // 64 weights of a row (K step J of its 256) to the integers s q as 32 fp16 pairs, exact.
@@ -212,11 +229,11 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
     int* first = reinterpret_cast<int*>(table + WX_TABLE);
     const int warp = uniform_warp(), lane = threadIdx.x & 31, chunks = a.K >> 8;
     wx_build(a, first);
-    const int total = first[a.ne] * a.n_tiles;
+    const int total = first[a.ne] * a.n_tiles * a.k_splits;
     const int mine = (int)blockIdx.x < total ? (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
     if (threadIdx.x < WX_TABLE && (int)threadIdx.x < mine) {
         const WxTile w = wx_find(a, first, blockIdx.x + threadIdx.x * gridDim.x);
-        table[threadIdx.x] = make_int4(w.slot0, w.slots, w.n0, w.brow);
+        table[threadIdx.x] = make_int4(w.slot0, w.slots, w.n0 | (w.sb0 / a.per_split) << 20, w.brow);
     }
     if (threadIdx.x == 0) {
         for (int s = 0; s < WX_SX; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
@@ -240,7 +257,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
         for (int i = 0; i < mine && ok; ++i) {
             const WxTile w = wx_tile_at(a, first, table, i);
             const int boxes = (w.slots + 7) / 8;
-            for (int sb = 0; sb < chunks; ++sb, ++it) {
+            for (int sb = w.sb0; sb < w.sb1; ++sb, ++it) {
                 if (it >= WX_SX) ok = mbar_wait_warp(&x_empty[s], ph ^ 1, a.status);
                 if (!ok) break;
                 if (elect_one()) {
@@ -262,7 +279,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
         for (int i = 0; i < mine && ok; ++i) {
             const WxTile w = wx_tile_at(a, first, table, i);
             const int brow = w.brow + w.n0 * TILE_N;
-            for (int sb = 0; sb < chunks; ++sb, ++it) {
+            for (int sb = w.sb0; sb < w.sb1; ++sb, ++it) {
                 if (it >= WX_SP) ok = mbar_wait_warp(&p_empty[p], ph ^ 1, a.status);
                 if (!ok) break;
                 if (elect_one()) {
@@ -283,7 +300,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
         for (int i = 0; i < mine && ok; ++i) {
             const WxTile w = wx_tile_at(a, first, table, i);
             const uint32_t idesc = umma_idesc_f16(WX_ROWS, ((w.slots + 7) / 8 * WX_BOX + 15) & ~15);
-            for (int sb = 0; sb < chunks; ++sb, ++ci) {
+            for (int sb = w.sb0; sb < w.sb1; ++sb, ++ci) {
                 const uint32_t as = ci & 1, d = tmem + as * WX_SET, op = tmem + WX_OPERAND + as * WX_SET;
                 ok = (ci < 2 || mbar_wait_warp(&acc_empty[as], ((ci >> 1) - 1) & 1, a.status)) &&
                      mbar_wait_warp(&x_full[s], ph, a.status) && mbar_wait_warp(&a_full[as], (ci >> 1) & 1, a.status);
@@ -313,7 +330,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
         float4 nx[3];
         auto source = [&](int i) {
             const WxTile w = wx_tile_at(a, first, table, i);
-            return reinterpret_cast<const float4*>(a.aux + (int64_t)(w.slot0 + min(slot_of(min(lane, WX_HALF - 1)), w.slots - 1)) * chunks * WX_AUX);
+            return reinterpret_cast<const float4*>(a.aux + (int64_t)(w.slot0 + min(slot_of(min(lane, WX_HALF - 1)), w.slots - 1)) * chunks * WX_AUX) + w.sb0 * 3;
         };
         const float4* src = mine > 0 ? source(0) : nullptr;
         if (mine > 0)
@@ -325,14 +342,14 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
             float acc[WX_HALF];
 #pragma unroll
             for (int j = 0; j < WX_HALF; ++j) acc[j] = 0.0f;
-            for (int sb = 0; sb < chunks; ++sb, ++ci) {
+            for (int sb = w.sb0; sb < w.sb1; ++sb, ++ci) {
                 __syncwarp();
                 if (lane < WX_HALF)
 #pragma unroll
                     for (int j = 0; j < 3; ++j) *reinterpret_cast<float4*>(aux + lane * WX_AUX + 4 * j) = nx[j];
                 src += 3;
-                if (sb + 1 == chunks && i + 1 < mine) src = source(i + 1);
-                if (sb + 1 < chunks || i + 1 < mine)
+                if (sb + 1 == w.sb1 && i + 1 < mine) src = source(i + 1);
+                if (sb + 1 < w.sb1 || i + 1 < mine)
 #pragma unroll
                     for (int j = 0; j < 3; ++j) nx[j] = src[j];
                 const uint32_t as = ci & 1;
@@ -392,10 +409,11 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
             } else {
                 if (!ok) break;
                 const int n = w.n0 * TILE_N + tid;
+                float* c = a.c + w.sb0 / a.per_split * a.split_stride;
                 if (n < a.N)
 #pragma unroll
                     for (int j = 0; j < WX_HALF; ++j)
-                        if (slot_of(j) < w.slots) a.c[(int64_t)(w.slot0 + slot_of(j)) * a.N + n] = acc[j];
+                        if (slot_of(j) < w.slots) c[(int64_t)(w.slot0 + slot_of(j)) * a.N + n] = acc[j];
             }
         }
     } else if (warp >= WX_FIRST_EXPAND) {
@@ -403,7 +421,11 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
         const uint32_t dst = tmem + WX_OPERAND + slot * 32 + ((uint32_t)(q * 32) << 16);
         const uint32_t row_at = smem_u32(sm_p) + (q * 32 + lane) * WX_SBB;
         uint32_t p = 0, ph = 0;
-        const uint32_t stages = (uint32_t)mine * chunks;
+        uint32_t stages = 0;
+        for (int i = 0; i < mine; ++i) {
+            const WxTile w = wx_tile_at(a, first, table, i);
+            stages += w.sb1 - w.sb0;
+        }
         for (uint32_t ci = 0; ci < stages; ++ci) {
             if (!mbar_wait_warp(&p_full[p], ph, a.status)) break;
             const uint32_t seg = row_at + p * WX_PACKED;
@@ -434,13 +456,13 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
 }
 
 template <bool SWIGLU>
-static int launch_wx(const WxArgs& a, int64_t NK) {
+static int launch_wx(const WxArgs& a, int64_t rows) {
     static bool configured = false;
     if (!configured) {
         B200_CUDA(cudaFuncSetAttribute(wx_kernel<SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, WX_SMEM));
         configured = true;
     }
-    const int64_t most = (NK / WX_CAP + std::min<int64_t>(a.ne, NK)) * a.n_tiles;      // an expert's last tile may be short
+    const int64_t most = (rows / WX_CAP + std::min<int64_t>(a.ne, rows)) * a.n_tiles * a.k_splits;      // an expert's last tile may be short
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)std::min<int64_t>(most, num_sms()));
     cfg.blockDim = dim3(WX_THREADS);
@@ -468,7 +490,7 @@ int moe_exact_forward(const float* x, const int32_t* grouped, const int32_t* off
     __half* cols = static_cast<__half*>(scratch);
     float* aux = reinterpret_cast<float*>(static_cast<char*>(scratch) + ((size_t)NK * 3 * std::max(d, E) * 2 + 255) / 256 * 256);
     WxArgs a;
-    a.offsets = offsets; a.aux = aux; a.ne = ne;
+    a.offsets = offsets; a.aux = aux; a.ne = ne; a.M = 0; a.k_splits = 1; a.split_stride = 0;
     a.status = stream_status_ptr();
     B200_REQUIRE(a.status, "moe_exact: status word allocation failed");
     for (int pass = 0; pass < 2; ++pass) {
@@ -482,11 +504,40 @@ int moe_exact_forward(const float* x, const int32_t* grouped, const int32_t* off
                                                                                        (int)NK, Kd, cols, aux);
         B200_LAUNCH_CHECK("wx_split_kernel");
         a.c = down ? y : act;
-        a.N = Nd; a.K = Kd; a.n_tiles = ceil_div(Nd, tile);
+        a.N = Nd; a.K = Kd; a.n_tiles = ceil_div(Nd, tile); a.per_split = Kd / 256;
         rc = down ? launch_wx<false>(a, NK) : launch_wx<true>(a, NK);
         if (rc) return rc;
     }
     return B200_OK;
+}
+
+// One Q4_K matrix for a few tens of tokens, exact to fp32: y [M, N] = x [M, K] . w [N, K]^T; K a multiple of 256, N of 4.
+// Few tiles: K is cut across CTAs and the partial sums are added in a fixed order.
+int linear_exact(const float* x, const void* w, float* y, int M, int K, int N) {
+    WxArgs a;
+    a.n_tiles = ceil_div(N, WX_ROWS);
+    const int chunks = K / 256, tiles = ceil_div(M, WX_CAP) * a.n_tiles;
+    a.per_split = ceil_div(chunks, std::max(1, std::min(chunks, num_sms() / tiles)));
+    a.k_splits = ceil_div(chunks, a.per_split);
+    a.split_stride = a.k_splits > 1 ? (int64_t)M * N : 0;
+    void *ws, *part = nullptr;
+    const size_t cols_bytes = ((size_t)M * 3 * K * 2 + 255) / 256 * 256;
+    int rc = workspace(WS_LINEAR).ensure(cols_bytes + (size_t)M * chunks * WX_AUX * 4 + 256, &ws);
+    if (!rc && a.k_splits > 1) rc = workspace(WS_SPLITK).ensure((size_t)a.k_splits * a.split_stride * 4 + 256, &part);
+    if (rc) return rc;
+    __half* cols = static_cast<__half*>(ws);
+    float* aux = reinterpret_cast<float*>(static_cast<char*>(ws) + cols_bytes);
+    if ((rc = make_tile_map(&a.map_x, cols, 3 * (int64_t)M, K, WX_BOX))) return rc;
+    if ((rc = make_packed_map(&a.map_w, w, N, (int64_t)chunks * WX_SBB, WX_SBB, WX_ROWS))) return rc;
+    a.map_w2 = a.map_w;
+    a.offsets = nullptr; a.aux = aux; a.ne = 1; a.M = M; a.N = N; a.K = K;
+    a.c = part ? static_cast<float*>(part) : y;
+    a.status = stream_status_ptr();
+    B200_REQUIRE(a.status, "linear_exact: status word allocation failed");
+    wx_split_kernel<<<(unsigned)ceil_div(M * chunks, 8), 256, 0, stream()>>>(x, nullptr, 1, M, K, cols, aux);
+    B200_LAUNCH_CHECK("wx_split_kernel");
+    if ((rc = launch_wx<false>(a, M))) return rc;
+    return part ? splitk_reduce(a.c, y, a.k_splits, a.split_stride, M, N, N) : B200_OK;
 }
 
 }  // namespace b200
