@@ -144,6 +144,7 @@ struct b200_decoder {
     cudaGraphExec_t graph = nullptr;
     const int32_t* graph_tok = nullptr;
     int32_t* graph_next = nullptr;
+    bool graph_own = false;                    // recorded on tok and next below instead of the caller's buffers
     cudaStream_t own_stream = nullptr;
     int launches = 0;
     int32_t *h_tok = nullptr, *h_next = nullptr;   // pinned staging for the host entry point
@@ -1126,8 +1127,15 @@ int b200_decoder_step(b200_decoder* dec, const int32_t* tokens_dev, int32_t* nex
         drop_graph(dec);
         dec->launches = 0;          // one eager step first: it sizes the workspaces again
     }
-    if (!dec->graph || dec->graph_tok != tokens_dev || dec->graph_next != next_dev) {
+    // The recording holds the addresses of the tokens and of the picks.  A caller that hands over other buffers at every
+    // step would have the step recorded every time (on the host, over 8 us per launch: 7.5 ms for a step of nine
+    // sequences whose kernels take 4): from the second address on it is recorded on the decoder's own two, and the
+    // tokens and picks are copied (8 bytes per sequence).
+    if (dec->graph && !dec->graph_own && (dec->graph_tok != tokens_dev || dec->graph_next != next_dev)) {
         drop_graph(dec);
+        dec->graph_own = true;
+    }
+    if (!dec->graph) {
         // Workspaces grow with cudaMalloc, which cannot run inside a capture.  The
         // first step of a configuration therefore runs eagerly (sizing every
         // workspace); the capture happens on the second.
@@ -1146,7 +1154,7 @@ int b200_decoder_step(b200_decoder* dec, const int32_t* tokens_dev, int32_t* nex
         cudaError_t e = cudaStreamBeginCapture(dec->own_stream, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             const unsigned long long before = g_kernel_launches;
-            rc = enqueue(dec, tokens_dev, next_dev);
+            rc = enqueue(dec, dec->graph_own ? dec->tok : tokens_dev, dec->graph_own ? dec->next : next_dev);
             dec->launches = (int)(g_kernel_launches - before);
             e = cudaStreamEndCapture(dec->own_stream, &g);
         }
@@ -1156,11 +1164,16 @@ int b200_decoder_step(b200_decoder* dec, const int32_t* tokens_dev, int32_t* nex
         e = cudaGraphInstantiate(&dec->graph, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return cuda_status(e, "decoder_step: cudaGraphInstantiate");
-        dec->graph_tok = tokens_dev;
-        dec->graph_next = next_dev;
+        dec->graph_tok = dec->graph_own ? dec->tok : tokens_dev;
+        dec->graph_next = dec->graph_own ? dec->next : next_dev;
         dec->ws_generation = workspace_generation();
     }
+    const size_t bytes = (size_t)dec->batch * sizeof(int32_t);
+    if (dec->graph_tok != tokens_dev)
+        B200_CUDA(cudaMemcpyAsync(dec->tok, tokens_dev, bytes, cudaMemcpyDeviceToDevice, stream()));
     B200_CUDA(cudaGraphLaunch(dec->graph, stream()));
+    if (dec->graph_next != next_dev)
+        B200_CUDA(cudaMemcpyAsync(next_dev, dec->next, bytes, cudaMemcpyDeviceToDevice, stream()));
     dec->position += 1;
     return B200_OK;
 }
