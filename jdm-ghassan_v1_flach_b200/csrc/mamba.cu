@@ -209,7 +209,7 @@ mamba_conv_step_kernel(const float* __restrict__ proj, const float* __restrict__
 // through `out`.  Six CTAs per SM: the kernel is a chain of load -> block reduction -> store
 // per row, so resident rows are what hides its latencies.
 // VEC (rows, pointers and strides of 16 bytes): four neighbours per load, all of a thread's loads under way before the
-// first exponential.  GN_TIMES
+// first exponential: 4096 rows of 3072 took 52 us by single floats, 24 so (17 at the copy rate).
 template <int PER, bool VEC = false>
 __global__ void __launch_bounds__(256, 6)
 mamba_gated_norm_kernel(const float* y, const float* __restrict__ gate, int64_t gate_stride,

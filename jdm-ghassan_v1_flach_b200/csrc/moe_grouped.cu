@@ -174,7 +174,10 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
                       int ne, int K, int SH, int kind) {
     const bool shared = sh_g && sh_u && sh_d && SH > 0;
     const size_t NK = (size_t)N * K;
-    const bool exact = kind == 3;                 // EXACT_RULE
+    // The exact tensor-core form costs about the same for one slot of an expert as for 24, and some 20 us of set-up; the
+    // digit engine costs by the slot.  Experts of 512 x 1536: 54 against 67 us at 9 tokens (1.2 slots per expert of
+    // the 64), 85 against 84 at 28; of 768 x 4096: 275 against 186 at 9 tokens already.
+    const bool exact = kind == 3 && (2 * NK >= 5 * (size_t)ne || (int64_t)E * d >= (1 << 21));
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
     const size_t o_idx = take(NK * 4), o_w = take(NK * 4), o_grp = take(NK * 4), o_inv = take(NK * 4),

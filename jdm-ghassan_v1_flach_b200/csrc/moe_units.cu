@@ -18,7 +18,8 @@
 // Bound by the engine's instructions (about 85 per 1024 weights with eight tokens, 137 and more before it) and
 // by how evenly the units spread: two CTAs per SM share the list of all (unit, tile) pairs in equal contiguous
 // ranges, so a unit's tokens are staged by the few CTAs whose range it is in.
-// 64 tokens, H-Tiny shape, Q4_K: 54 + 53 us before, UNITS_US.
+// 64 tokens, H-Tiny shape, Q4_K: 54 + 53 us before, 47 + 58 (beside the shared expert) now; Q4_K has a
+// faster form since (moe_exact.cu: 38 + 22), the other kinds, whose scales change every 32 of K, have not.
 #include "digit_tile.cuh"
 #include "gemm.cuh"
 

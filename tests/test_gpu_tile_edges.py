@@ -1,0 +1,139 @@
+"""GPU parity at the edges of the kernels' tiles: the few-token products, the exact tensor-core form for a few tens
+of tokens, the GEMM whose token tiles follow the row count, the router's tiles, the one-chunk scan and the recorded
+step of a caller whose buffers move."""
+import numpy as np
+import pytest
+import torch
+
+from cases import mamba_params, moe_case
+from model_util import TINY, CudaDecoder, make_model
+
+pytestmark = pytest.mark.gpu
+
+
+# K: one chunk of 256, a partly filled one, several parts of a contraction; N: below a tile of 16 rows, one over
+@pytest.mark.parametrize("kind", [-1, 0, 1, 2, 3])
+@pytest.mark.parametrize("M", [1, 3, 8, 9, 24, 25, 31])
+@pytest.mark.parametrize("K,N", [(256, 4), (288, 20), (2560, 132)])
+def test_few_token_products(oracle, kind, M, K, N):
+    from gpu_util import SUM_ORDER, close, dev, empty, host, ops
+    if kind == 3 and K % 256:
+        pytest.skip("Q4_K rows are multiples of 256 weights")
+    r = np.random.default_rng(100 * M + K + kind)
+    x = r.standard_normal((M, K)).astype(np.float32)
+    x[0, :32] *= 1e4                                    # one block far above the rest of its row
+    x[M - 1, 256:] = 0.0
+    w = (r.standard_normal(N * K) * 0.02).astype(np.float32)
+    y = empty((M, N))
+    if kind < 0:
+        w = w.astype(np.float16).reshape(N, K)
+        ops.linear_forward_fp16(dev(x), dev(w.view(np.uint16)), y, M, K, N)
+        want = (x.astype(np.float64) @ w.astype(np.float64).T).astype(np.float32)
+    else:
+        w = oracle.quantize(w, kind)
+        ops.linear_forward_q4(dev(x), dev(w), y, M, K, N, kind)
+        want = oracle.linear_exact(x, w, kind, M, K, N)
+    tol = dict(SUM_ORDER, atol=SUM_ORDER["atol"] * max(1.0, float(np.abs(want).max())))
+    np.testing.assert_allclose(host(y), want, **tol)
+
+
+# rows around one, two and three token tiles of 192 and around the 16 and 96 rows of a copy
+@pytest.mark.parametrize("kind", [1, 2, 3])
+@pytest.mark.parametrize("M", [33, 96, 97, 192, 193, 385])
+@pytest.mark.parametrize("K,N", [(256, 132), (768, 260)])
+def test_gemm_token_tiles(oracle, kind, M, K, N):
+    from gpu_util import dev, empty, fp16_close, host, ops
+    r = np.random.default_rng(M + K + kind)
+    x = r.standard_normal((M, K)).astype(np.float32)
+    w = oracle.quantize((r.standard_normal(N * K) * 0.02).astype(np.float32), kind)
+    y = empty((M, N))
+    ops.linear_forward_q4(dev(x), dev(w), y, M, K, N, kind)
+    w16 = oracle.dequantize(w, N * K, kind).reshape(N, K).view(np.float16).astype(np.float64)
+    want = (x.astype(np.float16).astype(np.float64) @ w16.T).astype(np.float32)
+    fp16_close(host(y), want, frac=1e-3)
+
+
+# the bias gathers the tokens: experts with none, one, a full tile (8 / 24 slots) and one more
+@pytest.mark.parametrize("kind", [2, 3])
+@pytest.mark.parametrize("N", [9, 24, 25, 48])
+@pytest.mark.parametrize("d,E", [(256, 512), (768, 256)])
+def test_expert_tiles(oracle, kind, N, d, E):
+    from gpu_util import SUM_ORDER, dev, empty, host, ops
+    ne, K = 8, 2
+    c = moe_case(oracle, N + d, N, d, E, ne, K, 0, kind, bias_sigma=2.0)
+    out, idx, w = empty((N, d)), empty((N, K), torch.int32), empty((N, K))
+    args = [dev(c[k]) for k in ("gates", "ups", "downs", "sh_g", "sh_u", "sh_d")]
+    ops.moe_forward_bias_half(dev(c["x"]), dev(c["router_w"]), dev(c["router_bias"]), *args, out, None, idx, w, None, None,
+                              None, N, d, E, ne, K, 0, kind)
+    want, _, widx, _ = oracle.moe_forward(c["x"], c["router_w"], c["router_bias"], c["gates"], c["ups"], c["downs"], None, None,
+                                          None, d, E, ne, K, 0, kind)
+    assert np.array_equal(host(idx), widx)
+    np.testing.assert_allclose(host(out), want, **SUM_ORDER)
+
+
+# one to eight tokens; the 8-, 16- and 32-token tiles of the many-token router; widths off its 64 columns
+@pytest.mark.parametrize("d,ne,K", [(260, 33, 3), (1536, 64, 6)])
+@pytest.mark.parametrize("N", [1, 7, 257, 600, 2401])
+def test_router_tiles(oracle, d, ne, K, N):
+    from gpu_util import dev, empty, host, ops
+    r = np.random.default_rng(d + N)
+    x = r.standard_normal((N, d)).astype(np.float32)
+    rw = (r.standard_normal((ne, d)) / np.sqrt(d)).astype(np.float32)
+    bias = (r.standard_normal(ne) * 0.5 / ne).astype(np.float32)
+    _, idx, w = oracle.moe_route(x, rw, bias, ne, K)
+    di, dw = empty((N, K), torch.int32), empty((N, K))
+    ops.moe_route(dev(x), dev(rw), dev(bias), empty((N, ne)), di, dw, N, d, ne, K)
+    assert np.array_equal(host(di), idx)
+    np.testing.assert_array_max_ulp(host(dw), w, maxulp=4)
+
+
+# a sequence of one chunk carries its state in the output kernel; 129 steps: two chunks
+@pytest.mark.parametrize("kind", [-2, 2])
+@pytest.mark.parametrize("d_state", [64, 128])
+@pytest.mark.parametrize("T", [65, 128, 129])
+def test_scan_chunks(oracle, kind, d_state, T):
+    from gpu_util import dev, empty, fp16_close, host, ops
+    r = np.random.default_rng(T + d_state)
+    B, d, heads, P, k = 2, 256, 3, 64, 4
+    p = mamba_params(oracle, r, d, heads, P, d_state, k, kind, 0.2)
+    x = r.standard_normal((B, T, d)).astype(np.float32)
+    state = (r.standard_normal((B, heads, P, d_state)) * 0.1).astype(np.float32)
+    names = ("w_in", "conv_w", "conv_b", "dt_bias", "a_log", "D", "norm_w", "w_out")
+    rest = (B, T, d, p["d_inner"], p["conv_dim"], heads, P, d_state, k, 1e-5)
+    want, want_state = oracle.mamba2_forward(x, *(p[n] for n in names), state, *rest, kind)
+    ds, out = dev(state), empty((B, T, d))
+    weights = [dev(p[n]) for n in names]
+    if kind == -2:
+        ops.mamba2_forward(dev(x), *weights, ds, out, *rest)
+    else:
+        ops.mamba2_forward_half(dev(x), *weights, ds, out, *rest, kind)
+    fp16_close(host(out), want)
+    fp16_close(host(ds), want_state)
+
+
+# buffers that stay, that move at every step, and that move and come back
+@pytest.mark.parametrize("fused,batch", [(1, 1), (0, 3), (0, 9)])
+def test_recorded_step_with_moving_buffers(oracle, fused, batch):
+    model = make_model(oracle, TINY, 4)
+    r = np.random.default_rng(5)
+    steps = r.integers(0, TINY["vocab"], (6, batch)).astype(np.int32)
+    outs = []
+    for moving in (False, True):
+        dec = CudaDecoder(model, batch=batch, max_ctx=64)
+        dec.configure(fused, 1)
+        tok, nxt = torch.zeros(batch, dtype=torch.int32, device="cuda"), torch.zeros(batch, dtype=torch.int32, device="cuda")
+        kept, got = [], []
+        for i, t in enumerate(steps):
+            if moving and i != 3:
+                tok, nxt = torch.zeros_like(tok), torch.zeros_like(nxt)
+                kept.append((tok, nxt))
+            tok.copy_(torch.from_numpy(t))
+            torch.cuda.synchronize()
+            dec.lib.b200_decoder_step(dec.handle, tok, nxt)
+            dec.lib.b200_synchronize()
+            got.append((nxt.cpu().numpy().copy(), dec.logits()))
+        outs.append(got)
+        dec.close()
+    for (na, la), (nb, lb) in zip(*outs):
+        assert np.array_equal(na, nb)
+        assert np.array_equal(la.view(np.uint32), lb.view(np.uint32))
