@@ -140,12 +140,16 @@ __device__ __forceinline__ void wx_build(const WxArgs& a, int* first) {
     }
     __syncthreads();
 }
+template <bool SPLIT>
 __device__ __noinline__ WxTile wx_find(const WxArgs& a, const int* first, int t) {
     WxTile w;
-    const int split = t % a.k_splits;
-    t /= a.k_splits;
-    w.sb0 = split * a.per_split;
-    w.sb1 = min(a.K >> 8, w.sb0 + a.per_split);
+    w.sb0 = 0;
+    w.sb1 = a.K >> 8;
+    if (SPLIT) {
+        w.sb0 = t % a.k_splits * a.per_split;
+        w.sb1 = min(w.sb1, w.sb0 + a.per_split);
+        t /= a.k_splits;
+    }
     const int tile = t / a.n_tiles;
     w.n0 = t - tile * a.n_tiles;
     int l = 0, h = a.ne;                      // the last expert whose first tile is <= tile owns it
@@ -160,9 +164,11 @@ __device__ __noinline__ WxTile wx_find(const WxArgs& a, const int* first, int t)
     w.brow = l * a.N;
     return w;
 }
+template <bool SPLIT>
 __device__ __forceinline__ WxTile wx_tile_at(const WxArgs& a, const int* first, const int4* table, int i) {
-    if (i >= WX_TABLE) return wx_find(a, first, blockIdx.x + i * gridDim.x);
+    if (i >= WX_TABLE) return wx_find<SPLIT>(a, first, blockIdx.x + i * gridDim.x);
     const int4 e = table[i];
+    if (!SPLIT) return WxTile{e.x, e.y, e.z, e.w, 0, a.K >> 8};
     const int sb0 = (e.z >> 20) * a.per_split;
     return WxTile{e.x, e.y, e.z & 0xFFFFF, e.w, sb0, min(a.K >> 8, sb0 + a.per_split)};
 }
@@ -211,7 +217,7 @@ __device__ __forceinline__ void tmem_ld12(uint32_t at, float (&v)[12]) {
     for (int i = 0; i < 12; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-template <bool SWIGLU>
+template <bool SWIGLU, bool SPLIT>
 __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant__ WxArgs a) {
     constexpr int TILE_N = SWIGLU ? WX_ROWS / 2 : WX_ROWS;
     extern __shared__ uint8_t smem_raw[];
@@ -233,11 +239,11 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
     int* first = reinterpret_cast<int*>(table + WX_TABLE);
     const int warp = uniform_warp(), lane = threadIdx.x & 31, chunks = a.K >> 8;
     wx_build(a, first);
-    const int total = first[a.ne] * a.n_tiles * a.k_splits;
+    const int total = first[a.ne] * a.n_tiles * (SPLIT ? a.k_splits : 1);
     const int mine = (int)blockIdx.x < total ? (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
     if (threadIdx.x < WX_TABLE && (int)threadIdx.x < mine) {
-        const WxTile w = wx_find(a, first, blockIdx.x + threadIdx.x * gridDim.x);
-        table[threadIdx.x] = make_int4(w.slot0, w.slots, w.n0 | (w.sb0 / a.per_split) << 20, w.brow);
+        const WxTile w = wx_find<SPLIT>(a, first, blockIdx.x + threadIdx.x * gridDim.x);
+        table[threadIdx.x] = make_int4(w.slot0, w.slots, SPLIT ? w.n0 | (w.sb0 / a.per_split) << 20 : w.n0, w.brow);
     }
     if (threadIdx.x == 0) {
         for (int s = 0; s < WX_SX; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
@@ -259,7 +265,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
         uint32_t it = 0, s = 0, ph = 0;
         bool ok = true;
         for (int i = 0; i < mine && ok; ++i) {
-            const WxTile w = wx_tile_at(a, first, table, i);
+            const WxTile w = wx_tile_at<SPLIT>(a, first, table, i);
             const int boxes = (w.slots + 7) / 8;
             for (int sb = w.sb0; sb < w.sb1; ++sb, ++it) {
                 if (it >= WX_SX) ok = mbar_wait_warp(&x_empty[s], ph ^ 1, a.status);
@@ -281,7 +287,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
         uint32_t it = 0, p = 0, ph = 0;
         bool ok = true;
         for (int i = 0; i < mine && ok; ++i) {
-            const WxTile w = wx_tile_at(a, first, table, i);
+            const WxTile w = wx_tile_at<SPLIT>(a, first, table, i);
             const int brow = w.brow + w.n0 * TILE_N;
             for (int sb = w.sb0; sb < w.sb1; ++sb, ++it) {
                 if (it >= WX_SP) ok = mbar_wait_warp(&p_empty[p], ph ^ 1, a.status);
@@ -299,18 +305,24 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
             for (uint32_t j = it > WX_SP ? it - WX_SP : 0; j < it; ++j)
                 if (!mbar_wait_warp(&p_full[j % WX_SP], (j / WX_SP) & 1, a.status)) break;
     } else if (warp == 1) {
-        uint32_t ci = 0, s = 0, ph = 0;
+        uint32_t ci = 0, s = 0, ph = 0, ready = 0;
         bool ok = true;
         for (int i = 0; i < mine && ok; ++i) {
-            const WxTile w = wx_tile_at(a, first, table, i);
+            const WxTile w = wx_tile_at<SPLIT>(a, first, table, i);
             const uint32_t idesc = umma_idesc_f16(WX_ROWS, ((w.slots + 7) / 8 * WX_BOX + 15) & ~15);
             for (int sb = w.sb0; sb < w.sb1; ++sb, ++ci) {
                 const uint32_t as = ci & 1, d = tmem + as * WX_SET, op = tmem + WX_OPERAND + as * WX_SET;
-                ok = (ci < 2 || mbar_wait_warp(&acc_empty[as], ((ci >> 1) - 1) & 1, a.status)) &&
-                     mbar_wait_warp(&x_full[s], ph, a.status) && mbar_wait_warp(&a_full[as], (ci >> 1) & 1, a.status);
+                if (!__all_sync(0xffffffffu, ready != 0))
+                    ok = (ci < 2 || mbar_wait_warp(&acc_empty[as], ((ci >> 1) - 1) & 1, a.status)) &&
+                         mbar_wait_warp(&x_full[s], ph, a.status) && mbar_wait_warp(&a_full[as], (ci >> 1) & 1, a.status);
                 if (!ok) break;
                 tc_fence_after();
                 const uint64_t desc = umma_smem_desc(smem_u32(sm_x + s * WX_X_STAGE));
+                // the next step's barriers are looked at before this one's products are issued: a wait costs a few
+                // hundred cycles even when there is nothing to wait for
+                const uint32_t sn = s + 1 == WX_SX ? 0 : s + 1, phn = s + 1 == WX_SX ? ph ^ 1 : ph, nx = ci + 1;
+                ready = (nx < 2 ? 1u : mbar_peek(&acc_empty[nx & 1], ((nx >> 1) - 1) & 1)) & mbar_peek(&x_full[sn], phn) &
+                        mbar_peek(&a_full[nx & 1], (nx >> 1) & 1);
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 16; ++k)          // 32 bytes of K per step: 2 in the descriptor's units
@@ -328,12 +340,12 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
         const int e = warp >= WX_SECOND_EPI, q = warp & 3, tid = q * 32 + lane;
         float* aux = sm_aux + (4 * e + q) * WX_HALF * WX_AUX;
         auto slot_of = [&](int l) { return 4 * (2 * (l >> 2) + e) + (l & 3); };        // of the group's l-th sum
-        uint32_t ci = 0, ti = 0;
+        uint32_t ci = 0, ti = 0, ready = 0;
         pdl_wait();
         // the next 256's scales and sums travel while this one's are used: a lane fetches one slot's
         float4 nx[3];
         auto source = [&](int i) {
-            const WxTile w = wx_tile_at(a, first, table, i);
+            const WxTile w = wx_tile_at<SPLIT>(a, first, table, i);
             return reinterpret_cast<const float4*>(a.aux + (int64_t)(w.slot0 + min(slot_of(min(lane, WX_HALF - 1)), w.slots - 1)) * chunks * WX_AUX) + w.sb0 * 3;
         };
         const float4* src = mine > 0 ? source(0) : nullptr;
@@ -341,7 +353,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
 #pragma unroll
             for (int j = 0; j < 3; ++j) nx[j] = src[j];
         for (int i = 0; i < mine; ++i, ++ti) {
-            const WxTile w = wx_tile_at(a, first, table, i);
+            const WxTile w = wx_tile_at<SPLIT>(a, first, table, i);
             bool ok = true;
             float acc[WX_HALF];
 #pragma unroll
@@ -357,8 +369,9 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
 #pragma unroll
                     for (int j = 0; j < 3; ++j) nx[j] = src[j];
                 const uint32_t as = ci & 1;
-                ok = mbar_wait_warp(&done[as], (ci >> 1) & 1, a.status);
+                if (!__all_sync(0xffffffffu, ready != 0)) ok = mbar_wait_warp(&done[as], (ci >> 1) & 1, a.status);
                 if (!ok) break;
+                ready = mbar_peek(&done[as ^ 1], ((ci + 1) >> 1) & 1);
                 tc_fence_after();
                 const uint4 hdr = sm_hdr[(ci % WX_HDR) * WX_ROWS + tid];
                 const float d = half_bits_to_float((uint16_t)(hdr.x & 0xFFFFu)), dmin = half_bits_to_float((uint16_t)(hdr.x >> 16));
@@ -413,7 +426,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
             } else {
                 if (!ok) break;
                 const int n = w.n0 * TILE_N + tid;
-                float* c = a.c + w.sb0 / a.per_split * a.split_stride;
+                float* c = SPLIT ? a.c + w.sb0 / a.per_split * a.split_stride : a.c;
                 if (n < a.N)
 #pragma unroll
                     for (int j = 0; j < WX_HALF; ++j)
@@ -424,14 +437,15 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
         const int slot = (warp - WX_FIRST_EXPAND) >> 2, q = warp & 3;
         const uint32_t dst = tmem + WX_OPERAND + slot * 32 + ((uint32_t)(q * 32) << 16);
         const uint32_t row_at = smem_u32(sm_p) + (q * 32 + lane) * WX_SBB;
-        uint32_t p = 0, ph = 0;
-        uint32_t stages = 0;
-        for (int i = 0; i < mine; ++i) {
-            const WxTile w = wx_tile_at(a, first, table, i);
+        uint32_t p = 0, ph = 0, p_ready = 0;
+        uint32_t stages = SPLIT ? 0 : (uint32_t)mine * chunks;
+        for (int i = 0; SPLIT && i < mine; ++i) {
+            const WxTile w = wx_tile_at<SPLIT>(a, first, table, i);
             stages += w.sb1 - w.sb0;
         }
         for (uint32_t ci = 0; ci < stages; ++ci) {
-            if (!mbar_wait_warp(&p_full[p], ph, a.status)) break;
+            if (!__all_sync(0xffffffffu, p_ready != 0) && !mbar_wait_warp(&p_full[p], ph, a.status)) break;
+            const uint32_t free_ahead = ci > 1 ? mbar_peek(&done[ci & 1], ((ci >> 1) - 1) & 1) : 1u;
             const uint32_t seg = row_at + p * WX_PACKED;
             uint32_t out[32];
             uint32_t d_dmin, mins;
@@ -442,8 +456,9 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_empty[p]);
             if (++p == WX_SP) { p = 0; ph ^= 1; }
+            p_ready = mbar_peek(&p_full[p], ph);
             // (ci - 2 done: the epilogue has read ci - 4, whose header is overwritten below)
-            if (ci > 1 && !mbar_wait_warp(&done[ci & 1], ((ci >> 1) - 1) & 1, a.status)) break;
+            if (!__all_sync(0xffffffffu, free_ahead != 0) && !mbar_wait_warp(&done[ci & 1], ((ci >> 1) - 1) & 1, a.status)) break;
             uint8_t* hd = reinterpret_cast<uint8_t*>(sm_hdr + (ci % WX_HDR) * WX_ROWS + q * 32 + lane);
             if (slot == 0) *reinterpret_cast<uint32_t*>(hd) = d_dmin;
             *reinterpret_cast<uint16_t*>(hd + 4 + 2 * slot) = (uint16_t)mins;
@@ -459,11 +474,11 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-template <bool SWIGLU>
+template <bool SWIGLU, bool SPLIT>
 static int launch_wx(const WxArgs& a, int64_t rows) {
     static bool configured = false;
     if (!configured) {
-        B200_CUDA(cudaFuncSetAttribute(wx_kernel<SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, WX_SMEM));
+        B200_CUDA(cudaFuncSetAttribute(wx_kernel<SWIGLU, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, WX_SMEM));
         configured = true;
     }
     const int64_t most = (rows / WX_CAP + std::min<int64_t>(a.ne, rows)) * a.n_tiles * a.k_splits;      // an expert's last tile may be short
@@ -477,7 +492,7 @@ static int launch_wx(const WxArgs& a, int64_t rows) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    B200_CUDA(cudaLaunchKernelEx(&cfg, wx_kernel<SWIGLU>, a));
+    B200_CUDA(cudaLaunchKernelEx(&cfg, wx_kernel<SWIGLU, SPLIT>, a));
     ++g_kernel_launches;
     return B200_OK;
 }
@@ -509,7 +524,7 @@ int moe_exact_forward(const float* x, const int32_t* grouped, const int32_t* off
         B200_LAUNCH_CHECK("wx_split_kernel");
         a.c = down ? y : act;
         a.N = Nd; a.K = Kd; a.n_tiles = ceil_div(Nd, tile); a.per_split = Kd / 256;
-        rc = down ? launch_wx<false>(a, NK) : launch_wx<true>(a, NK);
+        rc = down ? launch_wx<false, false>(a, NK) : launch_wx<true, false>(a, NK);
         if (rc) return rc;
     }
     return B200_OK;
@@ -540,7 +555,7 @@ int linear_exact(const float* x, const void* w, float* y, int M, int K, int N) {
     B200_REQUIRE(a.status, "linear_exact: status word allocation failed");
     wx_split_kernel<<<(unsigned)ceil_div(M * chunks, 8), 256, 0, stream()>>>(x, nullptr, 1, M, K, cols, aux);
     B200_LAUNCH_CHECK("wx_split_kernel");
-    if ((rc = launch_wx<false>(a, M))) return rc;
+    if ((rc = launch_wx<false, true>(a, M))) return rc;
     return part ? splitk_reduce(a.c, y, a.k_splits, a.split_stride, M, N, N) : B200_OK;
 }
 
