@@ -479,8 +479,54 @@ __global__ void __launch_bounds__(256) residual_rmsnorm_kernel(float* __restrict
     const int64_t r = blockIdx.x;
     float* xr = x + r * dim;
     const float* yr = y + r * dim;
-    float v[RRN_PER];
     double ss = 0.0;
+    float* o = out + r * dim;
+    auto inverse = [&]() {
+        ss = block_sum_d(ss, red);
+        const double inv_d = 1.0 / sqrt(ss / (double)dim + (double)eps);
+        return isfinite(inv_d) ? (float)inv_d : 0.0f;
+    };
+    auto clamp = [](float f) { return fminf(fmaxf(f, -65504.0f), 65504.0f); };
+    if (gridDim.x >= 1024 && ((uintptr_t)x | (uintptr_t)y | (uintptr_t)w | (uintptr_t)out | (uintptr_t)out16) % 16 == 0 && dim % 4 == 0) {
+        // four neighbours per access, every load of the row under way at once (4096 x 1536: 22.4 -> 19.9 us); a few
+        // hundred rows are latency, which the narrow form spreads over more threads (301 rows: 0.2 us the other way)
+        float4 v[RRN_PER / 4], d4[RRN_PER / 4];
+#pragma unroll
+        for (int j = 0; j < RRN_PER / 4; ++j) {
+            const int i = 4 * (j * 256 + threadIdx.x);
+            v[j] = d4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < dim) {
+                v[j] = *reinterpret_cast<const float4*>(xr + i);
+                d4[j] = *reinterpret_cast<const float4*>(yr + i);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < RRN_PER / 4; ++j) {
+            const int i = 4 * (j * 256 + threadIdx.x);
+            v[j] = make_float4(v[j].x + d4[j].x * s, v[j].y + d4[j].y * s, v[j].z + d4[j].z * s, v[j].w + d4[j].w * s);
+            if (i < dim) *reinterpret_cast<float4*>(xr + i) = v[j];
+            ss += (double)v[j].x * (double)v[j].x;
+            ss += (double)v[j].y * (double)v[j].y;
+            ss += (double)v[j].z * (double)v[j].z;
+            ss += (double)v[j].w * (double)v[j].w;
+        }
+        const float inv = inverse();
+#pragma unroll
+        for (int j = 0; j < RRN_PER / 4; ++j) {
+            const int i = 4 * (j * 256 + threadIdx.x);
+            if (i < dim) {
+                const float4 wv = *reinterpret_cast<const float4*>(w + i);
+                const float4 f = make_float4(v[j].x * inv * wv.x, v[j].y * inv * wv.y, v[j].z * inv * wv.z, v[j].w * inv * wv.w);
+                *reinterpret_cast<float4*>(o + i) = f;
+                if (out16) {
+                    const __half2 h[2] = {__floats2half2_rn(clamp(f.x), clamp(f.y)), __floats2half2_rn(clamp(f.z), clamp(f.w))};
+                    *reinterpret_cast<uint2*>(out16 + r * dim + i) = *reinterpret_cast<const uint2*>(h);
+                }
+            }
+        }
+        return;
+    }
+    float v[RRN_PER];
 #pragma unroll
     for (int j = 0; j < RRN_PER; ++j) {
         const int i = j * 256 + threadIdx.x;
@@ -491,17 +537,14 @@ __global__ void __launch_bounds__(256) residual_rmsnorm_kernel(float* __restrict
             ss += (double)v[j] * (double)v[j];
         }
     }
-    ss = block_sum_d(ss, red);
-    const double inv_d = 1.0 / sqrt(ss / (double)dim + (double)eps);
-    const float inv = isfinite(inv_d) ? (float)inv_d : 0.0f;
-    float* o = out + r * dim;
+    const float inv = inverse();
 #pragma unroll
     for (int j = 0; j < RRN_PER; ++j) {
         const int i = j * 256 + threadIdx.x;
         if (i < dim) {
             const float r2 = v[j] * inv * w[i];
             o[i] = r2;
-            if (out16) out16[r * dim + i] = __float2half_rn(fminf(fmaxf(r2, -65504.0f), 65504.0f));
+            if (out16) out16[r * dim + i] = __float2half_rn(clamp(r2));
         }
     }
 }
