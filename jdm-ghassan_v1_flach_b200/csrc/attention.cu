@@ -11,6 +11,7 @@
 // running (max, sum) per query head so no [H, len] score buffer is needed; the
 // caller's `scratch` argument is accepted and unused.
 #include <algorithm>
+#include <climits>
 
 #include <mutex>
 
@@ -297,23 +298,29 @@ template <int EPL>
 __global__ void __launch_bounds__(ATT_WARPS * 32)
 attn_prefill_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                     float* __restrict__ out, float* __restrict__ probs, int T, int H, int KV, int hd,
-                    float scale, int window, const int32_t* __restrict__ seg) {
+                    float scale, int window, const int32_t* __restrict__ seg, const int32_t* __restrict__ off, int below) {
     __shared__ float sm_o[ATT_WARPS][EPL * 32];
     __shared__ float sm_ml[ATT_WARPS][2];
     __shared__ float s_final[2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
     const int kvh = h / (H / KV);
+    int64_t row0 = (int64_t)b * T;
+    if (off) {                              // sequences of different lengths, packed; those from `below` steps on are not
+        row0 = off[b];                      // this launch's
+        T = off[b + 1] - off[b];
+        if (t >= T || T >= below) return;
+    }
     const int j0 = window > 0 ? max(0, t - window + 1) : 0;
-    const int32_t seg_t = seg ? seg[(int64_t)b * T + t] : 0;
+    const int32_t seg_t = seg ? seg[row0 + t] : 0;
     float qv[EPL], o[EPL];
-    load_row<EPL, false>(q, (((int64_t)b * T + t) * H + h) * hd, lane, qv);
+    load_row<EPL, false>(q, ((row0 + t) * H + h) * hd, lane, qv);
 #pragma unroll
     for (int i = 0; i < EPL; ++i) o[i] = 0.0f;
     float m = -INFINITY, l = 0.0f;
     for (int j = j0 + warp; j <= t; j += ATT_WARPS) {
-        if (seg && seg_t >= 0 && seg[(int64_t)b * T + j] != seg_t) continue;
-        const int64_t off = (((int64_t)b * T + j) * KV + kvh) * hd;
+        if (seg && seg_t >= 0 && seg[row0 + j] != seg_t) continue;
+        const int64_t off = ((row0 + j) * KV + kvh) * hd;
         float kv[EPL], vv[EPL];
         load_row<EPL, false>(k, off, lane, kv);
         load_row<EPL, false>(v, off, lane, vv);
@@ -347,7 +354,7 @@ attn_prefill_kernel(const float* __restrict__ q, const float* __restrict__ k, co
             for (int i = 0; i < EPL; ++i) acc[i] += sm_o[w][lane * EPL + i] * c;
         }
         const float inv = ll > 0.0f ? 1.0f / ll : 0.0f;
-        float* dst = out + (((int64_t)b * T + t) * H + h) * hd;
+        float* dst = out + ((row0 + t) * H + h) * hd;
 #pragma unroll
         for (int i = 0; i < EPL; ++i) dst[lane * EPL + i] = acc[i] * inv;
         if (lane == 0) { s_final[0] = mm; s_final[1] = inv; }
@@ -360,9 +367,9 @@ attn_prefill_kernel(const float* __restrict__ q, const float* __restrict__ k, co
         if (j < j0 || j > t) pr[j] = 0.0f;
     for (int j = j0 + warp; j <= t; j += ATT_WARPS) {
         float p = 0.0f;
-        if (!(seg && seg_t >= 0 && seg[(int64_t)b * T + j] != seg_t)) {
+        if (!(seg && seg_t >= 0 && seg[row0 + j] != seg_t)) {
             float kv[EPL];
-            load_row<EPL, false>(k, (((int64_t)b * T + j) * KV + kvh) * hd, lane, kv);
+            load_row<EPL, false>(k, ((row0 + j) * KV + kvh) * hd, lane, kv);
             float s = 0.0f;
 #pragma unroll
             for (int i = 0; i < EPL; ++i) s += qv[i] * kv[i];
@@ -378,11 +385,47 @@ attn_prefill_kernel(const float* __restrict__ q, const float* __restrict__ k, co
 // attention_flash.cu
 namespace b200 {
 int attention_flash(const float* q, const float* k, const float* v, float* out, int B, int T, int H, int KV, int hd,
-                    float scale, int window, const int32_t* seg);
-constexpr int FLASH_MIN_T = 128;
+                    float scale, int window, const int32_t* seg, const int32_t* off);
 }  // namespace b200
 
 using namespace b200;
+
+namespace b200 {
+
+// Causal attention inside each of B packed sequences (off: device, host_off: host [B + 1] first rows): each sequence by
+// the kernel that takes its length, all of a kernel's in one launch (one after the other, 64 short prompts were 256
+// launches of 10 us and twelve long ones 48 of 48 us, each a fraction of the SMs).
+int attention_ragged(const float* q, const float* k, const float* v, float* out, const int32_t* off, const int32_t* host_off,
+                     int B, int H, int KV, int hd, float scale) {
+    int rc = check_hd("attention_ragged", hd);
+    if (rc) return rc;
+    const bool flash = (hd == 64 || hd == 128) &&
+                       (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) == 0;
+    int longest = 0, short_longest = 0;
+    for (int b = 0; b < B; ++b) {
+        const int n = host_off[b + 1] - host_off[b];
+        longest = std::max(longest, n);
+        if (n < FLASH_MIN_T || !flash) short_longest = std::max(short_longest, n);
+    }
+    for (int b0 = 0; b0 < B; b0 += 32768) {
+        const int nb = std::min(B - b0, 32768);
+        if (flash && longest >= FLASH_MIN_T && (rc = attention_flash(q, k, v, out, nb, longest, H, KV, hd, scale, 0, nullptr, off + b0)))
+            return rc;
+        if (short_longest == 0) continue;
+        const dim3 grid(short_longest, H, nb);
+        const int below = flash ? FLASH_MIN_T : INT_MAX, threads = ATT_WARPS * 32;
+        switch (hd / 32) {
+            case 1: attn_prefill_kernel<1><<<grid, threads, 0, stream()>>>(q, k, v, out, nullptr, 0, H, KV, hd, scale, 0, nullptr, off + b0, below); break;
+            case 2: attn_prefill_kernel<2><<<grid, threads, 0, stream()>>>(q, k, v, out, nullptr, 0, H, KV, hd, scale, 0, nullptr, off + b0, below); break;
+            case 4: attn_prefill_kernel<4><<<grid, threads, 0, stream()>>>(q, k, v, out, nullptr, 0, H, KV, hd, scale, 0, nullptr, off + b0, below); break;
+            default: attn_prefill_kernel<8><<<grid, threads, 0, stream()>>>(q, k, v, out, nullptr, 0, H, KV, hd, scale, 0, nullptr, off + b0, below); break;
+        }
+        B200_LAUNCH_CHECK("attn_prefill_kernel");
+    }
+    return B200_OK;
+}
+
+}  // namespace b200
 
 extern "C" {
 
@@ -436,13 +479,13 @@ int b200_attention_forward_ex(const float* q, const float* k, const float* v, fl
     auto aligned16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (!probs && T >= FLASH_MIN_T && (hd == 64 || hd == 128) && aligned16(q) && aligned16(k) && aligned16(v) &&
         aligned16(out))
-        return attention_flash(q, k, v, out, B, T, H, KV, hd, scale, window, segment_ids);
+        return attention_flash(q, k, v, out, B, T, H, KV, hd, scale, window, segment_ids, nullptr);
     const dim3 grid(T, H, B);
     switch (hd / 32) {
-        case 1: attn_prefill_kernel<1><<<grid, ATT_WARPS * 32, 0, stream()>>>(q, k, v, out, probs, T, H, KV, hd, scale, window, segment_ids); break;
-        case 2: attn_prefill_kernel<2><<<grid, ATT_WARPS * 32, 0, stream()>>>(q, k, v, out, probs, T, H, KV, hd, scale, window, segment_ids); break;
-        case 4: attn_prefill_kernel<4><<<grid, ATT_WARPS * 32, 0, stream()>>>(q, k, v, out, probs, T, H, KV, hd, scale, window, segment_ids); break;
-        default: attn_prefill_kernel<8><<<grid, ATT_WARPS * 32, 0, stream()>>>(q, k, v, out, probs, T, H, KV, hd, scale, window, segment_ids); break;
+        case 1: attn_prefill_kernel<1><<<grid, ATT_WARPS * 32, 0, stream()>>>(q, k, v, out, probs, T, H, KV, hd, scale, window, segment_ids, nullptr, 0); break;
+        case 2: attn_prefill_kernel<2><<<grid, ATT_WARPS * 32, 0, stream()>>>(q, k, v, out, probs, T, H, KV, hd, scale, window, segment_ids, nullptr, 0); break;
+        case 4: attn_prefill_kernel<4><<<grid, ATT_WARPS * 32, 0, stream()>>>(q, k, v, out, probs, T, H, KV, hd, scale, window, segment_ids, nullptr, 0); break;
+        default: attn_prefill_kernel<8><<<grid, ATT_WARPS * 32, 0, stream()>>>(q, k, v, out, probs, T, H, KV, hd, scale, window, segment_ids, nullptr, 0); break;
     }
     B200_LAUNCH_CHECK("attn_prefill_kernel");
     return B200_OK;

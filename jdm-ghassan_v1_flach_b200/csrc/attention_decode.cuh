@@ -5,6 +5,8 @@
 
 namespace b200 {
 
+constexpr int FLASH_MIN_T = 128;             // steps from which a prompt takes the tensor-core kernel (attention_flash.cu)
+
 struct DecodeMmaArgs {
     const float* q = nullptr;                // [batch, H, hd]
     const uint16_t *kc = nullptr, *vc = nullptr;   // fp16 [rows, KV*hd]

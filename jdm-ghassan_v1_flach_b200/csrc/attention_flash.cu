@@ -15,6 +15,7 @@
 // transposing ones.  Scores and outputs live in mma.sync.m16n8k16 accumulator fragments,
 // and the score fragment of a 16-key slice is reused directly as the A operand of the
 // probability-times-value product.
+#include "attention_decode.cuh"
 #include <cuda_fp16.h>
 
 #include "mma_tile.cuh"
@@ -43,7 +44,7 @@ template <int HD>
 __global__ void __launch_bounds__(FA_THREADS)
 attn_flash_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                   float* __restrict__ out, int T, int H, int KV, float scale, int window,
-                  const int32_t* __restrict__ seg) {
+                  const int32_t* __restrict__ seg, const int32_t* __restrict__ off) {
     constexpr int LDK = HD + 8;
     __shared__ __align__(16) __half Ks[FA_BN * LDK];
     __shared__ __align__(16) __half Vs[FA_BN * LDK];
@@ -54,10 +55,15 @@ attn_flash_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     // its position, and the heavy ones should not be what the last wave is made of
     const int q0 = (gridDim.x - 1 - blockIdx.x) * FA_BM, h = blockIdx.y, b = blockIdx.z;
     const int kvh = h / (H / KV);
-    const int64_t qs = (int64_t)T * H * HD, kvs = (int64_t)T * KV * HD;
-    const float* qb = q + b * qs + (int64_t)h * HD;
-    const float* kb = k + b * kvs + (int64_t)kvh * HD;
-    const float* vb = v + b * kvs + (int64_t)kvh * HD;
+    int64_t row0 = (int64_t)b * T;
+    if (off) {                              // sequences of different lengths, packed; the short ones are not this kernel's
+        row0 = off[b];
+        T = off[b + 1] - off[b];
+        if (T < FLASH_MIN_T || q0 >= T) return;
+    }
+    const float* qb = q + row0 * H * HD + (int64_t)h * HD;
+    const float* kb = k + row0 * KV * HD + (int64_t)kvh * HD;
+    const float* vb = v + row0 * KV * HD + (int64_t)kvh * HD;
     const int r0 = q0 + warp * 16 + g, r1 = r0 + 8;        // this lane's two query rows
     const float qscale = scale * 1.44269504088896f;         // scores in log2 units: p = 2^(s - m)
 
@@ -80,8 +86,8 @@ attn_flash_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
         qa[ks][2] = pack_half2(x2.x * qscale, x2.y * qscale);
         qa[ks][3] = pack_half2(x3.x * qscale, x3.y * qscale);
     }
-    const int32_t seg0 = (seg && r0 < T) ? seg[(int64_t)b * T + r0] : -1;
-    const int32_t seg1 = (seg && r1 < T) ? seg[(int64_t)b * T + r1] : -1;
+    const int32_t seg0 = (seg && r0 < T) ? seg[row0 + r0] : -1;
+    const int32_t seg1 = (seg && r1 < T) ? seg[row0 + r1] : -1;
     const int lo0 = window > 0 ? max(0, r0 - window + 1) : 0, lo1 = window > 0 ? max(0, r1 - window + 1) : 0;
 
     float o[HD / 8][4];
@@ -103,7 +109,7 @@ attn_flash_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
             *reinterpret_cast<uint2*>(&Ks[key * LDK + c]) = make_uint2(pack_half2(kk.x, kk.y), pack_half2(kk.z, kk.w));
             *reinterpret_cast<uint2*>(&Vs[key * LDK + c]) = make_uint2(pack_half2(vv.x, vv.y), pack_half2(vv.z, vv.w));
         }
-        if (threadIdx.x < FA_BN) s_seg[threadIdx.x] = (seg && kv0 + threadIdx.x < T) ? seg[(int64_t)b * T + kv0 + threadIdx.x] : 0;
+        if (threadIdx.x < FA_BN) s_seg[threadIdx.x] = (seg && kv0 + threadIdx.x < T) ? seg[row0 + kv0 + threadIdx.x] : 0;
         __syncthreads();
 
         // tiles entirely in this warp's future (or before its window) contribute nothing
@@ -188,7 +194,7 @@ attn_flash_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
     const float inv0 = l0 > 0.0f ? 1.0f / l0 : 0.0f, inv1 = l1 > 0.0f ? 1.0f / l1 : 0.0f;
-    float* ob = out + b * qs + (int64_t)h * HD;
+    float* ob = out + row0 * H * HD + (int64_t)h * HD;
 #pragma unroll
     for (int d = 0; d < HD / 8; ++d) {
         const int c = d * 8 + 2 * t4;
@@ -197,12 +203,13 @@ attn_flash_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     }
 }
 
-// Returns B200_EUNSUPPORTED for head sizes it has no instance for.
+// Returns B200_EUNSUPPORTED for head sizes it has no instance for.  off (optional, device [B + 1]): first row of each
+// sequence, T then the longest one's steps.
 int attention_flash(const float* q, const float* k, const float* v, float* out, int B, int T, int H, int KV, int hd,
-                    float scale, int window, const int32_t* seg) {
+                    float scale, int window, const int32_t* seg, const int32_t* off) {
     const dim3 grid(ceil_div(T, FA_BM), H, B);
-    if (hd == 128) attn_flash_kernel<128><<<grid, FA_THREADS, 0, stream()>>>(q, k, v, out, T, H, KV, scale, window, seg);
-    else if (hd == 64) attn_flash_kernel<64><<<grid, FA_THREADS, 0, stream()>>>(q, k, v, out, T, H, KV, scale, window, seg);
+    if (hd == 128) attn_flash_kernel<128><<<grid, FA_THREADS, 0, stream()>>>(q, k, v, out, T, H, KV, scale, window, seg, off);
+    else if (hd == 64) attn_flash_kernel<64><<<grid, FA_THREADS, 0, stream()>>>(q, k, v, out, T, H, KV, scale, window, seg, off);
     else return fail(B200_EUNSUPPORTED, "attention_flash: head_dim %d", hd);
     B200_LAUNCH_CHECK("attn_flash_kernel");
     return B200_OK;

@@ -27,6 +27,10 @@ struct SeqLayout {
     const int32_t* host_off = nullptr;    // host copy of seq_off
 };
 
+// attention.cu: causal attention inside each of B packed sequences.
+int attention_ragged(const float* q, const float* k, const float* v, float* out, const int32_t* off, const int32_t* host_off,
+                     int B, int H, int KV, int hd, float scale);
+
 enum { PRO_NONE = 0, PRO_RMS = 1 };
 enum { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_INPROJ = 2 };
 

@@ -222,6 +222,9 @@ constexpr int RRN_PER = 16;      // row elements a thread keeps in registers: di
 __global__ void residual_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ y, float s,
                                         const float* __restrict__ w, float* __restrict__ out, int dim, float eps,
                                         __half* __restrict__ out16);
+__global__ void residual_rmsnorm4_kernel(float* __restrict__ x, const float* __restrict__ y, float s,
+                                        const float* __restrict__ w, float* __restrict__ out, int dim, float eps,
+                                        __half* __restrict__ out16);
 
 static int enqueue_step(b200_decoder* dec, const int32_t* tokens, int32_t* next) {
     const int B = dec->batch, d = dec->d;
@@ -487,45 +490,6 @@ __global__ void __launch_bounds__(256) residual_rmsnorm_kernel(float* __restrict
         return isfinite(inv_d) ? (float)inv_d : 0.0f;
     };
     auto clamp = [](float f) { return fminf(fmaxf(f, -65504.0f), 65504.0f); };
-    if (gridDim.x >= 1024 && ((uintptr_t)x | (uintptr_t)y | (uintptr_t)w | (uintptr_t)out | (uintptr_t)out16) % 16 == 0 && dim % 4 == 0) {
-        // four neighbours per access, every load of the row under way at once (4096 x 1536: 22.4 -> 19.9 us); a few
-        // hundred rows are latency, which the narrow form spreads over more threads (301 rows: 0.2 us the other way)
-        float4 v[RRN_PER / 4], d4[RRN_PER / 4];
-#pragma unroll
-        for (int j = 0; j < RRN_PER / 4; ++j) {
-            const int i = 4 * (j * 256 + threadIdx.x);
-            v[j] = d4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < dim) {
-                v[j] = *reinterpret_cast<const float4*>(xr + i);
-                d4[j] = *reinterpret_cast<const float4*>(yr + i);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < RRN_PER / 4; ++j) {
-            const int i = 4 * (j * 256 + threadIdx.x);
-            v[j] = make_float4(v[j].x + d4[j].x * s, v[j].y + d4[j].y * s, v[j].z + d4[j].z * s, v[j].w + d4[j].w * s);
-            if (i < dim) *reinterpret_cast<float4*>(xr + i) = v[j];
-            ss += (double)v[j].x * (double)v[j].x;
-            ss += (double)v[j].y * (double)v[j].y;
-            ss += (double)v[j].z * (double)v[j].z;
-            ss += (double)v[j].w * (double)v[j].w;
-        }
-        const float inv = inverse();
-#pragma unroll
-        for (int j = 0; j < RRN_PER / 4; ++j) {
-            const int i = 4 * (j * 256 + threadIdx.x);
-            if (i < dim) {
-                const float4 wv = *reinterpret_cast<const float4*>(w + i);
-                const float4 f = make_float4(v[j].x * inv * wv.x, v[j].y * inv * wv.y, v[j].z * inv * wv.z, v[j].w * inv * wv.w);
-                *reinterpret_cast<float4*>(o + i) = f;
-                if (out16) {
-                    const __half2 h[2] = {__floats2half2_rn(clamp(f.x), clamp(f.y)), __floats2half2_rn(clamp(f.z), clamp(f.w))};
-                    *reinterpret_cast<uint2*>(out16 + r * dim + i) = *reinterpret_cast<const uint2*>(h);
-                }
-            }
-        }
-        return;
-    }
     float v[RRN_PER];
 #pragma unroll
     for (int j = 0; j < RRN_PER; ++j) {
@@ -545,6 +509,59 @@ __global__ void __launch_bounds__(256) residual_rmsnorm_kernel(float* __restrict
             const float r2 = v[j] * inv * w[i];
             o[i] = r2;
             if (out16) out16[r * dim + i] = __float2half_rn(clamp(r2));
+        }
+    }
+}
+// The same by 16-byte accesses, for pointers and rows of that alignment.  From 1024 rows on: 4096 x 1536 22.4 -> 19.9 us;
+// fewer rows are latency, and this form's longer one (64 rows: 3.0 us there, 5.3 here).
+__global__ void __launch_bounds__(256) residual_rmsnorm4_kernel(float* __restrict__ x, const float* __restrict__ y, float s,
+                                                               const float* __restrict__ w, float* __restrict__ out,
+                                                               int dim, float eps, __half* __restrict__ out16) {
+    __shared__ double red[32];
+    const int64_t r = blockIdx.x;
+    float* xr = x + r * dim;
+    const float* yr = y + r * dim;
+    double ss = 0.0;
+    float* o = out + r * dim;
+    auto inverse = [&]() {
+        ss = block_sum_d(ss, red);
+        const double inv_d = 1.0 / sqrt(ss / (double)dim + (double)eps);
+        return isfinite(inv_d) ? (float)inv_d : 0.0f;
+    };
+    auto clamp = [](float f) { return fminf(fmaxf(f, -65504.0f), 65504.0f); };
+    // four neighbours per access, every load of the row under way at once
+    float4 v[RRN_PER / 4], d4[RRN_PER / 4];
+#pragma unroll
+    for (int j = 0; j < RRN_PER / 4; ++j) {
+        const int i = 4 * (j * 256 + threadIdx.x);
+        v[j] = d4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < dim) {
+            v[j] = *reinterpret_cast<const float4*>(xr + i);
+            d4[j] = *reinterpret_cast<const float4*>(yr + i);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < RRN_PER / 4; ++j) {
+        const int i = 4 * (j * 256 + threadIdx.x);
+        v[j] = make_float4(v[j].x + d4[j].x * s, v[j].y + d4[j].y * s, v[j].z + d4[j].z * s, v[j].w + d4[j].w * s);
+        if (i < dim) *reinterpret_cast<float4*>(xr + i) = v[j];
+        ss += (double)v[j].x * (double)v[j].x;
+        ss += (double)v[j].y * (double)v[j].y;
+        ss += (double)v[j].z * (double)v[j].z;
+        ss += (double)v[j].w * (double)v[j].w;
+    }
+    const float inv = inverse();
+#pragma unroll
+    for (int j = 0; j < RRN_PER / 4; ++j) {
+        const int i = 4 * (j * 256 + threadIdx.x);
+        if (i < dim) {
+            const float4 wv = *reinterpret_cast<const float4*>(w + i);
+            const float4 f = make_float4(v[j].x * inv * wv.x, v[j].y * inv * wv.y, v[j].z * inv * wv.z, v[j].w * inv * wv.w);
+            *reinterpret_cast<float4*>(o + i) = f;
+            if (out16) {
+                const __half2 h[2] = {__floats2half2_rn(clamp(f.x), clamp(f.y)), __floats2half2_rn(clamp(f.z), clamp(f.w))};
+                *reinterpret_cast<uint2*>(out16 + r * dim + i) = *reinterpret_cast<const uint2*>(h);
+            }
         }
     }
 }
@@ -605,8 +622,12 @@ static int prefill(b200_decoder* dec, const int32_t* tokens, int T, int32_t* nex
     // x += res_mult * y followed by the next norm; fused when the row fits the registers
     auto residual_norm = [&](const float* norm_w) -> int {
         if (norm_w && d <= RRN_PER * 256) {
-            residual_rmsnorm_kernel<<<(unsigned)NT, 256, 0, st>>>(x, y, dec->res_mult, norm_w, xb, d, dec->eps,
-                                                                  want16 ? xb16 : nullptr);
+            __half* x16 = want16 ? xb16 : nullptr;
+            const uintptr_t at16 = (uintptr_t)x | (uintptr_t)y | (uintptr_t)norm_w | (uintptr_t)xb | (uintptr_t)x16;
+            if (NT >= 1024 && d % 4 == 0 && at16 % 16 == 0)
+                residual_rmsnorm4_kernel<<<(unsigned)NT, 256, 0, st>>>(x, y, dec->res_mult, norm_w, xb, d, dec->eps, x16);
+            else
+                residual_rmsnorm_kernel<<<(unsigned)NT, 256, 0, st>>>(x, y, dec->res_mult, norm_w, xb, d, dec->eps, x16);
             B200_LAUNCH_CHECK("residual_rmsnorm_kernel");
             return B200_OK;
         }
@@ -641,13 +662,7 @@ static int prefill(b200_decoder* dec, const int32_t* tokens, int T, int32_t* nex
                 kv_prefill_packed_kernel<<<dim3(ceil_div(kvd, 256), (unsigned)NT), 256, 0, st>>>(
                     k, v, w.k_pages, w.v_pages, page_table, lay->seq, lay->pos, dec->max_pages, dec->page, kvd);
                 B200_LAUNCH_CHECK("kv_prefill_packed_kernel");
-                // causal attention inside each sequence: one call per sequence on its rows
-                for (int b = 0; b < B; ++b) {
-                    const int64_t r0 = lay->host_off[b];
-                    STEP(b200_attention_forward_ex(q + r0 * qd, k + r0 * kvd, v + r0 * kvd, at + r0 * qd, nullptr, 1,
-                                                   lay->host_off[b + 1] - lay->host_off[b], dec->H, dec->KV, dec->hd,
-                                                   dec->attn_scale, 0, nullptr));
-                }
+                STEP(attention_ragged(q, k, v, at, lay->seq_off, lay->host_off, B, dec->H, dec->KV, dec->hd, dec->attn_scale));
             }
             STEP(lin(at, w.wo, y, qd, d));
         }
