@@ -1,6 +1,7 @@
 // Fused decode-step kernels, part 1: the streamed single-matrix GEMV (RMSNorm
-// prologue; store / residual / Mamba in_proj+conv epilogues) and the Mamba-2 state
-// update that also emits the gated-norm statistics.
+// prologue; store / residual / Mamba in_proj+conv epilogues) for fp32 weights - fp16 and
+// packed ones run on the digit engine (decode_gemv.cu) - and the Mamba-2 state update that
+// also emits the gated-norm statistics.
 //
 // These fuse across the reference's op boundaries (rmsnorm_forward -> linear ->
 // add_inplace in Generator::decode_step_logits, inference/generator.cpp:253-436),

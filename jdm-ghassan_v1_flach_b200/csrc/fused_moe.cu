@@ -1,5 +1,5 @@
-// Fused decode-step kernels, part 2: the MoE layer for a few tokens in three
-// streamed kernels -
+// Fused decode-step kernels, part 2: the MoE layer for a few tokens over fp16 and fp32
+// experts (packed ones: decode_moe.cu) in three streamed kernels -
 //   phase 1  router logits in the reference's exact fp32 order + the shared
 //            expert's gate/up (SwiGLU activation); the CTA that finishes the last
 //            router tile does softmax / top-K / mixture weights

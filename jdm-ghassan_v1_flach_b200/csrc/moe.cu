@@ -757,7 +757,7 @@ int moe_forward(const float* x, const float* router_w, const float* router_bias,
     }
     // A decode batch: at most MOE_UNITS_MAX_ROWS rows per expert on average.  The experts'
     // rows would leave the 128-row tensor-core tiles nearly empty; they run as weight streams
-    // shared by their tokens instead (moe_units.cu).
+    // shared by their tokens instead (moe_exact.cu, moe_units.cu).
     if (N > 8 && N * K <= (int64_t)MOE_UNITS_MAX_ROWS * ne && kind != KIND_F32 && !s_gate && !s_up && !s_act && aligned16(x) &&
         aligned16(out) && aligned16(gates) && aligned16(ups) && aligned16(downs) && d % 8 == 0 &&
         (kind != 3 || (d % 256 == 0 && E % 256 == 0)) && ne <= 256 &&

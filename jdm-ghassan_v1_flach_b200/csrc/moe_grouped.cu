@@ -164,7 +164,7 @@ int moe_forward_grouped(const float* x, const float* router_w, const float* rout
 // ===========================================================================
 // A decode batch (more tokens than the token-major kernels take, fewer than fill the
 // tensor-core tiles of every expert): routing and permutation as above, the routed experts
-// through moe_units.cu, the shared expert as a GEMM on the side stream, the same k-ordered
+// through moe_exact.cu or moe_units.cu, the shared expert as a GEMM on the side stream, the same k-ordered
 // combination.
 // ===========================================================================
 int moe_combine(const float* y, const int32_t* inv, const float* w, float* out, int64_t N, int d, int K, bool accumulate);
