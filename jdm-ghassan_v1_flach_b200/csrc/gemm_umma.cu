@@ -564,6 +564,8 @@ int make_packed_map(CUtensorMap* out, const void* base, int64_t rows, int64_t ro
 // c[m, n] = sum over the splits, in split order (deterministic), of the partial products.
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ part, float* __restrict__ c, int splits,
                                                            int64_t stride, int M, int N, int64_t ldc) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int64_t total = (int64_t)M * N;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t m = i / N, o = m * ldc + (i - m * N);
@@ -575,10 +577,8 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
 
 int splitk_reduce(const float* part, float* c, int splits, int64_t stride, int M, int N, int64_t ldc) {
     const int64_t total = (int64_t)M * N;
-    splitk_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div64(total, 256), (int64_t)num_sms() * 8), 256, 0, stream()>>>(
-        part, c, splits, stride, M, N, ldc);
-    B200_LAUNCH_CHECK("splitk_reduce_kernel");
-    return B200_OK;
+    return launch_short(splitk_reduce_kernel, dim3((unsigned)std::min<int64_t>(ceil_div64(total, 256), (int64_t)num_sms() * 8)),
+                        dim3(256), part, c, splits, stride, M, N, ldc);
 }
 
 template <int EPI>

@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();
     const int mine = ((int)blockIdx.x < total ? total - (int)blockIdx.x + (int)gridDim.x - 1 : 0) / (int)gridDim.x;
     // every role walks the same tiles; sb0 .. sb1: a tile's range of K in units of 256
     auto range = [&](const WtTile& w, int& sb0, int& sb1) {

@@ -128,6 +128,8 @@ mamba_step_scan_stream_kernel(const float* __restrict__ bc, const float* __restr
                               const float* __restrict__ dt_bias, const float* __restrict__ a_log,
                               const float* __restrict__ Dv, float* __restrict__ ssm_state, float* __restrict__ y,
                               int dt_stride, MambaDims p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rows = p.n_heads * p.d_head;
     const int row0 = (blockIdx.x * SCAN_WARPS + warp) * SCAN_ROWS;
@@ -179,6 +181,8 @@ __global__ void __launch_bounds__(256)
 mamba_conv_step_kernel(const float* __restrict__ proj, const float* __restrict__ conv_w,
                        const float* __restrict__ conv_b, float* __restrict__ conv_state, float* __restrict__ bc,
                        int M, MambaDims p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)M * p.conv_dim) return;
     const int m = (int)(i / p.conv_dim), c = (int)(i - (int64_t)m * p.conv_dim);
@@ -559,17 +563,19 @@ int mamba2_step(const float* x, const void* w_in, const float* conv_w, const flo
         rc = linear(x, w_in, kind, proj, batch, p.d, p.proj);
         if (rc) return rc;
         const int64_t items = (int64_t)batch * p.conv_dim;
-        mamba_conv_step_kernel<<<(unsigned)ceil_div64(items, 256), 256, 0, stream()>>>(proj, conv_w, conv_b, conv_state,
-                                                                                       bc, batch, p);
-        B200_LAUNCH_CHECK("mamba_conv_step_kernel");
+        rc = launch_short(mamba_conv_step_kernel, dim3((unsigned)ceil_div64(items, 256)), dim3(256), proj, conv_w, conv_b, conv_state,
+                          bc, batch, p);
+        if (rc) return rc;
         if (p.d_state == 128 && p.d_head % SCAN_ROWS == 0 && (reinterpret_cast<uintptr_t>(ssm_state) & 15) == 0 &&
             (reinterpret_cast<uintptr_t>(bc) & 15) == 0 && p.conv_dim % 4 == 0 && p.d_inner % 4 == 0)
-            mamba_step_scan_stream_kernel<<<dim3(ceil_div(rows, SCAN_WARPS * SCAN_ROWS), batch), SCAN_WARPS * 32, 0, stream()>>>(
-                bc, proj + p.d_inner + p.conv_dim, dt_bias, a_log, D, ssm_state, y, p.proj, p);
-        else
+            rc = launch_short(mamba_step_scan_stream_kernel, dim3(ceil_div(rows, SCAN_WARPS * SCAN_ROWS), batch), dim3(SCAN_WARPS * 32),
+                              bc, proj + p.d_inner + p.conv_dim, dt_bias, a_log, D, ssm_state, y, p.proj, p);
+        else {
             mamba_step_scan_kernel<<<dim3(ceil_div(rows, SCAN_WARPS), batch), SCAN_WARPS * 32, 0, stream()>>>(
                 bc, proj + p.d_inner + p.conv_dim, dt_bias, a_log, D, ssm_state, y, p.proj, p);
-        B200_LAUNCH_CHECK("mamba_step_scan_kernel");
+            B200_LAUNCH_CHECK("mamba_step_scan_kernel");
+        }
+        if (rc) return rc;
         launch_gated_norm(y, proj, p.proj, norm_w, y, p.d_inner, p.eps, out_gemm ? y16 : nullptr, batch);
         B200_LAUNCH_CHECK("mamba_gated_norm_kernel");
         if (out_gemm) return linear_a16(y16, w_out, kind, out, batch, p.d_inner, p.d);

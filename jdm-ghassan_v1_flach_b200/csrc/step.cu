@@ -249,9 +249,9 @@ static int enqueue_step(b200_decoder* dec, const int32_t* tokens, int32_t* next)
     auto residual_norm = [&](const float* norm_w) -> int {
         f16_shadow_clear();
         if (d <= RRN_PER * 256) {
-            residual_rmsnorm_kernel<<<(unsigned)B, 256, 0, st>>>(dec->x, dec->proj, dec->res_mult, norm_w, dec->xb, d,
-                                                                dec->eps, rows16 ? dec->xb16 : nullptr);
-            B200_LAUNCH_CHECK("residual_rmsnorm_kernel");
+            const int lrc = launch_short(residual_rmsnorm_kernel, dim3((unsigned)B), dim3(256), dec->x, dec->proj, dec->res_mult,
+                                         norm_w, dec->xb, d, dec->eps, rows16 ? dec->xb16 : nullptr);
+            if (lrc) return lrc;
             if (rows16) f16_shadow_set(dec->xb, dec->xb16, B, d);
             return B200_OK;
         }
@@ -478,6 +478,8 @@ __global__ void last_rows_kernel(const float* __restrict__ src, float* __restric
 __global__ void __launch_bounds__(256) residual_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ y, float s,
                                                                const float* __restrict__ w, float* __restrict__ out,
                                                                int dim, float eps, __half* __restrict__ out16) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ double red[32];
     const int64_t r = blockIdx.x;
     float* xr = x + r * dim;

@@ -70,6 +70,24 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, uint32_t
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Host: a short kernel whose first instruction is pdl_wait(), launched so that it is set up while the kernel before it
+// ends (about a microsecond of a decode step's short kernels each).
+template <typename... P, typename... A>
+static int launch_short(void (*kern)(P...), dim3 grid, dim3 block, const A&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = stream();
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    B200_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+    ++g_kernel_launches;
+    return B200_OK;
+}
+
 // ---- activations in shared memory -------------------------------------------
 // x is stored "unit-major": the 32 activations a 32-weight unit multiplies are
 // contiguous, units are 36 floats apart so that eight lanes reading eight different
