@@ -484,6 +484,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
                 else if (slot == 1) wt_expand<KIND, 1>(seg, out);
                 else if (slot == 2) wt_expand<KIND, 2>(seg, out);
                 else wt_expand<KIND, 3>(seg, out);
+                __syncwarp();                             // every lane has read its row: the stage goes back to TMA
                 if (lane == 0) mbar_arrive(&p_empty[p]);
                 if (++p == S::SP) { p = 0; ph ^= 1; }
                 if (it > 0) ok = mbar_wait_warp(&a_empty[slot], (it - 1) & 1, a.status);
