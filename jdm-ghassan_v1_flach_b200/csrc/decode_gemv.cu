@@ -222,7 +222,8 @@ static int launch_dg(SgArgs a) {
         if (most <= 8)
             for (int G = std::min(most - 1, 4); G >= 1 && !smem; --G) fits(G, 2, SMEM_BUDGET);
         for (int G = std::min(most, 4); G >= 2 && !smem; --G) fits(G, most > G ? 2 : 1, DG_SMEM_MAX);
-        for (int sets = std::min(most, DG_MAX_SETS); sets >= 1 && !smem; --sets) fits(1, sets, DG_SMEM_MAX);
+        // (one set holds a whole share or nothing: a share of several rounds takes two at least, at half the rows if it must)
+        for (int sets = std::min(most, DG_MAX_SETS); sets >= std::min(most, 2) && !smem; --sets) fits(1, sets, DG_SMEM_MAX);
     }
     if (!smem) return fail(B200_EUNSUPPORTED, "stream_gemv: K = %d does not fit the shared-memory staging", a.K);
     auto kern = dg_gemv_kernel<KIND, MT, PRO, EPI>;

@@ -37,6 +37,27 @@ def test_few_token_products(oracle, kind, M, K, N):
     np.testing.assert_allclose(host(y), want, **tol)
 
 
+# Rows so wide that one tile of sixteen fills the shared memory, and more tiles than a round of the CTAs takes.
+@pytest.mark.parametrize("kind,K,M", [(-1, 4096, 1), (-1, 2304, 8), (-1, 5632, 2), (0, 4608, 8), (1, 4352, 8), (2, 4096, 8), (2, 6144, 1),
+                                      (2, 4608, 3), (3, 4608, 8), (3, 10496, 1)])
+def test_few_token_products_of_wide_rows(oracle, kind, K, M):
+    from gpu_util import SUM_ORDER, dev, empty, host, ops
+    N = 2388                                            # of 16 rows: one tile for each of 148 SMs and two over
+    r = np.random.default_rng(K + M)
+    x = r.standard_normal((M, K)).astype(np.float32)
+    w = (r.standard_normal(N * K) * 0.02).astype(np.float32)
+    y = empty((M, N))
+    if kind < 0:
+        w = w.astype(np.float16).reshape(N, K)
+        ops.linear_forward_fp16(dev(x), dev(w.view(np.uint16)), y, M, K, N)
+        want = (x.astype(np.float64) @ w.astype(np.float64).T).astype(np.float32)
+    else:
+        w = oracle.quantize(w, kind)
+        ops.linear_forward_q4(dev(x), dev(w), y, M, K, N, kind)
+        want = oracle.linear_exact(x, w, kind, M, K, N)
+    np.testing.assert_allclose(host(y), want, **SUM_ORDER)
+
+
 # rows around one, two and three token tiles of 192 and around the 16 and 96 rows of a copy
 @pytest.mark.parametrize("kind", [1, 2, 3])
 @pytest.mark.parametrize("M", [33, 96, 97, 192, 193, 385])
