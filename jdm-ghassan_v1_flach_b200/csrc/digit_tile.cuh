@@ -7,7 +7,8 @@
 // weights HBM can deliver in a microsecond.  Here a nibble word needs one AND to become an operand:
 //     x = 2^(e - 30) * sum_j 256^j D_j,   |x| < 2^e,  D_j signed bytes, j = 0 .. 3
 // with e the exponent of the largest of the token's 256 activations (so no activation loses more than
-// 2^-31 of that maximum; the fp16 pairs kept 22 bits of each), and for every 32-weight sub-block one
+// 2^-31 of that maximum; the fp16 pairs kept 22 bits of each; a NaN or an infinity among the 256 makes their
+// scale, and so the token's outputs, NaN), and for every 32-weight sub-block one
 // mma.m16n8k32 gives sum_k q_k D_jk exactly, the eight columns being the four digits of two tokens.
 // The 6-bit scale of the sub-block multiplies the integer (exact: at most 63 * 32 * 240 * 128 * 4 in 31
 // bits), so a super-block ends in one conversion and one multiply-add per digit, and the minimum terms of
@@ -94,20 +95,24 @@ __device__ __forceinline__ void dg_mma_f16k8(float (&c)[4], uint32_t a0, uint32_
                  : "r"(a0), "r"(a1), "r"(b0));
 }
 
+// The scale of a chunk of packed weights is 2^(e - DG_UNIT) and dg_value puts 2^DG_UNIT back on the finished sum: the
+// products and the minimum terms, each larger than their difference, and the digits, each up to 2^10 of its share of the
+// output, do not overflow where the output does not; 2^-90 2^-24 leaves room for a weight's scale above.
+constexpr int DG_UNIT = 24;
+
 // Lane l's eight activations 256 * chunk + 8 l .. of token m (zeros past K), staged by one whole warp.
 // mul: a factor of the token's contribution, folded into the scale (a mixture weight).
 template <int KIND, int MT>
 __device__ __forceinline__ void dg_stage(const DgX<KIND, MT>& xd, int chunk, int m, const float (&v)[8], float mul, int lane) {
-    float mx = 0.0f;
+    uint32_t bits = 0;                                                // of the largest magnitude: a NaN counts as one
 #pragma unroll
-    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
-    uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-    int e = (int)(bits >> 23) - 126;                                  // every |v| < 2^e
-    e = min(max(e, -90), 127);
+    for (int i = 0; i < 8; ++i) bits = max(bits, __float_as_uint(v[i]) & 0x7FFFFFFFu);
+    bits = __reduce_max_sync(0xffffffffu, bits);
+    const int e = min(max((int)(bits >> 23) - 126, -90), 128);        // every finite |v| < 2^e
     if (lane == 0) {
         // fp16 parts are kept at up to 2^10
-        const float unit = __uint_as_float((uint32_t)(127 + e - (KIND == KIND_F16 ? 10 : 0)) << 23);
-        sts_u32(xd.scale + (chunk * MT + m) * 4, __float_as_uint(unit * mul));
+        const float unit = __uint_as_float((uint32_t)(127 + e - (KIND == KIND_F16 ? 10 : DG_UNIT)) << 23);
+        sts_u32(xd.scale + (chunk * MT + m) * 4, bits >= 0x7F800000u ? 0x7FFFFFFFu : __float_as_uint(unit * mul));
     }
     if (KIND == KIND_F16) {
         const float up = __uint_as_float((uint32_t)(127 + 10 - e) << 23);
@@ -125,7 +130,7 @@ __device__ __forceinline__ void dg_stage(const DgX<KIND, MT>& xd, int chunk, int
         asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(at + DG_COL), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
         return;
     }
-    const float to_int = __uint_as_float((uint32_t)(127 + 30 - e) << 23), down = __uint_as_float((uint32_t)(127 - e) << 23);
+    const float to_int = __uint_as_float((uint32_t)(127 + 30 - e) << 23), down = to_int * 0x1p-30f;
     uint32_t w[2][4];
     float sum = 0.0f;
 #pragma unroll
@@ -345,7 +350,7 @@ __device__ __forceinline__ void dg_chunk(DgAcc<KIND, MT>& acc, uint32_t row_a, u
     }
 }
 
-// The warp's sums to red[16 rows][MT].  The minimum terms lie in other lanes than the products: they go first, the
+// The warp's sums to red[16 rows][MT] (packed weights: in units of 2^DG_UNIT).  The minimum terms lie in other lanes than the products: they go first, the
 // products' lanes add theirs (so the threads that add the parts up read one value per part).
 constexpr int dg_red_floats(int MT) { return 16 * MT; }
 template <int KIND, int MT>
@@ -390,7 +395,7 @@ __device__ __forceinline__ float dg_value(const float* red, int parts, int row, 
     float v = 0.0f;
 #pragma unroll 4
     for (int p = 0; p < parts; ++p, at += dg_red_floats(MT)) v += *at;
-    return v;
+    return KIND == KIND_F16 ? v : v * (float)(1 << DG_UNIT);
 }
 #endif
 

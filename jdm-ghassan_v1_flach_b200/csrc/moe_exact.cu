@@ -40,7 +40,7 @@ constexpr int WX_X_SUB = 3 * WX_CAP * 128;    // 64 of K
 constexpr int WX_X_STAGE = 4 * WX_X_SUB;      // 256 of K
 constexpr int WX_SX = 2, WX_SP = 5;
 constexpr int WX_HDR = 4;                     // ring of (d, dmin, eight minima) per weight row, from the expansion to the epilogue
-constexpr int WX_AUX = 12;                    // floats per slot and 256 of K: 2^e, -, -, -, eight sub-block sums
+constexpr int WX_AUX = 12;                    // floats per slot and 256 of K: 2^e, -, -, -, eight sub-block sums in units of 2^e
 constexpr int WX_SET = 128;                   // tensor-memory columns between the two accumulators, between the two operands
 constexpr int WX_OPERAND = 2 * WX_SET;
 constexpr int WX_FIRST_EXPAND = 8, WX_EXPAND_WARPS = 16;
@@ -79,26 +79,24 @@ wx_split_kernel(const float* __restrict__ x, const int32_t* __restrict__ grouped
     v[4] = hi4.x; v[5] = hi4.y; v[6] = hi4.z; v[7] = hi4.w;
     float mx = 0.0f, sum = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        mx = fmaxf(mx, fabsf(v[k]));
-        sum += v[k];
-    }
+    for (int k = 0; k < 8; ++k) mx = fmaxf(mx, fabsf(v[k]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);          // of the lane's 32 values
     const int e = min(max((__float_as_int(mx) >> 23) - 127, -126), 126);
     const float s = __int_as_float((e + 127) << 23), inv = __int_as_float((127 - e) << 23);
     __half p[3][8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         float r = v[k] * inv;
+        sum += r;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             p[j][k] = __float2half_rn(r);
             r = (r - __half2float(p[j][k])) * 2048.0f;
         }
     }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);          // of the lane's 32 values
 #pragma unroll
     for (int j = 0; j < 3; ++j)
         *reinterpret_cast<uint4*>(out + ((int64_t)slot * 3 + j) * K + 256 * c + 8 * lane) = *reinterpret_cast<const uint4*>(p[j]);
@@ -394,7 +392,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
                             const float t = fmaf(fmaf(v[3 * j + 2], 0x1p-11f, v[3 * j + 1]), 0x1p-11f, v[3 * j]);
                             const float lo = fmaf(m[3], s0.w, fmaf(m[2], s0.z, fmaf(m[1], s0.y, m[0] * s0.x)));
                             const float hi = fmaf(m[7], s1.w, fmaf(m[6], s1.z, fmaf(m[5], s1.y, m[4] * s1.x)));
-                            acc[4 * k + j] = fmaf(d * au[0].x, t, fmaf(-dmin, lo + hi, acc[4 * k + j]));
+                            acc[4 * k + j] = fmaf(au[0].x, fmaf(d, t, -dmin * (lo + hi)), acc[4 * k + j]);
                         }
                     }
                 }

@@ -115,6 +115,44 @@ def test_linear_fp16_and_fp32(oracle, M, K, N):
     np.testing.assert_allclose(host(y), oracle.linear(x, wf, -2, M, K, N), **SUM_ORDER)
 
 
+@pytest.mark.parametrize("kind", [-1, 0, 1, 2, 3])
+@pytest.mark.parametrize("M", [1, 2, 3, 8, 9])
+def test_linear_not_finite(oracle, kind, M):
+    """A NaN or an infinity shows in every output of its token and in no other token's; activations up to the end of
+    the fp32 range do not overflow on the way.  SUM_ORDER's relative bound, on the largest output as the terms cancel."""
+    from gpu_util import SUM_ORDER, dev, empty, host, ops
+    K, N = 512, 40
+    r = np.random.default_rng(M + kind)
+    w = (r.standard_normal(N * K) * 0.02).astype(np.float32)
+    wd = w.astype(np.float16).view(np.uint16).reshape(N, K) if kind < 0 else oracle.quantize(w, kind)
+    exact = oracle.linear_exact(np.eye(K, dtype=np.float32), wd, kind, K, K, N) if kind >= 0 else \
+        w.astype(np.float16).astype(np.float32).reshape(N, K).T
+
+    def product(x):
+        y = empty((M, N))
+        if kind < 0:
+            ops.linear_forward_fp16(dev(x), dev(wd), y, M, K, N)
+        else:
+            ops.linear_forward_q4(dev(x), dev(wd), y, M, K, N, kind)
+        return host(y)
+
+    base = r.standard_normal((M, K)).astype(np.float32)
+    for bad in (np.nan, np.inf, -np.inf):
+        for at in (0, 300):
+            x = base.copy()
+            x[M - 1, at] = bad
+            y = product(x)
+            assert not np.isfinite(y[M - 1]).any(), (bad, at)
+            assert np.isfinite(y[:M - 1]).all()
+    for scale in (1e38, 3.4e38, 1e-20):
+        x = np.clip(base.astype(np.float64), -1, 1) * scale
+        x = x.astype(np.float32)
+        want = x.astype(np.float64) @ exact.astype(np.float64)
+        fits = np.abs(want) < 3.3e38
+        tol = dict(SUM_ORDER, atol=SUM_ORDER["rtol"] * np.abs(want).max())
+        np.testing.assert_allclose(product(x).astype(np.float64)[fits], want[fits], **tol)
+
+
 def test_linear_argument_errors(oracle):
     from gpu_util import B200Error, empty, ops
     x, w, y = empty((1, 48)), empty(64, torch.uint8), empty((1, 2))

@@ -92,6 +92,23 @@ def test_expert_tiles(oracle, kind, N, d, E):
     np.testing.assert_allclose(host(out), want, **SUM_ORDER)
 
 
+# the decode step's kernels, the digit engine's units and the exact tensor-core form
+@pytest.mark.parametrize("kind", [0, 2, 3])
+@pytest.mark.parametrize("N", [1, 3, 8, 9, 24])
+def test_experts_of_a_token_that_is_not_finite(oracle, kind, N):
+    from gpu_util import dev, empty, host, ops
+    d, E, ne, K = 256, 256, 8, 2
+    c = moe_case(oracle, N, N, d, E, ne, K, 0, kind)
+    x = c["x"].copy()
+    x[N - 1, 5] = np.nan
+    out, idx, w = empty((N, d)), empty((N, K), torch.int32), empty((N, K))
+    args = [dev(c[k]) for k in ("gates", "ups", "downs", "sh_g", "sh_u", "sh_d")]
+    ops.moe_forward_bias_half(dev(x), dev(c["router_w"]), dev(c["router_bias"]), *args, out, None, idx, w, None, None, None, N, d, E,
+                              ne, K, 0, kind)
+    got = host(out)
+    assert np.isnan(got[N - 1]).all() and np.isfinite(got[:N - 1]).all()
+
+
 # one to eight tokens; the 8-, 16- and 32-token tiles of the many-token router; widths off its 64 columns
 @pytest.mark.parametrize("d,ne,K", [(260, 33, 3), (1536, 64, 6)])
 @pytest.mark.parametrize("N", [1, 7, 257, 600, 2401])
