@@ -379,7 +379,8 @@ __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_gateup_kernel(MoeFused
 }
 
 // ---- kernel 3 ------------------------------------------------------------------
-// grid (ctas, M).  A tile is 16 output rows: of sh_down (SH wide), then of each chosen expert's down (E wide).
+// grid (ctas, M).  A tile is R = 16 output rows: of sh_down (SH wide), then of each chosen expert's down (E wide); fewer
+// where 16 of all of these do not fit the shared memory (the products then leave operand rows unused).
 template <int KIND>
 __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_down_kernel(MoeFusedArgs a) {
     constexpr int W = dg_warps(1);
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_down_kernel(MoeFusedAr
     __shared__ int s_idx[16];
     __shared__ float s_w[16];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = blockIdx.y;
-    const int sc = dg_chunks(a.SH), ec = dg_chunks(a.E), chunks = sc + a.K * ec, G = a.n_stages;
+    const int sc = dg_chunks(a.SH), ec = dg_chunks(a.E), chunks = sc + a.K * ec, G = a.n_stages, R = a.rows_per_tile;
     const uint32_t rb_s = a.SH > 0 ? (uint32_t)row_bytes_of(KIND, a.SH) : 0, rb_e = (uint32_t)row_bytes_of(KIND, a.E);
     DgX<KIND, 1> xd;
     uint8_t* p = xd.carve(smem + (size_t)a.sets * G * a.stage_bytes, chunks);
@@ -398,14 +399,14 @@ __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_down_kernel(MoeFusedAr
     auto issue = [&](int r, int set) {
         const int n = min(G, n_my - r * G);
         uint32_t rows_all = 0;
-        for (int i = 0; i < n; ++i) rows_all += min(16, a.d - (first + (r * G + i) * step) * 16);
+        for (int i = 0; i < n; ++i) rows_all += min(R, a.d - (first + (r * G + i) * step) * R);
         mbar_expect_tx(&bar[set], rows_all * (rb_s + a.K * rb_e));
         for (int i = 0; i < n; ++i) {
-            const int r0 = (first + (r * G + i) * step) * 16, rows = min(16, a.d - r0);
+            const int r0 = (first + (r * G + i) * step) * R, rows = min(R, a.d - r0);
             uint8_t* dst = smem + (size_t)(set * G + i) * a.stage_bytes;
             if (a.SH > 0) tma_load_1d(dst, a.sh_d + (int64_t)r0 * rb_s, rows * rb_s, &bar[set]);
             for (int k = 0; k < a.K; ++k)
-                tma_load_1d(dst + 16 * (rb_s + k * rb_e), a.downs + ((int64_t)s_idx[k] * a.d + r0) * rb_e, rows * rb_e, &bar[set]);
+                tma_load_1d(dst + R * (rb_s + k * rb_e), a.downs + ((int64_t)s_idx[k] * a.d + r0) * rb_e, rows * rb_e, &bar[set]);
         }
     };
     if (threadIdx.x < 32) {
@@ -429,8 +430,8 @@ __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_down_kernel(MoeFusedAr
     dm_rounds<KIND, 1>(a, n_my, red, bar,
         [&] {
             pdl_wait();
-            const int col = (first + threadIdx.x / 16 * step) * 16 + (threadIdx.x & 15);      // this thread's first element
-            if (!a.out && threadIdx.x < 16 * (unsigned)min(G, n_my) && col < a.d) pre = a.resid[(int64_t)m * a.d + col];
+            const int row = threadIdx.x & 15, col = (first + threadIdx.x / 16 * step) * R + row;      // this thread's first element
+            if (!a.out && threadIdx.x < 16 * (unsigned)min(G, n_my) && row < R && col < a.d) pre = a.resid[(int64_t)m * a.d + col];
             for (int i = warp; i < chunks; i += W) {
                 float v[8], mul = 1.0f;
                 if (i < sc) {
@@ -446,6 +447,7 @@ __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_down_kernel(MoeFusedAr
         }, issue,
         [&](int stage, int part, DgAcc<KIND, 1>& acc) {
             const uint32_t base = smem_u32(smem) + stage * a.stage_bytes, cb = dg_row_chunk<KIND>();
+            const int ga = min(lane >> 2, R - 1), gb = min((lane >> 2) + 8, R - 1);
             for (int c = part; c < chunks; c += a.parts) {
                 uint32_t at, rb;
                 int cc = c, K = a.SH;
@@ -454,19 +456,19 @@ __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_down_kernel(MoeFusedAr
                     rb = rb_s;
                 } else {
                     const int k = dg_div(c - sc, a.ec_inv);
-                    at = base + 16 * (rb_s + k * rb_e);
+                    at = base + R * (rb_s + k * rb_e);
                     rb = rb_e;
                     cc = c - sc - k * ec;
                     K = a.E;
                 }
-                at += (lane >> 2) * rb + cc * cb;
-                dg_chunk<KIND, 1>(acc, at, at + 8 * rb, xd, c, min(8, (K >> 5) - 8 * cc), lane);
+                at += cc * cb;
+                dg_chunk<KIND, 1>(acc, at + ga * rb, at + gb * rb, xd, c, min(8, (K >> 5) - 8 * cc), lane);
             }
         },
         [&](int t0, int n, const float* rr) {
             for (int e = threadIdx.x; e < n * 16; e += W * 32) {
-                const int row = e % 16, i = e / 16, col = (first + (t0 + i) * step) * 16 + row;
-                if (col >= a.d) continue;
+                const int row = e % 16, i = e / 16, col = (first + (t0 + i) * step) * R + row;
+                if (row >= R || col >= a.d) continue;
                 const float v = dg_value<KIND, 1>(rr + i * a.parts * dg_red_floats(1), a.parts, row, 0);
                 const int64_t at = (int64_t)m * a.d + col;
                 if (a.out) a.out[at] = v;
@@ -528,10 +530,21 @@ static int dm_kind(const MoeFusedArgs& a) {
     const int t2 = a.K * (a.E / 8), g2 = std::min(t2, per_token);
     p2.per_inv = 0xFFFFFFFFu / (uint32_t)(a.E / 8) + 1u;      // exact quotients below 2^16 (E / 8 >= 4)
     const size_t s2 = dm_plan<KIND>(p2, t2, g2, 16 * rb_d, dg_chunks(a.d), 1, (size_t)dg_chunks(a.d) * 8, 0);
-    const int t3 = ceil_div(a.d, 16), g3 = std::min(t3, per_token);
     p3.ec_inv = dg_inv(std::min(255, dg_chunks(a.E)));
-    const size_t s3 = dm_plan<KIND>(p3, t3, g3, 16 * (rb_s + a.K * rb_e), dg_chunks(a.SH) + a.K * dg_chunks(a.E), 1, 0, 0);
-    if (!s1 || !s2 || !s3) return fail(B200_EUNSUPPORTED, "moe_fused: hidden size %d does not fit the shared-memory staging", a.d);
+    // The down rows of the shared and all K experts: 16 to a tile, fewer where those do not fit (Q8_0, experts of 1024 and
+    // eight of them: 4.5 KB of rows per output), while a copy still moves whole 16-byte words.
+    size_t s3 = 0;
+    int g3 = 0;
+    for (int R = TILE_ROWS; R >= 1 && !s3 && (R * rb_e) % 16 == 0 && (R * rb_s) % 16 == 0; R >>= 1) {
+        const int t3 = ceil_div(a.d, R);
+        g3 = std::min(t3, per_token);
+        p3.rows_per_tile = R;
+        s3 = dm_plan<KIND>(p3, t3, g3, R * (rb_s + a.K * rb_e), dg_chunks(a.SH) + a.K * dg_chunks(a.E), 1, 0, 0);
+    }
+    if (!s1 || !s2) return fail(B200_EUNSUPPORTED, "moe_fused: hidden size %d does not fit the shared-memory staging", a.d);
+    if (!s3)
+        return fail(B200_EUNSUPPORTED, "moe_fused: the down rows of %d experts of %d and a shared one of %d do not fit the shared-memory staging",
+                    a.K, a.E, a.SH);
     int rc = mt == 1 ? dm_kernel1<KIND, 1>(p1, s1, n_router + sh_ctas) : mt == 2 ? dm_kernel1<KIND, 2>(p1, s1, n_router + sh_ctas)
              : mt == 4 ? dm_kernel1<KIND, 4>(p1, s1, n_router + sh_ctas) : dm_kernel1<KIND, 8>(p1, s1, n_router + sh_ctas);
     if (rc) return rc;

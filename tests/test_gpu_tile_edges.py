@@ -92,6 +92,43 @@ def test_expert_tiles(oracle, kind, N, d, E):
     np.testing.assert_allclose(host(out), want, **SUM_ORDER)
 
 
+# Experts whose down rows do not fit sixteen to a tile: (kind, hidden, experts, width, top, shared width, sequences)
+WIDE_EXPERTS = [(2, 2048, 64, 1024, 8, 2048, 1), (2, 2048, 128, 768, 8, 0, 2), (0, 1024, 16, 1024, 8, 1024, 8), (1, 1024, 16, 1024, 8, 1024, 8),
+                (2, 512, 16, 1536, 16, 0, 5)]
+
+
+@pytest.mark.parametrize("kind,d,ne,E,K,SH,B", WIDE_EXPERTS)
+def test_fused_step_takes_wide_experts(kind, d, ne, E, K, SH, B):
+    import ctypes as C
+    from gpu_util import pkg
+    lib, h = pkg.lib(), C.c_void_p()
+    types = np.array([0], np.int32)
+    lib.b200_decoder_create(C.byref(h), B, 512, d, 1, types.ctypes.data, d // 64, d // 64, 64, -1, 2 * d // 64, 64, 64, 4, ne, K, E, SH, 32,
+                            16, kind, 1e-5, 1.0, 1.0, 0.0, 1.0)
+    try:
+        lib.b200_decoder_configure(h, 1, 0)
+    finally:
+        lib.b200_decoder_destroy(h)
+
+
+@pytest.mark.parametrize("kind,ne,E,K,SH,N", [(2, 8, 1024, 8, 2048, 1), (0, 8, 1024, 8, 1024, 8), (1, 8, 1024, 8, 1024, 8),
+                                              (2, 16, 1536, 16, 0, 1), (2, 16, 1536, 16, 0, 5)])
+def test_wide_experts(oracle, kind, ne, E, K, SH, N):
+    from gpu_util import SUM_ORDER, dev, empty, host, ops
+    d = 544                                             # tiles of two and eight rows over the CTAs in several rounds
+    c = moe_case(oracle, N + E, N, d, E, ne, K, SH, kind)
+    out, idx, w = empty((N, d)), empty((N, K), torch.int32), empty((N, K))
+    args = [dev(c[k]) for k in ("gates", "ups", "downs", "sh_g", "sh_u", "sh_d")]
+    ops.moe_forward_bias_half(dev(c["x"]), dev(c["router_w"]), dev(c["router_bias"]), *args, out, None, idx, w, None, None, None, N, d, E,
+                              ne, K, SH, kind)
+    oracle.set_weight_rounding(False)
+    want, _, widx, _ = oracle.moe_forward(c["x"], c["router_w"], c["router_bias"], c["gates"], c["ups"], c["downs"], c["sh_g"], c["sh_u"],
+                                          c["sh_d"], d, E, ne, K, SH, kind)
+    oracle.set_weight_rounding(True)
+    assert np.array_equal(host(idx), widx)
+    np.testing.assert_allclose(host(out), want, **SUM_ORDER)
+
+
 # the decode step's kernels, the digit engine's units and the exact tensor-core form
 @pytest.mark.parametrize("kind", [0, 2, 3])
 @pytest.mark.parametrize("N", [1, 3, 8, 9, 24])
