@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dg_gemv_kernel(SgArgs a)
     float nw[8];
     if (PRO == PRO_RMS) {
         const int c = MT == 1 ? warp : warp - dg_div(warp, a.chunks_inv) * chunks;
-        dg_load8<false>(a.norm_w, c * DG_CHUNK + 8 * lane, a.K, nw);
+        dg_norm8(a.norm_w, c * DG_CHUNK + 8 * lane, a.K, nw);
     }
     pdl_wait();
 
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dg_gemv_kernel(SgArgs a)
         float v[8];
         dg_load8<true>(a.x + (int64_t)m * a.x_stride, c * DG_CHUNK + 8 * lane, a.K, v);
         if (PRO == PRO_RMS) {
-            if (i != warp) dg_load8<false>(a.norm_w, c * DG_CHUNK + 8 * lane, a.K, nw);
+            if (i != warp) dg_norm8(a.norm_w, c * DG_CHUNK + 8 * lane, a.K, nw);
             double ss = 0.0;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -254,7 +254,7 @@ static int launch_dg_kind(const SgArgs& a, int pro, int epi) {
 
 // stream_gemv() for packed and fp16 weights; arguments checked there.
 int digit_gemv(SgArgs a, int kind, int pro, int epi) {
-    if ((reinterpret_cast<uintptr_t>(a.x) & 15) != 0 || (a.x_stride & 3) != 0 || (reinterpret_cast<uintptr_t>(a.norm_w) & 15) != 0)
+    if ((reinterpret_cast<uintptr_t>(a.x) & 15) != 0 || (a.x_stride & 3) != 0)
         return fail(B200_EUNSUPPORTED, "stream_gemv: activations must be 16-byte aligned");
     switch (kind) {
         case 0: return launch_dg_kind<0>(a, pro, epi);

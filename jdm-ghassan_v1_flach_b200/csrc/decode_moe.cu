@@ -66,7 +66,7 @@ __device__ __forceinline__ void dm_stage_norm(const MoeFusedArgs& a, const DgX<K
         dg_load8<true>(a.x + (int64_t)(m0 + m) * a.d, c * DG_CHUNK + 8 * lane, a.d, v);
         double ss = 0.0;
         if (a.norm_w) {
-            dg_load8<false>(a.norm_w, c * DG_CHUNK + 8 * lane, a.d, nw);
+            dg_norm8(a.norm_w, c * DG_CHUNK + 8 * lane, a.d, nw);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 ss += (double)v[j] * (double)v[j];
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(
                 if (g < groups) {
                     x = __ldcg(reinterpret_cast<const float4*>(a.x + (int64_t)m * a.d + 4 * g));
                     if (a.norm_w) {
-                        const float4 nw = *reinterpret_cast<const float4*>(a.norm_w + 4 * g);
+                        const float4 nw = dg_norm4(a.norm_w + 4 * g);
                         const float f = inv[m];
                         x = make_float4(x.x * f * nw.x, x.y * f * nw.y, x.z * f * nw.z, x.w * f * nw.w);
                     }
@@ -556,7 +556,7 @@ static int dm_kind(const MoeFusedArgs& a) {
 // moe_fused() for packed weights (kind 0 .. 3); sizes checked there.
 int moe_digit(const MoeFusedArgs& a, int kind) {
     auto bad = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
-    if (bad(a.x) || bad(a.norm_w) || bad(a.gates) || bad(a.ups) || bad(a.downs) || (a.SH > 0 && (bad(a.sh_g) || bad(a.sh_u) || bad(a.sh_d))))
+    if (bad(a.x) || bad(a.gates) || bad(a.ups) || bad(a.downs) || (a.SH > 0 && (bad(a.sh_g) || bad(a.sh_u) || bad(a.sh_d))))
         return fail(B200_EUNSUPPORTED, "moe_fused: tensors must be 16-byte aligned");
     switch (kind) {
         case 0: return dm_kind<0>(a);

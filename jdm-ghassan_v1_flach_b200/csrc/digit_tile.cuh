@@ -190,6 +190,20 @@ __device__ __forceinline__ void dg_load8(const float* x, int k, int K, float (&v
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
+// The same of a norm's weights, which the caller may have put at any address.
+__device__ __forceinline__ float4 dg_norm4(const float* w) {
+    if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) return *reinterpret_cast<const float4*>(w);
+    return make_float4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void dg_norm8(const float* w, int k, int K, float (&v)[8]) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (k < K) {
+        a = dg_norm4(w + k);
+        b = dg_norm4(w + k + 4);
+    }
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
 // One warp's accumulators for a 16-row tile.  Packed: f[q] the digit columns of tokens 2 q, 2 q + 1 (lane
 // (g, t): rows g, g + 8; token 2 q + t / 2, digits 2 (t & 1), + 1), mn the minimum terms (rows g,
 // g + 8; tokens 2 t, 2 t + 1).  fp16: f[q] the two parts of token 4 q + t.

@@ -212,3 +212,28 @@ def test_recorded_step_with_moving_buffers(oracle, fused, batch):
     for (na, la), (nb, lb) in zip(*outs):
         assert np.array_equal(na, nb)
         assert np.array_equal(la.view(np.uint32), lb.view(np.uint32))
+
+
+# norm weights where a caller's own packing put them: any address of a float
+@pytest.mark.parametrize("B", [1, 2, 5])
+@pytest.mark.parametrize("qkind", [2, 3])
+def test_fused_step_with_norm_weights_at_odd_addresses(oracle, B, qkind):
+    from model_util import T
+    m = make_model(oracle, dict(TINY, qkind=qkind), seed=4)
+    toks = np.random.default_rng(B).integers(0, TINY["vocab"], (3, B)).astype(np.int32)
+    got = []
+    for odd in (False, True):
+        dec = CudaDecoder(m, B, 16)
+        if odd:
+            for l, L in [(-1, m)] + list(enumerate(m["layers"])):
+                for name in ("final_norm", "attn_norm", "ffn_norm"):
+                    if name in L:
+                        t = torch.empty(L[name].size + 1, device="cuda")[1:]
+                        t.copy_(torch.from_numpy(L[name]))
+                        dec.keep.append(t)
+                        dec.lib.b200_decoder_set_tensor(dec.handle, l, T[name], t)
+        dec.configure(1, 0)
+        for t in toks:
+            dec.step_host(t)
+        got.append(dec.logits())
+    assert np.array_equal(got[0], got[1])
