@@ -133,3 +133,31 @@ def test_prefill(oracle, B, T, H, KV, hd):
         else:
             from gpu_util import fp16_close                  # 128 tokens and more: tensor-core kernel
             fp16_close(host(out2), host(out), frac=4e-3)
+
+
+# three heads to a KV head (their parts share one operand), eight (two operands); one piece, several, a ragged batch
+@pytest.mark.parametrize("H,KV,hd", [(12, 4, 64), (32, 8, 128), (8, 1, 128)])
+@pytest.mark.parametrize("lens", [(64, 65, 100), (300, 511), (1000, 2000), tuple(range(300, 4300, 125))])
+def test_paged_decode_error_is_that_of_fp32(H, KV, hd, lens):
+    """Against 64 bits.  At scores of unit variance a probability carries the roundings of the score's sum, its scaling, the
+    difference from the maximum and the exponential, an output that of its own sum: five of 2^-24, in the 2-norm."""
+    from gpu_util import ops
+    g = torch.Generator(device="cuda").manual_seed(H + len(lens))
+    page = 64
+    pages = [-(-n // page) for n in lens]
+    table = torch.zeros(len(lens), max(pages), dtype=torch.int32, device="cuda")
+    order = torch.randperm(sum(pages), device="cuda", generator=g)
+    q = torch.randn(len(lens), H, hd, device="cuda", generator=g)
+    k, v = (torch.randn(sum(pages) * page, KV * hd, device="cuda", generator=g).half() for _ in range(2))
+    want = torch.empty(len(lens), H, hd, dtype=torch.float64, device="cuda")
+    for b, n in enumerate(lens):
+        mine = order[sum(pages[:b]):sum(pages[:b + 1])]
+        table[b, :pages[b]] = mine.int()
+        rows = (mine[:, None] * page + torch.arange(page, device="cuda")).flatten()[:n]
+        kk, vv = (c[rows].double().view(n, KV, hd) for c in (k, v))
+        s = torch.einsum("kgd,nkd->kgn", q[b].double().view(KV, H // KV, hd), kk) / hd ** 0.5
+        want[b] = torch.einsum("kgn,nkd->kgd", torch.softmax(s, -1), vv).reshape(H, hd)
+    out = torch.full_like(q, float("nan"))
+    ops.attention_decode_paged_fp16(q, k.view(torch.int16), v.view(torch.int16), table, torch.tensor(lens, dtype=torch.int32, device="cuda"),
+                                    out, len(lens), max(pages), page, H, KV, hd, hd ** -0.5)
+    assert float((out.double() - want).norm() / want.norm()) < 5 * 2.0 ** -24
