@@ -9,11 +9,13 @@
 // with e the exponent of the largest of the token's 256 activations (so no activation loses more than
 // 2^-31 of that maximum; the fp16 pairs kept 22 bits of each; a NaN or an infinity among the 256 makes their
 // scale, and so the token's outputs, NaN), and for every 32-weight sub-block one
-// mma.m16n8k32 gives sum_k q_k D_jk exactly, the eight columns being the four digits of two tokens.
-// The 6-bit scale of the sub-block multiplies the integer (exact: at most 63 * 32 * 240 * 128 * 4 in 31
-// bits), so a super-block ends in one conversion and one multiply-add per digit, and the minimum terms of
-// its eight sub-blocks are one mma.m16n8k8 with the sub-block sums.  About 40 instructions per 1024
-// weights for one or two tokens, 85 for eight.
+// mma.m16n8k32 gives sum_k 16 (q_k - 8) D_jk exactly, the eight columns being the four digits of two tokens.
+// The 6-bit scale of the sub-block multiplies the integer (exact: at most 63 * 32 * 128 * 128 * 8 = 2^28), so a
+// super-block ends in one conversion and one multiply-add per digit.  What the centred integers leave of a
+// sub-block, (8 d s - dmin m) times the sum of its activations, is small beside the products and added in fp32.
+// (With q itself the products and the minimum terms are each two to three times their difference, and the last
+// bits of both showed: 3e-7 .. 5e-7 of the output's norm against 64 bits, 1e-7 .. 2e-7 so.)
+// About 40 instructions per 1024 weights for one or two tokens, 85 for eight.
 #pragma once
 
 #include "fused_common.cuh"
@@ -30,14 +32,14 @@ __host__ __device__ __forceinline__ int dg_div(int a, uint32_t inv) { return (in
 
 template <int KIND>
 struct DgKind {
-    static constexpr bool mins = KIND == 3 || KIND == 1;
+    static constexpr bool offset = KIND == 3 || KIND == 1;       // the centred weights have an offset per 32
     // Q4_0 and Q4_1 pair element j with j + 16 of a block in one byte: their operand words are those of
     // elements 4t and 16 + 4t; the other kinds use 8t and 8t + 4.
     static constexpr bool split16 = KIND == 0 || KIND == 1;
 };
 
 __host__ __device__ inline int dg_chunks(int K) { return (K + DG_CHUNK - 1) / DG_CHUNK; }
-// Staged activations of a chunk and token: four digit bytes each, the sub-block sums as two fp16 parts and the
+// Staged activations of a chunk and token: four digit bytes each, the sub-block sums and the
 // scale; for fp16 weights the two fp16 parts of each, in columns of their own.
 constexpr int DG_COL = DG_CHUNK * 2 + 64;     // bytes of an fp16 column: two neighbours fall into different halves of the banks
 template <int KIND>
@@ -49,7 +51,7 @@ int dg_parts(int tiles, int chunks, int warps);      // decode_gemv.cu
 
 #ifdef __CUDACC__
 // Packed weights: digits [sub-block][token][slot][32 bytes], slot = (digit + sub-block) & 3 (so that the stores
-// of a warp spread over the banks); sub-block sums * 2^-e [chunk][part][token][8]; scales [chunk][token].
+// of a warp spread over the banks); sub-block sums times the scale [chunk][token][8]; scales [chunk][token].
 // fp16 weights: columns [chunk][token][part][DG_COL bytes]; scales.
 template <int KIND, int MT>
 struct DgX {
@@ -77,27 +79,15 @@ __device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v) { asm volatile("
 __device__ __forceinline__ void sts_u2(uint32_t a, uint32_t x, uint32_t y) {
     asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ void sts_u16(uint32_t a, uint16_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(v) : "memory"); }
-template <bool SIGNED_A>
 __device__ __forceinline__ void dg_mma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b) {
-    if (SIGNED_A)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y), "r"(0));
-    else
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y), "r"(0));
-}
-__device__ __forceinline__ void dg_mma_f16k8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(b0));
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y), "r"(0));
 }
 
 // The scale of a chunk of packed weights is 2^(e - DG_UNIT) and dg_value puts 2^DG_UNIT back on the finished sum: the
-// products and the minimum terms, each larger than their difference, and the digits, each up to 2^10 of its share of the
-// output, do not overflow where the output does not; 2^-90 2^-24 leaves room for a weight's scale above.
+// products and the offsets, and the digits, each up to 2^10 of its share of the output, do not overflow where the output
+// does not; 2^-90 2^-24 leaves room for a weight's scale above.
 constexpr int DG_UNIT = 24;
 
 // Lane l's eight activations 256 * chunk + 8 l .. of token m (zeros past K), staged by one whole warp.
@@ -109,11 +99,10 @@ __device__ __forceinline__ void dg_stage(const DgX<KIND, MT>& xd, int chunk, int
     for (int i = 0; i < 8; ++i) bits = max(bits, __float_as_uint(v[i]) & 0x7FFFFFFFu);
     bits = __reduce_max_sync(0xffffffffu, bits);
     const int e = min(max((int)(bits >> 23) - 126, -90), 128);        // every finite |v| < 2^e
-    if (lane == 0) {
-        // fp16 parts are kept at up to 2^10
-        const float unit = __uint_as_float((uint32_t)(127 + e - (KIND == KIND_F16 ? 10 : DG_UNIT)) << 23);
-        sts_u32(xd.scale + (chunk * MT + m) * 4, bits >= 0x7F800000u ? 0x7FFFFFFFu : __float_as_uint(unit * mul));
-    }
+    // fp16 parts are kept at up to 2^10
+    float unit = __uint_as_float((uint32_t)(127 + e - (KIND == KIND_F16 ? 10 : DG_UNIT)) << 23) * mul;
+    if (bits >= 0x7F800000u) unit = __uint_as_float(0x7FFFFFFFu);
+    if (lane == 0) sts_u32(xd.scale + (chunk * MT + m) * 4, __float_as_uint(unit));
     if (KIND == KIND_F16) {
         const float up = __uint_as_float((uint32_t)(127 + 10 - e) << 23);
         uint32_t hi[4], lo[4];
@@ -162,15 +151,10 @@ __device__ __forceinline__ void dg_stage(const DgX<KIND, MT>& xd, int chunk, int
             sts_u2(a + 8 * l4, w[0][j], w[1][j]);
         }
     }
-    if (DgKind<KIND>::mins) {
+    if (DgKind<KIND>::offset) {
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        if (l4 == 0) {
-            const __half hi = __float2half_rn(sum), lo = __float2half_rn(sum - __half2float(hi));
-            const uint32_t a = xd.sum + (chunk * 2 * MT + m) * 16 + (lane >> 2) * 2;
-            sts_u16(a, __half_as_ushort(hi));
-            sts_u16(a + MT * 16, __half_as_ushort(lo));
-        }
+        if (l4 == 0) sts_u32(xd.sum + (chunk * MT + m) * 32 + (lane >> 2) * 4, __float_as_uint(sum * unit));
     }
 }
 
@@ -205,19 +189,20 @@ __device__ __forceinline__ void dg_norm8(const float* w, int k, int K, float (&v
 }
 
 // One warp's accumulators for a 16-row tile.  Packed: f[q] the digit columns of tokens 2 q, 2 q + 1 (lane
-// (g, t): rows g, g + 8; token 2 q + t / 2, digits 2 (t & 1), + 1), mn the minimum terms (rows g,
-// g + 8; tokens 2 t, 2 t + 1).  fp16: f[q] the two parts of token 4 q + t.
+// (g, t): rows g, g + 8; token 2 q + t / 2, digits 2 (t & 1), + 1), off the offsets of this lane's sub-blocks
+// (rows g, g + 8; each token).  fp16: f[q] the two parts of token 4 q + t.
 template <int KIND, int MT>
 struct DgAcc {
     static constexpr int NT = KIND == KIND_F16 ? (MT <= 4 ? 1 : 2) : (MT <= 2 ? 1 : MT / 2);
-    float f[NT][4], mn[4];
+    static constexpr int NO = DgKind<KIND>::offset ? MT : 1;
+    float f[NT][4], off[2][NO];
     __device__ __forceinline__ void clear() {
 #pragma unroll
         for (int q = 0; q < NT; ++q)
 #pragma unroll
             for (int i = 0; i < 4; ++i) f[q][i] = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mn[i] = 0.0f;
+        for (int i = 0; i < NO; ++i) off[0][i] = off[1][i] = 0.0f;
     }
 };
 
@@ -264,27 +249,33 @@ __device__ __forceinline__ void dg_chunk(DgAcc<KIND, MT>& acc, uint32_t row_a, u
 #pragma unroll
     for (int q = 0; q < NT; ++q) xs[q] = lds_f32(xd.scale + (xc * MT + (MT == 1 ? 0 : 2 * q + (t >> 1))) * 4);
     auto bfrag = [&](int s, int q) { return lds_u2(xo[s & 3] + (s * MT + 2 * q) * 128); };
-    uint32_t ma = 0, mb = 0;                                          // fp16 pairs of the minima of sub-blocks 2 t, 2 t + 1
-    float da, db, dma = 1.0f, dmb = 1.0f;
+    float oa[2] = {0.f, 0.f}, ob[2] = {0.f, 0.f};                      // offsets of sub-blocks 2 t, 2 t + 1 in the two rows
+    float da, db;
     if (KIND == 3) {
         const uint4 ha = lds_u4(row_a), hb = lds_u4(row_b);
         const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&ha.x)), fb = __half22float2(*reinterpret_cast<const __half2*>(&hb.x));
-        da = fa.x; db = fb.x; dma = fa.y; dmb = fb.y;
+        da = fa.x; db = fb.x;
         const uint32_t sca[2] = {ha.y & 0x3F3F3F3Fu, (ha.w & 0x0F0F0F0Fu) | ((ha.y >> 2) & 0x30303030u)};
         const uint32_t scb[2] = {hb.y & 0x3F3F3F3Fu, (hb.w & 0x0F0F0F0Fu) | ((hb.y >> 2) & 0x30303030u)};
         const uint32_t mna = t < 2 ? ha.z & 0x3F3F3F3Fu : ((ha.w >> 4) & 0x0F0F0F0Fu) | ((ha.z >> 2) & 0x30303030u);
         const uint32_t mnb = t < 2 ? hb.z & 0x3F3F3F3Fu : ((hb.w >> 4) & 0x0F0F0F0Fu) | ((hb.z >> 2) & 0x30303030u);
-        const uint32_t sel = (t & 1) ? 0x4342u : 0x4140u;
-        const __half2 k1024 = __half2half2(__ushort_as_half(0x6400));
-        const uint32_t pa = __byte_perm(mna, 0x64646464u, sel), pb = __byte_perm(mnb, 0x64646464u, sel);
-        const __half2 qa = __hsub2(*reinterpret_cast<const __half2*>(&pa), k1024), qb = __hsub2(*reinterpret_cast<const __half2*>(&pb), k1024);
-        ma = *reinterpret_cast<const uint32_t*>(&qa);
-        mb = *reinterpret_cast<const uint32_t*>(&qb);
-        int lo[NT][4], hi[NT][4];
+        // 8 d s - dmin m, both products exact
+        auto offsets = [&](uint32_t sc, uint32_t mn, float2 f, float (&o)[2]) {
+            const int sh = 16 * (t & 1);
+            sc >>= sh;
+            mn >>= sh;
+            const float d8 = 8.0f * f.x;
+            o[0] = __fsub_rn(d8 * (float)(sc & 0xFF), f.y * (float)(mn & 0xFF));
+            o[1] = __fsub_rn(d8 * (float)((sc >> 8) & 0xFF), f.y * (float)((mn >> 8) & 0xFF));
+        };
+        offsets(t < 2 ? sca[0] : sca[1], mna, fa, oa);
+        offsets(t < 2 ? scb[0] : scb[1], mnb, fb, ob);
+        int v[NT][4];
 #pragma unroll
         for (int q = 0; q < NT; ++q)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { lo[q][i] = 0; hi[q][i] = 0; }
+            for (int i = 0; i < 4; ++i) v[q][i] = 0;
+        auto high = [](uint32_t w) { return (w & 0xF0F0F0F0u) ^ 0x80808080u; };      // 16 (q - 8) as signed bytes
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const uint2 wa = lds_u2(row_a + 16 + 32 * j + 8 * t), wb = lds_u2(row_b + 16 + 32 * j + 8 * t);
@@ -293,30 +284,34 @@ __device__ __forceinline__ void dg_chunk(DgAcc<KIND, MT>& acc, uint32_t row_a, u
 #pragma unroll
             for (int q = 0; q < NT; ++q) {
                 int c[4];
-                dg_mma<false>(c, wa.x & 0x0F0F0F0Fu, wb.x & 0x0F0F0F0Fu, wa.y & 0x0F0F0F0Fu, wb.y & 0x0F0F0F0Fu, bfrag(2 * j, q));
-                lo[q][0] += sa0 * c[0]; lo[q][1] += sa0 * c[1]; lo[q][2] += sb0 * c[2]; lo[q][3] += sb0 * c[3];
-                dg_mma<false>(c, wa.x & 0xF0F0F0F0u, wb.x & 0xF0F0F0F0u, wa.y & 0xF0F0F0F0u, wb.y & 0xF0F0F0F0u, bfrag(2 * j + 1, q));
-                hi[q][0] += sa1 * c[0]; hi[q][1] += sa1 * c[1]; hi[q][2] += sb1 * c[2]; hi[q][3] += sb1 * c[3];
+                dg_mma(c, high(wa.x << 4), high(wb.x << 4), high(wa.y << 4), high(wb.y << 4), bfrag(2 * j, q));
+                v[q][0] += sa0 * c[0]; v[q][1] += sa0 * c[1]; v[q][2] += sb0 * c[2]; v[q][3] += sb0 * c[3];
+                dg_mma(c, high(wa.x), high(wb.x), high(wa.y), high(wb.y), bfrag(2 * j + 1, q));
+                v[q][0] += sa1 * c[0]; v[q][1] += sa1 * c[1]; v[q][2] += sb1 * c[2]; v[q][3] += sb1 * c[3];
             }
         }
 #pragma unroll
         for (int q = 0; q < NT; ++q) {
-            const float ea = da * xs[q], eb = db * xs[q], ga = ea * 0.0625f, gb = eb * 0.0625f;
-            acc.f[q][0] += ea * (float)lo[q][0] + ga * (float)hi[q][0];
-            acc.f[q][1] += ea * (float)lo[q][1] + ga * (float)hi[q][1];
-            acc.f[q][2] += eb * (float)lo[q][2] + gb * (float)hi[q][2];
-            acc.f[q][3] += eb * (float)lo[q][3] + gb * (float)hi[q][3];
+            const float ea = da * xs[q], eb = db * xs[q];
+            acc.f[q][0] += ea * (float)v[q][0];
+            acc.f[q][1] += ea * (float)v[q][1];
+            acc.f[q][2] += eb * (float)v[q][2];
+            acc.f[q][3] += eb * (float)v[q][3];
         }
     } else {
         constexpr int BB = q_block_bytes(KIND);
         if (KIND == 1) {
-            // m of blocks 2 t, 2 t + 1 (zero past the row's end: their sums are zero, but the bits may be anything)
-            auto pair = [&](uint32_t row) {
-                const uint32_t m0 = 2 * t < nb ? lds_u32(row + 2 * t * BB) >> 16 : 0u, m1 = 2 * t + 1 < nb ? lds_u32(row + (2 * t + 1) * BB) & 0xFFFF0000u : 0u;
-                return m0 | m1;
+            // m + 8 d of blocks 2 t, 2 t + 1 (zero past the row's end: their sums are zero, but the bits may be anything)
+            auto offset = [&](uint32_t row, int s) {
+                const uint32_t dm = s < nb ? lds_u32(row + s * BB) : 0u;
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&dm));
+                return fmaf(8.0f, f.x, f.y);
             };
-            ma = pair(row_a);
-            mb = pair(row_b);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                oa[i] = offset(row_a, 2 * t + i);
+                ob[i] = offset(row_b, 2 * t + i);
+            }
         }
         // bytes [a, a + 4) at any even address
         auto word = [&](uint32_t a) { return __funnelshift_r(lds_u32(a & ~3u), lds_u32((a & ~3u) + 4), (a & 2) * 8); };
@@ -335,9 +330,9 @@ __device__ __forceinline__ void dg_chunk(DgAcc<KIND, MT>& acc, uint32_t row_a, u
                 two(ra + 2 + 8 * t, a0, a2);
                 two(rb + 2 + 8 * t, a1, a3);
             } else {
-                uint32_t wa = KIND == 0 ? word(ra + 2 + 4 * t) : lds_u32(ra + 4 + 4 * t);
-                uint32_t wb = KIND == 0 ? word(rb + 2 + 4 * t) : lds_u32(rb + 4 + 4 * t);
-                if (KIND == 0) { wa ^= 0x88888888u; wb ^= 0x88888888u; }          // 16 (q - 8) as a signed byte
+                // 16 (q - 8) as signed bytes
+                const uint32_t wa = (KIND == 0 ? word(ra + 2 + 4 * t) : lds_u32(ra + 4 + 4 * t)) ^ 0x88888888u;
+                const uint32_t wb = (KIND == 0 ? word(rb + 2 + 4 * t) : lds_u32(rb + 4 + 4 * t)) ^ 0x88888888u;
                 a0 = (wa << 4) & 0xF0F0F0F0u; a1 = (wb << 4) & 0xF0F0F0F0u;
                 a2 = wa & 0xF0F0F0F0u; a3 = wb & 0xF0F0F0F0u;
             }
@@ -346,26 +341,26 @@ __device__ __forceinline__ void dg_chunk(DgAcc<KIND, MT>& acc, uint32_t row_a, u
 #pragma unroll
             for (int q = 0; q < NT; ++q) {
                 int c[4];
-                dg_mma<KIND != 1>(c, a0, a1, a2, a3, bfrag(s, q));
+                dg_mma(c, a0, a1, a2, a3, bfrag(s, q));
                 const float ea = da * xs[q], eb = db * xs[q];
                 acc.f[q][0] += ea * (float)c[0]; acc.f[q][1] += ea * (float)c[1];
                 acc.f[q][2] += eb * (float)c[2]; acc.f[q][3] += eb * (float)c[3];
             }
         }
     }
-    if (DgKind<KIND>::mins) {
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        const uint32_t at = xd.sum + (xc * 2 * MT + min(g, MT - 1)) * 16 + 4 * t;
-        dg_mma_f16k8(c, ma, mb, lds_u32(at));
-        dg_mma_f16k8(c, ma, mb, lds_u32(at + MT * 16));
-        const float x0 = lds_f32(xd.scale + (xc * MT + min(2 * t, MT - 1)) * 4), x1 = lds_f32(xd.scale + (xc * MT + min(2 * t + 1, MT - 1)) * 4);
-        acc.mn[0] += dma * x0 * c[0]; acc.mn[1] += dma * x1 * c[1];
-        acc.mn[2] += dmb * x0 * c[2]; acc.mn[3] += dmb * x1 * c[3];
+    if (DgKind<KIND>::offset) {
+        const uint32_t at = xd.sum + xc * MT * 32 + 8 * t;
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            const uint2 u = lds_u2(at + m * 32);
+            const float s0 = __uint_as_float(u.x), s1 = __uint_as_float(u.y);
+            acc.off[0][m] = fmaf(oa[1], s1, fmaf(oa[0], s0, acc.off[0][m]));
+            acc.off[1][m] = fmaf(ob[1], s1, fmaf(ob[0], s0, acc.off[1][m]));
+        }
     }
 }
 
-// The warp's sums to red[16 rows][MT] (packed weights: in units of 2^DG_UNIT).  The minimum terms lie in other lanes than the products: they go first, the
-// products' lanes add theirs (so the threads that add the parts up read one value per part).
+// The warp's sums to red[16 rows][MT] (packed weights: in units of 2^DG_UNIT).
 constexpr int dg_red_floats(int MT) { return 16 * MT; }
 template <int KIND, int MT>
 __device__ __forceinline__ void dg_finish(const DgAcc<KIND, MT>& acc, float* red, int lane) {
@@ -379,26 +374,25 @@ __device__ __forceinline__ void dg_finish(const DgAcc<KIND, MT>& acc, float* red
             }
         return;
     }
-    if (DgKind<KIND>::mins) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-            if (2 * t + i < MT) {
-                red[g * MT + 2 * t + i] = KIND == 3 ? -acc.mn[i] : acc.mn[i];
-                red[(g + 8) * MT + 2 * t + i] = KIND == 3 ? -acc.mn[2 + i] : acc.mn[2 + i];
-            }
-        __syncwarp();
-    }
-    const float scale = ((t & 1) ? 65536.0f : 1.0f) * (DgKind<KIND>::split16 ? 0x1p-34f : 0x1p-30f);
+    const float scale = ((t & 1) ? 65536.0f : 1.0f) * (KIND == 2 ? 0x1p-30f : 0x1p-34f);
 #pragma unroll
     for (int q = 0; q < DgAcc<KIND, MT>::NT; ++q) {
-        float a = (acc.f[q][0] + 256.0f * acc.f[q][1]) * scale, b = (acc.f[q][2] + 256.0f * acc.f[q][3]) * scale;
-        a += __shfl_xor_sync(0xffffffffu, a, 1);
-        b += __shfl_xor_sync(0xffffffffu, b, 1);
+        float v[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            v[r] = (acc.f[q][2 * r] + 256.0f * acc.f[q][2 * r + 1]) * scale;
+            if (DgKind<KIND>::offset) {
+                // the four lanes of a row hold the offsets of two sub-blocks each for every token: lanes 0, 1 take the first
+                // token of the pair from lanes 2, 3, which take the second
+                const float o0 = acc.off[r][2 * q], o1 = acc.off[r][MT == 1 ? 0 : 2 * q + 1];
+                v[r] += (t < 2 ? o0 : o1) + __shfl_xor_sync(0xffffffffu, t < 2 ? o1 : o0, 2);
+            }
+            v[r] += __shfl_xor_sync(0xffffffffu, v[r], 1);
+        }
         const int tok = 2 * q + (t >> 1);
         if ((t & 1) == 0 && tok < MT) {
-            float *ra = red + g * MT + tok, *rb = red + (g + 8) * MT + tok;
-            *ra = DgKind<KIND>::mins ? *ra + a : a;
-            *rb = DgKind<KIND>::mins ? *rb + b : b;
+            red[g * MT + tok] = v[0];
+            red[(g + 8) * MT + tok] = v[1];
         }
     }
 }

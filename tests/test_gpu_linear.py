@@ -153,6 +153,25 @@ def test_linear_not_finite(oracle, kind, M):
         np.testing.assert_allclose(product(x).astype(np.float64)[fits], want[fits], **tol)
 
 
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("M", [1, 2, 5, 8])
+@pytest.mark.parametrize("mean", [0.0, 1.0])
+def test_linear_few_tokens_error_is_that_of_fp32(oracle, kind, M, mean):
+    """Against 64 bits: an output's share of 256 weights is rounded in its conversion, its scaling and its addition, three
+    times 2^-25 of it on average; twice 2^-24 of the output's norm in all.  With a mean as large as the deviation the
+    weights' offsets add up over a block to a term as large as the products, which doubles it."""
+    from gpu_util import dev, empty, host, ops
+    K, N = 1536, 512
+    r = np.random.default_rng(M + kind)
+    w = _w(oracle, r, N, K, kind)
+    exact = oracle.linear_exact(np.eye(K, dtype=np.float32), w, kind, K, K, N).astype(np.float64)
+    x = (r.standard_normal((M, K)) + mean).astype(np.float32)
+    y = empty((M, N))
+    ops.linear_forward_q4(dev(x), dev(w), y, M, K, N, kind)
+    want = x.astype(np.float64) @ exact
+    assert np.linalg.norm(host(y) - want) < (1 + mean) * 2.0 ** -23 * np.linalg.norm(want)
+
+
 def test_linear_argument_errors(oracle):
     from gpu_util import B200Error, empty, ops
     x, w, y = empty((1, 48)), empty(64, torch.uint8), empty((1, 2))
