@@ -1,10 +1,12 @@
 // The routed Q4_K experts of a decode batch on tcgen05, exact to fp32: every expert's weights are expanded once
 // for all the tokens that chose it.
 //
-// A Q4_K weight is d (s q) - dmin m with s q <= 945, an integer that fp16 holds exactly; d and dmin are constant
-// over 256 of K.  So the tensor cores multiply the integers (expanded in registers, first operand in tensor memory,
-// as in gemm_wt.cu), one accumulation per 256 of K, and the epilogue multiplies it by the row's d and takes off
-// dmin times the eight sub-block minima m times the sums of the activations.  An activation is three fp16 columns,
+// A Q4_K weight is d s (q - 8) + (8 d s - dmin m) with |s (q - 8)| <= 504, an integer that fp16 holds exactly; d and
+// dmin are constant over 256 of K, s and m over 32.  So the tensor cores multiply the integers (expanded in registers,
+// first operand in tensor memory, as in gemm_wt.cu), one accumulation per 256 of K, and the epilogue multiplies it by
+// the row's d and adds the eight offsets times the sums of the activations.  (With s q and the minima alone the two terms
+// cancel, and the tensor cores, which cut the last bits off a sum, show: 6e-7 .. 1.2e-6 of the output's norm against 64 bits,
+// 2.6e-7 so.)  An activation is three fp16 columns,
 // x = 2^e (a + 2^-11 b + 2^-22 c) with 2^e from the maximum of its 256 (33 bits below it), which the epilogue adds up:
 // a tile of up to 24 slots of one expert is 72 columns.
 // Everything moves in steps of 256 of K (per 64, as gemm_wt.cu does, the roles' waits took 4300 cycles per 256).
@@ -39,7 +41,7 @@ constexpr int WX_BOX = 24;                    // rows of a TMA box of activation
 constexpr int WX_X_SUB = 3 * WX_CAP * 128;    // 64 of K
 constexpr int WX_X_STAGE = 4 * WX_X_SUB;      // 256 of K
 constexpr int WX_SX = 2, WX_SP = 5;
-constexpr int WX_HDR = 4;                     // ring of (d, dmin, eight minima) per weight row, from the expansion to the epilogue
+constexpr int WX_HDR = 4;                     // ring of eight offsets and d per weight row, from the expansion to the epilogue
 constexpr int WX_AUX = 12;                    // floats per slot and 256 of K: 2^e, -, -, -, eight sub-block sums in units of 2^e
 constexpr int WX_SET = 128;                   // tensor-memory columns between the two accumulators, between the two operands
 constexpr int WX_OPERAND = 2 * WX_SET;
@@ -49,7 +51,7 @@ constexpr int WX_THREADS = (WX_SECOND_EPI + 4) * 32;
 constexpr int WX_HALF = WX_CAP / 2;           // slots of an epilogue group
 constexpr int WX_MAX_EXPERTS = 256, WX_TABLE = 64;
 constexpr int WX_SWAP = 2 * WX_CAP * WX_ROWS * 4;     // SwiGLU: gate and up rows of a tile, double buffered
-constexpr int WX_SMEM = 1024 + WX_SX * WX_X_STAGE + WX_SP * WX_PACKED + WX_SWAP + 8 * WX_HALF * WX_AUX * 4 + WX_HDR * WX_ROWS * 16 + 512 +
+constexpr int WX_SMEM = 1024 + WX_SX * WX_X_STAGE + WX_SP * WX_PACKED + WX_SWAP + 8 * WX_HALF * WX_AUX * 4 + WX_HDR * WX_ROWS * 36 + 512 +
                         (WX_MAX_EXPERTS + 4) * 4 + WX_TABLE * 16;
 static_assert(WX_SMEM <= 227 * 1024, "the stages do not fit the shared memory of an SM");
 
@@ -171,30 +173,30 @@ __device__ __forceinline__ WxTile wx_tile_at(const WxArgs& a, const int* first, 
     return WxTile{e.x, e.y, e.z & 0xFFFFF, e.w, sb0, min(a.K >> 8, sb0 + a.per_split)};
 }
 
-// 64 weights of a row (K step J of its 256) to the integers s q as 32 fp16 pairs, exact.
-// d_dmin: the row's two factors; mins: the two minima of these 64, a byte each.
+// 64 weights of a row (K step J of its 256) to the integers s (q - 8) as 32 fp16 pairs, exact.
+// d: the row's factor; off: 8 d s - dmin m of the two 32.
 template <int J>
-__device__ __forceinline__ void wx_expand(uint32_t seg, uint32_t (&out)[32], uint32_t& d_dmin, uint32_t& mins) {
+__device__ __forceinline__ void wx_expand(uint32_t seg, uint32_t (&out)[32], float& d, float2& off) {
     auto vec = [&](int i) {
         uint4 v;
         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(seg + 16 * i));
         return v;
     };
     const uint4 hdr = vec(0), q0 = vec(1 + 2 * J), q1 = vec(2 + 2 * J);
-    d_dmin = hdr.x;
-    mins = 0;
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hdr.x));
+    d = f.x;
     const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
         int s, m;
         q4k_scale_min_regs(2 * J + hh, hdr.y, hdr.z, hdr.w, s, m);
-        mins |= (uint32_t)m << (8 * hh);
-        // high nibbles stay where they are: 1024 + 16 q, times s / 16
-        const __half2 sc2 = __half2half2(__hmul(__int2half_rn(s), __float2half(hh ? 0.0625f : 1.0f)));
-        const __half2 nsc = __half2half2(__int2half_rn((hh ? -64 : -1024) * s));
+        (hh ? off.y : off.x) = __fsub_rn(8.0f * f.x * (float)s, f.y * (float)m);      // both products exact
+        // high nibbles stay where they are, low ones move there: 1024 + 16 q, times s / 16, less 72 s
+        const __half2 sc2 = __half2half2(__hmul(__int2half_rn(s), __float2half(0.0625f)));
+        const __half2 nsc = __half2half2(__int2half_rn(-72 * s));
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const uint32_t x = words[i] & (hh ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
+            const uint32_t x = (hh ? words[i] : words[i] << 4) & 0xF0F0F0F0u;
             out[16 * hh + 2 * i] = wt_bits(__hfma2(wt_magic(x, WT_SEL_01), sc2, nsc));
             out[16 * hh + 2 * i + 1] = wt_bits(__hfma2(wt_magic(x, WT_SEL_23), sc2, nsc));
         }
@@ -224,8 +226,9 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
     uint8_t* sm_p = sm_x + WX_SX * WX_X_STAGE;
     float* swap = reinterpret_cast<float*>(sm_p + WX_SP * WX_PACKED);
     float* sm_aux = swap + WX_SWAP / 4;                                // [8 warps][WX_HALF][WX_AUX]
-    uint4* sm_hdr = reinterpret_cast<uint4*>(sm_aux + 8 * WX_HALF * WX_AUX);      // [WX_HDR][WX_ROWS]
-    uint64_t* x_full = reinterpret_cast<uint64_t*>(sm_hdr + WX_HDR * WX_ROWS);
+    float4* sm_off = reinterpret_cast<float4*>(sm_aux + 8 * WX_HALF * WX_AUX);    // [WX_HDR][2][WX_ROWS]
+    float* sm_d = reinterpret_cast<float*>(sm_off + WX_HDR * 2 * WX_ROWS);        // [WX_HDR][WX_ROWS]
+    uint64_t* x_full = reinterpret_cast<uint64_t*>(sm_d + WX_HDR * WX_ROWS);
     uint64_t* x_empty = x_full + WX_SX;
     uint64_t* p_full = x_empty + WX_SX;
     uint64_t* p_empty = p_full + WX_SP;
@@ -371,14 +374,8 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
                 if (!ok) break;
                 ready = mbar_peek(&done[as ^ 1], ((ci + 1) >> 1) & 1);
                 tc_fence_after();
-                const uint4 hdr = sm_hdr[(ci % WX_HDR) * WX_ROWS + tid];
-                const float d = half_bits_to_float((uint16_t)(hdr.x & 0xFFFFu)), dmin = half_bits_to_float((uint16_t)(hdr.x >> 16));
-                float m[8];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    m[j] = (float)((hdr.y >> (8 * j)) & 0xFFu);
-                    m[4 + j] = (float)((hdr.z >> (8 * j)) & 0xFFu);
-                }
+                const float d = sm_d[(ci % WX_HDR) * WX_ROWS + tid];
+                const float4 o0 = sm_off[(ci % WX_HDR) * 2 * WX_ROWS + tid], o1 = sm_off[((ci % WX_HDR) * 2 + 1) * WX_ROWS + tid];
                 const uint32_t tq = tmem + as * WX_SET + ((uint32_t)(q * 32) << 16);
 #pragma unroll
                 for (int k = 0; k < WX_HALF / 4; ++k) {
@@ -390,9 +387,9 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
                             const float4* au = reinterpret_cast<const float4*>(aux + (4 * k + j) * WX_AUX);
                             const float4 s0 = au[1], s1 = au[2];
                             const float t = fmaf(fmaf(v[3 * j + 2], 0x1p-11f, v[3 * j + 1]), 0x1p-11f, v[3 * j]);
-                            const float lo = fmaf(m[3], s0.w, fmaf(m[2], s0.z, fmaf(m[1], s0.y, m[0] * s0.x)));
-                            const float hi = fmaf(m[7], s1.w, fmaf(m[6], s1.z, fmaf(m[5], s1.y, m[4] * s1.x)));
-                            acc[4 * k + j] = fmaf(au[0].x, fmaf(d, t, -dmin * (lo + hi)), acc[4 * k + j]);
+                            const float lo = fmaf(o0.w, s0.w, fmaf(o0.z, s0.z, fmaf(o0.y, s0.y, o0.x * s0.x)));
+                            const float hi = fmaf(o1.w, s1.w, fmaf(o1.z, s1.z, fmaf(o1.y, s1.y, o1.x * s1.x)));
+                            acc[4 * k + j] = fmaf(au[0].x, fmaf(d, t, lo + hi), acc[4 * k + j]);
                         }
                     }
                 }
@@ -446,20 +443,20 @@ __global__ void __launch_bounds__(WX_THREADS, 1) wx_kernel(const __grid_constant
             const uint32_t free_ahead = ci > 1 ? mbar_peek(&done[ci & 1], ((ci >> 1) - 1) & 1) : 1u;
             const uint32_t seg = row_at + p * WX_PACKED;
             uint32_t out[32];
-            uint32_t d_dmin, mins;
-            if (slot == 0) wx_expand<0>(seg, out, d_dmin, mins);
-            else if (slot == 1) wx_expand<1>(seg, out, d_dmin, mins);
-            else if (slot == 2) wx_expand<2>(seg, out, d_dmin, mins);
-            else wx_expand<3>(seg, out, d_dmin, mins);
+            float d;
+            float2 off;
+            if (slot == 0) wx_expand<0>(seg, out, d, off);
+            else if (slot == 1) wx_expand<1>(seg, out, d, off);
+            else if (slot == 2) wx_expand<2>(seg, out, d, off);
+            else wx_expand<3>(seg, out, d, off);
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_empty[p]);
             if (++p == WX_SP) { p = 0; ph ^= 1; }
             p_ready = mbar_peek(&p_full[p], ph);
             // (ci - 2 done: the epilogue has read ci - 4, whose header is overwritten below)
             if (!__all_sync(0xffffffffu, free_ahead != 0) && !mbar_wait_warp(&done[ci & 1], ((ci >> 1) - 1) & 1, a.status)) break;
-            uint8_t* hd = reinterpret_cast<uint8_t*>(sm_hdr + (ci % WX_HDR) * WX_ROWS + q * 32 + lane);
-            if (slot == 0) *reinterpret_cast<uint32_t*>(hd) = d_dmin;
-            *reinterpret_cast<uint16_t*>(hd + 4 + 2 * slot) = (uint16_t)mins;
+            if (slot == 0) sm_d[(ci % WX_HDR) * WX_ROWS + q * 32 + lane] = d;
+            reinterpret_cast<float2*>(sm_off + ((ci % WX_HDR) * 2 + (slot >> 1)) * WX_ROWS + q * 32 + lane)[slot & 1] = off;
             tc_fence_after();
             tmem_st32(dst + (ci & 1) * WX_SET, out);
             tc_fence_before();

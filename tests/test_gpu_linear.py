@@ -172,6 +172,23 @@ def test_linear_few_tokens_error_is_that_of_fp32(oracle, kind, M, mean):
     assert np.linalg.norm(host(y) - want) < (1 + mean) * 2.0 ** -23 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("M", [9, 16, 31])
+def test_linear_tens_of_tokens_error(oracle, M):
+    """The exact tensor-core form of Q4_K against 64 bits: the tensor cores cut each of the sixteen additions of an accumulation
+    towards zero, by half of 2^-23 of the running sum on average, and the running sum grows as the root of its length: two
+    thirds of 16 half units, 5.3 of 2^-24, and one for the fp32 sums behind it."""
+    from gpu_util import dev, empty, host, ops
+    K, N = 1536, 512
+    r = np.random.default_rng(M)
+    w = _w(oracle, r, N, K, 3)
+    exact = oracle.linear_exact(np.eye(K, dtype=np.float32), w, 3, K, K, N).astype(np.float64)
+    x = r.standard_normal((M, K)).astype(np.float32)
+    y = empty((M, N))
+    ops.linear_forward_q4(dev(x), dev(w), y, M, K, N, 3)
+    want = x.astype(np.float64) @ exact
+    assert np.linalg.norm(host(y) - want) < 6.3 * 2.0 ** -24 * np.linalg.norm(want)
+
+
 def test_linear_argument_errors(oracle):
     from gpu_util import B200Error, empty, ops
     x, w, y = empty((1, 48)), empty(64, torch.uint8), empty((1, 2))
