@@ -55,7 +55,7 @@ int moe_units_forward(const float* x, const int32_t* grouped, const int32_t* off
                       const void* downs, float* act, float* y, void* units_scratch, int64_t N, int d, int E, int ne, int K,
                       int kind);
 // moe_exact.cu: the same for Q4_K on the large tensor cores; scratch: moe_exact_bytes.
-int linear_exact(const float* x, const void* w, float* y, int M, int K, int N);
+int linear_exact(const float* x, const void* w, float* y, int M, int K, int N, const void* w_up = nullptr);
 size_t moe_exact_bytes(int64_t NK, int d, int E);
 int moe_exact_forward(const float* x, const int32_t* grouped, const int32_t* offsets, const void* gates, const void* ups,
                       const void* downs, float* act, float* y, void* scratch, int64_t N, int d, int E, int ne, int K);

@@ -526,11 +526,13 @@ int moe_exact_forward(const float* x, const int32_t* grouped, const int32_t* off
 }
 
 // One Q4_K matrix for a few tens of tokens, exact to fp32: y [M, N] = x [M, K] . w [N, K]^T; K a multiple of 256, N of 4.
-// Few tiles: K is cut across CTAs and the partial sums are added in a fixed order.
-int linear_exact(const float* x, const void* w, float* y, int M, int K, int N) {
+// Few tiles: K is cut across CTAs and the partial sums are added in a fixed order.  With w_up: y = silu(x . w^T) * (x . w_up^T),
+// K whole (a gate and its up must be complete).
+int linear_exact(const float* x, const void* w, float* y, int M, int K, int N, const void* w_up) {
     WxArgs a;
-    a.n_tiles = ceil_div(N, WX_ROWS);
-    const int chunks = K / 256, tiles = ceil_div(M, WX_CAP) * a.n_tiles;
+    const int rows = w_up ? WX_ROWS / 2 : WX_ROWS;
+    a.n_tiles = ceil_div(N, rows);
+    const int chunks = K / 256, tiles = w_up ? num_sms() : ceil_div(M, WX_CAP) * a.n_tiles;
     a.per_split = ceil_div(chunks, std::max(1, std::min(chunks, num_sms() / tiles)));
     a.k_splits = ceil_div(chunks, a.per_split);
     a.split_stride = a.k_splits > 1 ? (int64_t)M * N : 0;
@@ -542,15 +544,15 @@ int linear_exact(const float* x, const void* w, float* y, int M, int K, int N) {
     __half* cols = static_cast<__half*>(ws);
     float* aux = reinterpret_cast<float*>(static_cast<char*>(ws) + cols_bytes);
     if ((rc = make_tile_map(&a.map_x, cols, 3 * (int64_t)M, K, WX_BOX))) return rc;
-    if ((rc = make_packed_map(&a.map_w, w, N, (int64_t)chunks * WX_SBB, WX_SBB, WX_ROWS))) return rc;
-    a.map_w2 = a.map_w;
+    if ((rc = make_packed_map(&a.map_w, w, N, (int64_t)chunks * WX_SBB, WX_SBB, rows))) return rc;
+    if ((rc = make_packed_map(&a.map_w2, w_up ? w_up : w, N, (int64_t)chunks * WX_SBB, WX_SBB, rows))) return rc;
     a.offsets = nullptr; a.aux = aux; a.ne = 1; a.M = M; a.N = N; a.K = K;
     a.c = part ? static_cast<float*>(part) : y;
     a.status = stream_status_ptr();
     B200_REQUIRE(a.status, "linear_exact: status word allocation failed");
     wx_split_kernel<<<(unsigned)ceil_div(M * chunks, 8), 256, 0, stream()>>>(x, nullptr, 1, M, K, cols, aux);
     B200_LAUNCH_CHECK("wx_split_kernel");
-    if ((rc = launch_wx<false, true>(a, M))) return rc;
+    if ((rc = w_up ? launch_wx<true, false>(a, M) : launch_wx<false, true>(a, M))) return rc;
     return part ? splitk_reduce(a.c, y, a.k_splits, a.split_stride, M, N, N) : B200_OK;
 }
 

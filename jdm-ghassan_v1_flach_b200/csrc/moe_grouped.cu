@@ -164,7 +164,7 @@ int moe_forward_grouped(const float* x, const float* router_w, const float* rout
 // ===========================================================================
 // A decode batch (more tokens than the token-major kernels take, fewer than fill the
 // tensor-core tiles of every expert): routing and permutation as above, the routed experts
-// through moe_exact.cu or moe_units.cu, the shared expert as a GEMM on the side stream, the same k-ordered
+// through moe_exact.cu or moe_units.cu, the shared expert beside them on the side stream, the same k-ordered
 // combination.
 // ===========================================================================
 int moe_combine(const float* y, const int32_t* inv, const float* w, float* out, int64_t N, int d, int K, bool accumulate);
@@ -178,12 +178,15 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
     // digit engine costs by the slot.  Experts of 512 x 1536: 54 against 67 us at 9 tokens (1.2 slots per expert of
     // the 64), 85 against 84 at 28; of 768 x 4096: 275 against 186 at 9 tokens already.
     const bool exact = kind == 3 && (2 * NK >= 5 * (size_t)ne || (int64_t)E * d >= (1 << 21));
+    // Below the row count from which products round their activations to fp16, the shared expert must not either: its GEMM
+    // would leave 9e-4 of the output's norm where the routed experts leave 3e-7.
+    const bool shared_exact = shared && kind == 3 && N < GEMM_MIN_ROWS;
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
     const size_t o_idx = take(NK * 4), o_w = take(NK * 4), o_grp = take(NK * 4), o_inv = take(NK * 4),
                  o_off = take((size_t)(ne + 1) * 4), o_units = take(exact ? moe_exact_bytes((int64_t)NK, d, E) : moe_units_table_bytes((int64_t)NK, ne)),
                  o_act = take(NK * E * 4), o_y = take(NK * d * 4),
-                 o_sh = shared ? take(moe_shared_scratch_bytes(N, d, SH)) : 0;
+                 o_sh = shared ? take(shared_exact ? (size_t)N * SH * 4 : moe_shared_scratch_bytes(N, d, SH)) : 0;
     void* wsp;
     int rc = workspace(WS_MOE).ensure(off + 256, &wsp);
     if (rc) return rc;
@@ -197,7 +200,13 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
     float* y = reinterpret_cast<float*>(base + o_y);
     if (shared) {
         if ((rc = side_begin())) return rc;
-        rc = moe_shared_expert(x, sh_g, sh_u, sh_d, out, N, d, SH, kind, base + o_sh);
+        if (shared_exact) {
+            float* sh_act = reinterpret_cast<float*>(base + o_sh);
+            rc = linear_exact(x, sh_g, sh_act, (int)N, d, SH, sh_u);
+            if (!rc) rc = linear_exact(sh_act, sh_d, out, (int)N, SH, d);
+        } else {
+            rc = moe_shared_expert(x, sh_g, sh_u, sh_d, out, N, d, SH, kind, base + o_sh);
+        }
         const int rc2 = side_end();
         if (rc) return rc;
         if (rc2) return rc2;

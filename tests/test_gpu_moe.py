@@ -103,6 +103,18 @@ def test_layer_decode_batch_without_shared_expert_is_fp32_tight(oracle, wkind, N
     assert np.array_equal(got["out"].view(np.uint32), again["out"].view(np.uint32))      # run-to-run bit-stable
 
 
+@pytest.mark.parametrize("d,E,ne,K,SH", [(512, 256, 64, 6, 256), (1536, 512, 64, 6, 1024)])
+@pytest.mark.parametrize("N", [9, 24, 25, 31])
+def test_layer_of_tens_of_tokens_is_fp32_tight(oracle, d, E, ne, K, SH, N):
+    """Q4_K below the row count from which products round to fp16 (32): the shared expert as exact as the routed ones."""
+    from gpu_util import SUM_ORDER
+    c = moe_case(oracle, 70 + N, N, d, E, ne, K, SH, 3)
+    got = _run(c, N, d, E, ne, K, SH, 3)
+    out, _, idx, _ = _oracle(oracle, c, d, E, ne, K, SH, 3)
+    assert np.array_equal(got["idx"], idx)
+    np.testing.assert_allclose(got["out"], out, **SUM_ORDER)
+
+
 def test_layer_config3_4096_tokens(oracle):
     """The prefill-sized case: routing checked on every token, outputs on a sample of
     tokens (a token's output depends on no other token), and run-to-run bit stability."""
