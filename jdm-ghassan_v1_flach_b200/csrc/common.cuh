@@ -68,6 +68,22 @@ struct NvtxRange {
 int side_begin();
 int side_end();
 int side_wait();
+// Joins when it goes out of scope after an error, so that nothing is left running beside what the caller does next (and
+// no capture ends with a branch open).
+struct SideJoin {
+    bool open = false;
+    int begin() {
+        const int rc = side_begin();
+        open = rc == 0;
+        return rc;
+    }
+    int wait() {
+        const bool was = open;
+        open = false;
+        return was ? side_wait() : 0;
+    }
+    ~SideJoin() { wait(); }
+};
 
 // Status word of the kernels with bounded waits (0 = ok).  Device pointer, allocated
 // on first use; the check reads it back (synchronising copy) and clears it.

@@ -50,6 +50,7 @@ int moe_experts_rows(const __half* rows16, const int32_t* offsets, const int32_t
                      float* const* y_groups = nullptr);
 // moe_units.cu: the routed experts of a decode batch as weight streams shared by the tokens
 // that chose them (few-token dot engine, exact dequantised weights).
+bool moe_units_takes(int d, int E, int kind);             // whether its tiles fit the shared memory
 size_t moe_units_table_bytes(int64_t NK, int ne);
 int moe_units_forward(const float* x, const int32_t* grouped, const int32_t* offsets, const void* gates, const void* ups,
                       const void* downs, float* act, float* y, void* units_scratch, int64_t N, int d, int E, int ne, int K,

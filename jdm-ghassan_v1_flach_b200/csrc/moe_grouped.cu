@@ -109,6 +109,7 @@ int moe_forward_grouped(const float* x, const float* router_w, const float* rout
     };
 
     for (int64_t t0 = 0; t0 < N; t0 += chunk) {
+        SideJoin side;
         const int T = (int)std::min<int64_t>(chunk, N - t0);
         const int64_t NK = (int64_t)T * K;
         const float* xc = x + t0 * d;
@@ -123,7 +124,7 @@ int moe_forward_grouped(const float* x, const float* router_w, const float* rout
         // The shared expert shares no data with routing, permutation, gather and the routed
         // experts until the combine: it runs on the side stream next to them, straight into out.
         if (shared) {
-            if ((rc = side_begin())) return rc;
+            if ((rc = side.begin())) return rc;
             rc = pack_rows_f16(xc, nullptr, 1, H(o_xs), T, d);
             if (!rc)
                 rc = gemm(GEMM_EPI_SWIGLU, H(o_xs), T, sh_g, sh_u, sg16, su16, SH, nullptr, 1, T, SH, d, nullptr,
@@ -152,7 +153,7 @@ int moe_forward_grouped(const float* x, const float* router_w, const float* rout
         rc = gemm(GEMM_EPI_STORE, H(o_act), NK, downs, nullptr, d16, nullptr, (int64_t)ne * d, offsets, ne, (int)NK, d, E,
                   y, nullptr, d);
         if (rc) return rc;
-        if (shared && (rc = side_wait())) return rc;
+        if ((rc = side.wait())) return rc;
         const int64_t total = (int64_t)T * (d >> 2);
         const int grid = (int)std::min<int64_t>(ceil_div64(total, 256), (int64_t)num_sms() * 16);
         moe_combine_kernel<<<grid, 256, 0, stream()>>>(y, inv, w, oc, T, K, d, shared ? 1 : 0);
@@ -178,6 +179,7 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
     // digit engine costs by the slot.  Experts of 512 x 1536: 54 against 67 us at 9 tokens (1.2 slots per expert of
     // the 64), 85 against 84 at 28; of 768 x 4096: 275 against 186 at 9 tokens already.
     const bool exact = kind == 3 && (2 * NK >= 5 * (size_t)ne || (int64_t)E * d >= (1 << 21));
+    if (!exact && !moe_units_takes(d, E, kind)) return B200_EUNSUPPORTED;       // before anything is launched
     // Below the row count from which products round their activations to fp16, the shared expert must not either: its GEMM
     // would leave 9e-4 of the output's norm where the routed experts leave 3e-7.
     const bool shared_exact = shared && kind == 3 && N < GEMM_MIN_ROWS;
@@ -198,8 +200,9 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
     int32_t* offsets = reinterpret_cast<int32_t*>(base + o_off);
     float* act = reinterpret_cast<float*>(base + o_act);
     float* y = reinterpret_cast<float*>(base + o_y);
+    SideJoin side;
     if (shared) {
-        if ((rc = side_begin())) return rc;
+        if ((rc = side.begin())) return rc;
         if (shared_exact) {
             float* sh_act = reinterpret_cast<float*>(base + o_sh);
             rc = linear_exact(x, sh_g, sh_act, (int)N, d, SH, sh_u);
@@ -218,7 +221,7 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
     rc = exact ? moe_exact_forward(x, grouped, offsets, gates, ups, downs, act, y, base + o_units, N, d, E, ne, K)
                : moe_units_forward(x, grouped, offsets, gates, ups, downs, act, y, base + o_units, N, d, E, ne, K, kind);
     if (rc) return rc;
-    if (shared && (rc = side_wait())) return rc;
+    if ((rc = side.wait())) return rc;
     return moe_combine(y, inv, w, out, N, d, K, shared);
 }
 

@@ -181,25 +181,31 @@ __global__ void __launch_bounds__(dg_warps(UNIT_SLOTS) * 32, 2) moe_units_kernel
     }
 }
 
+// Rows of a tile, tiles of a set, warps of a contraction; dynamic shared memory, 0 if the width does not fit.
 template <int KIND, bool DOWN>
-static int launch_units(MoeUnitArgs a) {
+static size_t plan_units(MoeUnitArgs& a) {
     const int Kd = DOWN ? a.E : a.d, N = DOWN ? a.d : a.E, chunks = dg_chunks(Kd);
     const size_t rb = row_bytes_of(KIND, Kd), x = (dg_x_bytes<KIND>(chunks, UNIT_SLOTS) + 15) & ~(size_t)15;
-    if (chunks > 255) return fail(B200_EUNSUPPORTED, "moe_units: width %d does not fit the shared-memory staging", Kd);
-    a.chunks_inv = dg_inv(chunks);
-    size_t smem = 0;
+    if (chunks > 255) return 0;
     for (const size_t budget : {(size_t)SMEM_BUDGET - 1024, (size_t)SMEM_BUDGET_FULL})
-        for (int R = DOWN ? 16 : 8; R >= 4 && !smem; R >>= 1)
-            for (int G = 8; G >= 1 && !smem; G >>= 1) {
+        for (int R = DOWN ? 16 : 8; R >= 4; R >>= 1)
+            for (int G = 8; G >= 1; G >>= 1) {
                 if ((R * rb) % 16 != 0 || ((N % R) * rb) % 16 != 0) continue;
                 a.part_rows = R;
                 a.G = G;
                 a.P = dg_parts(G, chunks, dg_warps(UNIT_SLOTS));
                 a.stage_bytes = (int)(((DOWN ? 1 : 2) * R * rb + 127) / 128 * 128);
                 const size_t need = 2 * (size_t)G * a.stage_bytes + x + (size_t)2 * G * a.P * dg_red_floats(UNIT_SLOTS) * 4 + 128;
-                if (need <= budget) smem = need;
+                if (need <= budget) return need;
             }
+    return 0;
+}
+template <int KIND, bool DOWN>
+static int launch_units(MoeUnitArgs a) {
+    const int Kd = DOWN ? a.E : a.d;
+    const size_t smem = plan_units<KIND, DOWN>(a);
     if (!smem) return fail(B200_EUNSUPPORTED, "moe_units: width %d does not fit the shared-memory staging", Kd);
+    a.chunks_inv = dg_inv(dg_chunks(Kd));
     a.p_inv = dg_inv(a.P);
     auto kern = moe_units_kernel<KIND, DOWN>;
     static bool configured = false;
@@ -210,6 +216,22 @@ static int launch_units(MoeUnitArgs a) {
     }
     const int per_sm = smem <= (size_t)SMEM_BUDGET ? 2 : 1;
     return launch_pdl(kern, dim3(per_sm * num_sms()), dim3(dg_warps(UNIT_SLOTS) * 32), smem, a);
+}
+template <int KIND>
+static bool units_take(int d, int E) {
+    MoeUnitArgs a;
+    a.d = d; a.E = E;
+    return plan_units<KIND, false>(a) && plan_units<KIND, true>(a);
+}
+bool moe_units_takes(int d, int E, int kind) {
+    switch (kind) {
+        case 0: return units_take<0>(d, E);
+        case 1: return units_take<1>(d, E);
+        case 2: return units_take<2>(d, E);
+        case 3: return units_take<3>(d, E);
+        case KIND_F16: return units_take<KIND_F16>(d, E);
+        default: return false;
+    }
 }
 template <int KIND>
 static int moe_units_kind(const MoeUnitArgs& a) {

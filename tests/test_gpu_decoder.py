@@ -230,3 +230,20 @@ def test_errors(oracle):
     with pytest.raises(B200Error, match="not set"):
         lib.b200_decoder_step_host(h, tok.ctypes.data, tok.ctypes.data)
     lib.b200_decoder_destroy(h)
+
+
+def test_recorded_step_of_experts_too_wide_for_the_unit_kernels(oracle):
+    """Nine sequences, rows too wide for the unit kernels' staging: the layer is refused there before anything is on the
+    second stream, so the recording of the step has no branch left open and its outputs are the eager step's."""
+    cfg = dict(TINY, hidden=7168, n_layers=1, layer_types=[0], qkind=2, n_experts=4, top_k=1, expert_dim=64, shared_dim=256,
+               mamba_heads=4, mamba_d_state=64)
+    m = make_model(oracle, cfg, seed=1)
+    toks = np.random.default_rng(2).integers(0, cfg["vocab"], (3, 9)).astype(np.int32)
+    got = []
+    for graph in (0, 1):
+        dec = CudaDecoder(m, 9, 8)
+        dec.configure(0, graph)
+        for t in toks:
+            dec.step_host(t)
+        got.append(dec.logits())
+    assert np.array_equal(got[0], got[1]) and np.isfinite(got[0]).all()
