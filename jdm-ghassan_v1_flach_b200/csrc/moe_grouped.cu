@@ -181,14 +181,16 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
     const bool exact = kind == 3 && (2 * NK >= 5 * (size_t)ne || (int64_t)E * d >= (1 << 21));
     if (!exact && !moe_units_takes(d, E, kind)) return B200_EUNSUPPORTED;       // before anything is launched
     // Below the row count from which products round their activations to fp16, the shared expert must not either: its GEMM
-    // would leave 9e-4 of the output's norm where the routed experts leave 3e-7.
-    const bool shared_exact = shared && kind == 3 && N < GEMM_MIN_ROWS;
+    // would leave 9e-4 of the output's norm where the routed experts leave 3e-7.  The kinds without the exact tensor-core
+    // form pay for it in passes of eight tokens (31 tokens, Q8_0, 512 x 1536: 106 us with the GEMM, 141 without), so they do it
+    // only for rows as wide as the layer took token by token in fp32 before (768 x 4096: 606, 530 with the GEMM; 3800 there).
+    const bool shared_exact = shared && N < GEMM_MIN_ROWS && (kind == 3 || d >= 4096);
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
     const size_t o_idx = take(NK * 4), o_w = take(NK * 4), o_grp = take(NK * 4), o_inv = take(NK * 4),
                  o_off = take((size_t)(ne + 1) * 4), o_units = take(exact ? moe_exact_bytes((int64_t)NK, d, E) : moe_units_table_bytes((int64_t)NK, ne)),
                  o_act = take(NK * E * 4), o_y = take(NK * d * 4),
-                 o_sh = shared ? take(shared_exact ? (size_t)N * SH * 4 : moe_shared_scratch_bytes(N, d, SH)) : 0;
+                 o_sh = shared ? take(shared_exact ? (size_t)N * SH * 8 : moe_shared_scratch_bytes(N, d, SH)) : 0;
     void* wsp;
     int rc = workspace(WS_MOE).ensure(off + 256, &wsp);
     if (rc) return rc;
@@ -205,8 +207,15 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
         if ((rc = side.begin())) return rc;
         if (shared_exact) {
             float* sh_act = reinterpret_cast<float*>(base + o_sh);
-            rc = linear_exact(x, sh_g, sh_act, (int)N, d, SH, sh_u);
-            if (!rc) rc = linear_exact(sh_act, sh_d, out, (int)N, SH, d);
+            if (kind == 3) {
+                rc = linear_exact(x, sh_g, sh_act, (int)N, d, SH, sh_u);
+            } else {
+                float* sh_up = sh_act + N * SH;
+                rc = linear(x, sh_g, kind, sh_act, (int)N, d, SH);
+                if (!rc) rc = linear(x, sh_u, kind, sh_up, (int)N, d, SH);
+                if (!rc) rc = b200_swiglu_forward(sh_act, sh_up, sh_act, N * SH);
+            }
+            if (!rc) rc = linear(sh_act, sh_d, kind, out, (int)N, SH, d);
         } else {
             rc = moe_shared_expert(x, sh_g, sh_u, sh_d, out, N, d, SH, kind, base + o_sh);
         }
