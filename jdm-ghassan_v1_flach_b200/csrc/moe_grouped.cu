@@ -176,9 +176,14 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
     const bool shared = sh_g && sh_u && sh_d && SH > 0;
     const size_t NK = (size_t)N * K;
     // The exact tensor-core form costs about the same for one slot of an expert as for 24, and some 20 us of set-up; the
-    // digit engine costs by the slot.  Experts of 512 x 1536: 54 against 67 us at 9 tokens (1.2 slots per expert of
-    // the 64), 85 against 84 at 28; of 768 x 4096: 275 against 186 at 9 tokens already.
-    const bool exact = kind == 3 && (2 * NK >= 5 * (size_t)ne || (int64_t)E * d >= (1 << 21));
+    // digit engine costs by the slot, and by the row's width once a unit's staged tokens leave it few rows to a tile.
+    // Layers with a shared expert, exact against digits, us (E x d; slots per expert):
+    //   512 x 1536: 76 / 68 (0.8)  78 / 70 (1.1)  78 / 80 (1.5)  88 / 96 (2.9)     256 x 1536: 66 / 63 (0.8)  68 / 72 (1.5)
+    //   768 x 1536: 90 / 78 (0.8)  98 / 96 (1.5)  98 / 102 (1.9)                  1024 x 2048: 119 / 104 (1.1)  129 / 137 (1.5)
+    //   768 x 2048: 92 / 86 (1.1)  100 / 104 (1.5)                                1536 x 2048: 106 / 96 (1.5)  115 / 121 (2.0)
+    //   512 x 2560: 96 / 98 (0.8)  106 / 109 (1.1)  105 / 117 (1.5)                512 x 4096: 117 / 115 (0.8)  135 / 150 (1.1)
+    //   768 x 4096: 180 / 205 (1.2)  229 / 270 (4.3)
+    const bool exact = kind == 3 && (2 * NK >= 3 * (size_t)ne || d >= 2560);
     if (!exact && !moe_units_takes(d, E, kind)) return B200_EUNSUPPORTED;       // before anything is launched
     // Below the row count from which products round their activations to fp16, the shared expert must not either: its GEMM
     // would leave 9e-4 of the output's norm where the routed experts leave 3e-7.  The kinds without the exact tensor-core

@@ -115,12 +115,13 @@ def test_layer_of_tens_of_tokens_is_fp32_tight(oracle, d, E, ne, K, SH, N):
     np.testing.assert_allclose(got["out"], out, **SUM_ORDER)
 
 
-@pytest.mark.parametrize("wkind", [0, 2])
+@pytest.mark.parametrize("wkind", [0, 2, 3])
 @pytest.mark.parametrize("N", [9, 31])
 def test_layer_of_tens_of_tokens_with_wide_rows(oracle, wkind, N):
-    """Rows of 4096: the unit kernels' staging takes a whole SM and four rows of gate and up; the shared expert stays fp32."""
+    """Rows of 4096: the unit kernels' staging takes a whole SM and four rows of gate and up, Q4_K goes to the exact form
+    however few slots an expert has; the shared expert stays fp32."""
     from gpu_util import SUM_ORDER
-    d, E, ne, K, SH = 4096, 64, 16, 2, 256
+    d, E, ne, K, SH = 4096, 256 if wkind == 3 else 64, 16, 2, 256
     c = moe_case(oracle, 80 + N, N, d, E, ne, K, SH, wkind)
     got = _run(c, N, d, E, ne, K, SH, wkind)
     out, _, idx, _ = _oracle(oracle, c, d, E, ne, K, SH, wkind)
