@@ -40,10 +40,10 @@ struct DgKind {
 
 __host__ __device__ inline int dg_chunks(int K) { return (K + DG_CHUNK - 1) / DG_CHUNK; }
 // Staged activations of a chunk and token: four digit bytes each, the sub-block sums and the
-// scale; for fp16 weights the two fp16 parts of each, in columns of their own.
+// scale; for fp16 weights the three fp16 parts of each (all 24 bits), in columns of their own.
 constexpr int DG_COL = DG_CHUNK * 2 + 64;     // bytes of an fp16 column: two neighbours fall into different halves of the banks
 template <int KIND>
-__host__ __device__ constexpr int dg_chunk_bytes() { return (KIND == KIND_F16 ? 2 * DG_COL : DG_CHUNK * 4 + 32) + 4; }
+__host__ __device__ constexpr int dg_chunk_bytes() { return (KIND == KIND_F16 ? 3 * DG_COL : DG_CHUNK * 4 + 32) + 4; }
 template <int KIND>
 __host__ __device__ inline size_t dg_x_bytes(int chunks, int tokens) { return (size_t)chunks * tokens * dg_chunk_bytes<KIND>() + 16; }
 
@@ -52,13 +52,13 @@ int dg_parts(int tiles, int chunks, int warps);      // decode_gemv.cu
 #ifdef __CUDACC__
 // Packed weights: digits [sub-block][token][slot][32 bytes], slot = (digit + sub-block) & 3 (so that the stores
 // of a warp spread over the banks); sub-block sums times the scale [chunk][token][8]; scales [chunk][token].
-// fp16 weights: columns [chunk][token][part][DG_COL bytes]; scales.
+// fp16 weights: columns [chunk][part][token][DG_COL bytes]; scales.
 template <int KIND, int MT>
 struct DgX {
     uint32_t dig, sum, scale;                 // shared addresses
     __device__ __forceinline__ uint8_t* carve(uint8_t* p, int chunks) {
         dig = smem_u32(p);
-        sum = dig + chunks * MT * (KIND == KIND_F16 ? 2 * DG_COL : DG_CHUNK * 4);
+        sum = dig + chunks * MT * (KIND == KIND_F16 ? 3 * DG_COL : DG_CHUNK * 4);
         scale = sum + (KIND == KIND_F16 ? 0 : chunks * MT * 32);
         return p + dg_x_bytes<KIND>(chunks, MT);
     }
@@ -105,18 +105,23 @@ __device__ __forceinline__ void dg_stage(const DgX<KIND, MT>& xd, int chunk, int
     if (lane == 0) sts_u32(xd.scale + (chunk * MT + m) * 4, __float_as_uint(unit));
     if (KIND == KIND_F16) {
         const float up = __uint_as_float((uint32_t)(127 + 10 - e) << 23);
-        uint32_t hi[4], lo[4];
+        uint32_t p[3][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const __half2 h = __floats2half2_rn(v[2 * i] * up, v[2 * i + 1] * up);
-            const float2 f = __half22float2(h);
-            const __half2 l = __floats2half2_rn(v[2 * i] * up - f.x, v[2 * i + 1] * up - f.y);
-            hi[i] = *reinterpret_cast<const uint32_t*>(&h);
-            lo[i] = *reinterpret_cast<const uint32_t*>(&l);
+            float2 r = make_float2(v[2 * i] * up, v[2 * i + 1] * up);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const __half2 h = __floats2half2_rn(r.x, r.y);
+                const float2 f = __half22float2(h);
+                p[j][i] = *reinterpret_cast<const uint32_t*>(&h);
+                r = make_float2(r.x - f.x, r.y - f.y);
+            }
         }
-        const uint32_t at = xd.dig + (chunk * MT + m) * 2 * DG_COL + 16 * lane;
-        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
-        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(at + DG_COL), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
+        const uint32_t at = xd.dig + (chunk * 3 * MT + m) * DG_COL + 16 * lane;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(at + j * MT * DG_COL), "r"(p[j][0]), "r"(p[j][1]), "r"(p[j][2]), "r"(p[j][3])
+                         : "memory");
         return;
     }
     const float to_int = __uint_as_float((uint32_t)(127 + 30 - e) << 23), down = to_int * 0x1p-30f;
@@ -190,10 +195,12 @@ __device__ __forceinline__ void dg_norm8(const float* w, int k, int K, float (&v
 
 // One warp's accumulators for a 16-row tile.  Packed: f[q] the digit columns of tokens 2 q, 2 q + 1 (lane
 // (g, t): rows g, g + 8; token 2 q + t / 2, digits 2 (t & 1), + 1), off the offsets of this lane's sub-blocks
-// (rows g, g + 8; each token).  fp16: f[q] the two parts of token 4 q + t.
+// (rows g, g + 8; each token).  fp16: the operand's eight columns are Wd
+// = 2, 4 or 8 tokens of 4, 2 or 1 parts; f[q] columns 2 t, 2 t + 1 (rows g, g + 8).
 template <int KIND, int MT>
 struct DgAcc {
-    static constexpr int NT = KIND == KIND_F16 ? (MT <= 4 ? 1 : 2) : (MT <= 2 ? 1 : MT / 2);
+    static constexpr int Wd = MT <= 2 ? 2 : MT;
+    static constexpr int NT = KIND == KIND_F16 ? (3 * Wd + 7) / 8 : (MT <= 2 ? 1 : MT / 2);
     static constexpr int NO = DgKind<KIND>::offset ? MT : 1;
     float f[NT][4], off[2][NO];
     __device__ __forceinline__ void clear() {
@@ -214,31 +221,37 @@ __device__ __forceinline__ void dg_chunk(DgAcc<KIND, MT>& acc, uint32_t row_a, u
     constexpr int NT = DgAcc<KIND, MT>::NT;
     const int g = lane >> 2, t = lane & 3, dgt = g & 3;
     if (KIND == KIND_F16) {
+        constexpr int Wd = DgAcc<KIND, MT>::Wd;
+        // a column past the third part repeats it (dg_finish leaves it out), one past the tokens repeats the last token
         uint32_t col[NT];
-        float c[NT][4];
+        float sum[NT][4];
 #pragma unroll
         for (int q = 0; q < NT; ++q) {
-            col[q] = xd.dig + (xc * MT + min(4 * q + (g >> 1), MT - 1)) * 2 * DG_COL + (g & 1) * DG_COL + 16 * t;
+            col[q] = xd.dig + ((xc * 3 + min((8 * q + g) / Wd, 2)) * MT + min(g % Wd, MT - 1)) * DG_COL + 16 * t;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) c[q][i] = 0.0f;
+            for (int i = 0; i < 4; ++i) sum[q][i] = 0.0f;
         }
+        // The tensor cores cut a sum's last bits off where an addition rounds them: 32 of K at a time.
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
             if (s >= nb) break;
             const uint4 a = lds_u4(row_a + 64 * s + 16 * t), b = lds_u4(row_b + 64 * s + 16 * t);
 #pragma unroll
             for (int q = 0; q < NT; ++q) {
+                float c[4] = {0.f, 0.f, 0.f, 0.f};
                 const uint4 x = lds_u4(col[q] + 64 * s);
-                mma_16816(c[q], a.x, b.x, a.y, b.y, x.x, x.y);
-                mma_16816(c[q], a.z, b.z, a.w, b.w, x.z, x.w);
+                mma_16816(c, a.x, b.x, a.y, b.y, x.x, x.y);
+                mma_16816(c, a.z, b.z, a.w, b.w, x.z, x.w);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sum[q][i] += c[i];
             }
         }
+        const uint32_t xs = xd.scale + xc * MT * 4;
+        const float x0 = lds_f32(xs + min(2 * t % Wd, MT - 1) * 4), x1 = lds_f32(xs + min(2 * t % Wd + 1, MT - 1) * 4);
 #pragma unroll
-        for (int q = 0; q < NT; ++q) {
-            const float xs = lds_f32(xd.scale + (xc * MT + min(4 * q + t, MT - 1)) * 4);
+        for (int q = 0; q < NT; ++q)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) acc.f[q][i] += xs * c[q][i];
-        }
+            for (int i = 0; i < 4; ++i) acc.f[q][i] += (i & 1 ? x1 : x0) * sum[q][i];
         return;
     }
     const uint32_t xb = xd.dig + xc * 8 * MT * 128 + 8 * t + (MT == 1 ? 0 : (g >> 2) * 128);
@@ -365,13 +378,30 @@ constexpr int dg_red_floats(int MT) { return 16 * MT; }
 template <int KIND, int MT>
 __device__ __forceinline__ void dg_finish(const DgAcc<KIND, MT>& acc, float* red, int lane) {
     const int g = lane >> 2, t = lane & 3;
-    if (KIND == KIND_F16) {
+    if constexpr (KIND == KIND_F16) {
+        constexpr int Wd = DgAcc<KIND, MT>::Wd;
+        float v[4];                           // tokens 2 t % Wd, + 1; rows g, g + 8
 #pragma unroll
-        for (int q = 0; q < DgAcc<KIND, MT>::NT; ++q)
-            if (4 * q + t < MT) {
-                red[g * MT + 4 * q + t] = acc.f[q][0] + acc.f[q][1];
-                red[(g + 8) * MT + 4 * q + t] = acc.f[q][2] + acc.f[q][3];
+        for (int i = 0; i < 4; ++i) {
+            if constexpr (Wd == 8) {
+                v[i] = acc.f[0][i] + (acc.f[1][i] + acc.f[2][i]);
+            } else if constexpr (Wd == 4) {   // f[0]: high parts in lanes 0, 1, middle ones in 2, 3; f[1]: low ones in 0, 1
+                v[i] = acc.f[0][i] + (t < 2 ? acc.f[1][i] : 0.0f);
+                v[i] += __shfl_xor_sync(0xffffffffu, v[i], 2);
+            } else {                          // lane t: part t
+                v[i] = t < 3 ? acc.f[0][i] : 0.0f;
+                v[i] += __shfl_xor_sync(0xffffffffu, v[i], 2);
+                v[i] += __shfl_xor_sync(0xffffffffu, v[i], 1);
             }
+        }
+        if (2 * t < Wd) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (2 * t + i < MT) {
+                    red[g * MT + 2 * t + i] = v[i];
+                    red[(g + 8) * MT + 2 * t + i] = v[2 + i];
+                }
+        }
         return;
     }
     const float scale = ((t & 1) ? 65536.0f : 1.0f) * (KIND == 2 ? 0x1p-30f : 0x1p-34f);

@@ -188,7 +188,7 @@ static size_t plan_units(MoeUnitArgs& a) {
     const size_t rb = row_bytes_of(KIND, Kd), x = (dg_x_bytes<KIND>(chunks, UNIT_SLOTS) + 15) & ~(size_t)15;
     if (chunks > 255) return 0;
     for (const size_t budget : {(size_t)SMEM_BUDGET - 1024, (size_t)SMEM_OPT_IN - 1024})        // two CTAs on an SM, or one
-        for (int R = DOWN ? 16 : 8; R >= 4; R >>= 1)
+        for (int R = DOWN ? 16 : 8; R >= 1; R >>= 1)
             for (int G = 8; G >= 1; G >>= 1) {
                 if ((R * rb) % 16 != 0 || ((N % R) * rb) % 16 != 0) continue;
                 a.part_rows = R;

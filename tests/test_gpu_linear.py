@@ -172,6 +172,23 @@ def test_linear_few_tokens_error_is_that_of_fp32(oracle, kind, M, mean):
     assert np.linalg.norm(host(y) - want) < (1 + mean) * 2.0 ** -23 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("K", [768, 4096])
+@pytest.mark.parametrize("M", [1, 2, 3, 8])
+def test_linear_fp16_few_tokens_error_is_that_of_fp32(K, M):
+    """fp16 weights against 64 bits: the activations' three fp16 parts hold all their bits, 32 of K are summed on the tensor
+    cores (two additions cut, by half of 2^-23 of the running sum on average), eight such sums and then the chunks of 256 added
+    in fp32, whose roundings grow as the root of their number: two and a half of 2^-24 in all."""
+    from gpu_util import dev, empty, host, ops
+    N = 512
+    r = np.random.default_rng(M + K)
+    w = (r.standard_normal((N, K)) * 0.02).astype(np.float16)
+    x = r.standard_normal((M, K)).astype(np.float32)
+    y = empty((M, N))
+    ops.linear_forward_fp16(dev(x), dev(w.view(np.uint16)), y, M, K, N)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    assert np.linalg.norm(host(y) - want) < 2.5 * 2.0 ** -24 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("M", [9, 16, 31])
 def test_linear_tens_of_tokens_error(oracle, M):
     """The exact tensor-core form of Q4_K against 64 bits: the tensor cores cut each of the sixteen additions of an accumulation
