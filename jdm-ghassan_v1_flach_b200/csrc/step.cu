@@ -397,7 +397,22 @@ static int enqueue_step_fused(b200_decoder* dec, const int32_t* tokens, int32_t*
     }
     SgArgs h = base(dec->lm_head, dec->vocab, d, dec->x, d);
     h.norm_w = dec->final_norm; h.y = dec->logits; h.y_stride = dec->vocab; h.out_scale = 1.0f / dec->logits_scaling;
-    STEP(stream_gemv(h, KIND_F16, PRO_RMS, EPI_STORE));
+    // all sequences at once where their staged rows leave room for the weights (eight of hidden sizes below 3840), else in
+    // groups; the step is refused only if one does not
+    int group = B;
+    for (SgArgs probe = h; group > 1; group = (group + 1) / 2) {
+        probe.dry = true;
+        probe.M = group;
+        if ((rc = stream_gemv(probe, KIND_F16, PRO_RMS, EPI_STORE)) == B200_OK) break;
+        if (rc != B200_EUNSUPPORTED) return rc;
+    }
+    for (int b = 0; b < B; b += group) {
+        SgArgs part = h;
+        part.M = std::min(group, B - b);
+        part.x += (int64_t)b * part.x_stride;
+        part.y += (int64_t)b * part.y_stride;
+        STEP(stream_gemv(part, KIND_F16, PRO_RMS, EPI_STORE));
+    }
     if (dry) return B200_OK;
     STEP(pick_next(dec, dec->logits, tokens, 1, next, 0, B));
 #undef STEP

@@ -247,3 +247,19 @@ def test_recorded_step_of_experts_too_wide_for_the_unit_kernels(oracle):
             dec.step_host(t)
         got.append(dec.logits())
     assert np.array_equal(got[0], got[1]) and np.isfinite(got[0]).all()
+
+
+@pytest.mark.parametrize("B", [5, 8])
+def test_fused_step_with_a_wide_lm_head(oracle, B):
+    """Hidden size 4096: eight sequences' staged rows leave no room for an lm_head row, so it goes in groups."""
+    cfg = dict(TINY, hidden=4096, n_layers=1, layer_types=[0], n_experts=4, top_k=1, mamba_heads=4, mamba_d_state=64)
+    m = make_model(oracle, cfg, seed=3)
+    toks = np.random.default_rng(B).integers(0, cfg["vocab"], (2, B)).astype(np.int32)
+    got = []
+    for fused in (0, 1):
+        dec = CudaDecoder(m, B, 8)
+        dec.configure(fused, 0)
+        for t in toks:
+            dec.step_host(t)
+        got.append(dec.logits())
+    np.testing.assert_allclose(got[1], got[0], rtol=1e-4, atol=1e-4 * np.abs(got[0]).max())
