@@ -95,8 +95,8 @@ mamba_step_scan_kernel(const float* __restrict__ bc, const float* __restrict__ d
     const float* Cv = Bv + p.d_state;
     float* s = ssm_state + ((int64_t)m * rows + row) * p.d_state;
     float acc = 0.0f;
-    if (p.d_state == 128) {
-        // one 128-bit access per lane covers the row (same products, same order per element)
+    if (p.d_state == 128 && (reinterpret_cast<uintptr_t>(s) & 15) == 0) {
+        // one 128-bit access per lane covers the row (same products per element)
         float4 sv = *reinterpret_cast<const float4*>(s + lane * 4);
         const float4 b4 = *reinterpret_cast<const float4*>(Bv + lane * 4);
         const float4 c4 = *reinterpret_cast<const float4*>(Cv + lane * 4);

@@ -83,6 +83,24 @@ def test_step_batched(oracle, batch):
         close(host(dcs)[b], wcs, batch, SUM_ORDER)
 
 
+@pytest.mark.parametrize("batch", [1, 2, 3])
+def test_step_with_the_state_at_any_float_address(oracle, batch):
+    from gpu_util import SUM_ORDER, dev, empty, host, ops
+    c = mamba_case(oracle, 250 + batch, B=batch, T=1, d=256, n_heads=4, d_head=64, d_state=128, k=4, wkind=3)
+    (x, w_in, conv_w, conv_b, dt_bias, a_log, D, norm_w, w_out, state,
+     _, _, d, d_inner, conv_dim, n_heads, d_head, d_state, k, eps) = c["args"]
+    got = []
+    for shift in (0, 1):
+        ss = torch.zeros(state.size + shift, device="cuda")[shift:]
+        ss.copy_(torch.from_numpy(np.ascontiguousarray(state).reshape(-1)))
+        dcs, out = torch.zeros(batch, conv_dim, k - 1, device="cuda"), empty((batch, d))
+        ops.mamba2_step_batched(dev(x[:, 0]), *_dev_params((w_in, conv_w, conv_b, dt_bias, a_log, D, norm_w, w_out)), dcs, ss, out, batch, d,
+                                d_inner, conv_dim, n_heads, d_head, d_state, k, eps, 3)
+        got.append((host(out), host(ss)))
+    np.testing.assert_allclose(got[1][0], got[0][0], **SUM_ORDER)
+    assert np.array_equal(got[1][1], got[0][1])
+
+
 @pytest.mark.parametrize("B,T", [(1, 1), (2, 7), (1, 33), (3, 64), (1, 300), (2, 513)])
 @pytest.mark.parametrize("wkind", [-2, 2, 3])
 def test_forward_sequence(oracle, B, T, wkind):
