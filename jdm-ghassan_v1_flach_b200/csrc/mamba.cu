@@ -513,10 +513,13 @@ template <int KIND>
 static int launch_inproj_conv(const float* x, const uint8_t* w_in, const float* conv_w, const float* conv_b,
                               float* conv_state, float* gate, float* bc, float* dt_raw, int M, const MambaDims& p) {
     const int grid = ceil_div(p.proj, GEMV_WARPS);
-    if (M == 1) mamba_inproj_conv_kernel<KIND, 1><<<grid, GEMV_THREADS, 0, stream()>>>(x, w_in, conv_w, conv_b, conv_state, gate, bc, dt_raw, M, p);
-    else if (M == 2) mamba_inproj_conv_kernel<KIND, 2><<<grid, GEMV_THREADS, 0, stream()>>>(x, w_in, conv_w, conv_b, conv_state, gate, bc, dt_raw, M, p);
-    else if (M <= 4) mamba_inproj_conv_kernel<KIND, 4><<<grid, GEMV_THREADS, 0, stream()>>>(x, w_in, conv_w, conv_b, conv_state, gate, bc, dt_raw, M, p);
-    else mamba_inproj_conv_kernel<KIND, 8><<<grid, GEMV_THREADS, 0, stream()>>>(x, w_in, conv_w, conv_b, conv_state, gate, bc, dt_raw, M, p);
+    auto go = [&](auto kern) { kern<<<grid, GEMV_THREADS, 0, stream()>>>(x, w_in, conv_w, conv_b, conv_state, gate, bc, dt_raw, M, p); };
+    if (M == 1) go(mamba_inproj_conv_kernel<KIND, 1>);
+    else if (M == 2) go(mamba_inproj_conv_kernel<KIND, 2>);
+    else if constexpr (KIND == KIND_F32) {                   // the other kinds of more sequences: mamba2_step's product of its own
+        if (M <= 4) go(mamba_inproj_conv_kernel<KIND, 4>);
+        else go(mamba_inproj_conv_kernel<KIND, 8>);
+    }
     B200_LAUNCH_CHECK("mamba_inproj_conv_kernel");
     return B200_OK;
 }

@@ -132,12 +132,10 @@ __device__ int draw_sorted(const uint64_t* keys, double* probs, int n, float tem
     return key_id(keys[limit - 1]);
 }
 
-// Candidate sets of up to CAND_SMEM_MAX entries: sort and draw in shared memory.  Input
-// either as (vals, ids) [rows, K] or as keys [rows, K].
+// Candidate sets (vals, ids) [rows, K] of up to CAND_SMEM_MAX entries: sort and draw in shared memory.
 __global__ void __launch_bounds__(256) draw_small_kernel(const float* __restrict__ vals, const int32_t* __restrict__ ids,
-                                                         const uint64_t* __restrict__ keys_in, int K, float temperature,
-                                                         float top_p, float min_p, uint64_t* __restrict__ rng,
-                                                         int32_t* __restrict__ next) {
+                                                         int K, float temperature, float top_p, float min_p,
+                                                         uint64_t* __restrict__ rng, int32_t* __restrict__ next) {
     __shared__ uint64_t keys[CAND_SMEM_MAX];
     __shared__ double probs[CAND_SMEM_MAX];
     const int r = blockIdx.x;
@@ -145,7 +143,7 @@ __global__ void __launch_bounds__(256) draw_small_kernel(const float* __restrict
     while (n2 < K) n2 <<= 1;
     for (int i = threadIdx.x; i < n2; i += blockDim.x) {
         uint64_t k = 0;      // below every real candidate
-        if (i < K) k = keys_in ? keys_in[(int64_t)r * K + i] : cand_key(vals[(int64_t)r * K + i], ids[(int64_t)r * K + i]);
+        if (i < K) k = cand_key(vals[(int64_t)r * K + i], ids[(int64_t)r * K + i]);
         keys[i] = k;
     }
     __syncthreads();
@@ -641,8 +639,7 @@ int b200_sample_candidates(const float* vals_dev, const int32_t* ids_dev, int K,
                            uint64_t* rng_state_dev, int32_t* next_dev) {
     B200_REQUIRE(vals_dev && ids_dev && cfg && rng_state_dev && next_dev, "sample_candidates: null pointer");
     B200_REQUIRE(K >= 1 && K <= CAND_SMEM_MAX && rows >= 1, "sample_candidates: K must be in [1, %d]", CAND_SMEM_MAX);
-    draw_small_kernel<<<rows, 256, 0, stream()>>>(vals_dev, ids_dev, nullptr, K, cfg->temperature, cfg->top_p, cfg->min_p,
-                                                  rng_state_dev, next_dev);
+    draw_small_kernel<<<rows, 256, 0, stream()>>>(vals_dev, ids_dev, K, cfg->temperature, cfg->top_p, cfg->min_p, rng_state_dev, next_dev);
     B200_LAUNCH_CHECK("draw_small_kernel");
     return B200_OK;
 }

@@ -70,8 +70,8 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, uint32_t
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Host: a short kernel whose first instruction is pdl_wait(), launched so that it is set up while the kernel before it
-// ends (about a microsecond of a decode step's short kernels each).
+// Host: a short kernel that lets its dependents start and then waits, before it touches memory, launched so that it is set up
+// while the kernel before it ends (about a microsecond of a decode step's short kernels each).
 template <typename... P, typename... A>
 static int launch_short(void (*kern)(P...), dim3 grid, dim3 block, const A&... args) {
     cudaLaunchConfig_t cfg = {};
