@@ -64,7 +64,8 @@ int b200_decoder_reset(b200_decoder* dec);
  * fused = 1: cross-op fusions (norm into the following projection's prologue,
  * residual add into the epilogue); returns B200_EUNSUPPORTED, leaving the mode
  * unchanged, when a matrix of the model cannot be cut into 16-byte-aligned row
- * tiles (the per-op mode has no such limit).
+ * tiles, or its tiles and the staged activations do not fit the shared memory (the
+ * per-op mode has no such limits).  Matrices must be 16-byte aligned, norm weights not.
  * fused = 2 (batch 1 only): the Mamba and MoE phases of the token run inside one
  * persistent cooperative kernel per run of layers between attention layers (all CTAs
  * resident, weights streamed across phase boundaries, bounded grid barriers); attention

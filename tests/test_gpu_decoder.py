@@ -263,3 +263,29 @@ def test_fused_step_with_a_wide_lm_head(oracle, B):
             dec.step_host(t)
         got.append(dec.logits())
     np.testing.assert_allclose(got[1], got[0], rtol=1e-4, atol=1e-4 * np.abs(got[0]).max())
+
+
+@pytest.mark.parametrize("qkind", [2, 3])
+def test_batches_of_any_size_agree_when_the_routing_is_held(oracle, qkind):
+    """The same sequence decoded alone, among 2, 5, 8, 9, 20 and 31: the step's kernels differ (digit engine of one to eight
+    columns, exact tensor-core form, units), the logits must not by more than fp32 rounding.  The router is switched off
+    (equal probabilities, the choice by the bias alone), as a near-tie that comes out the other way hides everything else.
+    Per layer five products, each off by up to 2^-22 of its norm, of independent signs: 2^-22 sqrt(5 * 4 layers) on the logits;
+    four times that where the products are the exact tensor-core form's (cut sums: 6.3 of 2^-24 each, one direction within a
+    product, so that layers' errors add up rather than cancel).  Q8_0 from 9 sequences on: the shared expert's fp16 GEMM (2^-11 per activation, averaged over the row: 5e-4)."""
+    m = make_model(oracle, dict(TINY, qkind=qkind), seed=11)
+    for i, L in enumerate(m["layers"]):
+        L["router"] = np.zeros_like(L["router"])
+        L["router_bias"] = np.random.default_rng(i).permutation(L["router_bias"].size).astype(np.float32)
+    toks = np.random.default_rng(5).integers(0, TINY["vocab"], (6, 31)).astype(np.int32)
+    want = None
+    for B in (1, 2, 5, 8, 9, 20, 31):
+        dec = CudaDecoder(m, B, 16)
+        dec.configure(1 if B <= 8 else 0, 0)
+        for t in toks:
+            dec.step_host(t[:B])
+        got = dec.logits()[0].astype(np.float64)
+        if want is None:
+            want = got
+        bound = 2.0 ** -22 * 20 ** 0.5 * (1 if B <= 8 else 4) if B <= 8 or qkind == 3 else 5e-4
+        assert np.linalg.norm(got - want) < bound * np.linalg.norm(want), (B, np.linalg.norm(got - want) / np.linalg.norm(want))
