@@ -665,7 +665,7 @@ def moe_sweep_bench(lib, sizes=(1, 64, 512, 4096)):
         out.append({"tokens": T, "ms_per_layer": ms, "experts_touched": touched, "weight_bytes": wbytes,
                     "achieved_gbs": gbs, "frac_of_hbm_peak": gbs / hbm_peak, "tflops": tfs,
                     "frac_of_dense_peak": tfs / tf_peak, "bound": bound,
-                    "operands": "fp32 (exact dequantised weights; the shared expert as an fp16 tensor-core GEMM from 9 tokens on)"
+                    "operands": "fp32 (exact dequantised weights; the shared expert as an fp16 tensor-core GEMM from 32 tokens on)"
                                 if T * K <= 12 * ne else "fp16 x in-kernel dequantised Q4_K, fp32 accumulation"})
     return out
 
@@ -1113,7 +1113,7 @@ def main():
             "warmup": W, "ms_per_step": ms_dev / args.steps, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic", "config": workload_config(cfg, args),
             "dtype_note": "the decode step computes in fp32 on exact dequantised weights (activations enter the "
-                          "dot products as fp16 head + tail pairs, 22 bits); every many-token block states its own operands",
+                          "dot products as integers of 31 bits, the fp16 lm_head as three fp16 parts, 33 bits); every many-token block states its own operands",
             "e2e": {"value": e2e_tok_s, "unit": "tok/s", "h2d_bytes_per_step": 4 * B, "d2h_bytes_per_step": 4 * B,
                     "ms_per_step": ms_e2e / args.steps},
             "gpu_launches": launches_per_step * args.steps,

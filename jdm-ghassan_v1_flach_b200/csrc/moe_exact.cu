@@ -17,11 +17,11 @@
 //   warps 8..23   expansion: four groups of four warps, 64 of the 256 each, into one of two operands
 // The SwiGLU form puts 64 gate rows and the same 64 up rows in one tile.  All waits are bounded (gemm_umma.cu).
 //
-// Bound by instructions issued (58 % of the slots: the expansion, the epilogue's sums) and the waits between the roles,
+// Bound by instructions issued (63 % of the slots: the expansion, the epilogue's sums) and the waits between the roles,
 // 1930 cycles per 128 rows x 256 of K, 2.2 times what the bytes alone take.  Tried without effect: a third accumulator,
 // packed rows by 16-byte asynchronous copies instead of TMA, deeper rings.
 // 64 tokens, H-Tiny: gate / up 47 us and down 58 on the digit engine (moe_units.cu), 38 and 22 here; 48 tokens, H-Small:
-// the layer 450 us before, 227 now.
+// the layer 450 us before, 237 now.
 #include <algorithm>
 
 #include "gemm.cuh"
