@@ -502,10 +502,24 @@ static EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-int make_tile_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, int box_rows) {
-    B200_REQUIRE(base && rows > 0 && K > 0 && K % 8 == 0, "tile map: K must be a positive multiple of 8");
+// box_steps 0: a 2-D map with boxes of 64 x box_rows.  Otherwise 3-D, [K / 64][rows][64], with boxes of box_steps runs of 64.
+static int encode_tile_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, int box_rows, int box_steps) {
+    B200_REQUIRE(base && rows > 0 && K > 0 && K % (box_steps ? GM_TILE_K : 8) == 0, "tile map: K must be a positive multiple of 8");
     B200_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, "tile map: base must be 16-byte aligned");
     B200_REQUIRE(box_rows >= 8 && box_rows <= 256, "tile map: bad box");
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return fail(B200_ECUDA, "tile map: the driver does not export cuTensorMapEncodeTiled");
+    const cuuint64_t dims[3] = {(cuuint64_t)(box_steps ? GM_TILE_K : K), (cuuint64_t)rows, (cuuint64_t)(K / GM_TILE_K)};
+    const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)GM_TILE_K * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)GM_TILE_K, (cuuint32_t)box_rows, (cuuint32_t)box_steps};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, box_steps ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(B200_ECUDA, "tile map: cuTensorMapEncodeTiled failed with %d", (int)r);
+    return B200_OK;
+}
+int make_tile_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, int box_rows) {
     typedef std::tuple<const void*, int64_t, int64_t, int> Key;
     static std::map<Key, CUtensorMap> cache;
     static std::mutex mu;
@@ -516,19 +530,14 @@ int make_tile_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, i
         *out = it->second;
         return B200_OK;
     }
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) return fail(B200_ECUDA, "tile map: the driver does not export cuTensorMapEncodeTiled");
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)GM_TILE_K, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(B200_ECUDA, "tile map: cuTensorMapEncodeTiled failed with %d", (int)r);
+    const int rc = encode_tile_map(out, base, rows, K, box_rows, 0);
+    if (rc) return rc;
     if (cache.size() > 4096) cache.clear();
     cache[key] = *out;
     return B200_OK;
+}
+int make_stage_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, int box_rows, int box_steps) {
+    return encode_tile_map(out, base, rows, K, box_rows, box_steps);
 }
 
 // Tensor map over packed rows viewed as 32-bit words: boxes of (box_bytes / 4) words

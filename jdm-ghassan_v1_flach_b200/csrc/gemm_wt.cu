@@ -12,19 +12,33 @@
 // Tensor memory: two accumulator sets of 192 columns (the epilogue of a tile under the main loop of the next) and
 // four operand slots of 32 columns (64 fp16 of K).  The SwiGLU form puts 64 gate rows and the same 64 up rows
 // in one tile and exchanges them through shared memory in the epilogue.
-//   warp 0        token rows by TMA (64 of K per stage, boxes of 96 and 32 rows)
+//   warp 0        token rows by TMA: one load per stage of 64 of K (128 for at most 96 rows), from one of twelve 3-D maps
 //   warp 2        packed rows by TMA (256 of K per stage)
-//   warp 1        MMA issue
+//   warp 1        MMA issue, a stage per round
 //   warps 4..7    epilogue: a lane holds one weight row, so a warp stores 32 consecutive outputs of a token
 //   warps 8..23   expansion: four groups of four warps, group = operand slot = K step mod 4
+// A stage of token rows has one pair of barriers for everything that its MMAs read and free: `full` counts the load and
+// the expanding warps' arrivals, `empty` one commit; the operand slots need none of their own.
 // Group lists (the MoE experts): rows of A cut into consecutive ranges by device offsets; a range is cut into
 // equal token tiles.  All waits are bounded; see gemm_umma.cu for what happens when one runs out.
 //
-// 4096 x 6448 x 1536 Q4_K: 106 us before, 90 now (both
-// with the 13 us that round the activations), a K step 600 cycles: what is left is the token rows' way from L2, 29 KB
-// per step and SM, where 256 weight rows per CTA would halve it but leave no room for a second accumulator set
-// (tried: the exposed epilogue cost more than the traffic).
+// What bounds it: with six warps at a scheduler an instruction of a role costs four to five cycles, so a role that does
+// little per K step still takes hundreds of cycles for it.  Clock stamps showed the loads of token rows (two to four TMA
+// instructions per K step with their addresses, a wait and two barriers) at some 600 cycles for 384 of tensor work, and the
+// MMA warp's round (a wait, four MMAs, two commits) at 430.  Hence one load and one commit per stage, stages of 128 where
+// the rows leave room, descriptors by their low word, and a look before the counted wait.  In us, before and after:
+//   8188 x 6448 x 1536 Q4_K  164.9 -> 142.4 (16 of them round the activations; 1290 TFLOP/s without)
+//   8188 x 1536 x 3072        107.6 -> 95.3      4096 x 6448 x 1536  93.2 -> 82.9
+//   64 experts of 1536 x 512, gate | up and down: 384 rows each 156.7 -> 142.3, 192: 101 -> 91, 48: 76.8 -> 56.4, 16: 70.7 -> 52.1
+//   72 experts of 4096 x 768, 72 rows each: 216 -> 157 (the weights' way from HBM: 60)
+// With the expansion left out the last takes 130: few rows are bound by the hand-overs between the roles and by issue slots.
+// Slower: two K steps per expanding warp and turn (the second one's expansion sits between two MMA rounds), stages of
+// constant number in the MMA warp (no difference once the loads are quick).
 #include <algorithm>
+#include <iterator>
+#include <map>
+#include <mutex>
+#include <tuple>
 
 #include "gemm.cuh"
 #include "linear.cuh"
@@ -38,8 +52,8 @@ int splitk_reduce(const float* part, float* c, int splits, int64_t stride, int M
 
 constexpr int WT_TOKENS = 192;                // most tokens of a tile
 constexpr int WT_ROWS = 128;                  // weight rows of a tile
-constexpr int WT_BOX = 32, WT_BIG_BOX = 96;   // token rows of a TMA box; one big box instead of three small ones: 5 %
-constexpr int WT_X_STAGE = WT_TOKENS * 128;   // 64 fp16 of K per token row
+constexpr int WT_BOX = 16;                    // token rows are loaded in multiples of this, the MMA's granularity of N
+constexpr int WT_X_STAGE = WT_TOKENS * 128;   // 64 fp16 of K per token row, or 128 of at most 96 rows
 constexpr int WT_SLOT0 = 2 * WT_TOKENS;       // first tensor-memory column of the operand slots
 constexpr int WT_SLOT = 32, WT_SLOTS = 4;
 constexpr int WT_SWAP = 2 * 2 * 16 * 64 * 4;  // SwiGLU epilogue: [buffer][half][token][row] floats
@@ -47,10 +61,12 @@ constexpr int WT_FIRST_EXPAND = 8;
 constexpr int WT_EXPAND_WARPS = 16;
 constexpr int WT_THREADS = (WT_FIRST_EXPAND + WT_EXPAND_WARPS) * 32;
 constexpr int WT_TABLE = 64;                  // a CTA's tiles worked out in advance; later ones on the way
+constexpr int WT_LISTS = (3 * 256 + 2) * 4;
 constexpr int WT_MAX_GROUPS = 256;            // group lists kept as a prefix table; longer ones are walked
 
 struct alignas(64) WtArgs {
-    CUtensorMap map_x, map_x_big, map_w, map_w2;
+    CUtensorMap map_x[WT_TOKENS / WT_BOX];    // a stage of 16, 32 .. 192 token rows in one load
+    CUtensorMap map_w, map_w2;
     const int32_t* offsets;                   // device [groups + 1], or null: one group of M rows
     const int32_t* group_map;                 // device [groups]: block of N weight rows a group uses (negative: skipped)
     int M, groups, N, K;
@@ -69,10 +85,10 @@ template <bool SWIGLU, int KIND>
 struct WtShape {
     static constexpr int SBB = 8 * (KIND == 3 ? 18 : q_block_bytes(KIND));     // bytes of 256 weights
     static constexpr int PACKED = WT_ROWS * SBB;
-    static constexpr int SX = 5;
-    static constexpr int SP = KIND == 2 ? 2 : 3;
+    static constexpr int SX = SWIGLU ? 5 : 6;                                 // at least 4: see the expansion
+    static constexpr int SP = KIND == 2 ? 2 : KIND == 1 && !SWIGLU ? 3 : 4;
     static constexpr int TILE_N = SWIGLU ? WT_ROWS / 2 : WT_ROWS;              // output columns of a tile
-    static constexpr int SMEM = SX * WT_X_STAGE + SP * PACKED + (SWIGLU ? WT_SWAP : 0) + 1024 + 256 + (WT_MAX_GROUPS + 2) * 4 + WT_TABLE * 24;
+    static constexpr int SMEM = SX * WT_X_STAGE + SP * PACKED + (SWIGLU ? WT_SWAP : 0) + 1024 + 256 + WT_LISTS + WT_TABLE * 24;
     static_assert(SMEM <= 227 * 1024, "the stages do not fit the shared memory of an SM");
 };
 
@@ -88,32 +104,37 @@ __device__ __forceinline__ void wt_cut(int rows, int i, int& first, int& count) 
     count = max(0, min(size, rows - first));
 }
 
-// first[g] = first token tile of group g; first[groups] = all of them.  All threads.
-__device__ __noinline__ void wt_build(const WtArgs& a, int* first) {
+// Group lists of at most WT_MAX_GROUPS: the offsets and each group's first token tile (first[groups] = all of them) in
+// shared memory, so that the searches below touch global memory once, and with one latency.  All threads.
+struct WtLists {
+    int first[WT_MAX_GROUPS + 1], offset[WT_MAX_GROUPS + 1], block[WT_MAX_GROUPS];
+};
+__device__ __forceinline__ void wt_build(const WtArgs& a, WtLists& l) {
     if (!a.offsets || a.groups > WT_MAX_GROUPS) return;
-    for (int g = threadIdx.x; g < a.groups; g += blockDim.x)
-        first[g] = (a.group_map && a.group_map[g] < 0) ? 0 : wt_tiles(a.offsets[g + 1] - a.offsets[g]);
+    for (int g = threadIdx.x; g <= a.groups; g += blockDim.x) {
+        l.offset[g] = a.offsets[g];
+        if (g < a.groups) l.block[g] = a.group_map ? a.group_map[g] : g;
+    }
     __syncthreads();
     if (threadIdx.x < 32) {
         int carry = 0;
         for (int g0 = 0; g0 < a.groups; g0 += 32) {
-            const int g = g0 + threadIdx.x, n = g < a.groups ? first[g] : 0;
+            const int g = g0 + threadIdx.x, n = g < a.groups && l.block[g] >= 0 ? wt_tiles(l.offset[g + 1] - l.offset[g]) : 0;
             int incl = n;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int up = __shfl_up_sync(0xffffffffu, incl, o);
                 if ((int)threadIdx.x >= o) incl += up;
             }
-            __syncwarp();
-            if (g < a.groups) first[g] = carry + incl - n;
+            if (g < a.groups) l.first[g] = carry + incl - n;
             carry += __shfl_sync(0xffffffffu, incl, 31);
         }
-        if (threadIdx.x == 0) first[a.groups] = carry;
+        if (threadIdx.x == 0) l.first[a.groups] = carry;
     }
     __syncthreads();
 }
 
-__device__ __noinline__ bool wt_find(const WtArgs& a, const int* first, int t, WtTile& w) {
+__device__ __forceinline__ bool wt_find(const WtArgs& a, const WtLists& l, int t, WtTile& w) {
     w.split = 0;
     if (a.k_splits > 1) {
         w.split = t % a.k_splits;
@@ -122,17 +143,21 @@ __device__ __noinline__ bool wt_find(const WtArgs& a, const int* first, int t, W
     const int slot = t / a.n_tiles;
     w.n0 = t - slot * a.n_tiles;              // weight tile; scaled by the caller's tile width
     w.group = 0;
+    w.brow = 0;
     int lo = 0, hi = a.M, i = slot;
     if (a.offsets) {
         if (a.groups <= WT_MAX_GROUPS) {
-            if (slot >= first[a.groups]) return false;
-            int l = 0, h = a.groups;          // the last group whose first tile is <= slot owns it
-            while (h - l > 1) {
-                const int mid = (l + h) >> 1;
-                if (first[mid] <= slot) l = mid; else h = mid;
+            if (slot >= l.first[a.groups]) return false;
+            int g = 0, h = a.groups;          // the last group whose first tile is <= slot owns it
+            while (h - g > 1) {
+                const int mid = (g + h) >> 1;
+                if (l.first[mid] <= slot) g = mid; else h = mid;
             }
-            w.group = l;
-            i = slot - first[l];
+            w.group = g;
+            i = slot - l.first[g];
+            lo = l.offset[g];
+            hi = l.offset[g + 1];
+            w.brow = l.block[g] * a.N;
         } else {
             int g = 0;
             for (; g < a.groups; ++g) {
@@ -142,29 +167,42 @@ __device__ __noinline__ bool wt_find(const WtArgs& a, const int* first, int t, W
             }
             if (g == a.groups) return false;
             w.group = g;
+            lo = a.offsets[g];
+            hi = a.offsets[g + 1];
+            w.brow = (a.group_map ? a.group_map[g] : g) * a.N;
         }
-        lo = a.offsets[w.group];
-        hi = a.offsets[w.group + 1];
     }
     wt_cut(hi - lo, i, w.row0, w.rows);
     w.row0 += lo;
-    w.brow = (a.group_map ? a.group_map[w.group] : w.group) * a.N;
     return w.rows > 0;
+}
+__device__ __noinline__ bool wt_find_late(const WtArgs& a, const WtLists& l, int t, WtTile& w) { return wt_find(a, l, t, w); }
+
+// A stage of token rows, and with it one round of the MMA warp, is 64 of K, or 128 where the tile's rows fill no more than
+// half of it (a ring of mostly empty stages is shorter than the latency that it has to cover): log2 of the K steps of 64.
+__host__ __device__ __forceinline__ int wt_unit(int rows) { return rows > WT_TOKENS / 2 ? 0 : 1; }
+__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
 }
 
 // Tile number i of this CTA.  The search (divisions, bisection) takes over a thousand cycles, which every role would
 // otherwise spend between two tiles of a few thousand: one thread per tile does it when the kernel starts.
-__device__ __forceinline__ void wt_fill(const WtArgs& a, const int* first, int* table, int total) {
+__device__ __forceinline__ void wt_fill(const WtArgs& a, const WtLists& l, int* table, int total) {
     const int t = blockIdx.x + threadIdx.x * gridDim.x;
     if (threadIdx.x < WT_TABLE && t < total) {
         WtTile w{0, 0, 0, 0, 0, 0};
-        if (!wt_find(a, first, t, w)) w.rows = 0;
+        if (!wt_find(a, l, t, w)) w.rows = 0;
         int* e = table + 6 * threadIdx.x;
         e[0] = w.group; e[1] = w.row0; e[2] = w.rows; e[3] = w.n0; e[4] = w.brow; e[5] = w.split;
     }
 }
-__device__ __forceinline__ bool wt_tile_at(const WtArgs& a, const int* first, const int* table, int i, WtTile& w) {
-    if (i >= WT_TABLE) return wt_find(a, first, blockIdx.x + i * gridDim.x, w);
+__device__ __forceinline__ bool wt_tile_at(const WtArgs& a, const WtLists& l, const int* table, int i, WtTile& w) {
+    if (i >= WT_TABLE) {
+        WtTile late;                          // its address is taken: w itself stays in registers
+        const bool ok = wt_find_late(a, l, blockIdx.x + i * gridDim.x, late);
+        w = late;
+        return ok;
+    }
     const int* e = table + 6 * i;
     w.group = e[0]; w.row0 = e[1]; w.rows = e[2]; w.n0 = e[3]; w.brow = e[4]; w.split = e[5];
     return w.rows > 0;
@@ -192,10 +230,14 @@ __device__ __forceinline__ void wt_expand(uint32_t seg, uint32_t (&out)[32]) {
         for (int hh = 0; hh < 2; ++hh) {
             int s, m;
             q4k_scale_min_regs(2 * J + hh, hdr.y, hdr.z, hdr.w, s, m);
+            // integers below 1024 become fp16 (and fp32) by their bits; conversions would take the slow pipe.
             // high nibbles stay where they are: 1024 + 16 q, times s / 16 (exact)
-            const __half2 sc2 = __half2half2(__hmul(__int2half_rn(s), __float2half(hh ? 0.0625f : 1.0f)));
-            const __half2 nsc = __half2half2(__int2half_rn((hh ? -64 : -1024) * s));                    // exact
-            const __half2 nm = __half2half2(__float2half_rn(-__fmul_rn(dmin, (float)m)));
+            const uint32_t sb = (uint32_t)s * 0x00010001u | 0x64006400u;
+            const __half2 s2 = __hsub2(*reinterpret_cast<const __half2*>(&sb), wt_half2(0x6400u));
+            const __half2 sc2 = hh ? __hmul2(s2, wt_half2(0x2C00u)) : s2;
+            const __half2 nsc = __hmul2(s2, wt_half2(hh ? 0xD400u : 0xE400u));                          // -64 s, -1024 s: exact
+            const float mf = __fsub_rn(__uint_as_float(0x4B000000u | (uint32_t)m), 8388608.0f);
+            const __half2 nm = __half2half2(__float2half_rn(-__fmul_rn(dmin, mf)));
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const uint32_t x = words[i] & (hh ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
@@ -264,25 +306,23 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
     uint8_t* sm_x = smem;
     uint8_t* sm_p = sm_x + S::SX * WT_X_STAGE;
     float* swap = reinterpret_cast<float*>(sm_p + S::SP * S::PACKED);
-    uint64_t* x_full = reinterpret_cast<uint64_t*>(sm_p + S::SP * S::PACKED + (SWIGLU ? WT_SWAP : 0));
-    uint64_t* x_empty = x_full + S::SX;
-    uint64_t* p_full = x_empty + S::SX;
+    uint64_t* full = reinterpret_cast<uint64_t*>(sm_p + S::SP * S::PACKED + (SWIGLU ? WT_SWAP : 0));
+    uint64_t* empty = full + S::SX;
+    uint64_t* p_full = empty + S::SX;
     uint64_t* p_empty = p_full + S::SP;
-    uint64_t* a_full = p_empty + S::SP;
-    uint64_t* a_empty = a_full + WT_SLOTS;
-    uint64_t* acc_full = a_empty + WT_SLOTS;
+    uint64_t* acc_full = p_empty + S::SP;
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-    int* first = reinterpret_cast<int*>(x_full) + 64;
-    int* table = first + WT_MAX_GROUPS + 2;
+    WtLists& lists = *reinterpret_cast<WtLists*>(reinterpret_cast<int*>(full) + 64);
+    int* table = reinterpret_cast<int*>(&lists + 1);
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int total = a.slots * a.n_tiles * a.k_splits, sb_all = a.K / 256;
-    wt_build(a, first);
-    wt_fill(a, first, table, total);
+    // what does not depend on the kernels before
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S::SX; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
+        tma_prefetch_map(&a.map_w);
+        if (SWIGLU) tma_prefetch_map(&a.map_w2);
+        for (int s = 0; s < S::SX; ++s) { mbar_init(&full[s], 1 + WT_EXPAND_WARPS); mbar_init(&empty[s], 1); }
         for (int s = 0; s < S::SP; ++s) { mbar_init(&p_full[s], 1); mbar_init(&p_empty[s], WT_EXPAND_WARPS); }
-        for (int s = 0; s < WT_SLOTS; ++s) { mbar_init(&a_full[s], 4); mbar_init(&a_empty[s], 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], 4); }
         mbar_fence_init();
     }
@@ -290,10 +330,12 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
     }
+    wt_build(a, lists);
+    wt_fill(a, lists, table, total);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    constexpr uint32_t tmem = 0;              // all 512 columns: the allocation starts at the first
     pdl_launch_dependents();
     const int mine = ((int)blockIdx.x < total ? total - (int)blockIdx.x + (int)gridDim.x - 1 : 0) / (int)gridDim.x;
     // every role walks the same tiles; sb0 .. sb1: a tile's range of K in units of 256
@@ -303,48 +345,53 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
     };
 
     if (warp == 0) {
+        const uint32_t x0 = smem_u32(sm_x), full0 = smem_u32(full);
         uint32_t it = 0, s = 0, ph = 0;
         bool ok = true;
         for (int i = 0; i < mine && ok; ++i) {
             WtTile w;
-            if (!wt_tile_at(a, first, table, i, w)) continue;
+            if (!wt_tile_at(a, lists, table, i, w)) continue;
             int sb0, sb1;
             range(w, sb0, sb1);
-            const int boxes = (w.rows + WT_BOX - 1) / WT_BOX;
-            for (int kb = 4 * sb0; kb < 4 * sb1; ++kb, ++it) {
-                if (it >= S::SX) ok = mbar_wait_warp(&x_empty[s], ph ^ 1, a.status);
-                if (!ok) break;
+            const int unit = wt_unit(w.rows), steps = 1 << unit, boxes = (w.rows + WT_BOX - 1) / WT_BOX;
+            const uint32_t bytes = (boxes * WT_BOX * 128) << unit;
+            const CUtensorMap* map = &a.map_x[boxes - 1];
+            const int row0 = w.row0, k1 = 4 * sb1;
+            for (int kb = 4 * sb0; kb < k1; kb += steps, ++it) {
+                if (it >= S::SX && !__all_sync(0xffffffffu, mbar_try(&empty[s], ph ^ 1))) {
+                    ok = mbar_wait_warp(&empty[s], ph ^ 1, a.status);
+                    if (!ok) break;
+                }
                 if (elect_one()) {
-                    mbar_expect_tx(&x_full[s], boxes * WT_BOX * 128);
-                    int b = 0;
-                    for (; b + 3 <= boxes; b += 3)
-                        tma_load_2d(sm_x + s * WT_X_STAGE + b * WT_BOX * 128, &a.map_x_big, kb * 64, w.row0 + b * WT_BOX, &x_full[s]);
-                    for (; b < boxes; ++b)
-                        tma_load_2d(sm_x + s * WT_X_STAGE + b * WT_BOX * 128, &a.map_x, kb * 64, w.row0 + b * WT_BOX, &x_full[s]);
+                    mbar_expect_tx(&full[s], bytes);
+                    tma_load_3d(x0 + s * WT_X_STAGE, map, 0, row0, kb, full0 + s * 8);
                 }
                 if (++s == S::SX) { s = 0; ph ^= 1; }
             }
         }
         if (!ok)
             for (uint32_t j = it > S::SX ? it - S::SX : 0; j < it; ++j)
-                if (!mbar_wait_warp(&x_full[j % S::SX], (j / S::SX) & 1, a.status)) break;
+                if (!mbar_wait_warp(&full[j % S::SX], (j / S::SX) & 1, a.status)) break;
     } else if (warp == 2) {
+        const uint32_t p0 = smem_u32(sm_p), full0 = smem_u32(p_full);
         uint32_t it = 0, p = 0, ph = 0;
         bool ok = true;
         for (int i = 0; i < mine && ok; ++i) {
             WtTile w;
-            if (!wt_tile_at(a, first, table, i, w)) continue;
+            if (!wt_tile_at(a, lists, table, i, w)) continue;
             int sb0, sb1;
             range(w, sb0, sb1);
             const int brow = w.brow + w.n0 * S::TILE_N;
             for (int sb = sb0; sb < sb1; ++sb, ++it) {
-                if (it >= S::SP) ok = mbar_wait_warp(&p_empty[p], ph ^ 1, a.status);
-                if (!ok) break;
+                if (it >= S::SP && !__all_sync(0xffffffffu, mbar_try(&p_empty[p], ph ^ 1))) {
+                    ok = mbar_wait_warp(&p_empty[p], ph ^ 1, a.status);
+                    if (!ok) break;
+                }
                 if (elect_one()) {
-                    uint8_t* dst = sm_p + p * S::PACKED;
+                    const uint32_t dst = p0 + p * S::PACKED, bar = full0 + p * 8;
                     mbar_expect_tx(&p_full[p], S::PACKED);
-                    tma_load_2d(dst, &a.map_w, sb * (S::SBB / 4), brow, &p_full[p]);
-                    if (SWIGLU) tma_load_2d(dst + S::PACKED / 2, &a.map_w2, sb * (S::SBB / 4), brow, &p_full[p]);
+                    tma_load_2d(dst, &a.map_w, sb * (S::SBB / 4), brow, bar);
+                    if (SWIGLU) tma_load_2d(dst + S::PACKED / 2, &a.map_w2, sb * (S::SBB / 4), brow, bar);
                 }
                 if (++p == S::SP) { p = 0; ph ^= 1; }
             }
@@ -353,11 +400,12 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
             for (uint32_t j = it > S::SP ? it - S::SP : 0; j < it; ++j)
                 if (!mbar_wait_warp(&p_full[j % S::SP], (j / S::SP) & 1, a.status)) break;
     } else if (warp == 1) {
-        uint32_t it = 0, ti = 0, s = 0;
+        const uint32_t desc0 = (uint32_t)umma_smem_desc(smem_u32(sm_x));
+        uint32_t ti = 0, s = 0, ph = 0;
         bool ok = true;
         for (int i = 0; i < mine && ok; ++i) {
             WtTile w;
-            if (!wt_tile_at(a, first, table, i, w)) continue;
+            if (!wt_tile_at(a, lists, table, i, w)) continue;
             int sb0, sb1;
             range(w, sb0, sb1);
             const uint32_t idesc = umma_idesc_f16(WT_ROWS, (w.rows + 15) & ~15), as = ti & 1;
@@ -365,29 +413,30 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
             if (!ok) break;
             tc_fence_after();
             const uint32_t d = tmem + as * WT_TOKENS;
-            // a slot's barrier stands for both operands (an expanding warp waits for the token rows before it
-            // arrives), and the next slot's is looked at before this one's MMAs are issued: a wait costs this warp
-            // some 200 cycles even when there is nothing to wait for, half a K step
-            uint32_t ready = mbar_peek(&a_full[it & (WT_SLOTS - 1)], (it / WT_SLOTS) & 1);
-            for (int kb = 4 * sb0; kb < 4 * sb1; ++kb, ++it) {
-                const uint32_t slot = it & (WT_SLOTS - 1), nxt = it + 1;
-                if (!__all_sync(0xffffffffu, ready != 0)) {
-                    ok = mbar_wait_warp(&a_full[slot], (it / WT_SLOTS) & 1, a.status);
-                    if (!ok) break;
-                }
-                tc_fence_after();
-                ready = mbar_peek(&a_full[nxt & (WT_SLOTS - 1)], (nxt / WT_SLOTS) & 1);
-                const uint64_t desc = umma_smem_desc(smem_u32(sm_x + s * WT_X_STAGE));
-                if (elect_one()) {
+            const int k0 = 4 * sb0, k1 = 4 * sb1;
+            const uint32_t step = (w.rows + WT_BOX - 1) / WT_BOX * (WT_BOX * 128 / 16);   // 64 of K of the rows loaded
+            auto rounds = [&](auto unit) {
+                constexpr int STEPS = 1 << decltype(unit)::value;
+                for (int kb = k0; kb < k1; kb += STEPS) {
+                    if (!__all_sync(0xffffffffu, mbar_try(&full[s], ph))) {
+                        ok = mbar_wait_warp(&full[s], ph, a.status);
+                        if (!ok) return;
+                    }
+                    tc_fence_after();
+                    const uint32_t op = WT_SLOT0 + (kb & (WT_SLOTS - 1)) * WT_SLOT, desc = desc0 + s * (WT_X_STAGE / 16);
+                    const uint32_t accumulate = kb > k0;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)       // 32 bytes of K per step: 2 in the descriptor's units
-                        umma_f16_ts(d, tmem + WT_SLOT0 + slot * WT_SLOT + k * 8, desc + 2 * k, idesc, kb > 4 * sb0 || k > 0);
-                    umma_commit(&a_empty[slot]);
-                    umma_commit(&x_empty[s]);
-                    if (kb == 4 * sb1 - 1) umma_commit(&acc_full[as]);
+                        for (int k = 0; k < 4 * STEPS; ++k)   // 32 bytes of K per step: 2 in the descriptor's units
+                            umma_f16_ts_lo(d, op + k * 8, desc + (k >> 2) * step + 2 * (k & 3), idesc, k > 0 ? 1u : accumulate);
+                        umma_commit(&empty[s]);
+                        if (kb + STEPS == k1) umma_commit(&acc_full[as]);
+                    }
+                    if (++s == S::SX) { s = 0; ph ^= 1; }
                 }
-                if (++s == S::SX) s = 0;
-            }
+            };
+            if (wt_unit(w.rows) == 0) rounds(std::integral_constant<int, 0>{});
+            else rounds(std::integral_constant<int, 1>{});
             ++ti;
         }
     } else if (warp >= 4 && warp < WT_FIRST_EXPAND) {
@@ -395,7 +444,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
         uint32_t ti = 0;
         for (int i = 0; i < mine; ++i) {
             WtTile w;
-            if (!wt_tile_at(a, first, table, i, w)) continue;
+            if (!wt_tile_at(a, lists, table, i, w)) continue;
             const uint32_t as = ti & 1;
             bool ok = mbar_wait(&acc_full[as], (ti >> 1) & 1, a.status);
             ok = __all_sync(0xffffffffu, ok && *reinterpret_cast<volatile int*>(a.status) == 0);
@@ -467,17 +516,21 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
         const int slot = (warp - WT_FIRST_EXPAND) >> 2, q = warp & 3;
         const uint32_t dst = tmem + WT_SLOT0 + slot * WT_SLOT + ((uint32_t)(q * 32) << 16);
         const uint32_t row_at = smem_u32(sm_p) + (q * 32 + lane) * S::SBB;
-        uint32_t it = 0, p = 0, ph = 0;                   // stages of 256 = K steps of this slot
-        uint32_t xs = slot, xph = 0;                      // the token rows' stage of its K step
+        uint32_t p = 0, ph = 0;
+        uint32_t base = 0, bph = 0;                       // the token rows' first stage of these 256 of K
+        uint32_t last = S::SX, lph = 0;                   // the stage whose MMAs read this slot last (SX: none)
         bool ok = true;
         for (int i = 0; i < mine && ok; ++i) {
             WtTile w;
-            if (!wt_tile_at(a, first, table, i, w)) continue;
+            if (!wt_tile_at(a, lists, table, i, w)) continue;
             int sb0, sb1;
             range(w, sb0, sb1);
-            for (int sb = sb0; sb < sb1; ++sb, ++it) {
-                ok = mbar_wait_warp(&p_full[p], ph, a.status);
-                if (!ok) break;
+            const int unit = wt_unit(w.rows);
+            for (int sb = sb0; sb < sb1; ++sb) {
+                if (!__all_sync(0xffffffffu, mbar_try(&p_full[p], ph))) {
+                    ok = mbar_wait_warp(&p_full[p], ph, a.status);
+                    if (!ok) break;
+                }
                 const uint32_t seg = row_at + p * S::PACKED;
                 uint32_t out[32];
                 if (slot == 0) wt_expand<KIND, 0>(seg, out);
@@ -487,17 +540,23 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
                 __syncwarp();                             // every lane has read its row: the stage goes back to TMA
                 if (lane == 0) mbar_arrive(&p_empty[p]);
                 if (++p == S::SP) { p = 0; ph ^= 1; }
-                if (it > 0) ok = mbar_wait_warp(&a_empty[slot], (it - 1) & 1, a.status);
-                if (!ok) break;
+                // The slot is free once the MMAs of four K steps ago are done.  With them every stage up to theirs has
+                // been through, so that with SX >= 4 this step's stage is in the phase that the arrival is meant for;
+                // and theirs cannot complete another phase before this step, so that the parity is not ambiguous.
+                if (last < S::SX && !__all_sync(0xffffffffu, mbar_try(&empty[last], lph))) {
+                    ok = mbar_wait_warp(&empty[last], lph, a.status);
+                    if (!ok) break;
+                }
                 tc_fence_after();
                 tmem_st32(dst, out);
                 tc_fence_before();
-                if (q == 0) ok = mbar_wait_warp(&x_full[xs], xph, a.status);
-                if (!ok) break;
-                xs += WT_SLOTS;
-                if (xs >= S::SX) { xs -= S::SX; xph ^= 1; }
+                const uint32_t at = base + (slot >> unit), over = at >= S::SX;
+                last = at - (over ? S::SX : 0);
+                lph = bph ^ over;
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&a_full[slot]);
+                if (lane == 0) mbar_arrive_n(&full[last], 4 >> unit);     // 16 in all, whatever the unit
+                base += WT_SLOTS >> unit;
+                if (base >= S::SX) { base -= S::SX; bph ^= 1; }
             }
         }
     }
@@ -507,6 +566,31 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
 }
 
 // ---- host side ------------------------------------------------------------------
+// The token rows' maps: [K / 64][rows][64], boxes of 16 (i + 1) rows and the K steps of their stage.
+static int make_stage_maps(CUtensorMap (&out)[WT_TOKENS / WT_BOX], const void* base, int64_t rows, int64_t K) {
+    struct Maps {
+        CUtensorMap m[WT_TOKENS / WT_BOX];
+    };
+    typedef std::tuple<const void*, int64_t, int64_t> Key;
+    static std::map<Key, Maps> cache;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    const Key key(base, rows, K);
+    auto it = cache.find(key);
+    if (it == cache.end()) {
+        Maps maps;
+        for (int i = 0; i < WT_TOKENS / WT_BOX; ++i) {
+            const int box = (i + 1) * WT_BOX;
+            const int rc = make_stage_map(&maps.m[i], base, rows, K, box, 1 << wt_unit(box));
+            if (rc) return rc;
+        }
+        if (cache.size() > 1024) cache.clear();
+        it = cache.emplace(key, maps).first;
+    }
+    std::copy(std::begin(it->second.m), std::end(it->second.m), out);
+    return B200_OK;
+}
+
 template <bool SWIGLU, int KIND>
 static int launch_wt(WtArgs& a, bool allow_split) {
     using S = WtShape<SWIGLU, KIND>;
@@ -552,9 +636,7 @@ int umma_gemm_q(int epi, int kind, const __half* A, int64_t a_rows, const void* 
     B200_REQUIRE(groups >= 1 && (offsets || groups == 1), "umma_gemm_q: groups need a device offsets array");
     B200_REQUIRE((group_map || b_rows >= (int64_t)groups * N) && a_rows >= M, "umma_gemm_q: operand shapes do not cover the groups");
     WtArgs a;
-    int rc = make_tile_map(&a.map_x, A, a_rows, K, WT_BOX);
-    if (rc) return rc;
-    rc = make_tile_map(&a.map_x_big, A, a_rows, K, WT_BIG_BOX);
+    int rc = make_stage_maps(a.map_x, A, a_rows, K);
     if (rc) return rc;
     const int64_t row_bytes = q_row_bytes(kind, K);
     const int sbb = 8 * (kind == 3 ? 18 : q_block_bytes(kind));

@@ -92,6 +92,22 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
         ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
+__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+// The same from a 3-D map (make_stage_map): x = 0, y = row, z = K in steps of 64.  Shared-memory addresses.
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
 // ---- warp-uniform roles ---------------------------------------------------------------
 // The tcgen05 and TMA instructions take descriptors and addresses in uniform registers.  A role run by one lane
 // of a divergent branch moves every operand there by hand, and its waits are divergent loops: 1150 cycles per
@@ -108,6 +124,12 @@ __device__ __forceinline__ uint32_t mbar_peek(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok;
+}
+// One look that may wait for the hardware's own short while.
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
 }
 // Bounded wait of a whole warp, with the same result in every lane.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status) {
@@ -131,5 +153,7 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 // Host: tensor map of a row-major fp16 matrix [rows, K] with boxes of 64 x box_rows
 // and the 128-byte swizzle.  Returns B200_OK or an error status.
 int make_tile_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, int box_rows);
+// The same as [K / 64][rows][64]: one load brings box_steps runs of 64 of box_rows rows, run after run.  Not cached.
+int make_stage_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, int box_rows, int box_steps);
 
 }  // namespace b200

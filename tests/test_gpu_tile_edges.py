@@ -75,6 +75,35 @@ def test_gemm_token_tiles(oracle, kind, M, K, N):
 
 
 # the bias gathers the tokens: experts with none, one, a full tile (8 / 24 slots) and one more
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("d,E", [(256, 256), (768, 512)])
+def test_expert_rows_of_mixed_sizes(oracle, kind, d, E):
+    """One group list with every form of a token tile: empty groups, one row, the multiples of 16 that a load brings and
+    their neighbours, tiles of one and of two K steps per stage in turn (96 | 97 rows), groups of several tiles.  Norm-wise
+    bound: weights within one fp16 ulp of their value in both products (2 x 2^-10) and fp16 activations between them (2^-11)."""
+    from gpu_util import dev, empty, host, ops
+    sizes = [0, 1, 15, 16, 17, 0, 95, 96, 97, 32, 33, 191, 192, 193, 300, 2, 48, 0]
+    ne, R = len(sizes), sum(sizes)
+    r = np.random.default_rng(kind)
+    rows = r.standard_normal((R, d)).astype(np.float16)
+    w = [oracle.quantize((r.standard_normal(ne * E * d) * 0.05).astype(np.float32), kind) for _ in range(3)]
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    y = empty((R, d))
+    ops.moe_experts_rows(dev(rows.view(np.uint16)), dev(off), None, ne, R, dev(w[0]), dev(w[1]), dev(w[2]), ne, y, d, E, kind)
+    got = host(y)
+    g, u, dn = (torch.from_numpy(oracle.dequantize(x, ne * E * d, kind).view(np.float16).astype(np.float64)).cuda() for x in w)
+    g, u, dn = g.view(ne, E, d), u.view(ne, E, d), dn.view(ne, d, E)
+    x = torch.from_numpy(rows.astype(np.float64)).cuda()
+    for e in range(ne):
+        xe = x[off[e]:off[e + 1]]
+        if len(xe):
+            act = (torch.nn.functional.silu(xe @ g[e].T) * (xe @ u[e].T)).half().double()
+            ref = (act @ dn[e].T).cpu().numpy()
+            mine = got[off[e]:off[e + 1]]
+            err = np.linalg.norm(mine - ref, axis=1) / np.linalg.norm(ref, axis=1)
+            assert err.max() < 2.5e-3, (e, sizes[e], err.max())
+
+
 @pytest.mark.parametrize("kind", [2, 3])
 @pytest.mark.parametrize("N", [9, 24, 25, 48])
 @pytest.mark.parametrize("d,E", [(256, 512), (768, 256)])
