@@ -65,15 +65,20 @@ struct NvtxRange {
     NvtxRange(const NvtxRange&) = delete;
     NvtxRange& operator=(const NvtxRange&) = delete;
 };
-int side_begin();
+int side_fork();
+int side_begin(bool forked = false);
 int side_end();
 int side_wait();
 // Joins when it goes out of scope after an error, so that nothing is left running beside what the caller does next (and
 // no capture ends with a branch open).
 struct SideJoin {
-    bool open = false;
+    bool open = false, forked = false;
+    int fork() {
+        forked = true;
+        return side_fork();
+    }
     int begin() {
-        const int rc = side_begin();
+        const int rc = side_begin(forked);
         open = rc == 0;
         return rc;
     }

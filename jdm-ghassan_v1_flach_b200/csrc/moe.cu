@@ -151,189 +151,93 @@ moe_route_kernel(const float* __restrict__ x, const float* __restrict__ router_w
 }
 
 // ---------------------------------------------------------------------------
-// Expert permutation: stable counting sort of slots s = t*K + k by expert.
-// Three kernels, no atomics on ordering: per-block histograms, a scan over
-// (expert, block), then a fill where each warp ranks its 32 slots with
-// __match_any_sync and warps are ordered through shared-memory prefix sums.
+// Expert permutation: stable counting sort of slots s = t*K + k by expert, one block per expert and one launch.  A block
+// reads all slots twice (from L2): counted below and at its expert, which gives the expert's offset and each warp's first
+// position, then placed in order.  No block waits for another.  The three kernels before it (histograms, a scan, ranked
+// placing) and the one for the inverse were bound by their launches: 24 576 slots of 64 experts 19.5 us and 4 for the
+// inverse, 12.3 now; 3102 slots 17.4 + 4 -> 6.2, a decode batch of 384 8.2 -> 6.1.
 // ---------------------------------------------------------------------------
-constexpr int PERM_THREADS = 256;
-constexpr int PERM_ITERS = 4;                              // slots per block = 256 * 4
-constexpr int PERM_CHUNK = PERM_THREADS * PERM_ITERS;
+constexpr int PERM_WARPS = 16;
 
-__global__ void __launch_bounds__(PERM_THREADS)
-perm_count_kernel(const int32_t* __restrict__ idx, int64_t NK, int ne, int32_t* __restrict__ block_counts) {
-    __shared__ int cnt[MOE_MAX_NE];
-    for (int e = threadIdx.x; e < ne; e += blockDim.x) cnt[e] = 0;
-    __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * PERM_CHUNK;
-    for (int it = 0; it < PERM_ITERS; ++it) {
-        const int64_t s = base + it * PERM_THREADS + threadIdx.x;
-        if (s < NK) atomicAdd(&cnt[idx[s]], 1);
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < ne; e += blockDim.x) block_counts[(int64_t)blockIdx.x * ne + e] = cnt[e];
-}
-
-// One block; thread e walks the blocks of expert e.  block_counts becomes the
-// first output position of (block, expert); offsets[ne+1] the expert boundaries.
-__global__ void perm_scan_kernel(int32_t* __restrict__ block_counts, int nblocks, int ne,
-                                 int32_t* __restrict__ offsets) {
-    __shared__ int total[MOE_MAX_NE + 1];
-    const int e = threadIdx.x;
-    if (e < ne) {
-        int run = 0;
-        for (int b = 0; b < nblocks; ++b) {
-            const int c = block_counts[(int64_t)b * ne + e];
-            block_counts[(int64_t)b * ne + e] = run;
-            run += c;
+__global__ void __launch_bounds__(PERM_WARPS * 32)
+perm_kernel(const int32_t* __restrict__ idx, int NK, int32_t* __restrict__ grouped, int32_t* __restrict__ inv,
+            int32_t* __restrict__ offsets) {
+    __shared__ int s_below[PERM_WARPS], s_at[PERM_WARPS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e = blockIdx.x;
+    // a warp's run of slots: whole 128s
+    const uint32_t run = (((uint32_t)NK + PERM_WARPS - 1) / PERM_WARPS + 127) & ~127u;
+    const uint32_t s0 = min((uint32_t)NK, warp * run), s1 = min((uint32_t)NK, s0 + run);
+    const bool wide = (reinterpret_cast<uintptr_t>(idx) & 15) == 0;
+    auto load = [&](uint32_t s, int (&v)[4]) {                     // slots s .. s + 3; past the end: no expert
+        if (wide && s + 4 <= s1) {
+            const int4 q = *reinterpret_cast<const int4*>(idx + s);
+            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = s + j < s1 ? idx[s + j] : MOE_MAX_NE;
         }
-        total[e] = run;
+    };
+    pdl_launch_dependents();
+    pdl_wait();
+    int below = 0, at = 0;
+#pragma unroll 2
+    for (uint32_t s = s0 + 4 * lane; s < s1; s += 128) {
+        int v[4];
+        load(s, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            below += v[j] < e;
+            at += v[j] == e;
+        }
+    }
+    below = __reduce_add_sync(0xffffffffu, below);
+    at = __reduce_add_sync(0xffffffffu, at);
+    if (lane == 0) {
+        s_below[warp] = below;
+        s_at[warp] = at;
     }
     __syncthreads();
+    int offset = 0, pos = 0;
+#pragma unroll
+    for (int w = 0; w < PERM_WARPS; ++w) {
+        offset += s_below[w];
+        pos += w < warp ? s_at[w] : 0;
+    }
     if (threadIdx.x == 0) {
-        int run = 0;
-        for (int i = 0; i < ne; ++i) { const int c = total[i]; total[i] = run; run += c; }
-        total[ne] = run;
+        offsets[e] = offset;
+        if (e == (int)gridDim.x - 1) offsets[e + 1] = NK;
     }
-    __syncthreads();
-    if (e <= ne) offsets[e] = total[e];
-    if (e < ne) {
-        const int off = total[e];
-        for (int b = 0; b < nblocks; ++b) block_counts[(int64_t)b * ne + e] += off;
-    }
-}
-
-__global__ void __launch_bounds__(PERM_THREADS)
-perm_fill_kernel(const int32_t* __restrict__ idx, int64_t NK, int ne, const int32_t* __restrict__ block_base,
-                 int32_t* __restrict__ grouped) {
-    constexpr int NW = PERM_THREADS / 32;
-    __shared__ int cursor[MOE_MAX_NE];
-    __shared__ int wcnt[NW][MOE_MAX_NE];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int e = threadIdx.x; e < ne; e += blockDim.x) cursor[e] = block_base[(int64_t)blockIdx.x * ne + e];
-    const int64_t base = (int64_t)blockIdx.x * PERM_CHUNK;
-    for (int it = 0; it < PERM_ITERS; ++it) {
-        for (int i = threadIdx.x; i < NW * ne; i += blockDim.x) (&wcnt[0][0])[(i / ne) * MOE_MAX_NE + (i % ne)] = 0;
-        __syncthreads();
-        const int64_t s = base + it * PERM_THREADS + threadIdx.x;
-        const bool live = s < NK;
-        const int e = live ? idx[s] : -1 - lane;              // dead lanes match nobody
-        const unsigned peers = __match_any_sync(0xffffffffu, e);
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        if (live && rank == 0) wcnt[warp][e] = __popc(peers);
-        __syncthreads();
-        if (live) {
-            int pos = cursor[e] + rank;
-            for (int w = 0; w < warp; ++w) pos += wcnt[w][e];
-            grouped[pos] = (int32_t)s;
+    pos += offset;
+    if (at == 0) return;                                      // whole warps
+    for (uint32_t s = s0 + 4 * lane; s - 4 * lane < s1; s += 128) {
+        int v[4];
+        load(s, v);
+        unsigned has[4];
+        int before = 0, total = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            has[j] = __ballot_sync(0xffffffffu, v[j] == e);
+            before += __popc(has[j] & ((1u << lane) - 1u));
+            total += __popc(has[j]);
         }
-        __syncthreads();
-        for (int ee = threadIdx.x; ee < ne; ee += blockDim.x) {
-            int add = 0;
+        int p = pos + before;
 #pragma unroll
-            for (int w = 0; w < NW; ++w) add += wcnt[w][ee];
-            cursor[ee] += add;
-        }
-        __syncthreads();
-    }
-}
-
-// Up to PERM_CHUNK slots (a decode batch): the three steps and the inverse in one block -
-// histogram, scan over the experts, the same ranked fill (cursor = the expert's offset).
-__global__ void __launch_bounds__(PERM_THREADS)
-perm_small_kernel(const int32_t* __restrict__ idx, int NK, int ne, int32_t* __restrict__ grouped,
-                  int32_t* __restrict__ inv, int32_t* __restrict__ offsets) {
-    constexpr int NW = PERM_THREADS / 32;
-    __shared__ int cursor[MOE_MAX_NE + 1];
-    __shared__ int wcnt[NW][MOE_MAX_NE];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int e = threadIdx.x; e <= ne; e += blockDim.x) cursor[e] = 0;
-    __syncthreads();
-    int mine[PERM_ITERS];
-#pragma unroll
-    for (int it = 0; it < PERM_ITERS; ++it) {
-        const int s = it * PERM_THREADS + threadIdx.x;
-        mine[it] = s < NK ? idx[s] : -1;
-        if (s < NK) atomicAdd(&cursor[mine[it]], 1);
-    }
-    __syncthreads();
-    if (warp == 0) {
-        // exclusive scan of the counts, 32 experts at a time
-        int run = 0;
-        for (int e0 = 0; e0 <= ne; e0 += 32) {
-            const int e = e0 + lane;
-            const int c = e < ne ? cursor[e] : 0;
-            int incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
+        for (int j = 0; j < 4; ++j)
+            if (v[j] == e) {
+                grouped[p] = (int32_t)(s + j);
+                if (inv) inv[s + j] = p;
+                ++p;
             }
-            if (e <= ne) {
-                cursor[e] = run + incl - c;
-                offsets[e] = run + incl - c;
-            }
-            run += __shfl_sync(0xffffffffu, incl, 31);
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < PERM_ITERS; ++it) {
-        if (it * PERM_THREADS >= NK) break;                   // uniform
-        for (int i = threadIdx.x; i < NW * MOE_MAX_NE; i += blockDim.x) (&wcnt[0][0])[i] = 0;
-        __syncthreads();
-        const int s = it * PERM_THREADS + threadIdx.x;
-        const bool live = s < NK;
-        const int e = live ? mine[it] : -1 - lane;            // dead lanes match nobody
-        const unsigned peers = __match_any_sync(0xffffffffu, e);
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        if (live && rank == 0) wcnt[warp][e] = __popc(peers);
-        __syncthreads();
-        if (live) {
-            int pos = cursor[e] + rank;
-            for (int w = 0; w < warp; ++w) pos += wcnt[w][e];
-            grouped[pos] = (int32_t)s;
-            if (inv) inv[s] = pos;
-        }
-        __syncthreads();
-        for (int ee = threadIdx.x; ee < ne; ee += blockDim.x) {
-            int add = 0;
-#pragma unroll
-            for (int w = 0; w < NW; ++w) add += wcnt[w][ee];
-            cursor[ee] += add;
-        }
-        __syncthreads();
+        pos += total;
     }
 }
 
-// grouped, offsets and (optionally) the inverse permutation in one launch when the slots fit one block.
-int moe_permutation_inv(const int32_t* idx, int64_t NK, int ne, int32_t* grouped, int32_t* inv, int32_t* offsets) {
-    B200_REQUIRE(idx && grouped && offsets, "moe_permutation: null pointer");
-    B200_REQUIRE(ne > 0 && ne <= MOE_MAX_NE, "moe_permutation: ne out of range");
-    if (NK < 0 || NK > PERM_CHUNK) return fail(B200_EUNSUPPORTED, "moe_permutation_inv: more slots than one block takes");
-    perm_small_kernel<<<1, PERM_THREADS, 0, stream()>>>(idx, (int)NK, ne, grouped, inv, offsets);
-    B200_LAUNCH_CHECK("perm_small_kernel");
-    return B200_OK;
-}
-int moe_permutation_small_max() { return PERM_CHUNK; }
-
-int moe_permutation(const int32_t* idx, int64_t NK, int ne, int32_t* grouped, int32_t* offsets) {
+// grouped [NK]: slots sorted by expert, stable; inv (optional): where each slot went; offsets [ne + 1].
+int moe_permutation(const int32_t* idx, int64_t NK, int ne, int32_t* grouped, int32_t* inv, int32_t* offsets) {
     B200_REQUIRE(idx && grouped && offsets, "moe_permutation: null pointer");
     B200_REQUIRE(ne > 0 && ne <= MOE_MAX_NE, "moe_permutation: ne out of range");
     B200_REQUIRE(NK >= 0 && NK < ((int64_t)1 << 31), "moe_permutation: slot count out of range");
-    if (NK <= PERM_CHUNK) return moe_permutation_inv(idx, NK, ne, grouped, nullptr, offsets);     // one block does it all
-    const int nblocks = (int)std::max<int64_t>(1, ceil_div64(NK, PERM_CHUNK));
-    void* wsp;
-    int rc = workspace(WS_PERM).ensure((size_t)nblocks * ne * sizeof(int32_t) + 256, &wsp);
-    if (rc) return rc;
-    int32_t* bc = static_cast<int32_t*>(wsp);
-    perm_count_kernel<<<nblocks, PERM_THREADS, 0, stream()>>>(idx, NK, ne, bc);
-    B200_LAUNCH_CHECK("perm_count_kernel");
-    perm_scan_kernel<<<1, 320, 0, stream()>>>(bc, nblocks, ne, offsets);
-    B200_LAUNCH_CHECK("perm_scan_kernel");
-    perm_fill_kernel<<<nblocks, PERM_THREADS, 0, stream()>>>(idx, NK, ne, bc, grouped);
-    B200_LAUNCH_CHECK("perm_fill_kernel");
-    return B200_OK;
+    return launch_short(perm_kernel, dim3(ne), dim3(PERM_WARPS * 32), idx, (int)NK, grouped, inv, offsets);
 }
 
 // ---------------------------------------------------------------------------
@@ -417,17 +321,17 @@ static int launch_experts(const MoeArgs& a) {
 }
 
 // ---------------------------------------------------------------------------
-// Router for many tokens.  The logit of (token, expert) keeps the reference's
-// sequential fp32 chain over groups of four (products and sums rounded one by one, so two
-// instructions per multiply-add: 22 us for 4096 tokens of 1536 x 64 experts), but the chains
-// of a tile advance together: token and router rows come through a ring of asynchronous copies,
-// 64 columns at a time, and a thread carries TPT tokens of one expert - a warp reads its
-// lanes' 32 expert rows (four wavefronts per group of columns) for TPT token rows (one each, the
-// same for all lanes), so at 8 tokens shared memory needs 12 cycles where the arithmetic needs 16.
-// 4096 tokens: 60 us with the register double buffer and 4 tokens per thread before, 55 beside the shared expert's
-// GEMM now.  A second kernel finishes each token with one warp.
+// Router for more than eight tokens.  The logit of (token, expert) keeps the reference's sequential fp32 chain over groups
+// of four (products and sums rounded one by one: eight instructions per group, 23 us of a chip's fp32 rate for 4096 tokens
+// of 1536 x 64 experts).  A thread carries TPT x EPT chains; token and expert rows come through a ring of asynchronous
+// copies, RT_K columns at a time and a thousand columns deep where a block has few chains, because the chains advance
+// faster than a cold load returns: the ring of three 64-column stages before it spent 1800 cycles per stage, a load's way.
+// In us (before, now), router alone, launches included: 64 tokens of 1536 x 64
+// 16.4 -> 14.3, 301 27.6 -> 20.5, 2048 44 -> 38; of 4096 x 72: 64 tokens 30 -> 25, 517 64 -> 50, 4096 210 -> 194; 4096 tokens of
+// 768 x 16 34 -> 19.5.  Larger thread tiles (4 x 4, 8 x 2) and packed additions were no faster: about two cycles a product or
+// sum whatever their number.
 // ---------------------------------------------------------------------------
-constexpr int RT_K = 64, RT_LD = RT_K + 4, RT_WARPS = 4, RT_THREADS = 32 * RT_WARPS, RT_STAGES = 3;
+constexpr int RT_K = 128, RT_LD = RT_K + 4, RT_THREADS = 256;
 
 // One warp routes token t from its logits; s: ne floats of shared scratch.
 template <int PER>
@@ -453,159 +357,113 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
             if (32 * i + lane < ne) probs_out[t * ne + 32 * i + lane] = v[i];
 }
 
-template <int TPT>
+// Two products, each rounded as __fmul_rn does, in one instruction (few warps: issue slots count).
+__device__ __forceinline__ void mul_pair(float a, float b, float c, float d, float& ac, float& bd) {
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(ac), "=f"(bd)
+        : "f"(a), "f"(b), "f"(c), "f"(d));
+}
+
+// Lanes: eight experts x four tokens; CW warps compute (one to a scheduler with the blocks that share an SM), all copy.
+template <int TPT, int EPT, int CW, int STAGES>
+struct RtShape {
+    static constexpr int LE = 8, LT = 4, TOK = LT * TPT * CW, EXP = LE * EPT, ROWS = TOK + EXP, STAGE = ROWS * RT_LD, SMEM = STAGES * STAGE * 4;
+};
+template <int TPT, int EPT, int CW, int STAGES>
 __global__ void __launch_bounds__(RT_THREADS)
 route_logits_kernel(const float* __restrict__ x, const float* __restrict__ router_w, float* __restrict__ logits,
-                    int64_t N, int d, int ne) {
-    constexpr int TOK = RT_WARPS * TPT, ROWS = TOK + 32, STAGE = ROWS * RT_LD;
+                    int64_t N, int d, int ne, const float* __restrict__ router_bias, float* __restrict__ probs_out,
+                    int32_t* __restrict__ idx_out, float* __restrict__ w_out, int K, int* __restrict__ counters) {
+    using S = RtShape<TPT, EPT, CW, STAGES>;
     extern __shared__ __align__(16) float rt_sm[];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t t0 = (int64_t)blockIdx.x * TOK;
-    const int e0 = blockIdx.y * 32;
-    // rows 0 .. TOK-1: tokens, then 32 experts; rows past the ends repeat the last one, columns past d are not read
-    const int c4 = (threadIdx.x % (RT_K / 4)) * 4, r0 = threadIdx.x / (RT_K / 4);
-    constexpr int STEP = RT_THREADS / (RT_K / 4), PER = ROWS / STEP;
-    static_assert(ROWS % STEP == 0, "rows of a stage per copying thread");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t t0 = (int64_t)blockIdx.x * S::TOK;
+    const int e0 = blockIdx.y * S::EXP;
+    // rows 0 .. TOK-1: tokens, then the experts; rows past the ends repeat the last one, columns past d are not read
+    constexpr int PER = S::ROWS / (RT_THREADS / 32);
+    static_assert(S::ROWS % (RT_THREADS / 32) == 0 && RT_K == 128, "a warp copies a row's 128 columns");
+    const float* src[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        const int row = warp + u * (RT_THREADS / 32);
+        src[u] = (row < S::TOK ? x + min(t0 + row, N - 1) * d : router_w + (int64_t)min(e0 + row - S::TOK, ne - 1) * d) + 4 * lane;
+    }
+    const uint32_t dst = smem_u32(rt_sm + warp * RT_LD + 4 * lane);
     const int chunks = (d + RT_K - 1) / RT_K;
     auto fetch = [&](int k) {
-        if (k < chunks) {
-            float* st = rt_sm + (k % RT_STAGES) * STAGE;
-            if (k * RT_K + c4 < d)
+        if (k < chunks && k * RT_K + 4 * lane < d) {
+            const uint32_t at = dst + (k % STAGES) * (S::STAGE * 4);
 #pragma unroll
-                for (int u = 0; u < PER; ++u) {
-                    const int row = r0 + u * STEP;
-                    const float* src = row < TOK ? x + min(t0 + row, N - 1) * d : router_w + (int64_t)min(e0 + row - TOK, ne - 1) * d;
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(st + row * RT_LD + c4)), "l"(src + k * RT_K + c4) : "memory");
-                }
+            for (int u = 0; u < PER; ++u)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + u * (RT_THREADS / 32) * RT_LD * 4), "l"(src[u] + k * RT_K) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float acc[TPT] = {};
+    const int te = lane % S::LE, tt = warp * S::LT * TPT + lane / S::LE;
+    float acc[TPT][EPT] = {};
 #pragma unroll
-    for (int k = 0; k < RT_STAGES - 1; ++k) fetch(k);
+    for (int k = 0; k < STAGES - 1; ++k) fetch(k);
+    pdl_launch_dependents();
     for (int k = 0; k < chunks; ++k) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(RT_STAGES - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();                               // the stage is here, and the one before it is free
-        fetch(k + RT_STAGES - 1);
-        const float* xs = rt_sm + (k % RT_STAGES) * STAGE + TPT * ty * RT_LD;
-        const float* ws = rt_sm + (k % RT_STAGES) * STAGE + (TOK + tx) * RT_LD;
+        fetch(k + STAGES - 1);
+        if (warp >= CW) continue;
+        const float* xs = rt_sm + (k % STAGES) * S::STAGE + tt * RT_LD;
+        const float* ws = rt_sm + (k % STAGES) * S::STAGE + (S::TOK + te) * RT_LD;
         const int kc = min(RT_K, d - k * RT_K);        // a multiple of 4
-        auto group = [&](int g) {
-            const float4 b = *reinterpret_cast<const float4*>(ws + g);
+        auto load = [&](int g, float4 (&a)[TPT], float4 (&b)[EPT]) {
 #pragma unroll
-            for (int i = 0; i < TPT; ++i) {
-                const float4 a = *reinterpret_cast<const float4*>(xs + i * RT_LD + g);
-                float s = __fadd_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
-                s = __fadd_rn(s, __fmul_rn(a.z, b.z));
-                s = __fadd_rn(s, __fmul_rn(a.w, b.w));
-                acc[i] = __fadd_rn(acc[i], s);
-            }
+            for (int j = 0; j < EPT; ++j) b[j] = *reinterpret_cast<const float4*>(ws + S::LE * j * RT_LD + g);
+#pragma unroll
+            for (int i = 0; i < TPT; ++i) a[i] = *reinterpret_cast<const float4*>(xs + S::LT * i * RT_LD + g);
         };
-        // whole chunks with the loads of later groups under the additions of earlier ones (the chains are serial)
-        if (kc == RT_K) {
+        auto group = [&](const float4 (&a)[TPT], const float4 (&b)[EPT]) {
 #pragma unroll
-            for (int g = 0; g < RT_K; g += 4) group(g);
-        } else {
-            for (int g = 0; g < kc; g += 4) group(g);
-        }
-    }
-    const int e = e0 + tx;
+            for (int i = 0; i < TPT; ++i)
 #pragma unroll
-    for (int i = 0; i < TPT; ++i) {
-        const int64_t t = t0 + TPT * ty + i;
-        if (t < N && e < ne) logits[t * ne + e] = acc[i];
-    }
-}
-template <int TPT>
-static int launch_route_logits(const float* x, const float* router_w, float* logits, int64_t N, int d, int ne) {
-    constexpr int SMEM = RT_STAGES * (RT_WARPS * TPT + 32) * RT_LD * 4;
-    static bool configured = false;
-    if (!configured) {
-        B200_CUDA(cudaFuncSetAttribute(route_logits_kernel<TPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-        configured = true;
-    }
-    const dim3 grid((unsigned)ceil_div64(N, RT_WARPS * TPT), ceil_div(ne, 32));
-    route_logits_kernel<TPT><<<grid, RT_THREADS, SMEM, stream()>>>(x, router_w, logits, N, d, ne);
-    B200_LAUNCH_CHECK("route_logits_kernel");
-    return B200_OK;
-}
-
-// A decode batch (tens of tokens): the tiled kernel above would occupy N / 8 x ne / 32 blocks -
-// 16 SMs for 64 tokens - each crawling along 1536-long chains.  Here a block takes 8 tokens x 8
-// experts (64 chains), and the two parts of a chain are split over its threads: the group sums
-// ((a0 b0 + a1 b1) + a2 b2) + a3 b3 of a 1024-column piece are independent and go to shared
-// memory four threads per chain; one thread per chain then adds them in order (the only
-// sequential part: one dependent add per group).  Same values, same order as the chains above.
-constexpr int RC_TOK = 8, RC_EXP = 8, RC_COLS = 1024, RC_LD = RC_COLS + 4, RC_GLD = RC_COLS / 4 + 1;
-constexpr size_t RC_SMEM = ((size_t)(RC_TOK + RC_EXP) * RC_LD + (size_t)RC_TOK * RC_EXP * RC_GLD) * 4;
-__global__ void __launch_bounds__(256)
-route_logits_chains_kernel(const float* __restrict__ x, const float* __restrict__ router_w, float* __restrict__ logits,
-                           int64_t N, int d, int ne, const float* __restrict__ router_bias, float* __restrict__ probs_out,
-                           int32_t* __restrict__ idx_out, float* __restrict__ w_out, int K, int* __restrict__ counters) {
-    extern __shared__ __align__(16) float rc_smem[];
-    float* xs = rc_smem;                                  // [RC_TOK][RC_LD]
-    float* ws = xs + RC_TOK * RC_LD;                      // [RC_EXP][RC_LD]
-    float* gs = ws + RC_EXP * RC_LD;                      // [64 chains][RC_GLD]
-    const int64_t t0 = (int64_t)blockIdx.x * RC_TOK;
-    const int e0 = blockIdx.y * RC_EXP;
-    const int c = threadIdx.x & 63, sub = threadIdx.x >> 6;          // chain, which quarter of its groups
-    const int tc = c & 7, ec = c >> 3;
-    float chain = 0.0f;
-    // A piece is at most 256 runs of four wide: one run per thread and row, all 16 loads in flight;
-    // the next piece is fetched into registers while the current one is worked on.
-    const int q = threadIdx.x, c4 = q * 4;
-    float4 v[RC_TOK + RC_EXP];
-    auto fetch = [&](int k0) {
-        const int q4 = min(RC_COLS, d - k0) >> 2;
-#pragma unroll
-        for (int row = 0; row < RC_TOK + RC_EXP; ++row) {
-            v[row] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (q < q4) {
-                if (row < RC_TOK) {
-                    if (t0 + row < N) v[row] = *reinterpret_cast<const float4*>(x + (t0 + row) * d + k0 + c4);
-                } else if (e0 + row - RC_TOK < ne) {
-                    v[row] = *reinterpret_cast<const float4*>(router_w + (int64_t)(e0 + row - RC_TOK) * d + k0 + c4);
+                for (int j = 0; j < EPT; ++j) {
+                    float px, py, pz, pw;
+                    mul_pair(a[i].x, a[i].y, b[j].x, b[j].y, px, py);
+                    mul_pair(a[i].z, a[i].w, b[j].z, b[j].w, pz, pw);
+                    float s = __fadd_rn(px, py);
+                    s = __fadd_rn(s, pz);
+                    s = __fadd_rn(s, pw);
+                    acc[i][j] = __fadd_rn(acc[i][j], s);
                 }
+        };
+        float4 a[2][TPT], b[2][EPT];
+        if (kc == RT_K) {
+            // the next group's loads under this one's arithmetic
+            load(0, a[0], b[0]);
+            constexpr int UNROLL = TPT * EPT == 1 ? 8 : 4;
+#pragma unroll UNROLL
+            for (int g = 0; g < RT_K; g += 8) {
+                load(g + 4, a[1], b[1]);
+                group(a[0], b[0]);
+                if (g + 8 < RT_K) load(g + 8, a[0], b[0]);
+                group(a[1], b[1]);
+            }
+        } else {
+            for (int g = 0; g < kc; g += 4) {
+                load(g, a[0], b[0]);
+                group(a[0], b[0]);
             }
         }
-    };
-    fetch(0);
-    for (int k0 = 0; k0 < d; k0 += RC_COLS) {
-        const int kc = min(RC_COLS, d - k0), q4 = kc >> 2;           // kc % 4 == 0
-        __syncthreads();                                             // the previous piece has been consumed
-        if (q < q4) {
+    }
+    if (warp < CW) {
 #pragma unroll
-            for (int row = 0; row < RC_TOK + RC_EXP; ++row)
-                *reinterpret_cast<float4*>((row < RC_TOK ? xs + row * RC_LD : ws + (row - RC_TOK) * RC_LD) + c4) = v[row];
-        }
-        __syncthreads();
-        if (k0 + RC_COLS < d) fetch(k0 + RC_COLS);
-        const float* xa = xs + tc * RC_LD;
-        const float* wb = ws + ec * RC_LD;
-        float* gc = gs + c * RC_GLD;
-#pragma unroll 4
-        for (int g = sub; g < q4; g += 4) {
-            const float4 a = *reinterpret_cast<const float4*>(xa + 4 * g);
-            const float4 b = *reinterpret_cast<const float4*>(wb + 4 * g);
-            float t = __fadd_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
-            t = __fadd_rn(t, __fmul_rn(a.z, b.z));
-            t = __fadd_rn(t, __fmul_rn(a.w, b.w));
-            gc[g] = t;
-        }
-        __syncthreads();
-        if (threadIdx.x < 64) {
-#pragma unroll 8
-            for (int g = 0; g < q4; ++g) chain = __fadd_rn(chain, gc[g]);
-        }
+        for (int i = 0; i < TPT; ++i)
+#pragma unroll
+            for (int j = 0; j < EPT; ++j) {
+                const int64_t t = t0 + tt + S::LT * i;
+                const int e = e0 + te + S::LE * j;
+                if (t < N && e < ne) logits[t * ne + e] = acc[i][j];
+            }
     }
-    if (threadIdx.x < 64) {
-        const int64_t t = t0 + tc;
-        const int e = e0 + ec;
-        if (t < N && e < ne) logits[t * ne + e] = chain;
-    }
-    // The block that completes a token group's last expert tile turns the group's logits into
-    // (idx, w), one warp per token: nobody waits - each block counts itself in after publishing
-    // its logits, and whoever counts last finds all of them (fence before the count and after it).
+    // The block that completes a token tile's last expert tile turns the tile's logits into (idx, w), one warp per token:
+    // nobody waits - each block counts itself in after publishing its logits, and whoever counts last finds all of them
+    // (fence before the count and after it).
     __shared__ int s_last;
     if (!counters) return;                                   // the caller finishes with route_finish_kernel
     __threadfence();
@@ -614,21 +472,37 @@ route_logits_chains_kernel(const float* __restrict__ x, const float* __restrict_
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int64_t t = t0 + warp;
-        if (warp < RC_TOK && t < N) {
-            float* s_p = rc_smem + (size_t)warp * MOE_MAX_NE;                         // the tiles are dead
-            if (ne <= 64) route_token<2>(logits, router_bias, probs_out, idx_out, w_out, t, ne, K, s_p, lane);
-            else route_token<8>(logits, router_bias, probs_out, idx_out, w_out, t, ne, K, s_p, lane);
-        }
-        if (threadIdx.x == 0) counters[blockIdx.x] = 0;       // ready for the next call
+    for (int i = warp; i < S::TOK; i += RT_THREADS / 32) {
+        const int64_t t = t0 + i;
+        if (t >= N) break;
+        float* s_p = rt_sm + (size_t)warp * MOE_MAX_NE;      // the tiles are dead
+        if (ne <= 64) route_token<2>(logits, router_bias, probs_out, idx_out, w_out, t, ne, K, s_p, lane);
+        else route_token<8>(logits, router_bias, probs_out, idx_out, w_out, t, ne, K, s_p, lane);
+        __syncwarp();
     }
+    if (threadIdx.x == 0) counters[blockIdx.x] = 0;           // ready for the next call
+}
+template <int TPT, int EPT, int CW, int STAGES>
+static int launch_route_logits(const float* x, const float* router_w, float* logits, int64_t N, int d, int ne, const float* router_bias,
+                               float* probs, int32_t* idx, float* w, int K, int* counters) {
+    using S = RtShape<TPT, EPT, CW, STAGES>;
+    static_assert(S::SMEM <= 227 * 1024 && S::SMEM >= RT_THREADS / 32 * MOE_MAX_NE * 4, "stages, and the finishing warps' scratch");
+    auto kern = route_logits_kernel<TPT, EPT, CW, STAGES>;
+    static bool configured = false;
+    if (!configured) {
+        B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
+        configured = true;
+    }
+    const dim3 grid((unsigned)ceil_div64(N, S::TOK), ceil_div(ne, S::EXP));
+    kern<<<grid, RT_THREADS, S::SMEM, stream()>>>(x, router_w, logits, N, d, ne, router_bias, probs, idx, w, K, counters);
+    B200_LAUNCH_CHECK("route_logits_kernel");
+    return B200_OK;
 }
 
 // Arrival counters of the kernel above (one per token group), zeroed once; every call leaves them zero.
 // Not created while the stream is being captured into a graph (an allocation and a memset on the
 // default stream do not belong there): the caller then runs the separate finishing kernel.
+constexpr int ROUTE_COUNTERS = 1024;
 static int* route_counters() {
     static int* p = nullptr;
     if (!p) {
@@ -637,8 +511,8 @@ static int* route_counters() {
             cudaGetLastError();
             return nullptr;
         }
-        if (cudaMalloc(&p, 4096) != cudaSuccess) { p = nullptr; cudaGetLastError(); return nullptr; }
-        if (cudaMemset(p, 0, 4096) != cudaSuccess) { cudaFree(p); p = nullptr; cudaGetLastError(); return nullptr; }
+        if (cudaMalloc(&p, ROUTE_COUNTERS * sizeof(int)) != cudaSuccess) { p = nullptr; cudaGetLastError(); return nullptr; }
+        if (cudaMemset(p, 0, ROUTE_COUNTERS * sizeof(int)) != cudaSuccess) { cudaFree(p); p = nullptr; cudaGetLastError(); return nullptr; }
     }
     return p;
 }
@@ -651,6 +525,8 @@ route_finish_kernel(const float* __restrict__ logits, const float* __restrict__ 
     __shared__ float s_p[RF_WARPS][32 * PER];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t t = (int64_t)blockIdx.x * RF_WARPS + warp;
+    pdl_launch_dependents();
+    pdl_wait();
     if (t < N) route_token<PER>(logits, router_bias, probs_out, idx_out, w_out, t, ne, K, s_p[warp], lane);
 }
 
@@ -661,35 +537,22 @@ int moe_route(const float* x, const float* router_w, const float* router_bias, f
         int rc = workspace(WS_ROUTE).ensure((size_t)N * ne * 4 + 256, &wsp);
         if (rc) return rc;
         float* logits = static_cast<float*>(wsp);
-        if (N <= 256) {
-            static bool configured = false;
-            if (!configured) {
-                B200_CUDA(cudaFuncSetAttribute(route_logits_chains_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)RC_SMEM));
-                configured = true;
-            }
-            int* counters = route_counters();
-            const dim3 grid((unsigned)ceil_div64(N, RC_TOK), ceil_div(ne, RC_EXP));
-            route_logits_chains_kernel<<<grid, 256, RC_SMEM, stream()>>>(x, router_w, logits, N, d, ne, router_bias, probs, idx,
-                                                                         w, K, counters);
-            B200_LAUNCH_CHECK("route_logits_chains_kernel");
-            if (counters) return B200_OK;
+        // One chain per thread in blocks of 8 x 8 (most blocks, least latency) or four in blocks of 32 x 16 (a third of the
+        // shared loads per product).  Times in units of some us, from 1536 columns and 64 experts: 128 / 256 / 517 / 1024 tokens
+        // take 14 / 18 / 29 / 41 us with the first and 24 / 24 / 24 / 26 with the second, 2048 take 66 and 38.
+        auto rounds = [&](int tok, int exp) { return ceil_div64(ceil_div64(N, tok) * ceil_div(ne, exp), num_sms()); };
+        int* counters = nullptr;
+        if (5 * rounds(8, 8) + 4 <= 12 * rounds(32, 16) + 7) {
+            if (N <= 8 * ROUTE_COUNTERS) counters = route_counters();
+            rc = launch_route_logits<1, 1, 2, 8>(x, router_w, logits, N, d, ne, router_bias, probs, idx, w, K, counters);
         } else {
-            // the smallest token tile that one wave of blocks covers: a thread's chains run side by side, so few
-            // tokens want many blocks and many tokens want each expert row read for as many of them as there are
-            const int e_tiles = ceil_div(ne, 32);
-            auto blocks = [&](int tpt) { return ceil_div64(N, RT_WARPS * tpt) * e_tiles; };
-            rc = blocks(2) <= num_sms()   ? launch_route_logits<2>(x, router_w, logits, N, d, ne)
-                 : blocks(4) <= num_sms() ? launch_route_logits<4>(x, router_w, logits, N, d, ne)
-                                          : launch_route_logits<8>(x, router_w, logits, N, d, ne);
-            if (rc) return rc;
+            rc = launch_route_logits<2, 2, 4, 4>(x, router_w, logits, N, d, ne, router_bias, probs, idx, w, K, nullptr);
         }
-        const unsigned blocks = (unsigned)ceil_div64(N, RF_WARPS);
-        if (ne <= 64) route_finish_kernel<2><<<blocks, RF_WARPS * 32, 0, stream()>>>(logits, router_bias, probs, idx, w, N, ne, K);
-        else if (ne <= 128) route_finish_kernel<4><<<blocks, RF_WARPS * 32, 0, stream()>>>(logits, router_bias, probs, idx, w, N, ne, K);
-        else route_finish_kernel<8><<<blocks, RF_WARPS * 32, 0, stream()>>>(logits, router_bias, probs, idx, w, N, ne, K);
-        B200_LAUNCH_CHECK("route_finish_kernel");
-        return B200_OK;
+        if (rc || counters) return rc;
+        const dim3 blocks((unsigned)ceil_div64(N, RF_WARPS)), threads(RF_WARPS * 32);
+        if (ne <= 64) return launch_short(route_finish_kernel<2>, blocks, threads, logits, router_bias, probs, idx, w, N, ne, K);
+        if (ne <= 128) return launch_short(route_finish_kernel<4>, blocks, threads, logits, router_bias, probs, idx, w, N, ne, K);
+        return launch_short(route_finish_kernel<8>, blocks, threads, logits, router_bias, probs, idx, w, N, ne, K);
     }
     // shared memory: x + as many group rows as fit in ~96 KB
     const int groups = d >> 2;
@@ -875,7 +738,7 @@ int b200_moe_forward_bias_half(const float* x, const float* router_w, const floa
                        w_cache, s_gate, s_up, s_act, N, d, E, ne, K, SH, tag_of_qkind(qkind));
 }
 int b200_moe_permutation(const int32_t* idx, int64_t NK, int ne, int32_t* grouped, int32_t* offsets) {
-    return moe_permutation(idx, NK, ne, grouped, offsets);
+    return moe_permutation(idx, NK, ne, grouped, nullptr, offsets);
 }
 
 }  // extern "C"

@@ -20,17 +20,9 @@ namespace b200 {
 
 int moe_route(const float* x, const float* router_w, const float* router_bias, float* probs, int32_t* idx, float* w,
               int64_t N, int d, int ne, int K);
-int moe_permutation(const int32_t* idx, int64_t NK, int ne, int32_t* grouped, int32_t* offsets);
-int moe_permutation_inv(const int32_t* idx, int64_t NK, int ne, int32_t* grouped, int32_t* inv, int32_t* offsets);
-int moe_permutation_small_max();
+int moe_permutation(const int32_t* idx, int64_t NK, int ne, int32_t* grouped, int32_t* inv, int32_t* offsets);
 
 constexpr int GROUPED_CHUNK_TOKENS = 8192;
-
-// inv[grouped[pos]] = pos
-__global__ void perm_inverse_kernel(const int32_t* __restrict__ grouped, int32_t* __restrict__ inv, int64_t NK) {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < NK) inv[grouped[p]] = (int32_t)p;
-}
 
 // out[t, :] = (shared ? out[t, :] : 0) + sum_k w[t,k] * y[inv[t*K + k], :]   (k ascending)
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ y, const int32_t* __restrict__ inv,
@@ -122,7 +114,12 @@ int moe_forward_grouped(const float* x, const float* router_w, const float* rout
         float* y = reinterpret_cast<float*>(base + o_y);
 
         // The shared expert shares no data with routing, permutation, gather and the routed
-        // experts until the combine: it runs on the side stream next to them, straight into out.
+        // experts until the combine: it runs on the side stream next to them, straight into out.  The router, which the
+        // routed experts wait for, is launched first: behind the shared expert's GEMM, whose CTAs take whole SMs, it
+        // started 25 to 45 us late.
+        if (shared && (rc = side.fork())) return rc;
+        rc = moe_route(xc, router_w, router_bias, probs_cache ? probs_cache + t0 * ne : nullptr, idx, w, T, d, ne, K);
+        if (rc) return rc;
         if (shared) {
             if ((rc = side.begin())) return rc;
             rc = pack_rows_f16(xc, nullptr, 1, H(o_xs), T, d);
@@ -138,12 +135,8 @@ int moe_forward_grouped(const float* x, const float* router_w, const float* rout
             if (rc) return rc;
             if (rc2) return rc2;
         }
-        rc = moe_route(xc, router_w, router_bias, probs_cache ? probs_cache + t0 * ne : nullptr, idx, w, T, d, ne, K);
+        rc = moe_permutation(idx, NK, ne, grouped, inv, offsets);
         if (rc) return rc;
-        rc = moe_permutation(idx, NK, ne, grouped, offsets);
-        if (rc) return rc;
-        perm_inverse_kernel<<<(unsigned)ceil_div64(NK, 256), 256, 0, stream()>>>(grouped, inv, NK);
-        B200_LAUNCH_CHECK("perm_inverse_kernel");
         rc = pack_rows_f16(xc, grouped, K, H(o_a), NK, d);
         if (rc) return rc;
         // routed experts
@@ -208,6 +201,9 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
     float* act = reinterpret_cast<float*>(base + o_act);
     float* y = reinterpret_cast<float*>(base + o_y);
     SideJoin side;
+    if (shared && (rc = side.fork())) return rc;
+    rc = moe_route(x, router_w, router_bias, probs_cache, idx, w, N, d, ne, K);
+    if (rc) return rc;
     if (shared) {
         if ((rc = side.begin())) return rc;
         if (shared_exact) {
@@ -228,8 +224,6 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
         if (rc) return rc;
         if (rc2) return rc2;
     }
-    rc = moe_route(x, router_w, router_bias, probs_cache, idx, w, N, d, ne, K);
-    if (rc) return rc;
     rc = moe_dispatch_perm(idx, N, ne, K, grouped, inv, offsets);
     if (rc) return rc;
     rc = exact ? moe_exact_forward(x, grouped, offsets, gates, ups, downs, act, y, base + o_units, N, d, E, ne, K)
@@ -261,12 +255,7 @@ int moe_dispatch_perm(const int32_t* idx, int64_t N, int ne, int K, int32_t* gro
     B200_REQUIRE(idx && grouped && inv && offsets, "moe_dispatch_perm: null pointer");
     const int64_t NK = N * K;
     if (NK <= 0) return B200_OK;
-    if (NK <= moe_permutation_small_max()) return moe_permutation_inv(idx, NK, ne, grouped, inv, offsets);
-    const int rc = moe_permutation(idx, NK, ne, grouped, offsets);
-    if (rc) return rc;
-    perm_inverse_kernel<<<(unsigned)ceil_div64(NK, 256), 256, 0, stream()>>>(grouped, inv, NK);
-    B200_LAUNCH_CHECK("perm_inverse_kernel");
-    return B200_OK;
+    return moe_permutation(idx, NK, ne, grouped, inv, offsets);
 }
 
 int moe_dispatch_pack(const float* x, const int32_t* idx, int64_t N, int d, int ne, int K, __half* rows16, int32_t* inv,
@@ -278,10 +267,8 @@ int moe_dispatch_pack(const float* x, const int32_t* idx, int64_t N, int d, int 
     int rc = workspace(WS_MOE).ensure((size_t)NK * 4 + 256, &wsp);
     if (rc) return rc;
     int32_t* grouped = static_cast<int32_t*>(wsp);
-    rc = moe_permutation(idx, NK, ne, grouped, offsets);
+    rc = moe_permutation(idx, NK, ne, grouped, inv, offsets);
     if (rc) return rc;
-    perm_inverse_kernel<<<(unsigned)ceil_div64(NK, 256), 256, 0, stream()>>>(grouped, inv, NK);
-    B200_LAUNCH_CHECK("perm_inverse_kernel");
     return pack_rows_f16(x, grouped, K, rows16, NK, d);
 }
 

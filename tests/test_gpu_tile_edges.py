@@ -191,6 +191,30 @@ def test_router_tiles(oracle, d, ne, K, N):
     np.testing.assert_array_max_ulp(host(dw), w, maxulp=4)
 
 
+# both tiles of the router and their ragged ends: one chain per thread up to some 500 tokens, 2 x 2 above, one column tile and
+# several, a last one of four columns; bit-exact as above
+@pytest.mark.parametrize("d,ne,K", [(128, 16, 2), (132, 72, 10), (1028, 256, 16)])
+@pytest.mark.parametrize("N", [9, 300, 1111])
+def test_router_thread_tiles(oracle, d, ne, K, N):
+    test_router_tiles(oracle, d, ne, K, N)
+
+
+# slots around a warp's 128 and a block's 2048, at a list that is no multiple of 16 bytes; experts without any
+@pytest.mark.parametrize("NK", [1, 127, 129, 2047, 2049, 40001])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_permutation_and_its_inverse(NK, shift):
+    from gpu_util import dev, empty, host, ops
+    ne = 72
+    r = np.random.default_rng(NK)
+    idx = r.choice(ne, size=NK + shift, p=r.dirichlet(np.full(ne, 0.3))).astype(np.int32)
+    rows16, inv, offsets = empty((NK, 32), torch.int16), empty(NK, torch.int32), empty(ne + 1, torch.int32)
+    didx, x = dev(idx), empty((NK, 32))
+    ops.moe_dispatch_pack(x, didx[shift:], NK, 32, ne, 1, rows16, inv, offsets)
+    want = np.argsort(idx[shift:], kind="stable")
+    assert np.array_equal(host(inv)[want], np.arange(NK))
+    assert np.array_equal(host(offsets), np.concatenate([[0], np.cumsum(np.bincount(idx[shift:], minlength=ne))]))
+
+
 # a sequence of one chunk carries its state in the output kernel; 129 steps: two chunks
 @pytest.mark.parametrize("kind", [-2, 2])
 @pytest.mark.parametrize("d_state", [64, 128])
