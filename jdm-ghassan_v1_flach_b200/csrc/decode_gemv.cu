@@ -102,23 +102,33 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dg_gemv_kernel(SgArgs a)
             if (lane == 0) inv[m] = 1.0f / sqrtf((float)(t / (double)a.in_dim) + a.eps);
         }
     }
-    for (int i = warp; i < chunks * a.M; i += W) {
-        const int m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
-        float v[8];
-        dg_load8<true>(a.x + (int64_t)m * a.x_stride, c * DG_CHUNK + 8 * lane, a.K, v);
-        if (PRO == PRO_RMS) {
-            if (i != warp) dg_norm8(a.norm_w, c * DG_CHUNK + 8 * lane, a.K, nw);
-            double ss = 0.0;
+    constexpr int B = dg_batch(MT);
+    const int all = chunks * a.M;
+    for (int i0 = warp; i0 < all; i0 += B * W) {
+        float v[B][8], nv[B][8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                ss += (double)v[j] * (double)v[j];
-                v[j] *= nw[j];
+        for (int q = 0; q < B; ++q) {
+            const int i = min(i0 + q * W, all - 1), m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
+            dg_load8<true>(a.x + (int64_t)m * a.x_stride, c * DG_CHUNK + 8 * lane, a.K, v[q]);
+            if (PRO == PRO_RMS && (q > 0 || i0 != warp)) dg_norm8(a.norm_w, c * DG_CHUNK + 8 * lane, a.K, nv[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+            const int i = i0 + q * W, m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
+            if (i >= all) break;
+            if (PRO == PRO_RMS) {
+                double ss = 0.0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    ss += (double)v[q][j] * (double)v[q][j];
+                    v[q][j] *= q == 0 && i0 == warp ? nw[j] : nv[q][j];
+                }
+                dg_stage<KIND, MT>(xd, c, m, v[q], 1.0f, lane);
+                ss = warp_sum_d(ss);
+                if (lane == 0) ssq[c * MT + m] = ss;
+            } else {
+                dg_stage<KIND, MT>(xd, c, m, v[q], 1.0f, lane);
             }
-            dg_stage<KIND, MT>(xd, c, m, v, 1.0f, lane);
-            ss = warp_sum_d(ss);
-            if (lane == 0) ssq[c * MT + m] = ss;
-        } else {
-            dg_stage<KIND, MT>(xd, c, m, v, 1.0f, lane);
         }
     }
     __syncthreads();
@@ -197,6 +207,8 @@ static int launch_dg(SgArgs a) {
     // share when it fits half an SM (the next kernel's CTA fits beside it and streams early), else two sets of
     // as much as does; a whole SM for long shares (an fp16 lm_head: two sets of two tiles, whose products take
     // less time than their 98 KB - one tile at a time, the barriers between them held the stream at 4.3 TB/s).
+    // From three tokens on the products outweigh the hand-over and two CTAs share an SM (a step of five sequences of H-Tiny:
+    // in_proj and out_proj 10.4 and 8.4 us with one, the conversation 38.5 ms; 36.7 with two).
     for (int R = TILE_ROWS; R >= 1 && !smem; R >>= 1) {
         if ((R * a.row_bytes) % 16 != 0) break;
         a.rows_per_tile = R;
@@ -204,7 +216,7 @@ static int launch_dg(SgArgs a) {
         a.t2 = a.t1 + ceil_div(a.N2, R);
         a.num_tiles = a.t2 + ceil_div(a.N3, R);
         a.stage_bytes = (int)((R * a.row_bytes + 127) / 128 * 128);
-        grid = std::min(a.num_tiles, num_sms());
+        grid = std::min(a.num_tiles, (KIND != KIND_F16 && MT > 2 ? 2 : 1) * num_sms());
         const int most = ceil_div(a.num_tiles, grid);
         a.share = a.num_tiles / grid;
         a.share_rem = a.num_tiles % grid;

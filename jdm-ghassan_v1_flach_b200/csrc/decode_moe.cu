@@ -13,7 +13,8 @@
 // 384 additions of four cycles - are serial; kernel 2 lets kernel 3 start only after its own wait, which
 // proves the routing of kernel 1 complete, so kernel 3 fetches its experts' rows while kernel 2 runs.
 // One token, H-Tiny shape, in the step's graph: 31 us before,
-// 16 now.
+// 16 now.  The layer by itself at 3, 5 and 8 tokens: 28, 42 and 57 us before the router's CTAs read all tokens at once, the chunks
+// were loaded four at a time and two CTAs shared an SM; 22, 27 and 36 now.
 #include "digit_tile.cuh"
 #include "route.cuh"
 
@@ -26,6 +27,13 @@ __host__ __device__ inline int dm_chain_stride(int d) { return ((d >> 2) + 31) /
 // The tile loop shared by the three kernels: rounds of up to G tiles through `sets` sets of stages, each tile's
 // chunks split over P warps.  issue(r, set): one thread starts round r's copies; dot(stage, part, acc): one warp's
 // share; epilogue(first tile, tiles, red): all threads. prepare() stages the activations, barrier included.
+// The epilogues' elements go to the threads from the last warp but one on: a round has few, and the first warps, which
+// always have products, go on to the next round's.
+template <int MT>
+__device__ __forceinline__ int dm_element() {
+    constexpr int T = dg_warps(MT) * 32;
+    return threadIdx.x >= T - 64 ? threadIdx.x - (T - 64) : threadIdx.x + 64;
+}
 template <int KIND, int MT, typename Prepare, typename Issue, typename Dot, typename Epi>
 __device__ __forceinline__ void dm_rounds(const MoeFusedArgs& a, int n_my, float* red, uint64_t* bar, Prepare prepare, Issue issue, Dot dot, Epi epilogue) {
     constexpr int W = dg_warps(MT);
@@ -59,24 +67,33 @@ __device__ __forceinline__ void dm_rounds(const MoeFusedArgs& a, int n_my, float
 // squares to ssq.  The norm factor itself is applied by the epilogue.
 template <int KIND, int MT>
 __device__ __forceinline__ void dm_stage_norm(const MoeFusedArgs& a, const DgX<KIND, MT>& xd, int m0, int n, double* ssq) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunks = dg_chunks(a.d);
-    for (int i = warp; i < chunks * n; i += dg_warps(MT)) {
-        const int m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
-        float v[8], nw[8];
-        dg_load8<true>(a.x + (int64_t)(m0 + m) * a.d, c * DG_CHUNK + 8 * lane, a.d, v);
-        double ss = 0.0;
-        if (a.norm_w) {
-            dg_norm8(a.norm_w, c * DG_CHUNK + 8 * lane, a.d, nw);
+    constexpr int W = dg_warps(MT), B = dg_batch(MT);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunks = dg_chunks(a.d), all = chunks * n;
+    for (int i0 = warp; i0 < all; i0 += B * W) {
+        float v[B][8], nw[B][8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                ss += (double)v[j] * (double)v[j];
-                v[j] *= nw[j];
-            }
+        for (int b = 0; b < B; ++b) {
+            const int i = min(i0 + b * W, all - 1), m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
+            dg_load8<true>(a.x + (int64_t)(m0 + m) * a.d, c * DG_CHUNK + 8 * lane, a.d, v[b]);
+            if (a.norm_w) dg_norm8(a.norm_w, c * DG_CHUNK + 8 * lane, a.d, nw[b]);
         }
-        dg_stage<KIND, MT>(xd, c, m, v, 1.0f, lane);
-        if (a.norm_w) {
-            ss = warp_sum_d(ss);
-            if (lane == 0) ssq[c * MT + m] = ss;
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const int i = i0 + b * W, m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
+            if (i >= all) break;
+            double ss = 0.0;
+            if (a.norm_w) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    ss += (double)v[b][j] * (double)v[b][j];
+                    v[b][j] *= nw[b][j];
+                }
+            }
+            dg_stage<KIND, MT>(xd, c, m, v[b], 1.0f, lane);
+            if (a.norm_w) {
+                ss = warp_sum_d(ss);
+                if (lane == 0) ssq[c * MT + m] = ss;
+            }
         }
     }
 }
@@ -186,16 +203,48 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(
                 dm_route<8>(a, gs, biases8, false, warp, lane);
             }
         }
+        // A thread's RG runs of four of every token stay in registers from the norm to the group sums where the row is
+        // narrow enough (W * 32 * RG runs), all loads under way together: read token by token, and twice, five tokens of
+        // 1536 took 16 500 cycles here (now the shared expert's CTAs, 12 000, are what the kernel takes).
+        constexpr int RG = MT <= 2 ? 1 : 2;
+        const int padded = (groups + 31) & ~31;                       // zeros up to whole runs of 32
+        const bool held = padded <= RG * W * 32;
+        float4 nw[RG], xv[MT][RG];
+        if (held)
+#pragma unroll
+            for (int q = 0; q < RG; ++q) {
+                const int g = threadIdx.x + q * W * 32;
+                nw[q] = a.norm_w && g < groups ? dg_norm4(a.norm_w + 4 * g) : make_float4(1.f, 1.f, 1.f, 1.f);
+            }
         pdl_wait();
+        auto load = [&](int m, int g) {
+            return g < groups ? __ldcg(reinterpret_cast<const float4*>(a.x + (int64_t)m * a.d + 4 * g)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        if (held)
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int q = 0; q < RG; ++q)
+                    if (m < a.M) xv[m][q] = load(m, threadIdx.x + q * W * 32);
         if (a.norm_w) {
-            for (int m = 0; m < a.M; ++m) {
-                double ss = 0.0;
-                for (int g = threadIdx.x; g < groups; g += W * 32) {
-                    const float4 v = __ldcg(reinterpret_cast<const float4*>(a.x + (int64_t)m * a.d + 4 * g));
-                    ss += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w;
+            auto square = [](float4 v) { return (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w; };
+            if (held) {
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    if (m >= a.M) break;
+                    double ss = 0.0;
+#pragma unroll
+                    for (int q = 0; q < RG; ++q) ss += square(xv[m][q]);
+                    ss = warp_sum_d(ss);
+                    if (lane == 0) red_d[m * W + warp] = ss;
                 }
-                ss = warp_sum_d(ss);
-                if (lane == 0) red_d[m * W + warp] = ss;
+            } else {
+                for (int m = 0; m < a.M; ++m) {
+                    double ss = 0.0;
+                    for (int g = threadIdx.x; g < groups; g += W * 32) ss += square(load(m, g));
+                    ss = warp_sum_d(ss);
+                    if (lane == 0) red_d[m * W + warp] = ss;
+                }
             }
             __syncthreads();
             if (threadIdx.x < a.M) {
@@ -208,30 +257,36 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(
         }
         __syncthreads();
         const bool ok = mbar_wait(&bar[0], 0, a.status);
-        // group sums ((a0 b0 + a1 b1) + a2 b2) + a3 b3 of every (token, expert); zeros up to whole runs of 32
-        const int padded = (groups + 31) & ~31;
-        for (int m = 0; m < a.M; ++m) {
-            for (int g = threadIdx.x; g < padded; g += W * 32) {
-                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (g < groups) {
-                    x = __ldcg(reinterpret_cast<const float4*>(a.x + (int64_t)m * a.d + 4 * g));
-                    if (a.norm_w) {
-                        const float4 nw = dg_norm4(a.norm_w + 4 * g);
-                        const float f = inv[m];
-                        x = make_float4(x.x * f * nw.x, x.y * f * nw.y, x.z * f * nw.z, x.w * f * nw.w);
-                    }
-                }
+        // group sums ((a0 b0 + a1 b1) + a2 b2) + a3 b3 of every (token, expert)
+        auto sums = [&](int m, int g, float4 x, float4 w) {
+            if (a.norm_w) {
+                const float f = inv[m];
+                x = make_float4(x.x * f * w.x, x.y * f * w.y, x.z * f * w.z, x.w * f * w.w);
+            }
 #pragma unroll
-                for (int e = 0; e < DM_ROUTER; ++e) {
-                    if (e < rows) {
-                        float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (g < groups) b = *reinterpret_cast<const float4*>(w_s + e * a.d + 4 * g);
-                        float t = __fadd_rn(__fmul_rn(x.x, b.x), __fmul_rn(x.y, b.y));
-                        t = __fadd_rn(t, __fmul_rn(x.z, b.z));
-                        gs[(m * DM_ROUTER + e) * stride + g] = __fadd_rn(t, __fmul_rn(x.w, b.w));
-                    }
+            for (int e = 0; e < DM_ROUTER; ++e) {
+                if (e < rows) {
+                    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (g < groups) b = *reinterpret_cast<const float4*>(w_s + e * a.d + 4 * g);
+                    float t = __fadd_rn(__fmul_rn(x.x, b.x), __fmul_rn(x.y, b.y));
+                    t = __fadd_rn(t, __fmul_rn(x.z, b.z));
+                    gs[(m * DM_ROUTER + e) * stride + g] = __fadd_rn(t, __fmul_rn(x.w, b.w));
                 }
             }
+        };
+        if (held) {
+#pragma unroll
+            for (int q = 0; q < RG; ++q) {
+                const int g = threadIdx.x + q * W * 32;
+                if (g < padded)
+#pragma unroll
+                    for (int m = 0; m < MT; ++m)
+                        if (m < a.M) sums(m, g, xv[m][q], nw[q]);
+            }
+        } else {
+            for (int m = 0; m < a.M; ++m)
+                for (int g = threadIdx.x; g < padded; g += W * 32)
+                    sums(m, g, load(m, g), a.norm_w && g < groups ? dg_norm4(a.norm_w + 4 * g) : make_float4(1.f, 1.f, 1.f, 1.f));
         }
         __syncthreads();
         // the ordered additions: one lane per chain, the next 32 sums on their way while 32 are added
@@ -300,7 +355,7 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(
             }
         },
         [&](int t0, int n, const float* rr) {
-            for (int e = threadIdx.x; e < n * 8 * MT; e += W * 32) {
+            for (int e = dm_element<MT>(); e < n * 8 * MT; e += W * 32) {
                 const int m = e % MT, row = e / MT % 8, i = e / (8 * MT);
                 if (m >= a.M) continue;
                 const float* re = rr + i * a.parts * dg_red_floats(MT);
@@ -369,7 +424,7 @@ __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_gateup_kernel(MoeFused
             }
         },
         [&](int t0, int n, const float* rr) {
-            for (int e = threadIdx.x; e < n * 8; e += W * 32) {
+            for (int e = dm_element<1>(); e < n * 8; e += W * 32) {
                 const int row = e % 8, i = e / 8, tile = first + (t0 + i) * step, k = __umulhi(tile, a.per_inv);
                 const float* re = rr + i * a.parts * dg_red_floats(1);
                 const float gt = dg_value<KIND, 1>(re, a.parts, row, 0) * inv[0], up = dg_value<KIND, 1>(re, a.parts, row + 8, 0) * inv[0];
@@ -430,8 +485,8 @@ __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_down_kernel(MoeFusedAr
     dm_rounds<KIND, 1>(a, n_my, red, bar,
         [&] {
             pdl_wait();
-            const int row = threadIdx.x & 15, col = (first + threadIdx.x / 16 * step) * R + row;      // this thread's first element
-            if (!a.out && threadIdx.x < 16 * (unsigned)min(G, n_my) && row < R && col < a.d) pre = a.resid[(int64_t)m * a.d + col];
+            const int el = dm_element<1>(), row = el & 15, col = (first + el / 16 * step) * R + row;      // this thread's first element
+            if (!a.out && el < 16 * min(G, n_my) && row < R && col < a.d) pre = a.resid[(int64_t)m * a.d + col];
             for (int i = warp; i < chunks; i += W) {
                 float v[8], mul = 1.0f;
                 if (i < sc) {
@@ -466,13 +521,13 @@ __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_down_kernel(MoeFusedAr
             }
         },
         [&](int t0, int n, const float* rr) {
-            for (int e = threadIdx.x; e < n * 16; e += W * 32) {
+            for (int e = dm_element<1>(); e < n * 16; e += W * 32) {
                 const int row = e % 16, i = e / 16, col = (first + (t0 + i) * step) * R + row;
                 if (row >= R || col >= a.d) continue;
                 const float v = dg_value<KIND, 1>(rr + i * a.parts * dg_red_floats(1), a.parts, row, 0);
                 const int64_t at = (int64_t)m * a.d + col;
                 if (a.out) a.out[at] = v;
-                else a.resid[at] = (t0 == 0 && e == (int)threadIdx.x ? pre : a.resid[at]) + v * a.res_mult;
+                else a.resid[at] = (t0 == 0 && e == dm_element<1>() ? pre : a.resid[at]) + v * a.res_mult;
             }
         });
 }
@@ -519,7 +574,10 @@ template <int KIND>
 static int dm_kind(const MoeFusedArgs& a) {
     const int mt = a.M == 1 ? 1 : a.M == 2 ? 2 : a.M <= 4 ? 4 : 8;
     const size_t rb_d = row_bytes_of(KIND, a.d), rb_e = row_bytes_of(KIND, a.E), rb_s = a.SH > 0 ? row_bytes_of(KIND, a.SH) : 0;
-    const int per_token = std::max(1, num_sms() / a.M);
+    // One CTA of kernels 2 and 3 on an SM for one token, so that the next kernel's fits beside it and fetches early.  Two for more:
+    // their time is a CTA's rounds of products (13 tiles each at five tokens), which twelve warps fill an SM with to 39 %
+    // of its issue slots.  Us for gate / up at 2, 3, 5, 8 tokens (H-Tiny): 7.3, 11.5, 17.3, 24.2 with one, 5.7, 6.5, 9.7, 14.3 with two.
+    const int per_token = std::max(1, (a.M > 1 ? 2 : 1) * num_sms() / a.M);
     // all three are planned before the first is launched: a layer runs whole or not at all
     MoeFusedArgs p1 = a, p2 = a, p3 = a;
     const int n_router = ceil_div(a.ne, DM_ROUTER), sh_tiles = a.SH / 8;

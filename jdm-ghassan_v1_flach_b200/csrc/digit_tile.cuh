@@ -26,6 +26,9 @@ namespace b200 {
 // and two tokens fit; more tokens need the accumulators of eight warps at 128.
 __host__ __device__ constexpr int dg_warps(int MT) { return MT <= 2 ? 12 : 8; }
 constexpr int DG_CHUNK = 256;                 // activations that share a scale
+// Chunks that a warp loads together before it stages them: the activations come from L2, and one after the other five tokens
+// of 1536 were four such ways for each warp.
+__host__ __device__ constexpr int dg_batch(int MT) { return MT == 1 ? 1 : MT == 2 ? 2 : 4; }
 // a / b for 0 <= a < 4096, 1 <= b < 256, inv = dg_inv(b): no division on the kernels' serial path
 __host__ __device__ constexpr uint32_t dg_inv(int b) { return ((1u << 20) + (uint32_t)b - 1) / (uint32_t)b; }
 __host__ __device__ __forceinline__ int dg_div(int a, uint32_t inv) { return (int)(((uint32_t)a * inv) >> 20); }

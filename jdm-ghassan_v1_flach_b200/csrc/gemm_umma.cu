@@ -31,6 +31,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <vector>
 
 #include "gemm.cuh"
 #include "umma.cuh"
@@ -536,8 +537,24 @@ int make_tile_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, i
     cache[key] = *out;
     return B200_OK;
 }
-int make_stage_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, int box_rows, int box_steps) {
-    return encode_tile_map(out, base, rows, K, box_rows, box_steps);
+int make_stage_maps(CUtensorMap* out, const void* base, int64_t rows, int64_t K, const StageBox* boxes, int n) {
+    typedef std::tuple<const void*, int64_t, int64_t, const StageBox*> Key;
+    static std::map<Key, std::vector<CUtensorMap>> cache;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    const Key key(base, rows, K, boxes);
+    auto it = cache.find(key);
+    if (it == cache.end()) {
+        std::vector<CUtensorMap> maps(n);
+        for (int i = 0; i < n; ++i) {
+            const int rc = encode_tile_map(&maps[i], base, rows, K, boxes[i].rows, boxes[i].steps);
+            if (rc) return rc;
+        }
+        if (cache.size() > 1024) cache.clear();
+        it = cache.emplace(key, std::move(maps)).first;
+    }
+    std::copy(it->second.begin(), it->second.end(), out);
+    return B200_OK;
 }
 
 // Tensor map over packed rows viewed as 32-bit words: boxes of (box_bytes / 4) words

@@ -35,10 +35,6 @@
 // Slower: two K steps per expanding warp and turn (the second one's expansion sits between two MMA rounds), stages of
 // constant number in the MMA warp (no difference once the loads are quick).
 #include <algorithm>
-#include <iterator>
-#include <map>
-#include <mutex>
-#include <tuple>
 
 #include "gemm.cuh"
 #include "linear.cuh"
@@ -180,7 +176,7 @@ __device__ __noinline__ bool wt_find_late(const WtArgs& a, const WtLists& l, int
 
 // A stage of token rows, and with it one round of the MMA warp, is 64 of K, or 128 where the tile's rows fill no more than
 // half of it (a ring of mostly empty stages is shorter than the latency that it has to cover): log2 of the K steps of 64.
-__host__ __device__ __forceinline__ int wt_unit(int rows) { return rows > WT_TOKENS / 2 ? 0 : 1; }
+__host__ __device__ constexpr int wt_unit(int rows) { return rows > WT_TOKENS / 2 ? 0 : 1; }
 __device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
 }
@@ -566,30 +562,14 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
 }
 
 // ---- host side ------------------------------------------------------------------
-// The token rows' maps: [K / 64][rows][64], boxes of 16 (i + 1) rows and the K steps of their stage.
-static int make_stage_maps(CUtensorMap (&out)[WT_TOKENS / WT_BOX], const void* base, int64_t rows, int64_t K) {
-    struct Maps {
-        CUtensorMap m[WT_TOKENS / WT_BOX];
-    };
-    typedef std::tuple<const void*, int64_t, int64_t> Key;
-    static std::map<Key, Maps> cache;
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lock(mu);
-    const Key key(base, rows, K);
-    auto it = cache.find(key);
-    if (it == cache.end()) {
-        Maps maps;
-        for (int i = 0; i < WT_TOKENS / WT_BOX; ++i) {
-            const int box = (i + 1) * WT_BOX;
-            const int rc = make_stage_map(&maps.m[i], base, rows, K, box, 1 << wt_unit(box));
-            if (rc) return rc;
-        }
-        if (cache.size() > 1024) cache.clear();
-        it = cache.emplace(key, maps).first;
+// The token rows' loads: 16 (i + 1) rows and the K steps of their stage.
+struct WtBoxes {
+    StageBox b[WT_TOKENS / WT_BOX];
+    constexpr WtBoxes() : b() {
+        for (int i = 0; i < WT_TOKENS / WT_BOX; ++i) b[i] = StageBox{(i + 1) * WT_BOX, 1 << wt_unit((i + 1) * WT_BOX)};
     }
-    std::copy(std::begin(it->second.m), std::end(it->second.m), out);
-    return B200_OK;
-}
+};
+static constexpr WtBoxes wt_boxes;
 
 template <bool SWIGLU, int KIND>
 static int launch_wt(WtArgs& a, bool allow_split) {
@@ -636,7 +616,7 @@ int umma_gemm_q(int epi, int kind, const __half* A, int64_t a_rows, const void* 
     B200_REQUIRE(groups >= 1 && (offsets || groups == 1), "umma_gemm_q: groups need a device offsets array");
     B200_REQUIRE((group_map || b_rows >= (int64_t)groups * N) && a_rows >= M, "umma_gemm_q: operand shapes do not cover the groups");
     WtArgs a;
-    int rc = make_stage_maps(a.map_x, A, a_rows, K);
+    int rc = make_stage_maps(a.map_x, A, a_rows, K, wt_boxes.b, WT_TOKENS / WT_BOX);
     if (rc) return rc;
     const int64_t row_bytes = q_row_bytes(kind, K);
     const int sbb = 8 * (kind == 3 ? 18 : q_block_bytes(kind));

@@ -153,7 +153,11 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 // Host: tensor map of a row-major fp16 matrix [rows, K] with boxes of 64 x box_rows
 // and the 128-byte swizzle.  Returns B200_OK or an error status.
 int make_tile_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, int box_rows);
-// The same as [K / 64][rows][64]: one load brings box_steps runs of 64 of box_rows rows, run after run.  Not cached.
-int make_stage_map(CUtensorMap* out, const void* base, int64_t rows, int64_t K, int box_rows, int box_steps);
+// n maps of the same matrix as [K / 64][rows][64]: a load of boxes[i] brings `steps` runs of 64 of `rows` rows, run after
+// run.  `boxes` is a table of static storage.
+struct StageBox {
+    int rows, steps;
+};
+int make_stage_maps(CUtensorMap* out, const void* base, int64_t rows, int64_t K, const StageBox* boxes, int n);
 
 }  // namespace b200
