@@ -176,13 +176,15 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
     //   768 x 2048: 92 / 86 (1.1)  100 / 104 (1.5)                                1536 x 2048: 106 / 96 (1.5)  115 / 121 (2.0)
     //   512 x 2560: 96 / 98 (0.8)  106 / 109 (1.1)  105 / 117 (1.5)                512 x 4096: 117 / 115 (0.8)  135 / 150 (1.1)
     //   768 x 4096: 180 / 205 (1.2)  229 / 270 (4.3)
-    const bool exact = kind == 3 && (2 * NK >= 3 * (size_t)ne || d >= 2560);
+    // (Up to eight tokens, which come here where the decode step's kernels refuse them: the digit engine, whose error is a third.)
+    const bool exact = kind == 3 && N > 8 && (2 * NK >= 3 * (size_t)ne || d >= 2560);
     if (!exact && !moe_units_takes(d, E, kind)) return B200_EUNSUPPORTED;       // before anything is launched
     // Below the row count from which products round their activations to fp16, the shared expert must not either: its GEMM
     // would leave 9e-4 of the output's norm where the routed experts leave 3e-7.  The kinds without the exact tensor-core
     // form pay for it in passes of eight tokens (31 tokens, Q8_0, 512 x 1536: 106 us with the GEMM, 141 without), so they do it
     // only for rows as wide as the layer took token by token in fp32 before (768 x 4096: 606, 530 with the GEMM; 3800 there).
-    const bool shared_exact = shared && N < GEMM_MIN_ROWS && (kind == 3 || d >= 4096);
+    // (Up to eight tokens always: their products have fp32 activations in every form.)
+    const bool shared_exact = shared && N < GEMM_MIN_ROWS && (kind == 3 || d >= 4096 || N <= 8);
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
     const size_t o_idx = take(NK * 4), o_w = take(NK * 4), o_grp = take(NK * 4), o_inv = take(NK * 4),
@@ -208,7 +210,7 @@ int moe_forward_units(const float* x, const float* router_w, const float* router
         if ((rc = side.begin())) return rc;
         if (shared_exact) {
             float* sh_act = reinterpret_cast<float*>(base + o_sh);
-            if (kind == 3) {
+            if (kind == 3 && N > 8) {
                 rc = linear_exact(x, sh_g, sh_act, (int)N, d, SH, sh_u);
             } else {
                 float* sh_up = sh_act + N * SH;

@@ -158,6 +158,26 @@ def test_wide_experts(oracle, kind, ne, E, K, SH, N):
     np.testing.assert_allclose(host(out), want, **SUM_ORDER)
 
 
+# Up to eight tokens of rows so wide that the decode step's kernels refuse them (eight tokens of 4096 beside two tiles): they
+# run as units, in fp32 on the exact weights as the others.  Two and four tokens still fit.
+@pytest.mark.parametrize("kind", [2, 3])
+@pytest.mark.parametrize("N", [2, 3, 5, 8])
+def test_few_tokens_of_wide_rows(oracle, kind, N):
+    from gpu_util import SUM_ORDER, dev, empty, host, ops
+    d, E, ne, K, SH = 4096, 256, 8, 2, 1536
+    c = moe_case(oracle, N + kind, N, d, E, ne, K, SH, kind)
+    out, idx, w = empty((N, d)), empty((N, K), torch.int32), empty((N, K))
+    args = [dev(c[k]) for k in ("gates", "ups", "downs", "sh_g", "sh_u", "sh_d")]
+    ops.moe_forward_bias_half(dev(c["x"]), dev(c["router_w"]), dev(c["router_bias"]), *args, out, None, idx, w, None, None, None, N, d, E,
+                              ne, K, SH, kind)
+    oracle.set_weight_rounding(False)
+    want, _, widx, _ = oracle.moe_forward(c["x"], c["router_w"], c["router_bias"], c["gates"], c["ups"], c["downs"], c["sh_g"], c["sh_u"],
+                                          c["sh_d"], d, E, ne, K, SH, kind)
+    oracle.set_weight_rounding(True)
+    assert np.array_equal(host(idx), widx)
+    np.testing.assert_allclose(host(out), want, **SUM_ORDER)
+
+
 # the decode step's kernels, the digit engine's units and the exact tensor-core form
 @pytest.mark.parametrize("kind", [0, 2, 3])
 @pytest.mark.parametrize("N", [1, 3, 8, 9, 24])
