@@ -445,6 +445,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) umma_gemm_kernel(const __grid_c
 // fp16 range.  One warp per row, 8 values per lane per step.
 __global__ void __launch_bounds__(256) pack_rows_f16_kernel(const float* __restrict__ src, const int32_t* __restrict__ row_map,
                                                            int div, __half* __restrict__ dst, int64_t rows, int K) {
+    pdl_launch_dependents();                  // the product's kernel sets itself up meanwhile
     const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (r >= rows) return;
     const int lane = threadIdx.x & 31;

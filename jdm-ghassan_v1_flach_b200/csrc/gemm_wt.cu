@@ -326,6 +326,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
     }
+    pdl_wait();                               // offsets, rows and everything that reads the output now: the kernels before
     wt_build(a, lists);
     wt_fill(a, lists, table, total);
     tc_fence_before();
@@ -600,8 +601,19 @@ static int launch_wt(WtArgs& a, bool allow_split) {
         if (rc) return rc;
         a.c = static_cast<float*>(wsp);
     }
-    kern<<<std::min(tiles * a.k_splits, num_sms()), WT_THREADS, S::SMEM, stream()>>>(a);
-    B200_LAUNCH_CHECK("umma_wt_kernel");
+    // set up (barriers, tensor memory, tensor maps: a microsecond) while the kernel before it ends
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::min(tiles * a.k_splits, num_sms()));
+    cfg.blockDim = dim3(WT_THREADS);
+    cfg.dynamicSmemBytes = S::SMEM;
+    cfg.stream = stream();
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    B200_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+    ++g_kernel_launches;
     return a.k_splits > 1 ? splitk_reduce(a.c, c, a.k_splits, a.split_stride, a.M, a.N, a.ldc) : B200_OK;
 }
 
