@@ -446,6 +446,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) umma_gemm_kernel(const __grid_c
 __global__ void __launch_bounds__(256) pack_rows_f16_kernel(const float* __restrict__ src, const int32_t* __restrict__ row_map,
                                                            int div, __half* __restrict__ dst, int64_t rows, int K) {
     pdl_launch_dependents();                  // the product's kernel sets itself up meanwhile
+    pdl_wait();
     const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (r >= rows) return;
     const int lane = threadIdx.x & 31;
@@ -478,9 +479,7 @@ int pack_rows_f16(const float* src, const int32_t* row_map, int div, __half* dst
     B200_REQUIRE((reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0,
                  "pack_rows_f16: buffers must be 16-byte aligned");
     if (rows == 0) return B200_OK;
-    pack_rows_f16_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, stream()>>>(src, row_map, div > 0 ? div : 1, dst, rows, K);
-    B200_LAUNCH_CHECK("pack_rows_f16_kernel");
-    return B200_OK;
+    return launch_short(pack_rows_f16_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), src, row_map, div > 0 ? div : 1, dst, rows, K);
 }
 
 // ===========================================================================

@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(256, 6)
 mamba_gated_norm_kernel(const float* y, const float* __restrict__ gate, int64_t gate_stride,
                         const float* __restrict__ norm_w, float* out, int d_inner, float eps,
                         __half* __restrict__ out16 = nullptr) {
+    short_begin();
     __shared__ double red[32];
     const int64_t r = blockIdx.x;
     const float* yr = y + r * d_inner;
@@ -296,20 +297,19 @@ mamba_gated_norm_kernel(const float* y, const float* __restrict__ gate, int64_t 
     }
 }
 
-static void launch_gated_norm(const float* y, const float* gate, int64_t gate_stride, const float* norm_w, float* out,
+static int launch_gated_norm(const float* y, const float* gate, int64_t gate_stride, const float* norm_w, float* out,
                               int d_inner, float eps, __half* out16, int64_t rows) {
     const unsigned g = (unsigned)rows;
     const uintptr_t at = (uintptr_t)y | (uintptr_t)gate | (uintptr_t)norm_w | (out16 ? (uintptr_t)out16 : (uintptr_t)out);
     const bool vec = d_inner % 4 == 0 && gate_stride % 4 == 0 && at % 16 == 0;
-#define B200_GATED(PER)                                                                                                                       \
-    (vec ? mamba_gated_norm_kernel<PER, true><<<g, 256, 0, stream()>>>(y, gate, gate_stride, norm_w, out, d_inner, eps, out16)                \
-         : mamba_gated_norm_kernel<PER><<<g, 256, 0, stream()>>>(y, gate, gate_stride, norm_w, out, d_inner, eps, out16))
-    if (d_inner <= 1024) B200_GATED(4);
-    else if (d_inner <= 2048) B200_GATED(8);
-    else if (d_inner <= 3072) B200_GATED(12);
-    else if (d_inner <= 4096) B200_GATED(16);
-#undef B200_GATED
-    else mamba_gated_norm_kernel<0><<<g, 256, 0, stream()>>>(y, gate, gate_stride, norm_w, out, d_inner, eps, nullptr);
+    auto go = [&](auto kern, __half* half_out) {
+        return launch_short(kern, dim3(g), dim3(256), y, gate, gate_stride, norm_w, out, d_inner, eps, half_out);
+    };
+    if (d_inner <= 1024) return vec ? go(mamba_gated_norm_kernel<4, true>, out16) : go(mamba_gated_norm_kernel<4>, out16);
+    if (d_inner <= 2048) return vec ? go(mamba_gated_norm_kernel<8, true>, out16) : go(mamba_gated_norm_kernel<8>, out16);
+    if (d_inner <= 3072) return vec ? go(mamba_gated_norm_kernel<12, true>, out16) : go(mamba_gated_norm_kernel<12>, out16);
+    if (d_inner <= 4096) return vec ? go(mamba_gated_norm_kernel<16, true>, out16) : go(mamba_gated_norm_kernel<16>, out16);
+    return go(mamba_gated_norm_kernel<0>, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -347,6 +347,7 @@ constexpr int CONV_TT = 8;
 __global__ void __launch_bounds__(256)
 mamba_conv_seq4_kernel(const float* __restrict__ proj, const float* __restrict__ conv_w, const float* __restrict__ conv_b,
                        float* __restrict__ bc, int T, MambaDims p, const int32_t* __restrict__ pos) {
+    short_begin();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (c >= p.conv_dim) return;
     const int t0 = blockIdx.y * CONV_TT, b = blockIdx.z;
@@ -579,8 +580,8 @@ int mamba2_step(const float* x, const void* w_in, const float* conv_w, const flo
             B200_LAUNCH_CHECK("mamba_step_scan_kernel");
         }
         if (rc) return rc;
-        launch_gated_norm(y, proj, p.proj, norm_w, y, p.d_inner, p.eps, out_gemm ? y16 : nullptr, batch);
-        B200_LAUNCH_CHECK("mamba_gated_norm_kernel");
+        rc = launch_gated_norm(y, proj, p.proj, norm_w, y, p.d_inner, p.eps, out_gemm ? y16 : nullptr, batch);
+        if (rc) return rc;
         if (out_gemm) return linear_a16(y16, w_out, kind, out, batch, p.d_inner, p.d);
         return linear(y, w_out, kind, out, batch, p.d_inner, p.d);
     }
@@ -605,8 +606,8 @@ int mamba2_step(const float* x, const void* w_in, const float* conv_w, const flo
     mamba_step_scan_kernel<<<dim3(ceil_div(rows, SCAN_WARPS), batch), SCAN_WARPS * 32, 0, stream()>>>(
         bc, dt_raw, dt_bias, a_log, D, ssm_state, y, p.n_heads, p);
     B200_LAUNCH_CHECK("mamba_step_scan_kernel");
-    launch_gated_norm(y, gate, p.d_inner, norm_w, y, p.d_inner, p.eps, nullptr, batch);
-    B200_LAUNCH_CHECK("mamba_gated_norm_kernel");
+    rc = launch_gated_norm(y, gate, p.d_inner, norm_w, y, p.d_inner, p.eps, nullptr, batch);
+    if (rc) return rc;
     return linear(y, w_out, kind, out, batch, p.d_inner, p.d);
 }
 
@@ -619,6 +620,7 @@ constexpr int SSD_MIN_STEPS = 64;
 // decode step expects after this sequence (zeros where the sequence is shorter).
 __global__ void mamba_conv_window_kernel(const float* __restrict__ proj, float* __restrict__ conv_state, int B, int T,
                                          MambaDims p, const int32_t* __restrict__ seq_off) {
+    short_begin();
     const int win = p.k - 1;
     const int64_t total = (int64_t)B * p.conv_dim * win;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -674,18 +676,18 @@ int mamba2_forward(const float* x, const void* w_in, const float* conv_w, const 
         auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
         if (p.k == 4 && p.conv_dim % 4 == 0 && p.d_inner % 4 == 0 && p.proj % 4 == 0 && al16(proj) && al16(bc) &&
             al16(conv_w) && (!conv_b || al16(conv_b)) && cB <= 65535 && ceil_div(cT, CONV_TT) <= 65535) {
-            mamba_conv_seq4_kernel<<<dim3(ceil_div(p.conv_dim / 4, 256), ceil_div(cT, CONV_TT), cB), 256, 0, stream()>>>(
-                proj, conv_w, conv_b, bc, cT, p, pos);
-            B200_LAUNCH_CHECK("mamba_conv_seq4_kernel");
+            rc = launch_short(mamba_conv_seq4_kernel, dim3(ceil_div(p.conv_dim / 4, 256), ceil_div(cT, CONV_TT), cB), dim3(256), proj,
+                              conv_w, conv_b, bc, cT, p, pos);
+            if (rc) return rc;
         } else {
             mamba_conv_seq_kernel<<<grid, 256, 0, stream()>>>(proj, conv_w, conv_b, bc, cB, cT, p, pos);
             B200_LAUNCH_CHECK("mamba_conv_seq_kernel");
         }
         if (conv_state_out && p.k > 1) {
             const int64_t n = (int64_t)B * p.conv_dim * (p.k - 1);
-            mamba_conv_window_kernel<<<(unsigned)std::min<int64_t>(ceil_div64(n, 256), 4096), 256, 0, stream()>>>(
-                proj, conv_state_out, B, T, p, lay ? lay->seq_off : nullptr);
-            B200_LAUNCH_CHECK("mamba_conv_window_kernel");
+            rc = launch_short(mamba_conv_window_kernel, dim3((unsigned)std::min<int64_t>(ceil_div64(n, 256), 4096)), dim3(256), proj,
+                              conv_state_out, B, T, p, lay ? lay->seq_off : nullptr);
+            if (rc) return rc;
         }
     }
     // Long sequences: the chunked form (all steps in parallel, a short carry over chunks);
@@ -737,8 +739,8 @@ int mamba2_forward(const float* x, const void* w_in, const float* conv_w, const 
             if (rc) return rc;
         }
     }
-    launch_gated_norm(y, proj, p.proj, norm_w, y, p.d_inner, p.eps, out_gemm ? y16 : nullptr, NT);
-    B200_LAUNCH_CHECK("mamba_gated_norm_kernel");
+    rc = launch_gated_norm(y, proj, p.proj, norm_w, y, p.d_inner, p.eps, out_gemm ? y16 : nullptr, NT);
+    if (rc) return rc;
     if (out_gemm) return linear_a16(y16, w_out, kind, out, (int)NT, p.d_inner, p.d);
     return linear(y, w_out, kind, out, (int)NT, p.d_inner, p.d);
 }

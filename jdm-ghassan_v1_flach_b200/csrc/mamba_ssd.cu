@@ -84,6 +84,7 @@ __device__ __forceinline__ float softplus_dt(float u) { return (u > 20.0f) ? u :
 // (ty, tx) of a 16 x 16 block owns a 4 x 4 block of its quadrant.  fp32 throughout.
 __global__ void __launch_bounds__(SSD_THREADS)
 ssd_cb_kernel(const float* __restrict__ bc, float* __restrict__ G, int T, MambaDims p, const int2* __restrict__ tab) {
+    short_begin();
     extern __shared__ float sm[];
     constexpr int H = SSD_Q / 2;
     const int N = p.d_state, ld = N + 1;
@@ -270,6 +271,7 @@ ssd_chunk_state_kernel(const float* __restrict__ proj, const float* __restrict__
 __global__ void __launch_bounds__(256)
 ssd_carry_kernel(float* __restrict__ chunk_state, const float* __restrict__ decay, float* __restrict__ state, int B,
                  int NC, MambaDims p, const int32_t* __restrict__ seq_chunk0) {
+    short_begin();
     const int per = p.d_head * p.d_state;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= per) return;
@@ -489,6 +491,7 @@ __global__ void __launch_bounds__(SSD_THREADS, 4)
 ssd_chunk_state16_kernel(const float* __restrict__ proj, const float* __restrict__ bc, const float* __restrict__ dt_bias,
                          const float* __restrict__ a_log, float* __restrict__ dtcum, float* __restrict__ chunk_state,
                          float* __restrict__ decay, int T, int NC, MambaDims p, const int2* __restrict__ tab, int64_t NT) {
+    short_begin();
     extern __shared__ __align__(16) uint8_t sm16[];
     constexpr int P = SSD_P;
     const int N = N_ ? N_ : p.d_state, ldb = N + 8;
@@ -590,6 +593,7 @@ ssd_chunk_out16_kernel(const float* __restrict__ bc, const float* __restrict__ G
                        const float* __restrict__ chunk_state, const float* __restrict__ decay, float* __restrict__ state,
                      const float* __restrict__ Dv, float* __restrict__ y, int T,
                        int NC, MambaDims p, const int2* __restrict__ tab, int64_t NT) {
+    short_begin();
     extern __shared__ __align__(16) uint8_t sm16[];
     constexpr int P = SSD_P;
     const int N = N_ ? N_ : p.d_state, ldc = N + 8;
@@ -783,19 +787,20 @@ int mamba_ssd_scan(const float* proj, const float* bc, const float* dt_bias, con
     B200_REQUIRE(NC <= 65535 * 32 && B <= 65535 && p.n_heads <= 65535, "mamba_ssd_scan: grid too large");
     const int gz = lay ? 1 : B;
     // (the upper right quadrant of every G is never written and never read: s <= t only)
-    ssd_cb_kernel<<<dim3(3 * NC, gz), SSD_THREADS, smem_cb, stream()>>>(bc, G, T, p, tab);
-    B200_LAUNCH_CHECK("ssd_cb_kernel");
+    rc = launch_short_smem(ssd_cb_kernel, dim3(3 * NC, gz), dim3(SSD_THREADS), smem_cb, bc, G, T, p, tab);
+    if (rc) return rc;
     const dim3 grid(NC, p.n_heads, gz);
     const bool half_tiles = !precise && N % 32 == 0;
     const size_t smem_st16 = (size_t)(SSD_Q * (N + 8) + SSD_Q * SSD_LDX16) * 2 + 2 * SSD_Q * 4;
     const size_t smem_out16 = (size_t)std::max(SSD_Q * (N + 8) + P * (N + 8), SSD_Q * SSD_LDM16 + SSD_Q * SSD_LDX16) * 2 + 3 * SSD_Q * 4;
     if (half_tiles)
-        N == 128 ? ssd_chunk_state16_kernel<128><<<grid, SSD_THREADS, smem_st16, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT)
-                 : ssd_chunk_state16_kernel<0><<<grid, SSD_THREADS, smem_st16, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
+        rc = launch_short_smem(N == 128 ? ssd_chunk_state16_kernel<128> : ssd_chunk_state16_kernel<0>, grid, dim3(SSD_THREADS), smem_st16, proj, bc,
+                                 dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
     else if (precise)
         ssd_chunk_state_kernel<true><<<grid, SSD_THREADS, smem_st, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
     else
         ssd_chunk_state_kernel<false><<<grid, SSD_THREADS, smem_st, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
+    if (rc) return rc;
     B200_LAUNCH_CHECK("ssd_chunk_state_kernel");
     // 64 sequences of one chunk: 295 us in the carry, its blocks each a chain of three dependent loads, and a second
     // way of the chunk states through memory
@@ -805,17 +810,18 @@ int mamba_ssd_scan(const float* proj, const float* bc, const float* dt_bias, con
         for (int b = 0; b < B && !carry; ++b) carry = lay->host_off[b + 1] - lay->host_off[b] > SSD_Q;
     }
     if (carry) {
-        ssd_carry_kernel<<<dim3((unsigned)ceil_div(p.d_head * p.d_state, 256), (unsigned)p.n_heads, (unsigned)B), 256, 0, stream()>>>(
-            cstate, decay, state, B, NC, p, lay ? lay->seq_chunk0 : nullptr);
-        B200_LAUNCH_CHECK("ssd_carry_kernel");
+        rc = launch_short(ssd_carry_kernel, dim3((unsigned)ceil_div(p.d_head * p.d_state, 256), (unsigned)p.n_heads, (unsigned)B), dim3(256),
+                            cstate, decay, state, B, NC, p, lay ? lay->seq_chunk0 : nullptr);
+        if (rc) return rc;
     }
     if (half_tiles)
-        N == 128 ? ssd_chunk_out16_kernel<128><<<grid, SSD_THREADS, smem_out16, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT)
-                 : ssd_chunk_out16_kernel<0><<<grid, SSD_THREADS, smem_out16, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
+        rc = launch_short_smem(N == 128 ? ssd_chunk_out16_kernel<128> : ssd_chunk_out16_kernel<0>, grid, dim3(SSD_THREADS), smem_out16, bc, G, dtcum,
+                                 cstate, decay, state, D, y, T, NC, p, tab, NT);
     else if (precise)
         ssd_chunk_out_kernel<true><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
     else
         ssd_chunk_out_kernel<false><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
+    if (rc) return rc;
     B200_LAUNCH_CHECK("ssd_chunk_out_kernel");
     return B200_OK;
 }

@@ -15,6 +15,7 @@
 // 3 cuBLAS calls per expert and synchronises with the host for the group offsets.
 #include "gemm.cuh"
 #include "linear.cuh"
+#include "stream.cuh"
 
 namespace b200 {
 
@@ -28,6 +29,7 @@ constexpr int GROUPED_CHUNK_TOKENS = 8192;
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ y, const int32_t* __restrict__ inv,
                                                          const float* __restrict__ w, float* __restrict__ out, int N,
                                                          int K, int d, int has_shared) {
+    short_begin();
     const int d4 = d >> 2;
     const int64_t total = (int64_t)N * d4;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -149,8 +151,8 @@ int moe_forward_grouped(const float* x, const float* router_w, const float* rout
         if ((rc = side.wait())) return rc;
         const int64_t total = (int64_t)T * (d >> 2);
         const int grid = (int)std::min<int64_t>(ceil_div64(total, 256), (int64_t)num_sms() * 16);
-        moe_combine_kernel<<<grid, 256, 0, stream()>>>(y, inv, w, oc, T, K, d, shared ? 1 : 0);
-        B200_LAUNCH_CHECK("moe_combine_kernel");
+        rc = launch_short(moe_combine_kernel, dim3(grid), dim3(256), y, inv, w, oc, T, K, d, shared ? 1 : 0);
+        if (rc) return rc;
     }
     return B200_OK;
 }
