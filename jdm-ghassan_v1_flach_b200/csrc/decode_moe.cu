@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(
         // 1536 took 16 500 cycles here (now the shared expert's CTAs, 12 000, are what the kernel takes).
         constexpr int RG = MT <= 2 ? 1 : 2;
         const int padded = (groups + 31) & ~31;                       // zeros up to whole runs of 32
-        const bool held = padded <= RG * W * 32;
+        const bool held = (MT > 2 || a.norm_w) && padded <= RG * W * 32;     // (one read is all there is without a norm)
         float4 nw[RG], xv[MT][RG];
         if (held)
 #pragma unroll

@@ -601,7 +601,9 @@ static int launch_wt(WtArgs& a, bool allow_split) {
         if (rc) return rc;
         a.c = static_cast<float*>(wsp);
     }
-    // set up (barriers, tensor memory, tensor maps: a microsecond) while the kernel before it ends
+    // Set up (barriers, tensor memory, tensor maps: a microsecond) while the kernel before it ends: the projections, which have
+    // the device to themselves (64 sequences 102.7 -> 100.1 ms).  Not the experts' products, routed and shared beside each other:
+    // CTAs that wait hold SMs that the other stream's could use (five ragged prompts and steps 37.0 ms, 37.8 with them).
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)std::min(tiles * a.k_splits, num_sms()));
     cfg.blockDim = dim3(WT_THREADS);
@@ -611,7 +613,7 @@ static int launch_wt(WtArgs& a, bool allow_split) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = !SWIGLU && !a.offsets && allow_split ? 1 : 0;
     B200_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
     ++g_kernel_launches;
     return a.k_splits > 1 ? splitk_reduce(a.c, c, a.k_splits, a.split_stride, a.M, a.N, a.ldc) : B200_OK;
