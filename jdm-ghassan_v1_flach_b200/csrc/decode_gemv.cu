@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dg_gemv_kernel(SgArgs a)
         float v[B][8], nv[B][8];
 #pragma unroll
         for (int q = 0; q < B; ++q) {
-            const int i = min(i0 + q * W, all - 1), m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
+            const int i = i0 + q * W, m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
+            if (i >= all) break;
             dg_load8<true>(a.x + (int64_t)m * a.x_stride, c * DG_CHUNK + 8 * lane, a.K, v[q]);
             if (PRO == PRO_RMS && (q > 0 || i0 != warp)) dg_norm8(a.norm_w, c * DG_CHUNK + 8 * lane, a.K, nv[q]);
         }

@@ -73,7 +73,8 @@ __device__ __forceinline__ void dm_stage_norm(const MoeFusedArgs& a, const DgX<K
         float v[B][8], nw[B][8];
 #pragma unroll
         for (int b = 0; b < B; ++b) {
-            const int i = min(i0 + b * W, all - 1), m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
+            const int i = i0 + b * W, m = MT == 1 ? 0 : dg_div(i, a.chunks_inv), c = i - m * chunks;
+            if (i >= all) break;
             dg_load8<true>(a.x + (int64_t)(m0 + m) * a.d, c * DG_CHUNK + 8 * lane, a.d, v[b]);
             if (a.norm_w) dg_norm8(a.norm_w, c * DG_CHUNK + 8 * lane, a.d, nw[b]);
         }
