@@ -15,6 +15,7 @@ namespace b200 {
 
 constexpr int DG_MAX_SETS = 4;
 constexpr size_t DG_SMEM_MAX = 224 * 1024;
+constexpr size_t DG_SMEM_TWO = SMEM_BUDGET - 128;     // of two CTAs on an SM: the kernel's static variables come on top
 
 template <int KIND, int MT, int PRO, int EPI>
 __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dg_gemv_kernel(SgArgs a) {
@@ -195,50 +196,64 @@ int dg_parts(int tiles, int chunks, int warps) {
     return best;
 }
 
-template <int KIND, int MT, int PRO, int EPI>
-static int launch_dg(SgArgs a) {
-    constexpr int W = dg_warps(MT);
+// A launch's CTAs and their dynamic shared memory (0: K does not fit); fills the tiling of a.
+struct DgPlan { int grid = 0; size_t smem = 0; };
+template <int KIND>
+static DgPlan dg_plan(SgArgs& a, int mt, bool norm) {
     const int chunks = dg_chunks(a.K);
-    if (chunks > 255) return fail(B200_EUNSUPPORTED, "stream_gemv: K = %d does not fit the shared-memory staging", a.K);
+    DgPlan plan;
+    if (chunks > 255) return plan;
     a.chunks_inv = dg_inv(chunks);
-    const size_t fixed = dg_x_bytes<KIND>(chunks, MT) + 16 + (size_t)(PRO == PRO_RMS ? chunks : 0) * MT * 8 + 128;
-    int grid = 0;
-    size_t smem = 0;
+    const size_t fixed = dg_x_bytes<KIND>(chunks, mt) + 16 + (size_t)(norm ? chunks : 0) * mt * 8 + 128;
     // Rows per tile: 16, fewer only for rows so wide that a tile would not fit.  Stages: the CTA's whole
     // share when it fits half an SM (the next kernel's CTA fits beside it and streams early), else two sets of
     // as much as does; a whole SM for long shares (an fp16 lm_head: two sets of two tiles, whose products take
     // less time than their 98 KB - one tile at a time, the barriers between them held the stream at 4.3 TB/s).
-    // From three tokens on the products outweigh the hand-over and two CTAs share an SM (a step of five sequences of H-Tiny:
-    // in_proj and out_proj 10.4 and 8.4 us with one, the conversation 38.5 ms; 36.7 with two).
-    for (int R = TILE_ROWS; R >= 1 && !smem; R >>= 1) {
-        if ((R * a.row_bytes) % 16 != 0) break;
+    auto tile = [&](int R, int ctas) {
         a.rows_per_tile = R;
         a.t1 = ceil_div(a.N, R);
         a.t2 = a.t1 + ceil_div(a.N2, R);
         a.num_tiles = a.t2 + ceil_div(a.N3, R);
         a.stage_bytes = (int)((R * a.row_bytes + 127) / 128 * 128);
-        grid = std::min(a.num_tiles, (KIND != KIND_F16 && MT > 2 ? 2 : 1) * num_sms());
-        const int most = ceil_div(a.num_tiles, grid);
-        a.share = a.num_tiles / grid;
-        a.share_rem = a.num_tiles % grid;
-        auto fits = [&](int G, int sets, size_t budget) {
-            a.n_stages = G;
-            a.sets = sets;
-            a.parts = dg_parts(G, chunks, W);
-            a.parts_inv = dg_inv(a.parts);
-            const size_t need = (size_t)sets * G * a.stage_bytes + fixed + (size_t)2 * G * a.parts * dg_red_floats(MT) * 4;
-            if (need > budget) return false;
-            smem = need;
-            return true;
-        };
-        if (most <= 8 && fits(most, 1, SMEM_BUDGET)) break;
-        if (most <= 8)
-            for (int G = std::min(most - 1, 4); G >= 1 && !smem; --G) fits(G, 2, SMEM_BUDGET);
-        for (int G = std::min(most, 4); G >= 2 && !smem; --G) fits(G, most > G ? 2 : 1, DG_SMEM_MAX);
+        plan.grid = std::min(a.num_tiles, ctas);
+        a.share = a.num_tiles / plan.grid;
+        a.share_rem = a.num_tiles % plan.grid;
+        return ceil_div(a.num_tiles, plan.grid);
+    };
+    auto fits = [&](int G, int sets, size_t budget) {
+        a.n_stages = G;
+        a.sets = sets;
+        a.parts = dg_parts(G, chunks, dg_warps(mt));
+        a.parts_inv = dg_inv(a.parts);
+        const size_t need = (size_t)sets * G * a.stage_bytes + fixed + (size_t)2 * G * a.parts * dg_red_floats(mt) * 4;
+        if (need > budget) return false;
+        plan.smem = need;
+        return true;
+    };
+    auto half = [&](int most, size_t budget) {
+        if (most > 8 || fits(most, 1, budget)) return;
+        for (int G = std::min(most - 1, 4); G >= 1 && !plan.smem; --G) fits(G, 2, budget);
+    };
+    // From three tokens on the products outweigh the hand-over and two CTAs share an SM, where two of them fit: else the
+    // grid is two waves, which both stage all activations, and no CTA of the next kernel is set up beside them.  Us a call in a
+    // row with one CTA an SM and with two.  They fit: 1536 -> 6448 in Q4_K, 5 tokens 9.0 / 7.7; 2560 -> 10448, 3 tokens 11.0 /
+    // 9.3.  They do not: 2560 -> 10448, 5 tokens 11.7 / 14.6; 4096 -> 16768, 8 tokens 25.2 / 31.2, in Q8_0 64.7 / 69.3.
+    if (KIND != KIND_F16 && mt > 2 && (TILE_ROWS * a.row_bytes) % 16 == 0) half(tile(TILE_ROWS, 2 * num_sms()), DG_SMEM_TWO);
+    for (int R = TILE_ROWS; R >= 1 && !plan.smem; R >>= 1) {
+        if ((R * a.row_bytes) % 16 != 0) break;
+        const int most = tile(R, num_sms());
+        half(most, SMEM_BUDGET);
+        for (int G = std::min(most, 4); G >= 2 && !plan.smem; --G) fits(G, most > G ? 2 : 1, DG_SMEM_MAX);
         // (one set holds a whole share or nothing: a share of several rounds takes two at least, at half the rows if it must)
-        for (int sets = std::min(most, DG_MAX_SETS); sets >= std::min(most, 2) && !smem; --sets) fits(1, sets, DG_SMEM_MAX);
+        for (int sets = std::min(most, DG_MAX_SETS); sets >= std::min(most, 2) && !plan.smem; --sets) fits(1, sets, DG_SMEM_MAX);
     }
-    if (!smem) return fail(B200_EUNSUPPORTED, "stream_gemv: K = %d does not fit the shared-memory staging", a.K);
+    return plan;
+}
+
+template <int KIND, int MT, int PRO, int EPI>
+static int launch_dg(SgArgs a) {
+    const DgPlan plan = dg_plan<KIND>(a, MT, PRO == PRO_RMS);
+    if (!plan.smem) return fail(B200_EUNSUPPORTED, "stream_gemv: K = %d does not fit the shared-memory staging", a.K);
     auto kern = dg_gemv_kernel<KIND, MT, PRO, EPI>;
     static bool configured = false;
     if (!configured) {
@@ -246,15 +261,17 @@ static int launch_dg(SgArgs a) {
         if (rc) return rc;
         configured = true;
     }
-    return launch_pdl(kern, dim3(grid), dim3(W * 32), smem, a);
+    return launch_pdl(kern, dim3(plan.grid), dim3(dg_warps(MT) * 32), plan.smem, a);
 }
 
 template <int KIND, int PRO, int EPI>
 static int launch_dg_mt(const SgArgs& a) {
-    if (a.M == 1) return launch_dg<KIND, 1, PRO, EPI>(a);
-    if (a.M == 2) return launch_dg<KIND, 2, PRO, EPI>(a);
-    if (a.M <= 4) return launch_dg<KIND, 4, PRO, EPI>(a);
-    return launch_dg<KIND, 8, PRO, EPI>(a);
+    switch (dg_tokens(a.M)) {
+        case 1: return launch_dg<KIND, 1, PRO, EPI>(a);
+        case 2: return launch_dg<KIND, 2, PRO, EPI>(a);
+        case 4: return launch_dg<KIND, 4, PRO, EPI>(a);
+        default: return launch_dg<KIND, 8, PRO, EPI>(a);
+    }
 }
 template <int KIND>
 static int launch_dg_kind(const SgArgs& a, int pro, int epi) {
@@ -279,3 +296,18 @@ int digit_gemv(SgArgs a, int kind, int pro, int epi) {
 }
 
 }  // namespace b200
+
+// The launch of one matrix's product as it would be planned, for tests: CTAs and dynamic shared memory of a CTA.
+extern "C" int b200_digit_gemv_plan(int kind, int M, int N, int K, int norm, int* ctas, int* smem) {
+    using namespace b200;
+    SgArgs a;
+    a.M = M;
+    a.N = N;
+    a.K = K;
+    a.row_bytes = row_bytes_of(kind, K);
+    const int mt = dg_tokens(M);
+    const DgPlan plan = kind == KIND_F16 ? dg_plan<KIND_F16>(a, mt, norm) : dg_plan<0>(a, mt, norm);
+    *ctas = plan.grid;
+    *smem = (int)plan.smem;
+    return plan.smem ? B200_OK : B200_EUNSUPPORTED;
+}

@@ -535,15 +535,17 @@ __global__ void __launch_bounds__(dg_warps(1) * 32, 2) dm_down_kernel(MoeFusedAr
 
 // ---- host side -----------------------------------------------------------------
 // Stages and contraction split for `share` tiles per CTA of tile_bytes each: the whole share in half an SM, or two
-// sets of as much as fits there, or the same in a whole SM.  Returns the dynamic shared memory, 0 if nothing fits.
+// sets of as much as fits there, or the same in a whole SM (unless two CTAs are to share it).  Returns the dynamic
+// shared memory, 0 if nothing fits.
 template <int KIND>
-static size_t dm_plan(MoeFusedArgs& a, int tiles, int ctas, size_t tile_bytes, int chunks, int mt, size_t fixed, size_t floor_bytes) {
+static size_t dm_plan(MoeFusedArgs& a, int tiles, int ctas, size_t tile_bytes, int chunks, int mt, size_t fixed, size_t floor_bytes, bool share = false) {
     const int most = ctas ? ceil_div(tiles, ctas) : 0;
     a.share = ctas ? tiles / ctas : 0;
     a.share_rem = ctas ? tiles % ctas : 0;
     a.stage_bytes = (int)((tile_bytes + 127) / 128 * 128);
     if (chunks > 255) return 0;
-    for (const size_t budget : {(size_t)SMEM_BUDGET - 2048, (size_t)SMEM_BUDGET_FULL - 2048})
+    for (const size_t budget : {(size_t)SMEM_BUDGET - 2048, (size_t)SMEM_BUDGET_FULL - 2048}) {
+        if (share && budget > SMEM_BUDGET) break;
         for (int G = std::max(1, std::min(most, 8)); G >= 1; --G) {
             a.n_stages = G;
             a.sets = G >= most ? 1 : 2;
@@ -553,6 +555,7 @@ static size_t dm_plan(MoeFusedArgs& a, int tiles, int ctas, size_t tile_bytes, i
                                                           (size_t)2 * G * a.parts * dg_red_floats(mt) * 4);
             if (need <= budget) return need;
         }
+    }
     return 0;
 }
 template <typename Kern>
@@ -571,45 +574,76 @@ static int dm_kernel1(MoeFusedArgs a, size_t smem, int grid) {
     return dm_launch(dm_router_shared_kernel<KIND, MT>, configured, dim3(grid), dg_warps(MT) * 32, smem, a);
 }
 
+// The three launches of a layer: arguments with their tiling, CTAs (per token in the second and third) and dynamic shared
+// memory (0: does not fit).
+struct DmPlan {
+    MoeFusedArgs p1, p2, p3;
+    int g1 = 0, g2 = 0, g3 = 0;
+    size_t s1 = 0, s2 = 0, s3 = 0;
+};
 template <int KIND>
-static int dm_kind(const MoeFusedArgs& a) {
-    const int mt = a.M == 1 ? 1 : a.M == 2 ? 2 : a.M <= 4 ? 4 : 8;
+static DmPlan dm_plan_layer(const MoeFusedArgs& a) {
+    DmPlan p;
+    p.p1 = p.p2 = p.p3 = a;
     const size_t rb_d = row_bytes_of(KIND, a.d), rb_e = row_bytes_of(KIND, a.E), rb_s = a.SH > 0 ? row_bytes_of(KIND, a.SH) : 0;
     // One CTA of kernels 2 and 3 on an SM for one token, so that the next kernel's fits beside it and fetches early.  Two for more:
     // their time is a CTA's rounds of products (13 tiles each at five tokens), which twelve warps fill an SM with to 39 %
     // of its issue slots.  Us for gate / up at 2, 3, 5, 8 tokens (H-Tiny): 7.3, 11.5, 17.3, 24.2 with one, 5.7, 6.5, 9.7, 14.3 with two.
-    const int per_token = std::max(1, (a.M > 1 ? 2 : 1) * num_sms() / a.M);
-    // all three are planned before the first is launched: a layer runs whole or not at all
-    MoeFusedArgs p1 = a, p2 = a, p3 = a;
+    // One again where two do not fit: the second would be a second wave, which stages its token again.  The layer in us with such a
+    // second wave and without: 4096 x 768 in Q8_0 (gate / up), two tokens 134.6 / 128.7, in Q4_K (down) 77.2 / 72.6; 1536 x 1024 with
+    // eight experts in Q4_K (down), five tokens 61.6 / 57.3; 1536 x 512 in Q8_0 (down), four tokens 33.4 / 31.8.  (2560 x 512 in
+    // Q8_0, two tokens 27.5 / 29.8: 160 tiles per token for 74 CTAs are three to some, and two waves even that out.)
+    auto per_token = [&](int per_sm) { return std::max(1, per_sm * num_sms() / a.M); };
+    const int most_per_sm = a.M > 1 ? 2 : 1;
     const int n_router = ceil_div(a.ne, DM_ROUTER), sh_tiles = a.SH / 8;
     const int sh_ctas = std::min(sh_tiles, std::max(8, num_sms() - n_router));
     const size_t router_bytes = (size_t)DM_ROUTER * a.d * 4 + std::max<size_t>((size_t)DM_ROUTER * a.M * dm_chain_stride(a.d) * 4, (size_t)a.M * a.ne * 4);
-    p1.chunks_inv = dg_inv(std::min(255, dg_chunks(a.d)));
-    const size_t s1 = dm_plan<KIND>(p1, sh_tiles, sh_ctas, sh_ctas ? 16 * rb_d : 0, sh_ctas ? dg_chunks(a.d) : 1, mt, (size_t)dg_chunks(a.d) * mt * 8, router_bytes);
-    const int t2 = a.K * (a.E / 8), g2 = std::min(t2, per_token);
-    p2.per_inv = 0xFFFFFFFFu / (uint32_t)(a.E / 8) + 1u;      // exact quotients below 2^16 (E / 8 >= 4)
-    const size_t s2 = dm_plan<KIND>(p2, t2, g2, 16 * rb_d, dg_chunks(a.d), 1, (size_t)dg_chunks(a.d) * 8, 0);
-    p3.ec_inv = dg_inv(std::min(255, dg_chunks(a.E)));
+    const int mt = dg_tokens(a.M);
+    p.p1.chunks_inv = dg_inv(std::min(255, dg_chunks(a.d)));
+    p.g1 = n_router + sh_ctas;
+    p.s1 = dm_plan<KIND>(p.p1, sh_tiles, sh_ctas, sh_ctas ? 16 * rb_d : 0, sh_ctas ? dg_chunks(a.d) : 1, mt, (size_t)dg_chunks(a.d) * mt * 8, router_bytes);
+    const int t2 = a.K * (a.E / 8);
+    p.p2.per_inv = 0xFFFFFFFFu / (uint32_t)(a.E / 8) + 1u;      // exact quotients below 2^16 (E / 8 >= 4)
+    auto gate_up = [&](int n, bool share) {
+        p.g2 = std::min(t2, per_token(n));
+        p.s2 = dm_plan<KIND>(p.p2, t2, p.g2, 16 * rb_d, dg_chunks(a.d), 1, (size_t)dg_chunks(a.d) * 8, 0, share);
+    };
+    if (most_per_sm == 2) gate_up(2, true);
+    if (!p.s2) gate_up(1, false);
+    if (!p.s2 && most_per_sm == 2) gate_up(2, false);      // rows so wide that two tiles do not fit a whole SM, and one to each of two waves
+    p.p3.ec_inv = dg_inv(std::min(255, dg_chunks(a.E)));
     // The down rows of the shared and all K experts: 16 to a tile, fewer where those do not fit (Q8_0, experts of 1024 and
     // eight of them: 4.5 KB of rows per output), while a copy still moves whole 16-byte words.
-    size_t s3 = 0;
-    int g3 = 0;
-    for (int R = TILE_ROWS; R >= 1 && !s3 && (R * rb_e) % 16 == 0 && (R * rb_s) % 16 == 0; R >>= 1) {
+    auto down = [&](int R, int n, bool share) {
         const int t3 = ceil_div(a.d, R);
-        g3 = std::min(t3, per_token);
-        p3.rows_per_tile = R;
-        s3 = dm_plan<KIND>(p3, t3, g3, R * (rb_s + a.K * rb_e), dg_chunks(a.SH) + a.K * dg_chunks(a.E), 1, 0, 0);
-    }
-    if (!s1 || !s2) return fail(B200_EUNSUPPORTED, "moe_fused: hidden size %d does not fit the shared-memory staging", a.d);
-    if (!s3)
+        p.g3 = std::min(t3, per_token(n));
+        p.p3.rows_per_tile = R;
+        p.s3 = dm_plan<KIND>(p.p3, t3, p.g3, R * (rb_s + a.K * rb_e), dg_chunks(a.SH) + a.K * dg_chunks(a.E), 1, 0, 0, share);
+    };
+    auto copies = [&](int R) { return (R * rb_e) % 16 == 0 && (R * rb_s) % 16 == 0; };
+    if (most_per_sm == 2 && copies(TILE_ROWS)) down(TILE_ROWS, 2, true);
+    for (int R = TILE_ROWS; R >= 1 && !p.s3 && copies(R); R >>= 1) down(R, 1, false);
+    return p;
+}
+template <int KIND>
+static int dm_kind(const MoeFusedArgs& a) {
+    // all three are planned before the first is launched: a layer runs whole or not at all
+    const DmPlan p = dm_plan_layer<KIND>(a);
+    if (!p.s1 || !p.s2) return fail(B200_EUNSUPPORTED, "moe_fused: hidden size %d does not fit the shared-memory staging", a.d);
+    if (!p.s3)
         return fail(B200_EUNSUPPORTED, "moe_fused: the down rows of %d experts of %d and a shared one of %d do not fit the shared-memory staging",
                     a.K, a.E, a.SH);
-    int rc = mt == 1 ? dm_kernel1<KIND, 1>(p1, s1, n_router + sh_ctas) : mt == 2 ? dm_kernel1<KIND, 2>(p1, s1, n_router + sh_ctas)
-             : mt == 4 ? dm_kernel1<KIND, 4>(p1, s1, n_router + sh_ctas) : dm_kernel1<KIND, 8>(p1, s1, n_router + sh_ctas);
+    int rc;
+    switch (dg_tokens(a.M)) {
+        case 1: rc = dm_kernel1<KIND, 1>(p.p1, p.s1, p.g1); break;
+        case 2: rc = dm_kernel1<KIND, 2>(p.p1, p.s1, p.g1); break;
+        case 4: rc = dm_kernel1<KIND, 4>(p.p1, p.s1, p.g1); break;
+        default: rc = dm_kernel1<KIND, 8>(p.p1, p.s1, p.g1); break;
+    }
     if (rc) return rc;
     static bool c2 = false, c3 = false;
-    rc = dm_launch(dm_gateup_kernel<KIND>, c2, dim3(g2, a.M), dg_warps(1) * 32, s2, p2);
-    return rc ? rc : dm_launch(dm_down_kernel<KIND>, c3, dim3(g3, a.M), dg_warps(1) * 32, s3, p3);
+    rc = dm_launch(dm_gateup_kernel<KIND>, c2, dim3(p.g2, a.M), dg_warps(1) * 32, p.s2, p.p2);
+    return rc ? rc : dm_launch(dm_down_kernel<KIND>, c3, dim3(p.g3, a.M), dg_warps(1) * 32, p.s3, p.p3);
 }
 
 // moe_fused() for packed weights (kind 0 .. 3); sizes checked there.
@@ -626,3 +660,23 @@ int moe_digit(const MoeFusedArgs& a, int kind) {
 }
 
 }  // namespace b200
+
+// The three launches of a layer as they would be planned, for tests: CTAs and dynamic shared memory of a CTA of each.
+extern "C" int b200_moe_digit_plan(int kind, int M, int d, int E, int ne, int K, int SH, int* ctas, int* smem) {
+    using namespace b200;
+    MoeFusedArgs a;
+    a.M = M;
+    a.d = d;
+    a.E = E;
+    a.ne = ne;
+    a.K = K;
+    a.SH = SH;
+    const DmPlan p = kind == 0 ? dm_plan_layer<0>(a) : kind == 1 ? dm_plan_layer<1>(a) : kind == 2 ? dm_plan_layer<2>(a) : dm_plan_layer<3>(a);
+    const int g[3] = {p.g1, p.g2 * M, p.g3 * M};
+    const size_t s[3] = {p.s1, p.s2, p.s3};
+    for (int i = 0; i < 3; ++i) {
+        ctas[i] = g[i];
+        smem[i] = (int)s[i];
+    }
+    return p.s1 && p.s2 && p.s3 ? B200_OK : B200_EUNSUPPORTED;
+}

@@ -25,6 +25,8 @@ namespace b200 {
 // Warps of a CTA: two CTAs of consecutive kernels share an SM, so twelve warps leave 80 registers, which one
 // and two tokens fit; more tokens need the accumulators of eight warps at 128.
 __host__ __device__ constexpr int dg_warps(int MT) { return MT <= 2 ? 12 : 8; }
+// Token columns of the instance that takes M tokens.
+inline int dg_tokens(int M) { return M <= 2 ? M : M <= 4 ? 4 : 8; }
 constexpr int DG_CHUNK = 256;                 // activations that share a scale
 // Chunks that a warp loads together before it stages them: the activations come from L2, and one after the other five tokens
 // of 1536 were four such ways for each warp.  A batch's places past the last chunk load nothing: repeating the last chunk

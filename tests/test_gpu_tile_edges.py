@@ -37,6 +37,21 @@ def test_few_token_products(oracle, kind, M, K, N):
     np.testing.assert_allclose(host(y), want, **tol)
 
 
+# More tiles than SMs, on both sides of the line from which two CTAs no longer fit an SM's shared memory.
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("M", [3, 4, 5, 8])
+@pytest.mark.parametrize("K", [1536, 2560])
+def test_few_token_products_of_one_and_two_ctas(oracle, kind, M, K):
+    from gpu_util import SUM_ORDER, dev, empty, host, ops
+    N = 4772                                            # of 16 rows: two tiles for each of 148 SMs and three over, the last with four rows
+    r = np.random.default_rng(K + 10 * M + kind)
+    x = r.standard_normal((M, K)).astype(np.float32)
+    w = oracle.quantize((r.standard_normal(N * K) * 0.02).astype(np.float32), kind)
+    y = empty((M, N))
+    ops.linear_forward_q4(dev(x), dev(w), y, M, K, N, kind)
+    np.testing.assert_allclose(host(y), oracle.linear_exact(x, w, kind, M, K, N), **SUM_ORDER)
+
+
 # Rows so wide that one tile of sixteen fills the shared memory, and more tiles than a round of the CTAs takes.
 @pytest.mark.parametrize("kind,K,M", [(-1, 4096, 1), (-1, 2304, 8), (-1, 5632, 2), (0, 4608, 8), (1, 4352, 8), (2, 4096, 8), (2, 6144, 1),
                                       (2, 4608, 3), (3, 4608, 8), (3, 10496, 1)])
