@@ -796,12 +796,14 @@ int mamba_ssd_scan(const float* proj, const float* bc, const float* dt_bias, con
     if (half_tiles)
         rc = launch_short_smem(N == 128 ? ssd_chunk_state16_kernel<128> : ssd_chunk_state16_kernel<0>, grid, dim3(SSD_THREADS), smem_st16, proj, bc,
                                  dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
-    else if (precise)
-        ssd_chunk_state_kernel<true><<<grid, SSD_THREADS, smem_st, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
-    else
-        ssd_chunk_state_kernel<false><<<grid, SSD_THREADS, smem_st, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
+    else {
+        if (precise)
+            ssd_chunk_state_kernel<true><<<grid, SSD_THREADS, smem_st, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
+        else
+            ssd_chunk_state_kernel<false><<<grid, SSD_THREADS, smem_st, stream()>>>(proj, bc, dt_bias, a_log, dtcum, cstate, decay, T, NC, p, tab, NT);
+        B200_LAUNCH_CHECK("ssd_chunk_state_kernel");
+    }
     if (rc) return rc;
-    B200_LAUNCH_CHECK("ssd_chunk_state_kernel");
     // 64 sequences of one chunk: 295 us in the carry, its blocks each a chain of three dependent loads, and a second
     // way of the chunk states through memory
     bool carry = NC > 1;
@@ -817,12 +819,14 @@ int mamba_ssd_scan(const float* proj, const float* bc, const float* dt_bias, con
     if (half_tiles)
         rc = launch_short_smem(N == 128 ? ssd_chunk_out16_kernel<128> : ssd_chunk_out16_kernel<0>, grid, dim3(SSD_THREADS), smem_out16, bc, G, dtcum,
                                  cstate, decay, state, D, y, T, NC, p, tab, NT);
-    else if (precise)
-        ssd_chunk_out_kernel<true><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
-    else
-        ssd_chunk_out_kernel<false><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
+    else {
+        if (precise)
+            ssd_chunk_out_kernel<true><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
+        else
+            ssd_chunk_out_kernel<false><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
+        B200_LAUNCH_CHECK("ssd_chunk_out_kernel");
+    }
     if (rc) return rc;
-    B200_LAUNCH_CHECK("ssd_chunk_out_kernel");
     return B200_OK;
 }
 

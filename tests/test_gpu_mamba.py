@@ -170,6 +170,35 @@ def test_forward_then_steps_continue_state(oracle):
     np.testing.assert_allclose(host(dstate), st, rtol=5e-4, atol=5e-6)
 
 
+# fp16 tiles (state 64 and 128), fp32 tiles of the chunked scan (state 16), and fewer steps than it takes
+@pytest.mark.parametrize("T,d_state", [(300, 128), (300, 64), (300, 16), (33, 128)])
+def test_forward_counts_its_launches(oracle, T, d_state):
+    """b200_kernel_launches() goes up by the kernels that the call enqueues, as a capture of it records them."""
+    from cuda.bindings import runtime as rt
+    from gpu_util import dev, empty, ops, pkg
+    c = mamba_case(oracle, T + d_state, B=1, T=T, d=256, n_heads=4, d_head=64, d_state=d_state, k=4, wkind=3)
+    a = c["args"]
+    args = [dev(a[0]), *_dev_params(a[1:9]), dev(a[9]), empty((1, T, a[12])), *a[10:], 3]
+    lib, stream = pkg.lib(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    lib.b200_set_stream(stream.cuda_stream)
+    try:
+        ops.mamba2_forward_half(*args)                                    # workspaces
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            before = lib.b200_kernel_launches()
+            ops.mamba2_forward_half(*args)
+            counted = lib.b200_kernel_launches() - before
+    finally:
+        lib.b200_set_stream(None)
+    raw = rt.cudaGraph_t(graph.raw_cuda_graph())
+    n = rt.cudaGraphGetNodes(raw)[2]
+    nodes = rt.cudaGraphGetNodes(raw, n)[1]
+    kernels = sum(rt.cudaGraphNodeGetType(v)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for v in nodes)
+    assert counted == kernels > 4
+
+
 def test_argument_errors():
     from gpu_util import B200Error, empty, ops
     t = empty(4096)
