@@ -146,12 +146,11 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dg_gemv_kernel(SgArgs a)
     }
 
     const uint32_t ra = min(lane >> 2, a.rows_per_tile - 1) * (uint32_t)a.row_bytes, rb = min((lane >> 2) + 8, a.rows_per_tile - 1) * (uint32_t)a.row_bytes;
-    bool ok = true;
     for (int r = 0, set = 0, parity = 0; r < rounds; ++r) {
         const int n = min(G, n_my - r * G);
         float* rr = red + (size_t)(r & 1) * G * P * dg_red_floats(MT);
         if (r > 0 && EPI == EPI_RESIDUAL && (int)threadIdx.x < n * ELEMS && element(r, threadIdx.x, s0, n0, m0)) epi.prefetch(a, n0, m0);
-        ok = ok && mbar_wait(&bar[set], parity, a.status);
+        const bool ok = mbar_wait(&bar[set], parity, a.status);
         if (ok) {
             for (int u = warp; u < n * P; u += W) {
                 const int tile = dg_div(u, a.parts_inv), part = u - tile * P;
@@ -165,7 +164,13 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dg_gemv_kernel(SgArgs a)
                 dg_finish<KIND, MT>(acc, rr + u * dg_red_floats(MT), lane);
             }
         }
-        if (!__syncthreads_and(ok)) break;
+        if (!__syncthreads_and(ok)) {
+            // a wait that ran out: no copy of this CTA may be left under way
+            if (threadIdx.x == 0)
+                for (int t = 0; t < min(a.sets, rounds); ++t)
+                    for (int par = 0; par < 2 && !mbar_wait(&bar[t], par, a.status); ++par) {}
+            break;
+        }
         if (threadIdx.x == 0 && r + a.sets < rounds) issue(r + a.sets, set);
         for (int e = threadIdx.x; e < n * ELEMS; e += W * 32) {
             const float* re = rr + e / ELEMS * P * dg_red_floats(MT);
@@ -180,10 +185,6 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dg_gemv_kernel(SgArgs a)
             parity ^= 1;
         }
     }
-    // a wait that ran out: no copy of this CTA may be left under way
-    if (!ok && threadIdx.x == 0)
-        for (int set = 0; set < min(a.sets, rounds); ++set)
-            for (int par = 0; par < 2 && !mbar_wait(&bar[set], par, a.status); ++par) {}
 }
 
 // Warps per tile's contraction: fewest passes of the warps over `tiles` tiles, ties to fewer parts.
