@@ -170,7 +170,9 @@ __device__ __noinline__ void dm_route(const MoeFusedArgs& a, float* scratch, con
 }
 
 // ---- kernel 1 ------------------------------------------------------------------
-template <int KIND, int MT>
+// NORM: a norm may be in front (a.norm_w says).  One token without one has an instance of its own: its serial path is the whole
+// kernel, and the code for a held row, which it never takes, cost it 0.3 us.
+template <int KIND, int MT, bool NORM>
 __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(MoeFusedArgs a) {
     constexpr int W = dg_warps(MT);
     extern __shared__ __align__(128) uint8_t smem[];
@@ -209,13 +211,14 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(
         // 1536 took 16 500 cycles here (now the shared expert's CTAs, 12 000, are what the kernel takes).
         constexpr int RG = MT <= 2 ? 1 : 2;
         const int padded = (groups + 31) & ~31;                       // zeros up to whole runs of 32
-        const bool held = (MT > 2 || a.norm_w) && padded <= RG * W * 32;     // (one read is all there is without a norm)
+        const bool norm = NORM && a.norm_w;
+        const bool held = (MT > 2 || norm) && padded <= RG * W * 32;     // (one read is all there is without a norm)
         float4 nw[RG], xv[MT][RG];
         if (held)
 #pragma unroll
             for (int q = 0; q < RG; ++q) {
                 const int g = threadIdx.x + q * W * 32;
-                nw[q] = a.norm_w && g < groups ? dg_norm4(a.norm_w + 4 * g) : make_float4(1.f, 1.f, 1.f, 1.f);
+                nw[q] = norm && g < groups ? dg_norm4(a.norm_w + 4 * g) : make_float4(1.f, 1.f, 1.f, 1.f);
             }
         pdl_wait();
         auto load = [&](int m, int g) {
@@ -227,7 +230,7 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(
 #pragma unroll
                 for (int q = 0; q < RG; ++q)
                     if (m < a.M) xv[m][q] = load(m, threadIdx.x + q * W * 32);
-        if (a.norm_w) {
+        if (norm) {
             auto square = [](float4 v) { return (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w; };
             if (held) {
 #pragma unroll
@@ -260,7 +263,7 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(
         const bool ok = mbar_wait(&bar[0], 0, a.status);
         // group sums ((a0 b0 + a1 b1) + a2 b2) + a3 b3 of every (token, expert)
         auto sums = [&](int m, int g, float4 x, float4 w) {
-            if (a.norm_w) {
+            if (norm) {
                 const float f = inv[m];
                 x = make_float4(x.x * f * w.x, x.y * f * w.y, x.z * f * w.z, x.w * f * w.w);
             }
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dm_router_shared_kernel(
         } else {
             for (int m = 0; m < a.M; ++m)
                 for (int g = threadIdx.x; g < padded; g += W * 32)
-                    sums(m, g, load(m, g), a.norm_w && g < groups ? dg_norm4(a.norm_w + 4 * g) : make_float4(1.f, 1.f, 1.f, 1.f));
+                    sums(m, g, load(m, g), norm && g < groups ? dg_norm4(a.norm_w + 4 * g) : make_float4(1.f, 1.f, 1.f, 1.f));
         }
         __syncthreads();
         // the ordered additions: one lane per chain, the next 32 sums on their way while 32 are added
@@ -568,10 +571,10 @@ static int dm_launch(Kern kern, bool& configured, dim3 grid, int threads, size_t
     return launch_pdl(kern, grid, dim3(threads), smem, a);
 }
 
-template <int KIND, int MT>
+template <int KIND, int MT, bool NORM = true>
 static int dm_kernel1(MoeFusedArgs a, size_t smem, int grid) {
     static bool configured = false;
-    return dm_launch(dm_router_shared_kernel<KIND, MT>, configured, dim3(grid), dg_warps(MT) * 32, smem, a);
+    return dm_launch(dm_router_shared_kernel<KIND, MT, NORM>, configured, dim3(grid), dg_warps(MT) * 32, smem, a);
 }
 
 // The three launches of a layer: arguments with their tiling, CTAs (per token in the second and third) and dynamic shared
@@ -635,7 +638,7 @@ static int dm_kind(const MoeFusedArgs& a) {
                     a.K, a.E, a.SH);
     int rc;
     switch (dg_tokens(a.M)) {
-        case 1: rc = dm_kernel1<KIND, 1>(p.p1, p.s1, p.g1); break;
+        case 1: rc = a.norm_w ? dm_kernel1<KIND, 1>(p.p1, p.s1, p.g1) : dm_kernel1<KIND, 1, false>(p.p1, p.s1, p.g1); break;
         case 2: rc = dm_kernel1<KIND, 2>(p.p1, p.s1, p.g1); break;
         case 4: rc = dm_kernel1<KIND, 4>(p.p1, p.s1, p.g1); break;
         default: rc = dm_kernel1<KIND, 8>(p.p1, p.s1, p.g1); break;
