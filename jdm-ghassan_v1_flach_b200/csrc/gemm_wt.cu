@@ -333,12 +333,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     constexpr uint32_t tmem = 0;              // all 512 columns: the allocation starts at the first
-    // The next kernel's blocks go wherever there is room, as soon as every CTA has come here: on the few SMs that have no CTA of
-    // this kernel or are done with it early, up to eight of them on one, where they wait and then run crowded.  So only for a decode
-    // batch, whose next kernel is short.  After more rows it is launched when the CTAs have ended, on all SMs.  In us, always
-    // launched early and now: 8192 -> 4096, 1000 rows 124 -> 76; 4096 -> 6144, 517 rows 40.5 -> 24.6; 3072 -> 1536, 2000 rows
-    // 32.2 -> 21.6; never and now: 3072 -> 1536, 32 rows 12.4 -> 10.9; 2560 -> 10448, 64 rows 15.1 -> 14.3.
-    if (a.M <= WT_TOKENS) pdl_launch_dependents();
+    pdl_launch_dependents();
     const int mine = ((int)blockIdx.x < total ? total - (int)blockIdx.x + (int)gridDim.x - 1 : 0) / (int)gridDim.x;
     // every role walks the same tiles; sb0 .. sb1: a tile's range of K in units of 256
     auto range = [&](const WtTile& w, int& sb0, int& sb1) {
