@@ -15,7 +15,7 @@ enum { GEMM_EPI_STORE = 0, GEMM_EPI_SWIGLU = 1 };
 constexpr int GEMM_MIN_ROWS = 32;
 
 // dst[r, :] = fp16(src[(row_map ? row_map[r] / div : r), :]); K % 8 == 0.
-int pack_rows_f16(const float* src, const int32_t* row_map, int div, __half* dst, int64_t rows, int K);
+int pack_rows_f16(const float* src, const int32_t* row_map, int div, __half* dst, int64_t rows, int K, bool early = true);
 // The fp16 copy a producer registered for exactly these rows (f16_shadow_set), or null; see gemm_umma.cu.
 void f16_shadow_set(const float* src, const __half* rows16, int64_t rows, int K);
 void f16_shadow_clear();

@@ -474,12 +474,17 @@ const __half* f16_shadow_find(const float* src, int64_t rows, int K) {
     return (src && g_f16_shadow.src == src && g_f16_shadow.rows == rows && g_f16_shadow.K == K) ? g_f16_shadow.rows16 : nullptr;
 }
 
-int pack_rows_f16(const float* src, const int32_t* row_map, int div, __half* dst, int64_t rows, int K) {
+// early: set up while the kernel before it ends.
+int pack_rows_f16(const float* src, const int32_t* row_map, int div, __half* dst, int64_t rows, int K, bool early) {
     B200_REQUIRE(src && dst && rows >= 0 && K > 0 && K % 8 == 0, "pack_rows_f16: K must be a positive multiple of 8");
     B200_REQUIRE((reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0,
                  "pack_rows_f16: buffers must be 16-byte aligned");
     if (rows == 0) return B200_OK;
-    return launch_short(pack_rows_f16_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), src, row_map, div > 0 ? div : 1, dst, rows, K);
+    const dim3 grid((unsigned)((rows + 7) / 8));
+    if (early) return launch_short(pack_rows_f16_kernel, grid, dim3(256), src, row_map, div > 0 ? div : 1, dst, rows, K);
+    pack_rows_f16_kernel<<<grid, 256, 0, stream()>>>(src, row_map, div > 0 ? div : 1, dst, rows, K);
+    B200_LAUNCH_CHECK("pack_rows_f16_kernel");
+    return B200_OK;
 }
 
 // ===========================================================================

@@ -153,7 +153,12 @@ int linear(const float* x, const void* w, int kind, float* y, int M, int K, int 
         const __half* a16 = f16_shadow_find(x, M, K);       // rows a fused norm has already written as fp16
         if (!a16) {
             __half* packed = static_cast<__half*>(ws);
-            rc = pack_rows_f16(x, nullptr, 1, packed, M, K);
+            // The kernel before may be a product, whose CTAs leave room for these blocks only on the few SMs that have none of
+            // them or are done early: launched before its end, up to eight of them wait on one SM and then run crowded there.
+            // So only small inputs are launched so.  In us, rounding and product, all launched early and now: 1000 rows 8192 -> 4096
+            // 124 -> 76 and 768 -> 3224 14.9 -> 12.3; 4096 -> 6144, 517 rows 40.5 -> 24.5; 3072 -> 1536, 2000 rows 32.2 -> 22.5.  No
+            // difference: 1536 -> 6448, 300 rows 12.5 / 12.4; a small layer by itself, 379 rows of 768, would be 2 % slower.
+            rc = pack_rows_f16(x, nullptr, 1, packed, M, K, (int64_t)M * K <= 1 << 19);
             if (rc) return rc;
             a16 = packed;
         }
