@@ -16,6 +16,7 @@ namespace b200 {
 constexpr int DG_MAX_SETS = 4;
 constexpr size_t DG_SMEM_MAX = 224 * 1024;
 constexpr size_t DG_SMEM_TWO = SMEM_BUDGET - 128;     // of two CTAs on an SM: the kernel's static variables come on top
+constexpr size_t DG_SMEM_THIRD = 77 * 1024;           // from here on a third CTA does not fit
 
 template <int KIND, int MT, int PRO, int EPI>
 __global__ void __launch_bounds__(dg_warps(MT) * 32, 2) dg_gemv_kernel(SgArgs a) {
@@ -197,10 +198,11 @@ int dg_parts(int tiles, int chunks, int warps) {
     return best;
 }
 
-// A launch's CTAs and their dynamic shared memory (0: K does not fit); fills the tiling of a.
+// A launch's CTAs and their dynamic shared memory (0: K does not fit); fills the tiling of a.  plain: a product by itself,
+// without the norm or the epilogues of a decode step.
 struct DgPlan { int grid = 0; size_t smem = 0; };
 template <int KIND>
-static DgPlan dg_plan(SgArgs& a, int mt, bool norm) {
+static DgPlan dg_plan(SgArgs& a, int mt, bool norm, bool plain) {
     const int chunks = dg_chunks(a.K);
     DgPlan plan;
     if (chunks > 255) return plan;
@@ -236,10 +238,19 @@ static DgPlan dg_plan(SgArgs& a, int mt, bool norm) {
         for (int G = std::min(most - 1, 4); G >= 1 && !plan.smem; --G) fits(G, 2, budget);
     };
     // From three tokens on the products outweigh the hand-over and two CTAs share an SM, where two of them fit: else the
-    // grid is two waves, which both stage all activations, and no CTA of the next kernel is set up beside them.  Us a call in a
-    // row with one CTA an SM and with two.  They fit: 1536 -> 6448 in Q4_K, 5 tokens 9.0 / 7.7; 2560 -> 10448, 3 tokens 11.0 /
-    // 9.3.  They do not: 2560 -> 10448, 5 tokens 11.7 / 14.6; 4096 -> 16768, 8 tokens 25.2 / 31.2, in Q8_0 64.7 / 69.3.
-    if (KIND != KIND_F16 && mt > 2 && (TILE_ROWS * a.row_bytes) % 16 == 0) half(tile(TILE_ROWS, 2 * num_sms()), DG_SMEM_TWO);
+    // grid is two waves, which both stage all activations, and no CTA of the next kernel is set up beside them.  A step of 3, 5 and 8
+    // sequences with one CTA an SM and with two: H-Tiny in Q4_K 1611 / 1586, 2236 / 2160 and 2817 / 2740 us, in Q8_0 1878 / 1836, 2755 /
+    // 2596 and 3405 / 3254, the small model in Q4_K 268 / 261, 310 / 306 and 351 / 346.  They do not fit (us a call in a row):
+    // 2560 -> 10448, 5 tokens 11.7 / 14.6; 4096 -> 16768, 8 tokens 25.2 / 31.2, in Q8_0 64.7 / 69.3.
+    // Products by themselves keep one CTA an SM where its share is one set in half an SM, beside which the next call fetches its
+    // weights: from a graph, on other weights each, 1536 -> 6448 in Q4_K, 3, 5, 8 tokens 4.4 / 5.1, 5.9 / 7.1, 6.7 / 8.0; 768 -> 3224 in
+    // Q8_0, 5 tokens 3.7 / 4.2.  A share that does not fit so: 2560 -> 10448 in Q4_K, 3 tokens 10.6 / 9.0; 512 -> 24000, 5 tokens 7.3 / 6.4.
+    const bool whole = (TILE_ROWS * a.row_bytes) % 16 == 0;
+    if (plain && whole) {
+        const int most = tile(TILE_ROWS, num_sms());
+        if (most <= 8) fits(most, 1, SMEM_BUDGET);
+    }
+    if (KIND != KIND_F16 && mt > 2 && whole && !plan.smem) half(tile(TILE_ROWS, 2 * num_sms()), DG_SMEM_TWO);
     for (int R = TILE_ROWS; R >= 1 && !plan.smem; R >>= 1) {
         if ((R * a.row_bytes) % 16 != 0) break;
         const int most = tile(R, num_sms());
@@ -253,16 +264,23 @@ static DgPlan dg_plan(SgArgs& a, int mt, bool norm) {
 
 template <int KIND, int MT, int PRO, int EPI>
 static int launch_dg(SgArgs a) {
-    const DgPlan plan = dg_plan<KIND>(a, MT, PRO == PRO_RMS);
+    const DgPlan plan = dg_plan<KIND>(a, MT, PRO == PRO_RMS, PRO == PRO_NONE && EPI == EPI_STORE);
     if (!plan.smem) return fail(B200_EUNSUPPORTED, "stream_gemv: K = %d does not fit the shared-memory staging", a.K);
     auto kern = dg_gemv_kernel<KIND, MT, PRO, EPI>;
+    // Where the instance's registers let a third CTA on an SM (56 of twelve warps), the CTAs of two kernels crowd on some SMs while others
+    // have none: two tokens, 1536 -> 1536 in Q8_0 4.3 us with three, 3.7 with two; 3072 -> 1536 in Q4_0 7.4 and 5.9; a step of H-Tiny in
+    // Q8_0, one sequence 1587 and 1541.  Shared memory that it does not use keeps it out.
+    static size_t least = 0;
     static bool configured = false;
     if (!configured) {
         int rc = allow_smem(kern);
         if (rc) return rc;
+        cudaFuncAttributes at;
+        B200_CUDA(cudaFuncGetAttributes(&at, kern));
+        if (3 * dg_warps(MT) * 32 * ((at.numRegs + 7) / 8 * 8) <= 65536) least = DG_SMEM_THIRD;
         configured = true;
     }
-    return launch_pdl(kern, dim3(plan.grid), dim3(dg_warps(MT) * 32), plan.smem, a);
+    return launch_pdl(kern, dim3(plan.grid), dim3(dg_warps(MT) * 32), std::max(plan.smem, least), a);
 }
 
 template <int KIND, int PRO, int EPI>
@@ -299,7 +317,7 @@ int digit_gemv(SgArgs a, int kind, int pro, int epi) {
 }  // namespace b200
 
 // The launch of one matrix's product as it would be planned, for tests: CTAs and dynamic shared memory of a CTA.
-extern "C" int b200_digit_gemv_plan(int kind, int M, int N, int K, int norm, int* ctas, int* smem) {
+extern "C" int b200_digit_gemv_plan(int kind, int M, int N, int K, int norm, int plain, int* ctas, int* smem) {
     using namespace b200;
     SgArgs a;
     a.M = M;
@@ -307,7 +325,7 @@ extern "C" int b200_digit_gemv_plan(int kind, int M, int N, int K, int norm, int
     a.K = K;
     a.row_bytes = row_bytes_of(kind, K);
     const int mt = dg_tokens(M);
-    const DgPlan plan = kind == KIND_F16 ? dg_plan<KIND_F16>(a, mt, norm) : dg_plan<0>(a, mt, norm);
+    const DgPlan plan = kind == KIND_F16 ? dg_plan<KIND_F16>(a, mt, norm, plain) : dg_plan<0>(a, mt, norm, plain);
     *ctas = plan.grid;
     *smem = (int)plan.smem;
     return plan.smem ? B200_OK : B200_EUNSUPPORTED;

@@ -596,8 +596,14 @@ static DmPlan dm_plan_layer(const MoeFusedArgs& a) {
     // second wave and without: 4096 x 768 in Q8_0 (gate / up), two tokens 134.6 / 128.7, in Q4_K (down) 77.2 / 72.6; 1536 x 1024 with
     // eight experts in Q4_K (down), five tokens 61.6 / 57.3; 1536 x 512 in Q8_0 (down), four tokens 33.4 / 31.8.  (2560 x 512 in
     // Q8_0, two tokens 27.5 / 29.8: 160 tiles per token for 74 CTAs are three to some, and two waves even that out.)
+    // A layer by itself (not in a decode step) is shorter with one where the second CTA takes little: gate / up of less than seven
+    // products of a chunk for a CTA, and down of three tiles and more in one set of half an SM, beside which the next
+    // kernel's CTA fits.  Us from a graph, on other weights each, two and one: 768 x 512, two tokens in Q4_K 15.5 / 12.3, in Q8_0 15.6 /
+    // 13.4 (gate / up); 4096 x 256, two tokens in Q4_K 24.1 / 20.6; 768 x 512, eight tokens 18.4 / 16.7; 2048 x 1024, three tokens
+    // 21.8 / 19.8 (down).  On the other side: 768 x 512, three tokens 13.0 / 13.2 (gate / up); 2560 x 512, three tokens 27.1 / 30.1 (down).
     auto per_token = [&](int per_sm) { return std::max(1, per_sm * num_sms() / a.M); };
     const int most_per_sm = a.M > 1 ? 2 : 1;
+    const bool alone = a.out != nullptr;
     const int n_router = ceil_div(a.ne, DM_ROUTER), sh_tiles = a.SH / 8;
     const int sh_ctas = std::min(sh_tiles, std::max(8, num_sms() - n_router));
     const size_t router_bytes = (size_t)DM_ROUTER * a.d * 4 + std::max<size_t>((size_t)DM_ROUTER * a.M * dm_chain_stride(a.d) * 4, (size_t)a.M * a.ne * 4);
@@ -611,7 +617,7 @@ static DmPlan dm_plan_layer(const MoeFusedArgs& a) {
         p.g2 = std::min(t2, per_token(n));
         p.s2 = dm_plan<KIND>(p.p2, t2, p.g2, 16 * rb_d, dg_chunks(a.d), 1, (size_t)dg_chunks(a.d) * 8, 0, share);
     };
-    if (most_per_sm == 2) gate_up(2, true);
+    if (most_per_sm == 2 && !(alone && t2 * dg_chunks(a.d) < 7 * per_token(1))) gate_up(2, true);
     if (!p.s2) gate_up(1, false);
     if (!p.s2 && most_per_sm == 2) gate_up(2, false);      // rows so wide that two tiles do not fit a whole SM, and one to each of two waves
     p.p3.ec_inv = dg_inv(std::min(255, dg_chunks(a.E)));
@@ -624,7 +630,13 @@ static DmPlan dm_plan_layer(const MoeFusedArgs& a) {
         p.s3 = dm_plan<KIND>(p.p3, t3, p.g3, R * (rb_s + a.K * rb_e), dg_chunks(a.SH) + a.K * dg_chunks(a.E), 1, 0, 0, share);
     };
     auto copies = [&](int R) { return (R * rb_e) % 16 == 0 && (R * rb_s) % 16 == 0; };
-    if (most_per_sm == 2 && copies(TILE_ROWS)) down(TILE_ROWS, 2, true);
+    if (most_per_sm == 2 && copies(TILE_ROWS)) {
+        if (alone && ceil_div(a.d, TILE_ROWS) > 2 * per_token(1)) {
+            down(TILE_ROWS, 1, true);
+            if (p.p3.sets != 1) p.s3 = 0;
+        }
+        if (!p.s3) down(TILE_ROWS, 2, true);
+    }
     for (int R = TILE_ROWS; R >= 1 && !p.s3 && copies(R); R >>= 1) down(R, 1, false);
     return p;
 }
@@ -665,9 +677,11 @@ int moe_digit(const MoeFusedArgs& a, int kind) {
 }  // namespace b200
 
 // The three launches of a layer as they would be planned, for tests: CTAs and dynamic shared memory of a CTA of each.
-extern "C" int b200_moe_digit_plan(int kind, int M, int d, int E, int ne, int K, int SH, int* ctas, int* smem) {
+extern "C" int b200_moe_digit_plan(int kind, int M, int d, int E, int ne, int K, int SH, int alone, int* ctas, int* smem) {
     using namespace b200;
+    static float out;
     MoeFusedArgs a;
+    if (alone) a.out = &out;
     a.M = M;
     a.d = d;
     a.E = E;
