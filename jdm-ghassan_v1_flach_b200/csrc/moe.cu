@@ -622,8 +622,10 @@ int moe_forward(const float* x, const float* router_w, const float* router_bias,
     // rows would leave the 128-row tensor-core tiles nearly empty; they run as weight streams
     // shared by their tokens instead (moe_exact.cu, moe_units.cu).
     // (Up to eight tokens come here where the three kernels above refuse them: 3, 5, 8 tokens of 768 x 4096 in Q8_0 took 397, 638
-    // and 1000 us token by token.)
-    if ((N > 8 || (kind >= 0 && kind <= 3)) && N * K <= (int64_t)MOE_UNITS_MAX_ROWS * ne && kind != KIND_F32 && !s_gate && !s_up && !s_act && aligned16(x) &&
+    // and 1000 us token by token.  Not in place, which every other form for few tokens takes: the units' shared expert writes out
+    // beside the routed experts that read x.)
+    const bool in_place = x < out + N * d && out < x + N * d;
+    if ((N > 8 || (kind >= 0 && kind <= 3 && !in_place)) && N * K <= (int64_t)MOE_UNITS_MAX_ROWS * ne && kind != KIND_F32 && !s_gate && !s_up && !s_act && aligned16(x) &&
         aligned16(out) && aligned16(gates) && aligned16(ups) && aligned16(downs) && d % 8 == 0 &&
         (kind != 3 || (d % 256 == 0 && E % 256 == 0)) && ne <= 256 &&
         (!shared || (aligned16(sh_g) && aligned16(sh_u) && aligned16(sh_d) && (kind == KIND_F16 || SH % 256 == 0)))) {

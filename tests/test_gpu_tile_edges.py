@@ -176,7 +176,7 @@ def test_wide_experts(oracle, kind, ne, E, K, SH, N):
 # Up to eight tokens of rows so wide that the decode step's kernels refuse them (eight tokens of 4096 beside two tiles): they
 # run as units, in fp32 on the exact weights as the others.  Two and four tokens still fit.
 @pytest.mark.parametrize("kind", [2, 3])
-@pytest.mark.parametrize("N", [2, 3, 5, 8])
+@pytest.mark.parametrize("N", [2, 3, 4, 5, 8])
 def test_few_tokens_of_wide_rows(oracle, kind, N):
     from gpu_util import SUM_ORDER, dev, empty, host, ops
     d, E, ne, K, SH = 4096, 256, 8, 2, 1536
@@ -191,6 +191,26 @@ def test_few_tokens_of_wide_rows(oracle, kind, N):
     oracle.set_weight_rounding(True)
     assert np.array_equal(host(idx), widx)
     np.testing.assert_allclose(host(out), want, **SUM_ORDER)
+
+
+# Up to eight tokens may be written over x, whatever the row's width and with or without the last elements of x in front of out.
+@pytest.mark.parametrize("kind", [2, 3])
+@pytest.mark.parametrize("N,d", [(5, 4096), (8, 4096), (8, 512)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_few_tokens_in_place(oracle, kind, N, d, shift):
+    from gpu_util import SUM_ORDER, dev, empty, host, ops
+    E, ne, K, SH = 256, 8, 2, 1536
+    c = moe_case(oracle, N + kind, N, d, E, ne, K, SH, kind)
+    args = [dev(c[k]) for k in ("router_w", "router_bias", "gates", "ups", "downs", "sh_g", "sh_u", "sh_d")]
+    got = []
+    for over in (False, True):
+        room = empty(((N + shift) * d,))
+        x = room[: N * d]
+        x.copy_(dev(c["x"]).view(-1))
+        out = room[shift * d:] if over else empty((N * d,))
+        ops.moe_forward_bias_half(x, *args, out, None, None, None, None, None, None, N, d, E, ne, K, SH, kind)
+        got.append(host(out))
+    np.testing.assert_allclose(got[1], got[0], **SUM_ORDER)
 
 
 # the decode step's kernels, the digit engine's units and the exact tensor-core form
