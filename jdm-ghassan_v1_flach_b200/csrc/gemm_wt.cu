@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
             const CUtensorMap* map = &a.map_x[boxes - 1];
             const int row0 = w.row0, k1 = 4 * sb1;
             for (int kb = 4 * sb0; kb < k1; kb += steps, ++it) {
-                if (it >= S::SX && !__all_sync(0xffffffffu, mbar_try(&empty[s], ph ^ 1))) {
+                if (it >= S::SX && !__all_sync(0xffffffffu, mbar_try_wait(&empty[s], ph ^ 1))) {
                     ok = mbar_wait_warp(&empty[s], ph ^ 1, a.status);
                     if (!ok) break;
                 }
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
             range(w, sb0, sb1);
             const int brow = w.brow + w.n0 * S::TILE_N;
             for (int sb = sb0; sb < sb1; ++sb, ++it) {
-                if (it >= S::SP && !__all_sync(0xffffffffu, mbar_try(&p_empty[p], ph ^ 1))) {
+                if (it >= S::SP && !__all_sync(0xffffffffu, mbar_try_wait(&p_empty[p], ph ^ 1))) {
                     ok = mbar_wait_warp(&p_empty[p], ph ^ 1, a.status);
                     if (!ok) break;
                 }
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
             auto rounds = [&](auto unit) {
                 constexpr int STEPS = 1 << decltype(unit)::value;
                 for (int kb = k0; kb < k1; kb += STEPS) {
-                    if (!__all_sync(0xffffffffu, mbar_try(&full[s], ph))) {
+                    if (!__all_sync(0xffffffffu, mbar_try_wait(&full[s], ph))) {
                         ok = mbar_wait_warp(&full[s], ph, a.status);
                         if (!ok) return;
                     }
@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
             range(w, sb0, sb1);
             const int unit = wt_unit(w.rows);
             for (int sb = sb0; sb < sb1; ++sb) {
-                if (!__all_sync(0xffffffffu, mbar_try(&p_full[p], ph))) {
+                if (!__all_sync(0xffffffffu, mbar_try_wait(&p_full[p], ph))) {
                     ok = mbar_wait_warp(&p_full[p], ph, a.status);
                     if (!ok) break;
                 }
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) umma_wt_kernel(const __grid_con
                 // The slot is free once the MMAs of four K steps ago are done.  With them every stage up to theirs has
                 // been through, so that with SX >= 4 this step's stage is in the phase that the arrival is meant for;
                 // and theirs cannot complete another phase before this step, so that the parity is not ambiguous.
-                if (last < S::SX && !__all_sync(0xffffffffu, mbar_try(&empty[last], lph))) {
+                if (last < S::SX && !__all_sync(0xffffffffu, mbar_try_wait(&empty[last], lph))) {
                     ok = mbar_wait_warp(&empty[last], lph, a.status);
                     if (!ok) break;
                 }
@@ -573,7 +573,7 @@ struct WtBoxes {
 static constexpr WtBoxes wt_boxes;
 
 template <bool SWIGLU, int KIND>
-static int launch_wt(WtArgs& a, bool allow_split) {
+static int launch_wt(WtArgs& a, bool allow_split, bool early) {
     using S = WtShape<SWIGLU, KIND>;
     auto kern = umma_wt_kernel<SWIGLU, KIND>;
     static bool configured = false;
@@ -613,7 +613,7 @@ static int launch_wt(WtArgs& a, bool allow_split) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = !SWIGLU && !a.offsets && allow_split ? 1 : 0;
+    cfg.numAttrs = early ? 1 : 0;
     B200_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
     ++g_kernel_launches;
     return a.k_splits > 1 ? splitk_reduce(a.c, c, a.k_splits, a.split_stride, a.M, a.N, a.ldc) : B200_OK;
@@ -622,7 +622,7 @@ static int launch_wt(WtArgs& a, bool allow_split) {
 // See gemm.cuh.
 int umma_gemm_q(int epi, int kind, const __half* A, int64_t a_rows, const void* B, const void* B2, int64_t b_rows,
                 const int32_t* offsets, int groups, int M, int N, int K, float* c, __half* c16, int64_t ldc,
-                float scale, const int32_t* group_map, float* const* group_c, bool allow_split_k) {
+                float scale, const int32_t* group_map, float* const* group_c, bool allow_split_k, bool early) {
     if (M <= 0 || N <= 0) return B200_OK;
     B200_REQUIRE(kind >= 0 && kind <= 3, "umma_gemm_q: unknown kind %d", kind);
     B200_REQUIRE(!group_c || (offsets && epi == GEMM_EPI_STORE), "umma_gemm_q: per-group outputs need the grouped store form");
@@ -651,10 +651,10 @@ int umma_gemm_q(int epi, int kind, const __half* A, int64_t a_rows, const void* 
     a.status = stream_status_ptr();
     B200_REQUIRE(a.status, "umma_gemm_q: status word allocation failed");
     switch (kind) {
-        case 0: return swiglu ? launch_wt<true, 0>(a, allow_split_k) : launch_wt<false, 0>(a, allow_split_k);
-        case 1: return swiglu ? launch_wt<true, 1>(a, allow_split_k) : launch_wt<false, 1>(a, allow_split_k);
-        case 2: return swiglu ? launch_wt<true, 2>(a, allow_split_k) : launch_wt<false, 2>(a, allow_split_k);
-        default: return swiglu ? launch_wt<true, 3>(a, allow_split_k) : launch_wt<false, 3>(a, allow_split_k);
+        case 0: return swiglu ? launch_wt<true, 0>(a, allow_split_k, early) : launch_wt<false, 0>(a, allow_split_k, early);
+        case 1: return swiglu ? launch_wt<true, 1>(a, allow_split_k, early) : launch_wt<false, 1>(a, allow_split_k, early);
+        case 2: return swiglu ? launch_wt<true, 2>(a, allow_split_k, early) : launch_wt<false, 2>(a, allow_split_k, early);
+        default: return swiglu ? launch_wt<true, 3>(a, allow_split_k, early) : launch_wt<false, 3>(a, allow_split_k, early);
     }
 }
 

@@ -115,7 +115,7 @@ int linear_a16(const void* a16, const void* w, int kind, float* y, int M, int K,
     const __half* a = static_cast<const __half*>(a16);
     if (kind == KIND_F16)
         return umma_gemm(GEMM_EPI_STORE, a, M, static_cast<const __half*>(w), nullptr, N, nullptr, 1, M, N, K, y, nullptr, N, 1.0f);
-    return umma_gemm_q(GEMM_EPI_STORE, kind, a, M, w, nullptr, N, nullptr, 1, M, N, K, y, nullptr, N, 1.0f);
+    return umma_gemm_q(GEMM_EPI_STORE, kind, a, M, w, nullptr, N, nullptr, 1, M, N, K, y, nullptr, N, 1.0f, nullptr, nullptr, true, true);
 }
 
 int linear(const float* x, const void* w, int kind, float* y, int M, int K, int N) {
@@ -163,7 +163,7 @@ int linear(const float* x, const void* w, int kind, float* y, int M, int K, int 
             a16 = packed;
         }
         if (in_kernel)
-            return umma_gemm_q(GEMM_EPI_STORE, kind, a16, M, w, nullptr, N, nullptr, 1, M, N, K, y, nullptr, N, 1.0f);
+            return umma_gemm_q(GEMM_EPI_STORE, kind, a16, M, w, nullptr, N, nullptr, 1, M, N, K, y, nullptr, N, 1.0f, nullptr, nullptr, true, true);
         const __half* b16 = static_cast<const __half*>(w);
         if (kind != KIND_F16) {
             uint16_t* scratch = reinterpret_cast<uint16_t*>(static_cast<char*>(ws) + a_bytes);
