@@ -534,7 +534,6 @@ __global__ void __launch_bounds__(256) residual_rmsnorm_kernel(float* __restrict
 __global__ void __launch_bounds__(256) residual_rmsnorm4_kernel(float* __restrict__ x, const float* __restrict__ y, float s,
                                                                const float* __restrict__ w, float* __restrict__ out,
                                                                int dim, float eps, __half* __restrict__ out16) {
-    short_begin();
     __shared__ double red[32];
     const int64_t r = blockIdx.x;
     float* xr = x + r * dim;
@@ -642,8 +641,11 @@ static int prefill(b200_decoder* dec, const int32_t* tokens, int T, int32_t* nex
         if (norm_w && d <= RRN_PER * 256) {
             __half* x16 = want16 ? xb16 : nullptr;
             const uintptr_t at16 = (uintptr_t)x | (uintptr_t)y | (uintptr_t)norm_w | (uintptr_t)xb | (uintptr_t)x16;
-            if (NT >= 1024 && d % 4 == 0 && at16 % 16 == 0)
-                return launch_short(residual_rmsnorm4_kernel, dim3((unsigned)NT), dim3(256), x, y, dec->res_mult, norm_w, xb, d, dec->eps, x16);
+            if (NT >= 1024 && d % 4 == 0 && at16 % 16 == 0) {
+                residual_rmsnorm4_kernel<<<(unsigned)NT, 256, 0, st>>>(x, y, dec->res_mult, norm_w, xb, d, dec->eps, x16);
+                B200_LAUNCH_CHECK("residual_rmsnorm4_kernel");
+                return B200_OK;
+            }
             return launch_short(residual_rmsnorm_kernel, dim3((unsigned)NT), dim3(256), x, y, dec->res_mult, norm_w, xb, d, dec->eps, x16);
         }
         residual_kernel<<<res_grid, 256, 0, st>>>(x, y, dec->res_mult, NT * d);

@@ -70,10 +70,10 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, uint32_t
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// A short kernel's first statement.  Only a grid of about two blocks to an SM is worth overlapping with its neighbours: the
+// A short kernel's first statement.  Only a grid of at most three blocks to an SM is worth overlapping with its neighbours: the
 // early blocks of a larger one's successor hold SMs that its last wave could use (4096 tokens: 1 % slower so, 64 sequences 2 %
-// faster with the small grids alone).
-constexpr int SHORT_BLOCKS = 444;
+// faster with the small grids alone).  Of a B200's 148 SMs, not num_sms(): the kernel asks too.
+constexpr int SHORT_BLOCKS = 3 * 148;
 __device__ __forceinline__ void short_begin() {
     if (gridDim.x * gridDim.y * gridDim.z <= SHORT_BLOCKS) pdl_launch_dependents();
     pdl_wait();
