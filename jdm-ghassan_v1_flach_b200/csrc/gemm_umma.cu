@@ -481,10 +481,7 @@ int pack_rows_f16(const float* src, const int32_t* row_map, int div, __half* dst
                  "pack_rows_f16: buffers must be 16-byte aligned");
     if (rows == 0) return B200_OK;
     const dim3 grid((unsigned)((rows + 7) / 8));
-    if (early) return launch_short(pack_rows_f16_kernel, grid, dim3(256), src, row_map, div > 0 ? div : 1, dst, rows, K);
-    pack_rows_f16_kernel<<<grid, 256, 0, stream()>>>(src, row_map, div > 0 ? div : 1, dst, rows, K);
-    B200_LAUNCH_CHECK("pack_rows_f16_kernel");
-    return B200_OK;
+    return launch_waiting(early && short_grid(grid), pack_rows_f16_kernel, grid, dim3(256), 0, src, row_map, div > 0 ? div : 1, dst, rows, K);
 }
 
 // ===========================================================================

@@ -786,10 +786,19 @@ int mamba_ssd_scan(const float* proj, const float* bc, const float* dt_bias, con
     B200_REQUIRE(smem_cb <= 160 * 1024 && smem_st <= 160 * 1024 && smem_out <= 160 * 1024, "mamba_ssd_scan: shared memory");
     B200_REQUIRE(NC <= 65535 * 32 && B <= 65535 && p.n_heads <= 65535, "mamba_ssd_scan: grid too large");
     const int gz = lay ? 1 : B;
-    // (the upper right quadrant of every G is never written and never read: s <= t only)
-    rc = launch_short_smem(ssd_cb_kernel, dim3(3 * NC, gz), dim3(SSD_THREADS), smem_cb, bc, G, T, p, tab);
-    if (rc) return rc;
     const dim3 grid(NC, p.n_heads, gz);
+    // Kernels that start early take the SMs that in_proj leaves, and with few blocks so does everything behind them: convolution,
+    // states and outputs ran crowded on a third of the device while the projection had the rest.  Where the heads' grids have at
+    // most two blocks to an SM, the first of these kernels is launched when the convolution has ended, so that all find all SMs
+    // free; the outputs too for narrow states.  In us before any kernel started early, with all early, and now: layer of 768, state 64
+    // 130 / 300 / 600 steps 61 / 64 / 65, 70 / 81 / 88, 59 / 62 / 67; of 1536, state 128 79 / 82 / 105, 90 / 97 / 103, 75 / 79 / 98.  Prompts of 600
+    // tokens 1575 and 11476, 1332 and 9735, 1240 and 9219.  With the outputs of wide states launched so: 301 tokens 7553 -> 7628; with
+    // larger grids: 1000 tokens 10752 -> 10872.
+    const bool few = (int64_t)NC * p.n_heads * gz <= 2 * 148;
+    // (the upper right quadrant of every G is never written and never read: s <= t only)
+    const dim3 grid_cb(3 * NC, gz);
+    rc = launch_waiting(!few && short_grid(grid_cb), ssd_cb_kernel, grid_cb, dim3(SSD_THREADS), smem_cb, bc, G, T, p, tab);
+    if (rc) return rc;
     const bool half_tiles = !precise && N % 32 == 0;
     const size_t smem_st16 = (size_t)(SSD_Q * (N + 8) + SSD_Q * SSD_LDX16) * 2 + 2 * SSD_Q * 4;
     const size_t smem_out16 = (size_t)std::max(SSD_Q * (N + 8) + P * (N + 8), SSD_Q * SSD_LDM16 + SSD_Q * SSD_LDX16) * 2 + 3 * SSD_Q * 4;
@@ -817,8 +826,8 @@ int mamba_ssd_scan(const float* proj, const float* bc, const float* dt_bias, con
         if (rc) return rc;
     }
     if (half_tiles)
-        rc = launch_short_smem(N == 128 ? ssd_chunk_out16_kernel<128> : ssd_chunk_out16_kernel<0>, grid, dim3(SSD_THREADS), smem_out16, bc, G, dtcum,
-                                 cstate, decay, state, D, y, T, NC, p, tab, NT);
+        rc = launch_waiting((!few || N == 128) && short_grid(grid), N == 128 ? ssd_chunk_out16_kernel<128> : ssd_chunk_out16_kernel<0>, grid,
+                            dim3(SSD_THREADS), smem_out16, bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);
     else {
         if (precise)
             ssd_chunk_out_kernel<true><<<grid, SSD_THREADS, smem_out, stream()>>>(bc, G, dtcum, cstate, decay, state, D, y, T, NC, p, tab, NT);

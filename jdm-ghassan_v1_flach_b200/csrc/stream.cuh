@@ -79,10 +79,10 @@ __device__ __forceinline__ void short_begin() {
     pdl_wait();
 }
 
-// Host: a short kernel that lets its dependents start and then waits, before it touches memory, launched so that it is set up
-// while the kernel before it ends (about a microsecond of a decode step's short kernels each).
+// Host: a kernel that lets its dependents start and then waits, before it touches memory; early: launched so that it is set up while
+// the kernel before it ends (about a microsecond of a decode step's short kernels each).
 template <typename... P, typename... A>
-static int launch_short_smem(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, const A&... args) {
+static int launch_waiting(bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, const A&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -92,10 +92,15 @@ static int launch_short_smem(void (*kern)(P...), dim3 grid, dim3 block, size_t s
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = (int64_t)grid.x * grid.y * grid.z <= SHORT_BLOCKS ? 1 : 0;
+    cfg.numAttrs = early ? 1 : 0;
     B200_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
     ++g_kernel_launches;
     return B200_OK;
+}
+inline bool short_grid(dim3 grid) { return (int64_t)grid.x * grid.y * grid.z <= SHORT_BLOCKS; }
+template <typename... P, typename... A>
+static int launch_short_smem(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, const A&... args) {
+    return launch_waiting(short_grid(grid), kern, grid, block, smem, args...);
 }
 template <typename... P, typename... A>
 static int launch_short(void (*kern)(P...), dim3 grid, dim3 block, const A&... args) {
