@@ -47,7 +47,7 @@ struct Workspace {
     int ensure(size_t need, void** out);
     void release();
 };
-enum { WS_LINEAR = 0, WS_MOE = 1, WS_MAMBA = 2, WS_ATTN = 3, WS_SAMPLE = 4, WS_ROUTE = 5, WS_PREFILL = 6, WS_SPLITK = 7, WS_COUNT = 8 };
+enum { WS_LINEAR = 0, WS_MOE = 1, WS_MAMBA = 2, WS_ATTN = 3, WS_SAMPLE = 4, WS_ROUTE = 5, WS_PREFILL = 6, WS_SPLITK = 7, WS_PERM = 8, WS_COUNT = 9 };
 Workspace& workspace(int which);
 unsigned long long workspace_generation();   // changes whenever a workspace address goes stale
 

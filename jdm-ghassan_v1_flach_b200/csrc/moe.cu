@@ -232,12 +232,126 @@ perm_kernel(const int32_t* __restrict__ idx, int NK, int32_t* __restrict__ group
     }
 }
 
+// Many slots: every block above reads all of them twice, 0.27 us a thousand, whatever the device has to spare.
+// Here each slot is read twice in all, by three kernels: per-block histograms, a scan over (expert, block), and a fill where each warp
+// ranks its 32 slots with __match_any_sync and warps are ordered through shared-memory prefix sums.
+// In us, the kernel above and these, 24 576 / 100 000 / 655 360 / 4 000 000 slots: 4 experts 7 / 28 / 170 / 1022 and 11 / 25 / 215 / 1215; 16
+// experts 7 / 28 / 169 / 1015 and 12 / 25 / 135 / 1040; 64 experts 7 / 27 / 165 / 990 and 11 / 22 / 100 / 1124; 256 experts 12 / 44 / 266 / 1597
+// and 15 / 25 / 193 / 1134.
+constexpr int SORT_THREADS = 256;
+constexpr int SORT_ITERS = 4;                              // slots per block = 256 * 4
+constexpr int SORT_CHUNK = SORT_THREADS * SORT_ITERS;
+
+__global__ void __launch_bounds__(SORT_THREADS)
+sort_count_kernel(const int32_t* __restrict__ idx, int64_t NK, int ne, int32_t* __restrict__ block_counts) {
+    __shared__ int cnt[MOE_MAX_NE];
+    for (int e = threadIdx.x; e < ne; e += blockDim.x) cnt[e] = 0;
+    __syncthreads();
+    const int64_t base = (int64_t)blockIdx.x * SORT_CHUNK;
+    for (int it = 0; it < SORT_ITERS; ++it) {
+        const int64_t s = base + it * SORT_THREADS + threadIdx.x;
+        const int e = s < NK ? idx[s] : -1;
+        if ((unsigned)e < (unsigned)ne) atomicAdd(&cnt[e], 1);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < ne; e += blockDim.x) block_counts[(int64_t)blockIdx.x * ne + e] = cnt[e];
+}
+
+// One block; thread e walks the blocks of expert e.  block_counts becomes the
+// first output position of (block, expert); offsets[ne+1] the expert boundaries.
+__global__ void sort_scan_kernel(int32_t* __restrict__ block_counts, int nblocks, int ne,
+                                 int32_t* __restrict__ offsets) {
+    __shared__ int total[MOE_MAX_NE + 1];
+    const int e = threadIdx.x;
+    if (e < ne) {
+        int run = 0;
+        for (int b = 0; b < nblocks; ++b) {
+            const int c = block_counts[(int64_t)b * ne + e];
+            block_counts[(int64_t)b * ne + e] = run;
+            run += c;
+        }
+        total[e] = run;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int run = 0;
+        for (int i = 0; i < ne; ++i) { const int c = total[i]; total[i] = run; run += c; }
+        total[ne] = run;
+    }
+    __syncthreads();
+    if (e <= ne) offsets[e] = total[e];
+    if (e < ne) {
+        const int off = total[e];
+        for (int b = 0; b < nblocks; ++b) block_counts[(int64_t)b * ne + e] += off;
+    }
+}
+
+__global__ void __launch_bounds__(SORT_THREADS)
+sort_fill_kernel(const int32_t* __restrict__ idx, int64_t NK, int ne, const int32_t* __restrict__ block_base,
+                 int32_t* __restrict__ grouped) {
+    constexpr int NW = SORT_THREADS / 32;
+    __shared__ int cursor[MOE_MAX_NE];
+    __shared__ int wcnt[NW][MOE_MAX_NE];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int e = threadIdx.x; e < ne; e += blockDim.x) cursor[e] = block_base[(int64_t)blockIdx.x * ne + e];
+    const int64_t base = (int64_t)blockIdx.x * SORT_CHUNK;
+    for (int it = 0; it < SORT_ITERS; ++it) {
+        for (int i = threadIdx.x; i < NW * ne; i += blockDim.x) (&wcnt[0][0])[(i / ne) * MOE_MAX_NE + (i % ne)] = 0;
+        __syncthreads();
+        const int64_t s = base + it * SORT_THREADS + threadIdx.x;
+        int e = s < NK ? idx[s] : -1;
+        const bool live = (unsigned)e < (unsigned)ne;
+        if (!live) e = -1 - lane;              // dead lanes match nobody
+        const unsigned peers = __match_any_sync(0xffffffffu, e);
+        const int rank = __popc(peers & ((1u << lane) - 1u));
+        if (live && rank == 0) wcnt[warp][e] = __popc(peers);
+        __syncthreads();
+        if (live) {
+            int pos = cursor[e] + rank;
+            for (int w = 0; w < warp; ++w) pos += wcnt[w][e];
+            grouped[pos] = (int32_t)s;
+        }
+        __syncthreads();
+        for (int ee = threadIdx.x; ee < ne; ee += blockDim.x) {
+            int add = 0;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) add += wcnt[w][ee];
+            cursor[ee] += add;
+        }
+        __syncthreads();
+    }
+}
+
+// inv[grouped[pos]] = pos
+__global__ void sort_inverse_kernel(const int32_t* __restrict__ grouped, int32_t* __restrict__ inv, int64_t NK) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < NK) inv[grouped[p]] = (int32_t)p;
+}
+
 // grouped [NK]: slots sorted by expert, stable; inv (optional): where each slot went; offsets [ne + 1].
 int moe_permutation(const int32_t* idx, int64_t NK, int ne, int32_t* grouped, int32_t* inv, int32_t* offsets) {
     B200_REQUIRE(idx && grouped && offsets, "moe_permutation: null pointer");
     B200_REQUIRE(ne > 0 && ne <= MOE_MAX_NE, "moe_permutation: ne out of range");
     B200_REQUIRE(NK >= 0 && NK < ((int64_t)1 << 31), "moe_permutation: slot count out of range");
-    return launch_short(perm_kernel, dim3(ne), dim3(PERM_WARPS * 32), idx, (int)NK, grouped, inv, offsets);
+    const bool two = ne > num_sms();                               // blocks of the one kernel on an SM
+    const bool many = NK * (two ? 2 : 1) >= (inv ? 110000 : 90000) && (NK < 1 << 18 || (ne >= 16 && NK < 1 << 21) || two);
+    if (!many) return launch_short(perm_kernel, dim3(ne), dim3(PERM_WARPS * 32), idx, (int)NK, grouped, inv, offsets);
+    const int nblocks = (int)ceil_div64(NK, SORT_CHUNK);
+    void* wsp;
+    int rc = workspace(WS_PERM).ensure((size_t)nblocks * ne * sizeof(int32_t) + 256, &wsp);
+    if (rc) return rc;
+    int32_t* bc = static_cast<int32_t*>(wsp);
+    sort_count_kernel<<<nblocks, SORT_THREADS, 0, stream()>>>(idx, NK, ne, bc);
+    B200_LAUNCH_CHECK("sort_count_kernel");
+    sort_scan_kernel<<<1, 320, 0, stream()>>>(bc, nblocks, ne, offsets);
+    B200_LAUNCH_CHECK("sort_scan_kernel");
+    sort_fill_kernel<<<nblocks, SORT_THREADS, 0, stream()>>>(idx, NK, ne, bc, grouped);
+    B200_LAUNCH_CHECK("sort_fill_kernel");
+    if (inv) {
+        sort_inverse_kernel<<<(unsigned)ceil_div64(NK, 256), 256, 0, stream()>>>(grouped, inv, NK);
+        B200_LAUNCH_CHECK("sort_inverse_kernel");
+    }
+    return B200_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -321,14 +435,14 @@ static int launch_experts(const MoeArgs& a) {
 }
 
 // ---------------------------------------------------------------------------
-// Router for more than eight tokens.  The logit of (token, expert) keeps the reference's sequential fp32 chain over groups
+// Router.  The logit of (token, expert) keeps the reference's sequential fp32 chain over groups
 // of four (products and sums rounded one by one: eight instructions per group, 23 us of a chip's fp32 rate for 4096 tokens
 // of 1536 x 64 experts).  A thread carries TPT x EPT chains; token and expert rows come through a ring of asynchronous
 // copies, RT_K columns at a time and a thousand columns deep where a block has few chains, because the chains advance
 // faster than a cold load returns: the ring of three 64-column stages before it spent 1800 cycles per stage, a load's way.
 // In us (before, now), router alone, launches included: 64 tokens of 1536 x 64
 // 16.4 -> 14.3, 301 27.6 -> 20.5, 2048 44 -> 38; of 4096 x 72: 64 tokens 30 -> 25, 517 64 -> 50, 4096 210 -> 194; 4096 tokens of
-// 768 x 16 34 -> 19.5.  Larger thread tiles (4 x 4, 8 x 2) and packed additions were no faster: about two cycles a product or
+// 768 x 16 34 -> 19.5.  (A layer's few tokens have the router of decode_moe.cu, unless it refuses their width.)  Larger thread tiles (4 x 4, 8 x 2) and packed additions were no faster: about two cycles a product or
 // sum whatever their number.
 // ---------------------------------------------------------------------------
 constexpr int RT_K = 128, RT_LD = RT_K + 4, RT_THREADS = 256;

@@ -89,7 +89,6 @@ def test_gemm_token_tiles(oracle, kind, M, K, N):
     fp16_close(host(y), want, frac=1e-3)
 
 
-# the bias gathers the tokens: experts with none, one, a full tile (8 / 24 slots) and one more
 @pytest.mark.parametrize("kind", [0, 1, 2, 3])
 @pytest.mark.parametrize("d,E", [(256, 256), (768, 512)])
 def test_expert_rows_of_mixed_sizes(oracle, kind, d, E):
@@ -119,6 +118,7 @@ def test_expert_rows_of_mixed_sizes(oracle, kind, d, E):
             assert err.max() < 2.5e-3, (e, sizes[e], err.max())
 
 
+# the bias gathers the tokens: experts with none, one, a full tile (8 / 24 slots) and one more
 @pytest.mark.parametrize("kind", [2, 3])
 @pytest.mark.parametrize("N", [9, 24, 25, 48])
 @pytest.mark.parametrize("d,E", [(256, 512), (768, 256)])
@@ -230,7 +230,7 @@ def test_experts_of_a_token_that_is_not_finite(oracle, kind, N):
     assert np.isnan(got[N - 1]).all() and np.isfinite(got[:N - 1]).all()
 
 
-# one to eight tokens; the 8-, 16- and 32-token tiles of the many-token router; widths off its 64 columns
+# one to eight tokens; the 8- and 32-token tiles of the router; widths off its 128 columns
 @pytest.mark.parametrize("d,ne,K", [(260, 33, 3), (1536, 64, 6)])
 @pytest.mark.parametrize("N", [1, 7, 257, 600, 2401])
 def test_router_tiles(oracle, d, ne, K, N):
@@ -246,16 +246,17 @@ def test_router_tiles(oracle, d, ne, K, N):
     np.testing.assert_array_max_ulp(host(dw), w, maxulp=4)
 
 
-# both tiles of the router and their ragged ends: one chain per thread up to some 500 tokens, 2 x 2 above, one column tile and
-# several, a last one of four columns; bit-exact as above
+# the tiles of the router and their ragged ends: one chain per thread up to some 500 tokens, 2 x 2 above, one
+# column tile and several, a last one of four columns; bit-exact as above
 @pytest.mark.parametrize("d,ne,K", [(128, 16, 2), (132, 72, 10), (1028, 256, 16)])
 @pytest.mark.parametrize("N", [9, 300, 1111])
 def test_router_thread_tiles(oracle, d, ne, K, N):
     test_router_tiles(oracle, d, ne, K, N)
 
 
-# slots around a warp's 128 and a block's 2048, at a list that is no multiple of 16 bytes; experts without any
-@pytest.mark.parametrize("NK", [1, 127, 129, 2047, 2049, 40001])
+# slots around a warp's 128 and a block's 2048, on both sides of the line to the three kernels for many; at a list that is no multiple
+# of 16 bytes; experts without any
+@pytest.mark.parametrize("NK", [1, 127, 129, 2047, 2049, 40001, 109999, 110001])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_permutation_and_its_inverse(NK, shift):
     from gpu_util import dev, empty, host, ops
