@@ -613,6 +613,87 @@ static int launch_route_logits(const float* x, const float* router_w, float* log
     return B200_OK;
 }
 
+// Tokens times experts enough to fill the device with blocks of 32 x 32: a thread carries eight tokens of one expert.  A warp reads its
+// lanes' 32 expert rows (four wavefronts per group of columns) for eight token rows (one each, the same for all lanes), so that
+// shared memory needs 12 cycles where the arithmetic needs 16.  In us, the form above and this one: 4096 and 16 384 tokens of 1536 x 64
+// 58 / 54 and 195 / 164, 1024 and 4096 of 2048 x 256 77 / 70 and 252 / 212, 2048 of 8192 x 128 285 / 262; fewer tokens: 2048 of 1536 x 64 32 / 38,
+// 700 of 2048 x 256 61 / 70, 1500 of 8192 x 128 222 / 263.  Not where a third of the experts' columns would be idle.
+constexpr int RW_K = 64, RW_LD = RW_K + 4, RW_WARPS = 4, RW_THREADS = 32 * RW_WARPS, RW_STAGES = 3, RW_TOKENS = 8;
+__global__ void __launch_bounds__(RW_THREADS)
+route_logits_wide_kernel(const float* __restrict__ x, const float* __restrict__ router_w, float* __restrict__ logits,
+                    int64_t N, int d, int ne) {
+    constexpr int TOK = RW_WARPS * RW_TOKENS, ROWS = TOK + 32, STAGE = ROWS * RW_LD;
+    extern __shared__ __align__(16) float rw_sm[];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t t0 = (int64_t)blockIdx.x * TOK;
+    const int e0 = blockIdx.y * 32;
+    // rows 0 .. TOK-1: tokens, then 32 experts; rows past the ends repeat the last one, columns past d are not read
+    const int c4 = (threadIdx.x % (RW_K / 4)) * 4, r0 = threadIdx.x / (RW_K / 4);
+    constexpr int STEP = RW_THREADS / (RW_K / 4), PER = ROWS / STEP;
+    static_assert(ROWS % STEP == 0, "rows of a stage per copying thread");
+    const int chunks = (d + RW_K - 1) / RW_K;
+    auto fetch = [&](int k) {
+        if (k < chunks) {
+            float* st = rw_sm + (k % RW_STAGES) * STAGE;
+            if (k * RW_K + c4 < d)
+#pragma unroll
+                for (int u = 0; u < PER; ++u) {
+                    const int row = r0 + u * STEP;
+                    const float* src = row < TOK ? x + min(t0 + row, N - 1) * d : router_w + (int64_t)min(e0 + row - TOK, ne - 1) * d;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(st + row * RW_LD + c4)), "l"(src + k * RW_K + c4) : "memory");
+                }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[RW_TOKENS] = {};
+#pragma unroll
+    for (int k = 0; k < RW_STAGES - 1; ++k) fetch(k);
+    for (int k = 0; k < chunks; ++k) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(RW_STAGES - 2) : "memory");
+        __syncthreads();                               // the stage is here, and the one before it is free
+        fetch(k + RW_STAGES - 1);
+        const float* xs = rw_sm + (k % RW_STAGES) * STAGE + RW_TOKENS * ty * RW_LD;
+        const float* ws = rw_sm + (k % RW_STAGES) * STAGE + (TOK + tx) * RW_LD;
+        const int kc = min(RW_K, d - k * RW_K);        // a multiple of 4
+        auto group = [&](int g) {
+            const float4 b = *reinterpret_cast<const float4*>(ws + g);
+#pragma unroll
+            for (int i = 0; i < RW_TOKENS; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(xs + i * RW_LD + g);
+                float s = __fadd_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+                s = __fadd_rn(s, __fmul_rn(a.z, b.z));
+                s = __fadd_rn(s, __fmul_rn(a.w, b.w));
+                acc[i] = __fadd_rn(acc[i], s);
+            }
+        };
+        // whole chunks with the loads of later groups under the additions of earlier ones (the chains are serial)
+        if (kc == RW_K) {
+#pragma unroll
+            for (int g = 0; g < RW_K; g += 4) group(g);
+        } else {
+            for (int g = 0; g < kc; g += 4) group(g);
+        }
+    }
+    const int e = e0 + tx;
+#pragma unroll
+    for (int i = 0; i < RW_TOKENS; ++i) {
+        const int64_t t = t0 + RW_TOKENS * ty + i;
+        if (t < N && e < ne) logits[t * ne + e] = acc[i];
+    }
+}
+static int launch_route_logits_wide(const float* x, const float* router_w, float* logits, int64_t N, int d, int ne) {
+    constexpr int SMEM = RW_STAGES * (RW_WARPS * RW_TOKENS + 32) * RW_LD * 4;
+    static bool configured = false;
+    if (!configured) {
+        B200_CUDA(cudaFuncSetAttribute(route_logits_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        configured = true;
+    }
+    const dim3 grid((unsigned)ceil_div64(N, RW_WARPS * RW_TOKENS), ceil_div(ne, 32));
+    route_logits_wide_kernel<<<grid, RW_THREADS, SMEM, stream()>>>(x, router_w, logits, N, d, ne);
+    B200_LAUNCH_CHECK("route_logits_wide_kernel");
+    return B200_OK;
+}
+
 // Arrival counters of the kernel above (one per token group), zeroed once; every call leaves them zero.
 // Not created while the stream is being captured into a graph (an allocation and a memset on the
 // default stream do not belong there): the caller then runs the separate finishing kernel.
@@ -656,7 +737,10 @@ int moe_route(const float* x, const float* router_w, const float* router_bias, f
         // take 14 / 18 / 29 / 41 us with the first and 24 / 24 / 24 / 26 with the second, 2048 take 66 and 38.
         auto rounds = [&](int tok, int exp) { return ceil_div64(ceil_div64(N, tok) * ceil_div(ne, exp), num_sms()); };
         int* counters = nullptr;
-        if (5 * rounds(8, 8) + 4 <= 12 * rounds(32, 16) + 7) {
+        const int64_t wide = ceil_div64(N, RW_WARPS * RW_TOKENS) * ceil_div(ne, 32);
+        if (2 * wide > 3 * num_sms() && 6 * 32 * ceil_div(ne, 32) < 7 * 16 * ceil_div(ne, 16)) {
+            rc = launch_route_logits_wide(x, router_w, logits, N, d, ne);
+        } else if (5 * rounds(8, 8) + 4 <= 12 * rounds(32, 16) + 7) {
             if (N <= 8 * ROUTE_COUNTERS) counters = route_counters();
             rc = launch_route_logits<1, 1, 2, 8>(x, router_w, logits, N, d, ne, router_bias, probs, idx, w, K, counters);
         } else {

@@ -246,11 +246,17 @@ def test_router_tiles(oracle, d, ne, K, N):
     np.testing.assert_array_max_ulp(host(dw), w, maxulp=4)
 
 
-# the tiles of the router and their ragged ends: one chain per thread up to some 500 tokens, 2 x 2 above, one
+# the tiles of the router and their ragged ends: one chain per thread up to some 500 tokens, 2 x 2 above, 8 x 1 for many experts, one
 # column tile and several, a last one of four columns; bit-exact as above
 @pytest.mark.parametrize("d,ne,K", [(128, 16, 2), (132, 72, 10), (1028, 256, 16)])
 @pytest.mark.parametrize("N", [9, 300, 1111])
 def test_router_thread_tiles(oracle, d, ne, K, N):
+    test_router_tiles(oracle, d, ne, K, N)
+
+
+# 8 x 1 tiles: the last token and expert tiles with one row, a last column tile of four
+@pytest.mark.parametrize("d,ne,K,N", [(68, 64, 6, 3585), (256, 97, 4, 1793)])
+def test_router_wide_tiles(oracle, d, ne, K, N):
     test_router_tiles(oracle, d, ne, K, N)
 
 
