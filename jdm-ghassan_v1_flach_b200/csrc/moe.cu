@@ -734,7 +734,8 @@ int moe_route(const float* x, const float* router_w, const float* router_bias, f
         float* logits = static_cast<float*>(wsp);
         // One chain per thread in blocks of 8 x 8 (most blocks, least latency) or four in blocks of 32 x 16 (a third of the
         // shared loads per product).  Times in units of some us, from 1536 columns and 64 experts: 128 / 256 / 517 / 1024 tokens
-        // take 14 / 18 / 29 / 41 us with the first and 24 / 24 / 24 / 26 with the second, 2048 take 66 and 38.
+        // take 14 / 18 / 29 / 41 us with the first and 24 / 24 / 24 / 26 with the second, 2048 take 66 and 38.  (The fixed terms are those
+        // of that width; wider rows come to the second form early: 517 tokens of 4096 x 72 are 85 blocks of it, 44 us.)
         auto rounds = [&](int tok, int exp) { return ceil_div64(ceil_div64(N, tok) * ceil_div(ne, exp), num_sms()); };
         int* counters = nullptr;
         const int64_t wide = ceil_div64(N, RW_WARPS * RW_TOKENS) * ceil_div(ne, 32);
